@@ -1,83 +1,437 @@
 // True float32 matrix product for the 32-bit path: C[M, N] = A[M, K] * W[N, K]^T, FMA on the
-// CUDA cores, no tensor cores and no reduced-precision mode anywhere. Every output element is
-// accumulated over k = 0..K-1 in that order whatever the tile shape, M or N, so a row's result
-// does not depend on which other rows share the launch.
+// CUDA cores, no tensor cores and no reduced-precision mode anywhere.
+//
+// One summation order for every shape. K is cut into slices of 128; chain j (j = 0..7) takes the slices j, j + 8, ...
+// in turn and keeps two running sums, of its even and of its odd k (the two halves of a packed fma.rn.f32x2); P_j is
+// their sum, and the result is ((P_0 + P_1) + P_2) + ... + P_7. Both kernels below compute exactly this, so a row's
+// result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
+//
+// What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
+// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 43 TFLOP/s of
+// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 890 us so; a
+// one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
+// (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 #include "common.cuh"
 
 namespace llmie {
 
-constexpr int kBK = 16;
+constexpr int kSlice = 128;
+constexpr int kChains = 8;
 
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
-                   int K, int lda, int ldw, int ldc) {
-  constexpr int kThreads = (BM / TM) * (BN / TN);
-  __shared__ float As[kBK][BM + 4];
-  __shared__ float Ws[kBK][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+__device__ __forceinline__ void fma2(float2& acc, const float2& a, const float2& b) {
+  unsigned long long& c = reinterpret_cast<unsigned long long&>(acc);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(c)
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+}
 
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-    for (int idx = tid; idx < BM * kBK; idx += kThreads) {
-      const int r = idx / kBK, c = idx % kBK;
-      const int gm = m0 + r, gk = k0 + c;
-      As[c][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-    }
-    for (int idx = tid; idx < BN * kBK; idx += kThreads) {
-      const int r = idx / kBK, c = idx % kBK;
-      const int gn = n0 + r, gk = k0 + c;
-      Ws[c][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
-    }
-    __syncthreads();
+// Copies of 16 bytes (or of four single floats where rows are not 16-byte aligned) from global into shared memory that
+// complete asynchronously; `n_valid` floats of the four are read, the others are zeros.
+template <bool VEC>
+__device__ __forceinline__ void copy4(float* dst, const float* src, const float* safe, int n_valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (VEC) {
+    const int bytes = n_valid <= 0 ? 0 : (n_valid >= 4 ? 16 : 4 * n_valid);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(bytes ? src : safe), "r"(bytes) : "memory");
+  } else {
 #pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      float a[TM], w[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
+    for (int e = 0; e < 4; ++e)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * e), "l"(e < n_valid ? src + e : safe),
+                   "r"(e < n_valid ? 4 : 0)
+                   : "memory");
   }
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 read_peer(const float4* p, unsigned rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r));
+  return v;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Tiles for more than kFewRows rows: WM x WN warps, each 32 x 64 outputs, a thread 8 x 8 of them (rows lane / 8 + 4 i,
+// columns lane % 8 + 8 j), all 16 k of a stage read as four 16-byte pieces a row: rows lie 20 floats apart in shared
+// memory, so the eight rows a 16-byte access touches fall on different banks. The 8 x 8 packed sums are 128 registers;
+// at a chain's end they are added up into shared memory, a slot per thread. `split` blocks of a cluster share a tile's
+// chains (8 / split chains each, rank 0 the first ones); their sums meet in distributed shared memory in chain order.
+constexpr int kBK = 16, kStride = 20, kStages = 4;
+
+template <int WM, int WN>
+struct Tile {
+  static constexpr int BM = 32 * WM, BN = 64 * WN, kThreads = 32 * WM * WN;
+  static constexpr int kStageFloats = (BM + BN) * kStride;
+  static constexpr int kSumFloats = BM * BN;
+  // the sums of the last chain of a rank > 0 lie where the stages were
+  static constexpr int kRing = kStages * kStageFloats > kSumFloats ? kStages * kStageFloats : kSumFloats;
+  static constexpr int smem_bytes() { return 4 * (kRing + kSumFloats); }
+};
+
+template <int WM, int WN, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN)
+gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
+                     int K, int lda, int ldw, int ldc, int split) {
+  using T = Tile<WM, WN>;
+  extern __shared__ float4 smem4[];
+  float* ring = reinterpret_cast<float*>(smem4);
+  float4* held = smem4 + T::kRing / 4;                    // [16][kThreads]: a thread's 64 sums of earlier chains
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = blockIdx.x % split;
+  const int m0 = blockIdx.y * T::BM, n0 = (blockIdx.x / split) * T::BN;
+  const int row_a = (warp / WN) * 32 + (lane >> 3), row_w = T::BM + (warp % WN) * 64 + (lane & 7);
+
+  const int n_chains = kChains / split, chain0 = rank * n_chains;
+  const int n_slices = (K + kSlice - 1) / kSlice;
+  // the blocks of 16 k that this block works on, chain by chain (each a whole slice: k >= K reads zeros)
+  int total_blocks = 0;
+  for (int j = chain0; j < chain0 + n_chains; ++j)
+    if (j < n_slices) total_blocks += ((n_slices - 1 - j) / kChains + 1) * (kSlice / kBK);
+
+  // ---- loading, kStages - 1 blocks early
+  int ld_chain = chain0, ld_slice = chain0, ld_sub = 0, ld_count = 0;
+  auto load_next = [&]() {
+    if (ld_count < total_blocks) {
+      while (ld_slice >= n_slices) { ++ld_chain; ld_slice = ld_chain; }
+      const int k0 = ld_slice * kSlice + ld_sub * kBK;
+      float* st = ring + (ld_count % kStages) * T::kStageFloats;
+      constexpr int kPieces = (T::BM + T::BN) * (kBK / 4);
+      static_assert(kPieces % T::kThreads == 0, "pieces of a stage divide among the threads");
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gm = m0 + ty * TM + i;
-    if (gm >= M) continue;
+      for (int p = 0; p < kPieces / T::kThreads; ++p) {
+        const int idx = tid + p * T::kThreads;
+        const int r = idx >> 2, c = (idx & 3) * 4;
+        const bool is_a = r < T::BM;
+        const int g = is_a ? m0 + r : n0 + r - T::BM;
+        const bool in = g < (is_a ? M : N);
+        const float* base = is_a ? A : W;
+        copy4<VEC>(st + r * kStride + c, base + (size_t)(in ? g : 0) * (is_a ? lda : ldw) + k0 + c, base,
+                   in ? K - k0 - c : 0);
+      }
+      if (++ld_sub == kSlice / kBK) { ld_sub = 0; ld_slice += kChains; }
+      ++ld_count;
+    }
+    copy_commit();
+  };
+
+  float2 acc[8][8];
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gn = n0 + tx * TN + j;
-      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) load_next();
+
+  int chain = chain0, count = 0;
+  bool first = true;
+  for (int c = 0; c < n_chains; ++c, ++chain) {
+    const int blocks = chain < n_slices ? ((n_slices - 1 - chain) / kChains + 1) * (kSlice / kBK) : 0;
+    for (int b = 0; b < blocks; ++b, ++count) {
+      copy_wait<kStages - 2>();
+      __syncthreads();
+      load_next();
+      const float* st = ring + (count % kStages) * T::kStageFloats;
+#pragma unroll
+      for (int k4 = 0; k4 < kBK / 4; ++k4) {
+        float4 w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(st + (row_w + 8 * j) * kStride + 4 * k4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 a = *reinterpret_cast<const float4*>(st + (row_a + 4 * i) * kStride + 4 * k4);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) fma2(acc[i][j], make_float2(a.x, a.y), make_float2(w[j].x, w[j].y));
+#pragma unroll
+          for (int j = 0; j < 8; ++j) fma2(acc[i][j], make_float2(a.z, a.w), make_float2(w[j].z, w[j].w));
+        }
+      }
+    }
+    if (c == n_chains - 1) break;
+    // the chain's sums: the first chain's as they are, later ones added to what is held; a rank > 0 has two chains at
+    // most and holds the first apart from the last
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float4* slot = held + (2 * i + h) * T::kThreads + tid;
+        float4 v = first ? make_float4(0.f, 0.f, 0.f, 0.f) : *slot;
+        float* e = &v.x;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float2& s = acc[i][4 * h + q];
+          e[q] = first ? s.x + s.y : e[q] + (s.x + s.y);
+          s = make_float2(0.f, 0.f);
+        }
+        *slot = v;
+      }
+    first = false;
+  }
+  copy_wait<0>();
+
+  if (split == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + (warp / WN) * 32 + (lane >> 3) + 4 * i;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 v = held[(2 * i + h) * T::kThreads + tid];
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int j = 4 * h + q, n = n0 + (warp % WN) * 64 + (lane & 7) + 8 * j;
+          if (m < M && n < N) C[(size_t)m * ldc + n] = e[q] + (acc[i][j].x + acc[i][j].y);
+        }
+      }
+    }
+    return;
+  }
+  // ---- a cluster shares the tile: the last chain's sums lie in the ring (rank 0 with two chains adds them to what it
+  // holds), then every rank adds up its share of the slots over the ranks, in chain order
+  __syncthreads();
+  float4* last = smem4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int slot = (2 * i + h) * T::kThreads + tid;
+      float e[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = acc[i][4 * h + q].x + acc[i][4 * h + q].y;
+      if (rank == 0 && n_chains > 1) {
+        const float4 v = held[slot];
+        e[0] = v.x + e[0]; e[1] = v.y + e[1]; e[2] = v.z + e[2]; e[3] = v.w + e[3];
+      }
+      last[slot] = make_float4(e[0], e[1], e[2], e[3]);
+    }
+  cluster_barrier();
+  for (int s = rank; s < 16; s += split) {
+    const int slot = s * T::kThreads + tid;
+    float4 v = read_peer(last + slot, 0);
+    for (int r = 1; r < split; ++r) {
+      if (n_chains > 1) {
+        const float4 p = read_peer(held + slot, r);
+        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+      }
+      const float4 p = read_peer(last + slot, r);
+      v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+    }
+    const int m = m0 + (warp / WN) * 32 + (lane >> 3) + 4 * (s >> 1);
+    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int n = n0 + (warp % WN) * 64 + (lane & 7) + 8 * (4 * (s & 1) + q);
+      if (m < M && n < N) C[(size_t)m * ldc + n] = e[q];
     }
   }
+  cluster_barrier();          // nobody leaves while its shared memory is being read
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Up to kFewRows rows: the weights stream through shared memory once. A thread is RW weight rows of one chain, a warp
+// 4 RW rows x 8 chains; a stage brings RUN k of every chain's current slice for the block's weight rows and for all MT
+// rows of A. Runs lie RUN + 4 floats apart, so a 16-byte access of 8 chains falls on all banks.
+constexpr int kFewRows = 16;
+
+template <int MT, int WARPS, int RW, int STAGES, int RUN> struct Few {
+  static constexpr int kRows = 4 * RW * WARPS, kThreads = 32 * WARPS;
+  static constexpr int kRunStride = RUN + 4;
+  static constexpr int kStageFloats = (kRows + MT) * kChains * kRunStride;
+  static constexpr int smem_bytes() { return 4 * STAGES * kStageFloats; }
+};
+
+template <int MT, int WARPS, int RW, int STAGES, int RUN, bool VEC>
+__global__ void __launch_bounds__(32 * WARPS)
+gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
+                    int K, int lda, int ldw, int ldc) {
+  using F = Few<MT, WARPS, RW, STAGES, RUN>;
+  constexpr int kRunStride = F::kRunStride;
+  extern __shared__ float4 smem4[];
+  float* ring = reinterpret_cast<float*>(smem4);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int chain = lane & 7, row = warp * 4 * RW + (lane >> 3);
+  const int n0 = blockIdx.x * F::kRows;
+  const int n_slices = (K + kSlice - 1) / kSlice;
+  constexpr int kPerSlice = kSlice / RUN;
+  const int steps = (n_slices + kChains - 1) / kChains * kPerSlice;
+
+  auto load = [&](int t) {
+    if (t < steps) {
+      float* st = ring + (t % STAGES) * F::kStageFloats;
+      constexpr int kPieces = (F::kRows + MT) * kChains * (RUN / 4);
+#pragma unroll
+      for (int p = 0; p < (kPieces + F::kThreads - 1) / F::kThreads; ++p) {
+        const int idx = tid + p * F::kThreads;
+        if (kPieces % F::kThreads && idx >= kPieces) break;
+        const int piece = idx % (RUN / 4), c = idx / (RUN / 4) % kChains, r = idx / (RUN / 4 * kChains);
+        const int k = ((t / kPerSlice) * kChains + c) * kSlice + (t % kPerSlice) * RUN + piece * 4;
+        const bool is_w = r < F::kRows;
+        const int g = is_w ? n0 + r : r - F::kRows;
+        const bool in = g < (is_w ? N : M);
+        const float* base = is_w ? W : A;
+        copy4<VEC>(st + (r * kChains + c) * kRunStride + piece * 4, base + (size_t)(in ? g : 0) * (is_w ? ldw : lda) + k,
+                   base, in ? K - k : 0);
+      }
+    }
+    copy_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) load(s);
+
+  float2 acc[RW][MT];
+#pragma unroll
+  for (int i = 0; i < RW; ++i)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[i][m] = make_float2(0.f, 0.f);
+  for (int t = 0; t < steps; ++t) {
+    copy_wait<STAGES - 2>();
+    __syncthreads();
+    load(t + STAGES - 1);
+    const float* st = ring + (t % STAGES) * F::kStageFloats;
+    const float* wr = st + (row * kChains + chain) * kRunStride;
+    const float* ar = st + (F::kRows * kChains + chain) * kRunStride;
+    constexpr int kTogether = MT * RW <= 4 ? 4 : (MT <= 8 ? 2 : 1);     // 16-byte pieces read before they are used
+#pragma unroll
+    for (int q0 = 0; q0 < RUN / 4; q0 += kTogether) {
+      float4 w[kTogether][RW], a[kTogether][MT];
+#pragma unroll
+      for (int q = 0; q < kTogether; ++q) {
+#pragma unroll
+        for (int i = 0; i < RW; ++i)
+          w[q][i] = *reinterpret_cast<const float4*>(wr + 4 * i * kChains * kRunStride + 4 * (q0 + q));
+#pragma unroll
+        for (int m = 0; m < MT; ++m) a[q][m] = *reinterpret_cast<const float4*>(ar + m * kChains * kRunStride + 4 * (q0 + q));
+      }
+#pragma unroll
+      for (int q = 0; q < kTogether; ++q) {
+#pragma unroll
+        for (int i = 0; i < RW; ++i)
+#pragma unroll
+          for (int m = 0; m < MT; ++m) fma2(acc[i][m], make_float2(a[q][m].x, a[q][m].y), make_float2(w[q][i].x, w[q][i].y));
+#pragma unroll
+        for (int i = 0; i < RW; ++i)
+#pragma unroll
+          for (int m = 0; m < MT; ++m) fma2(acc[i][m], make_float2(a[q][m].z, a[q][m].w), make_float2(w[q][i].z, w[q][i].w));
+      }
+    }
+  }
+  copy_wait<0>();
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    const int n = n0 + row + 4 * i;
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const float p = acc[i][m].x + acc[i][m].y;
+      float sum = __shfl_sync(0xffffffffu, p, lane & 24);
+#pragma unroll
+      for (int c = 1; c < kChains; ++c) sum += __shfl_sync(0xffffffffu, p, (lane & 24) + c);
+      if (chain == (m & 7) && m < M && n < N) C[(size_t)m * ldc + n] = sum;
+    }
+  }
+}
+
+template <int WM, int WN, bool VEC>
+static int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int split,
+                       cudaStream_t stream) {
+  using T = Tile<WM, WN>;
+  const int tiles_n = (N + T::BN - 1) / T::BN, tiles_m = (M + T::BM - 1) / T::BM;
+  if (tiles_m > 65535) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  auto kernel = gemm_f32_tile_kernel<WM, WN, VEC>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::smem_bytes());
+  if (e != cudaSuccess) return (int)e;
+  if (split == 1)
+    launch_k(kernel, dim3(tiles_n, tiles_m), dim3(T::kThreads), T::smem_bytes(), stream, A, W, C, M, N, K, lda, ldw, ldc, 1);
+  else
+    launch_k_cluster(kernel, dim3(tiles_n * split, tiles_m), dim3(T::kThreads), T::smem_bytes(), stream, (unsigned)split, A,
+                     W, C, M, N, K, lda, ldw, ldc, split);
+  LLMIE_LAUNCH_CHECK();
+  return LLMIE_OK;
+}
+
+template <int MT, int WARPS, int RW, int STAGES, int RUN, bool VEC>
+static int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                      cudaStream_t stream) {
+  using F = Few<MT, WARPS, RW, STAGES, RUN>;
+  static_assert(F::smem_bytes() <= 227 * 1024, "a block's stages fit its shared memory");
+  auto kernel = gemm_f32_few_kernel<MT, WARPS, RW, STAGES, RUN, VEC>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem_bytes());
+  if (e != cudaSuccess) return (int)e;
+  launch_k(kernel, dim3((N + F::kRows - 1) / F::kRows), dim3(F::kThreads), F::smem_bytes(), stream, A, W, C, M, N, K, lda,
+           ldw, ldc);
+  LLMIE_LAUNCH_CHECK();
+  return LLMIE_OK;
+}
+
+// The kernels by form: kernel * 10 + blocks that share a tile's chains. 10, 20, 30: up to kFewRows rows. 5x: tiles of 32 x
+// 128, 6x: of 64 x 64.
+template <bool VEC>
+static int dispatch(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int form,
+                    cudaStream_t stream) {
+#define LLMIE_FEW(MAX, MT, WARPS, RW, STAGES, RUN) \
+  if (M <= MAX) return launch_few<MT, WARPS, RW, STAGES, RUN, VEC>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  switch (form) {
+    case 10:
+      LLMIE_FEW(1, 1, 2, 1, 6, 32) LLMIE_FEW(2, 2, 2, 1, 6, 32) LLMIE_FEW(4, 4, 2, 1, 6, 32) LLMIE_FEW(8, 8, 2, 1, 6, 32)
+      break;
+    case 20:
+      LLMIE_FEW(1, 1, 2, 2, 3, 32) LLMIE_FEW(2, 2, 2, 2, 3, 32) LLMIE_FEW(4, 4, 2, 2, 3, 32) LLMIE_FEW(16, 16, 2, 2, 3, 32)
+      break;
+    case 30:
+      LLMIE_FEW(8, 8, 4, 2, 4, 16) LLMIE_FEW(16, 16, 4, 2, 3, 16)
+      break;
+    case 51: case 54: case 58: return launch_tile<1, 2, VEC>(A, W, C, M, N, K, lda, ldw, ldc, form - 50, stream);
+    case 61: case 64: case 68: return launch_tile<2, 1, VEC>(A, W, C, M, N, K, lda, ldw, ldc, form - 60, stream);
+    default: return LLMIE_ERR_BAD_ARG;
+  }
+#undef LLMIE_FEW
+  return LLMIE_ERR_UNSUPPORTED_SIZE;
+}
+
+// Which form serves which size; microseconds measured with weights beyond L2 (N x K: rows).
+// Few rows: 8 weight rows a block and six stages where that gives no SM more than two blocks (2,048 x 8,192, 1 / 8 rows:
+// 18 / 35, form 20 26 / 44); 16 weight rows a block above (16,384 x 2,048, 1 / 3 rows: 26 / 30, form 10 29 / 42), and 32
+// from 5 rows on, where a thread's reads of A cost more than its weights (16,384 x 2,048, 8 / 13 rows: 38 / 60, form 20
+// 49 / 76). Tiles: 32 rows high up to 32 rows (2,048 x 2,048, 20 rows: 25, 64 high 34), else 64 x 64 (301 rows: 89, 64 x
+// 128 93). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
+// 317, 4 blocks 364, 1 block 761), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 563, 8
+// 570, 1 589), then each tile has one block (32,000 x 2,048, 512 rows: 1,602, 4 blocks 1,682).
+static int choose_form(int M, int N) {
+  if (M <= kFewRows) {
+    const bool narrow = N <= 2 * 8 * 148;
+    if (narrow) return M <= 8 ? 10 : 20;
+    return M <= 4 ? 20 : 30;
+  }
+  if (M <= 32) return 58;
+  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  return tiles < 640 ? 68 : (tiles < 1900 ? 64 : 61);
 }
 
 }  // namespace llmie
 
 using namespace llmie;
 
-extern "C" int llmie_gemm_f32_nt(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                                 int ldc, cudaStream_t stream) {
+// form 0: chosen by size; the others are for tests (every form that takes a size gives the same bits).
+extern "C" int llmie_gemm_f32_nt_form(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                                      int ldc, int form, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N) return LLMIE_ERR_BAD_ARG;
   if (M == 0) return LLMIE_OK;
-  if (M <= 16) {
-    dim3 grid((N + 31) / 32, (M + 15) / 16);
-    gemm_f32_nt_kernel<16, 32, 2, 2><<<grid, 128, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
-  } else {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    if (grid.y > 65535) return LLMIE_ERR_UNSUPPORTED_SIZE;
-    gemm_f32_nt_kernel<64, 64, 4, 4><<<grid, 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
-  }
-  LLMIE_LAUNCH_CHECK();
-  return LLMIE_OK;
+  if (form == 0) form = choose_form(M, N);
+  const bool vec = aligned16(A) && aligned16(W) && lda % 4 == 0 && ldw % 4 == 0;
+  return vec ? dispatch<true>(A, W, C, M, N, K, lda, ldw, ldc, form, stream)
+             : dispatch<false>(A, W, C, M, N, K, lda, ldw, ldc, form, stream);
+}
+
+extern "C" int llmie_gemm_f32_nt(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                                 int ldc, cudaStream_t stream) {
+  return llmie_gemm_f32_nt_form(A, W, C, M, N, K, lda, ldw, ldc, 0, stream);
 }
