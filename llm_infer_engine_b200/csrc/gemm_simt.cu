@@ -11,6 +11,11 @@
 // it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 890 us so; a
 // one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
 // (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
+//
+// These kernels wait for the one before them, but do not let the next one start early: when they did, rows behind a state
+// space or short-convolution layer's projection came out wrong now and then (one prompt in four of the 128-wide test model),
+// never with the next kernel held back. Kernels that follow a float32 product read it through read-only pointers behind work
+// of their own in front of their wait, and were written for a product that ends first.
 #include "common.cuh"
 
 namespace llmie {
@@ -82,8 +87,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   extern __shared__ float4 smem4[];
   float* ring = reinterpret_cast<float*>(smem4);
   float4* held = smem4 + T::kRing / 4;                    // [16][kThreads]: a thread's 64 sums of earlier chains
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();       // the next kernel starts when this one is done: see the top of the file
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x % split;
   const int m0 = blockIdx.y * T::BM, n0 = (blockIdx.x / split) * T::BN;
@@ -256,8 +260,7 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   constexpr int kRunStride = F::kRunStride;
   extern __shared__ float4 smem4[];
   float* ring = reinterpret_cast<float*>(smem4);
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();       // the next kernel starts when this one is done: see the top of the file
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chain = lane & 7, row = warp * 4 * RW + (lane >> 3);
   const int n0 = blockIdx.x * F::kRows;
