@@ -122,31 +122,54 @@ grouped_gemm_kernel(const GroupedArgs p) {
 }
 
 // ------------------------------------------------------------------------------------------
-// The same products for bfloat16 inputs on the tensor cores (mma.sync m16n8k16, float32 accumulators): tiles of
-// BM x 64 outputs, four warps. With BM = 64 a warp owns 16 rows and all 64 columns; with BM = 16 (few rows a group:
-// one-token steps, where the weights are what is streamed) the warps share out the columns and the K step is longer.
-// A row's sums depend on that row and the weights alone (the rows of an mma are independent), so here too a result
-// does not depend on what else is in the launch. `vec`: K, the leading dimensions and the group strides are multiples
-// of 8 elements and the bases 16-byte aligned, so tiles are fetched 16 bytes at a time; otherwise element by element.
-__device__ __forceinline__ void gg_mma(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
-                                       unsigned b1) {
+// The same products for bfloat16 inputs on the tensor cores (mma.sync m16n8k16, float32 accumulators): tiles of BM x 64
+// outputs (64 gate and 64 up columns with DUAL), four warps that share out the columns. A row's sums depend on that row
+// and the weights alone (the rows of an mma are independent, and every tile height adds up k in the same order), so here
+// too a result does not depend on what else is in the launch.
+//
+// With a few rows a group (the experts of a batched one-token step) the weights' stream is what bounds it, with many rows
+// and a short K (the heads of a latent attention layer) the rows' way in and out. So: K steps of 64 arrive in a ring of
+// asynchronous copies, 16 bytes each, two steps ahead; fragments come by ldmatrix from rows of 128 bytes whose
+// eight pieces are exchanged by the row's number (no two rows of an 8 x 8 block share a bank); only the 16-row slices of a
+// tile that hold rows are multiplied; and results leave through shared memory in whole rows.
+// `vec`: K, the leading dimensions and the group strides are multiples of 8 elements and the bases 16-byte aligned;
+// otherwise the tiles are brought element by element. `cvec`: the same of C, for 16-byte stores.
+__device__ __forceinline__ void gg_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void gg_ldmatrix(unsigned (&r)[4], unsigned addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
 }
 
-template <typename TC, int BM, int BK, bool DUAL>
+constexpr int kMmaBK = 64, kMmaBN = 64;
+
+template <int BM, bool DUAL>
+struct MmaTile {
+  static constexpr int kRows = BM + (DUAL ? 2 : 1) * kMmaBN;            // rows of 128 bytes a stage holds
+  static constexpr int kStageBytes = kRows * 2 * kMmaBK;
+  // 16 rows: gate and up together in 3 stages, four blocks an SM, so that 16 experts' 512 blocks are all resident (2,048 x
+  // 2 x 2,048, 24 to 64 rows: 50 us of 41 for the weights; 5 stages, two blocks an SM, 63); one matrix in 5 (26 us of
+  // 20.5; 3 stages 35: what is in flight counts). 64 rows: 3 stages (2: 10 to 30 % slower; the same 40 rows 82 / 40 us).
+  static constexpr int kStages = BM == 16 && !DUAL ? 5 : 3;
+  static constexpr int kOutPitch = kMmaBN + 4;                          // floats between two rows on their way out
+  static constexpr int kOutBytes = BM * kOutPitch * 4;
+  static constexpr int smem_bytes() { return kStages * kStageBytes > kOutBytes ? kStages * kStageBytes : kOutBytes; }
+};
+
+template <typename TC, int BM, bool DUAL>
 __global__ void __launch_bounds__(128)
-grouped_gemm_mma_kernel(const GroupedArgs p, const int vec) {
-  constexpr int BN = 64, PITCH = BK + 8, NW = DUAL ? 2 : 1, CH = BK / 8;
-  constexpr int NT = BM == 64 ? 8 : 2;                 // n-tiles of 8 columns a warp owns
-  __shared__ __align__(16) __nv_bfloat16 As[BM][PITCH];
-  __shared__ __align__(16) __nv_bfloat16 Ws[NW][BN][PITCH];
+grouped_gemm_mma_kernel(const GroupedArgs p, const int vec, const int cvec) {
+  using T = MmaTile<BM, DUAL>;
+  constexpr int NW = DUAL ? 2 : 1, kSlices = BM / 16, BK = kMmaBK, BN = kMmaBN;
+  extern __shared__ __align__(128) unsigned char gg_smem[];
   __shared__ int rowA[BM], rowC[BM];
   pdl_launch_dependents();
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
   const int tile = blockIdx.y;
   int group = blockIdx.z;
   if (p.tile_group) {
@@ -154,6 +177,7 @@ grouped_gemm_mma_kernel(const GroupedArgs p, const int vec) {
     if (group < 0) return;
   }
   const int m0 = tile * BM, n0 = blockIdx.x * BN;
+  int last_row = 0;
   for (int r = tid; r < BM; r += 128) {
     const int pos = m0 + r;
     int ra = -1, rc = -1;
@@ -164,115 +188,149 @@ grouped_gemm_mma_kernel(const GroupedArgs p, const int vec) {
     }
     rowA[r] = ra;
     rowC[r] = rc;
+    if (ra >= 0) last_row = r + 1;
   }
+  // slices of 16 rows that hold a row (the positions of a tile are filled from its start; a gap costs time only)
+  const int slices = BM == 16 ? 1 : (__syncthreads_or(last_row > 48) ? 4 : __syncthreads_or(last_row > 32) ? 3
+                                     : __syncthreads_or(last_row > 16) ? 2 : 1);
   __syncthreads();
   const __nv_bfloat16* A = reinterpret_cast<const __nv_bfloat16*>(p.A) + (size_t)group * p.a_gcs;
   const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(p.W) + (size_t)group * p.w_gs;
-  const int row0 = BM == 64 ? warp * 16 : 0;
-  const int nt0 = BM == 64 ? 0 : warp * 2;
-  float acc[NW][NT][4];
+  const unsigned base = (unsigned)__cvta_generic_to_shared(gg_smem);
+  const int steps = (p.K + BK - 1) / BK;
+
+  // a thread brings piece tid % 8 of the stage's rows tid / 8 + 16 j
+  auto load = [&](int s) {
+    if (s < steps) {
+      const int k = s * BK + (tid & 7) * 8;
+      const unsigned stage = base + (s % T::kStages) * T::kStageBytes;
+#pragma unroll
+      for (int j = 0; j < T::kRows / 16; ++j) {
+        const int r = (tid >> 3) + 16 * j;
+        if (r < BM && r >= 16 * slices) continue;
+        const __nv_bfloat16* src = nullptr;
+        if (r < BM) {
+          if (rowA[r] >= 0) src = A + (size_t)rowA[r] * p.lda;
+        } else {
+          const int n = n0 + (r - BM) % BN;
+          if (n < p.N) src = W + (size_t)(n + ((r - BM) >= BN ? p.N : 0)) * p.ldw;
+        }
+        const unsigned dst = stage + r * 2 * BK + (((tid & 7) ^ (r & 7)) << 4);
+        if (vec) {
+          const int bytes = src && k < p.K ? 16 : 0;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(bytes ? src + k : W), "r"(bytes)
+                       : "memory");
+        } else {
+          alignas(16) __nv_bfloat16 e[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) e[i] = src && k + i < p.K ? src[k + i] : __float2bfloat16_rn(0.f);
+          *reinterpret_cast<uint4*>(gg_smem + (dst - base)) = *reinterpret_cast<const uint4*>(e);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[NW][kSlices][2][4];
 #pragma unroll
   for (int s = 0; s < NW; ++s)
 #pragma unroll
-    for (int i = 0; i < NT; ++i) acc[s][i][0] = acc[s][i][1] = acc[s][i][2] = acc[s][i][3] = 0.f;
-
-  // eight consecutive elements of a row from column gk on (zeros beyond K or for a row that is not there)
-  auto fetch = [&](const __nv_bfloat16* row, bool there, int gk) -> uint4 {
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (!there || gk >= p.K) return v;
-    if (vec) return *reinterpret_cast<const uint4*>(row + gk);
-    __nv_bfloat16 e[8];
+    for (int i = 0; i < kSlices; ++i)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) e[i] = gk + i < p.K ? row[gk + i] : __float2bfloat16_rn(0.f);
-    return *reinterpret_cast<const uint4*>(e);
-  };
-
-  // The next K step's pieces are requested into registers before this step's products, so that the loads are in flight
-  // while the tensor cores work: with few rows a group the weights' stream is all there is to wait for.
-  constexpr int A_PER = BM * CH / 128 > 0 ? BM * CH / 128 : 1, W_PER = BN * CH / 128;
-  static_assert((BM * CH) % 128 == 0 || BM * CH < 128, "whole rounds of the block's threads");
-  uint4 ra[A_PER], rw[NW][W_PER];
-  auto request = [&](int k0) {
+      for (int j = 0; j < 2; ++j) acc[s][i][j][0] = acc[s][i][j][1] = acc[s][i][j][2] = acc[s][i][j][3] = 0.f;
 #pragma unroll
-    for (int j = 0; j < A_PER; ++j) {
-      const int c = tid + j * 128;
-      if (c < BM * CH) {
-        const int r = c / CH, kc = (c % CH) * 8;
-        const int row = rowA[r];
-        ra[j] = fetch(A + (size_t)(row < 0 ? 0 : row) * p.lda, row >= 0, k0 + kc);
+  for (int s = 0; s < T::kStages - 1; ++s) load(s);
+
+  // this lane's row within an ldmatrix of A (rows 0-15, then the same rows of the next 8 k) and of W (8 columns, their
+  // next 8 k, the next 8 columns, their next 8 k)
+  const int a_row = lane & 15, a_k = lane >> 4;
+  const int w_row = BM + warp * 16 + (lane & 7) + ((lane >> 4) << 3), w_k = (lane >> 3) & 1;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(T::kStages - 2) : "memory");
+    __syncthreads();
+    load(s + T::kStages - 1);
+    const unsigned stage = base + (s % T::kStages) * T::kStageBytes;
+#pragma unroll
+    for (int kk = 0; kk < BK / 16; ++kk) {
+      unsigned b[NW][4];
+#pragma unroll
+      for (int q = 0; q < NW; ++q) gg_ldmatrix(b[q], stage + (w_row + q * BN) * 2 * BK + (((2 * kk + w_k) ^ (w_row & 7)) << 4));
+#pragma unroll
+      for (int i = 0; i < kSlices; ++i) {
+        if (i < slices) {
+          unsigned a[4];
+          gg_ldmatrix(a, stage + (16 * i + a_row) * 2 * BK + (((2 * kk + a_k) ^ (a_row & 7)) << 4));
+#pragma unroll
+          for (int q = 0; q < NW; ++q) {
+            gg_mma(acc[q][i][0], a, b[q][0], b[q][1]);
+            gg_mma(acc[q][i][1], a, b[q][2], b[q][3]);
+          }
+        }
       }
     }
-#pragma unroll
-    for (int j = 0; j < W_PER; ++j) {
-      const int c = tid + j * 128;
-      const int r = c / CH, kc = (c % CH) * 8;
-      const int gn = n0 + r;
-      rw[0][j] = fetch(W + (size_t)gn * p.ldw, gn < p.N, k0 + kc);
-      if (DUAL) rw[NW - 1][j] = fetch(W + (size_t)(gn + p.N) * p.ldw, gn < p.N, k0 + kc);
-    }
-  };
-  request(0);
-  for (int k0 = 0; k0 < p.K; k0 += BK) {
-#pragma unroll
-    for (int j = 0; j < A_PER; ++j) {
-      const int c = tid + j * 128;
-      if (c < BM * CH) *reinterpret_cast<uint4*>(&As[c / CH][(c % CH) * 8]) = ra[j];
-    }
-#pragma unroll
-    for (int j = 0; j < W_PER; ++j) {
-      const int c = tid + j * 128;
-      *reinterpret_cast<uint4*>(&Ws[0][c / CH][(c % CH) * 8]) = rw[0][j];
-      if (DUAL) *reinterpret_cast<uint4*>(&Ws[NW - 1][c / CH][(c % CH) * 8]) = rw[NW - 1][j];
-    }
-    __syncthreads();
-    if (k0 + BK < p.K) request(k0 + BK);
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 16) {
-      const unsigned a0 = *reinterpret_cast<const unsigned*>(&As[row0 + g][kk + 2 * t]);
-      const unsigned a1 = *reinterpret_cast<const unsigned*>(&As[row0 + g + 8][kk + 2 * t]);
-      const unsigned a2 = *reinterpret_cast<const unsigned*>(&As[row0 + g][kk + 2 * t + 8]);
-      const unsigned a3 = *reinterpret_cast<const unsigned*>(&As[row0 + g + 8][kk + 2 * t + 8]);
-#pragma unroll
-      for (int s = 0; s < NW; ++s)
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          const unsigned b0 = *reinterpret_cast<const unsigned*>(&Ws[s][(nt0 + i) * 8 + g][kk + 2 * t]);
-          const unsigned b1 = *reinterpret_cast<const unsigned*>(&Ws[s][(nt0 + i) * 8 + g][kk + 2 * t + 8]);
-          gg_mma(acc[s][i], a0, a1, a2, a3, b0, b1);
-        }
-    }
-    __syncthreads();
   }
-  TC* C = reinterpret_cast<TC*>(p.C) + (size_t)group * p.c_gcs;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+
+  // out through shared memory (the ring is done with): results as float32, whole rows of 64 columns
+  float* out = reinterpret_cast<float*>(gg_smem);
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int rc = rowC[row0 + g + 8 * half];
-    if (rc < 0) continue;
+  for (int i = 0; i < kSlices; ++i) {
+    if (i >= slices) break;
 #pragma unroll
-    for (int i = 0; i < NT; ++i)
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int gn = n0 + (nt0 + i) * 8 + 2 * t + e;
-        if (gn >= p.N) continue;
-        float v = acc[0][i][2 * half + e];
+      for (int e = 0; e < 4; ++e) {
+        float v = acc[0][i][j][e];
         if (DUAL) {
-          const float gt = to_f32(from_f32<TC>(v)), up = to_f32(from_f32<TC>(acc[NW - 1][i][2 * half + e]));
+          const float gt = to_f32(from_f32<TC>(v)), up = to_f32(from_f32<TC>(acc[NW - 1][i][j][e]));
           v = apply_act(gt, p.act) * up;
         } else if (p.act) {
           v = apply_act(to_f32(from_f32<TC>(v)), p.act);
         }
-        C[(size_t)rc * p.ldc + gn] = from_f32<TC>(v);
+        out[(16 * i + (lane >> 2) + 8 * (e >> 1)) * T::kOutPitch + warp * 16 + 8 * j + 2 * (lane & 3) + (e & 1)] = v;
       }
   }
+  __syncthreads();
+  TC* C = reinterpret_cast<TC*>(p.C) + (size_t)group * p.c_gcs;
+  constexpr int kPer = 16 / (int)sizeof(TC), kPieces = BN / kPer;
+  for (int idx = tid; idx < 16 * slices * kPieces; idx += 128) {
+    const int r = idx / kPieces, c = idx % kPieces * kPer;
+    const int rc = rowC[r];
+    if (rc < 0 || n0 + c >= p.N) continue;
+    const float* v = out + r * T::kOutPitch + c;
+    TC* dst = C + (size_t)rc * p.ldc + n0 + c;
+    if (cvec && n0 + c + kPer <= p.N) {
+      alignas(16) TC e[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) e[i] = from_f32<TC>(v[i]);
+      *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(e);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (n0 + c + i < p.N) dst[i] = from_f32<TC>(v[i]);
+    }
+  }
+}
+
+template <typename TC, int BM, bool DUAL>
+static int launch_mma_tile(const GroupedArgs& p, dim3 grid, int vec, int cvec, cudaStream_t stream) {
+  using T = MmaTile<BM, DUAL>;
+  auto kernel = grouped_gemm_mma_kernel<TC, BM, DUAL>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::smem_bytes());
+  if (e != cudaSuccess) return (int)e;
+  launch_k(kernel, grid, dim3(128), T::smem_bytes(), stream, p, vec, cvec);
+  return LLMIE_OK;
 }
 
 template <typename TC, bool DUAL>
 static int launch_grouped_mma(const GroupedArgs& p, int n_tiles, int groups_z, bool small, int vec, cudaStream_t stream) {
-  dim3 grid((p.N + 63) / 64, n_tiles, groups_z);
+  dim3 grid((p.N + kMmaBN - 1) / kMmaBN, n_tiles, groups_z);
   if (grid.y > 65535 || grid.z > 65535) return LLMIE_ERR_UNSUPPORTED_SIZE;
-  if (small) launch_k(grouped_gemm_mma_kernel<TC, 16, 64, DUAL>, grid, dim3(128), 0, stream, p, vec);
-  else launch_k(grouped_gemm_mma_kernel<TC, 64, 32, DUAL>, grid, dim3(128), 0, stream, p, vec);
-  return LLMIE_OK;
+  constexpr int kPer = 16 / (int)sizeof(TC);
+  const int cvec = p.ldc % kPer == 0 && p.c_gcs % kPer == 0 && aligned16(p.C);
+  return small ? launch_mma_tile<TC, 16, DUAL>(p, grid, vec, cvec, stream)
+               : launch_mma_tile<TC, 64, DUAL>(p, grid, vec, cvec, stream);
 }
 
 template <typename TA, typename TC, bool DUAL>

@@ -148,14 +148,15 @@ class RoutedExperts(FeedForward):
             ops.moe_route(x, self.w_router, self.b_router, ids, weights, self.route_mode, self.correction,
                           self.weight_scale, self.groups)
             n_pairs = T * top
-            small = n_pairs <= ops.GROUPED_SMALL_ROWS
+            library = self._library and ops.library_grouped_mm_ok(n_pairs, w, self.w_down)
+            small = not library and ops.routed_tiles_small(n_pairs, E, w.dtype)
             tile = ops.grouped_tile_rows(small)
             n_tiles = ops.moe_max_tiles(n_pairs, E, tile)
             index = torch.empty(2 * n_tiles * tile + n_tiles, dtype=torch.int32, device=dev)
             sorted_token, sorted_pair = index[:n_tiles * tile], index[n_tiles * tile:2 * n_tiles * tile]
             tile_group = index[2 * n_tiles * tile:]
             shared = None
-            if self._library and ops.library_grouped_mm_ok(n_pairs, w, self.w_down):
+            if library:
                 # prompts: each expert's rows side by side, the two products by the library's grouped GEMM
                 extra = torch.empty(E + n_pairs, dtype=torch.int32, device=dev)
                 group_end, pair_pos = extra[:E], extra[E:]
