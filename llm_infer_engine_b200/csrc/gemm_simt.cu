@@ -7,8 +7,8 @@
 // result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
 //
 // What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
-// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 43 TFLOP/s of
-// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 890 us so; a
+// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 46 TFLOP/s of
+// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 830 us so; a
 // one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
 // (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 //
@@ -67,11 +67,13 @@ __device__ __forceinline__ float4 read_peer(const float4* p, unsigned rank) {
 // memory, so the eight rows a 16-byte access touches fall on different banks. The 8 x 8 packed sums are 128 registers;
 // at a chain's end they are added up into shared memory, a slot per thread. `split` blocks of a cluster share a tile's
 // chains (8 / split chains each, rank 0 the first ones); their sums meet in distributed shared memory in chain order.
-constexpr int kBK = 16, kStride = 20, kStages = 4;
+constexpr int kBK = 16, kStride = 20;
 
 template <int WM, int WN>
 struct Tile {
   static constexpr int BM = 32 * WM, BN = 64 * WN, kThreads = 32 * WM * WN;
+  // 32 x 128: three stages, so that four blocks share an SM (32,000 x 2,048, 20 rows: 127 us, 143 with four stages)
+  static constexpr int kStages = WM == 1 ? 3 : 4;
   static constexpr int kStageFloats = (BM + BN) * kStride;
   static constexpr int kSumFloats = BM * BN;
   // the sums of the last chain of a rank > 0 lie where the stages were
@@ -100,27 +102,63 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
   for (int j = chain0; j < chain0 + n_chains; ++j)
     if (j < n_slices) total_blocks += ((n_slices - 1 - j) / kChains + 1) * (kSlice / kBK);
 
-  // ---- loading, kStages - 1 blocks early
-  int ld_chain = chain0, ld_slice = chain0, ld_sub = 0, ld_count = 0;
+  // ---- loading, T::kStages - 1 blocks early. A thread brings piece tid % 4 of the rows tid / 4 + kStep p: rows of A first,
+  // then of W. What is left of each piece is an address and a copy, in tiles whose rows are all there; looking at every
+  // piece's row and k took two instructions for every three of the products.
+  constexpr int kStep = T::kThreads / 4, kPiecesA = T::BM / kStep, kPiecesW = T::BN / kStep;
+  static_assert(T::BM % kStep == 0 && T::BN % kStep == 0, "a piece's row is one of A's or one of W's for all threads");
+  const int ld_row = tid >> 2, ld_c = (tid & 3) * 4;
+  const bool rows_there = m0 + T::BM <= M && n0 + T::BN <= N;
+  // how many of this thread's rows there are (they come in order), and its first ones
+  const int a_there = M - m0 - ld_row, w_there = N - n0 - ld_row;        // row p is there if p * kStep is below
+  const float* a_src = A + (size_t)(a_there > 0 ? m0 + ld_row : 0) * lda + ld_c;
+  const float* w_src = W + (size_t)(w_there > 0 ? n0 + ld_row : 0) * ldw + ld_c;
+  int ld_chain = chain0, ld_slice = chain0, ld_sub = 0, ld_count = 0, ld_stage = 0;
   auto load_next = [&]() {
     if (ld_count < total_blocks) {
       while (ld_slice >= n_slices) { ++ld_chain; ld_slice = ld_chain; }
       const int k0 = ld_slice * kSlice + ld_sub * kBK;
-      float* st = ring + (ld_count % kStages) * T::kStageFloats;
-      constexpr int kPieces = (T::BM + T::BN) * (kBK / 4);
-      static_assert(kPieces % T::kThreads == 0, "pieces of a stage divide among the threads");
+      float* st = ring + ld_stage * T::kStageFloats + ld_row * kStride + ld_c;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(st);
+      if (VEC && k0 + kBK <= K) {
+        const float* a = a_src + k0;
+        const float* w = w_src + k0;
+        if (rows_there) {
 #pragma unroll
-      for (int p = 0; p < kPieces / T::kThreads; ++p) {
-        const int idx = tid + p * T::kThreads;
-        const int r = idx >> 2, c = (idx & 3) * 4;
-        const bool is_a = r < T::BM;
-        const int g = is_a ? m0 + r : n0 + r - T::BM;
-        const bool in = g < (is_a ? M : N);
-        const float* base = is_a ? A : W;
-        copy4<VEC>(st + r * kStride + c, base + (size_t)(in ? g : 0) * (is_a ? lda : ldw) + k0 + c, base,
-                   in ? K - k0 - c : 0);
+          for (int p = 0; p < kPiecesA; ++p)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + p * kStep * kStride * 4),
+                         "l"(a + (size_t)p * kStep * lda) : "memory");
+#pragma unroll
+          for (int p = 0; p < kPiecesW; ++p)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (T::BM + p * kStep) * kStride * 4),
+                         "l"(w + (size_t)p * kStep * ldw) : "memory");
+        } else {
+#pragma unroll
+          for (int p = 0; p < kPiecesA; ++p) {
+            const bool in = p * kStep < a_there;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + p * kStep * kStride * 4),
+                         "l"(in ? a + (size_t)p * kStep * lda : a), "r"(in ? 16 : 0) : "memory");
+          }
+#pragma unroll
+          for (int p = 0; p < kPiecesW; ++p) {
+            const bool in = p * kStep < w_there;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (T::BM + p * kStep) * kStride * 4),
+                         "l"(in ? w + (size_t)p * kStep * ldw : w), "r"(in ? 16 : 0) : "memory");
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int p = 0; p < kPiecesA + kPiecesW; ++p) {
+          const bool is_a = p < kPiecesA;
+          const int g = is_a ? m0 + ld_row + p * kStep : n0 + ld_row + (p - kPiecesA) * kStep;
+          const bool in = g < (is_a ? M : N);
+          const float* base = is_a ? A : W;
+          copy4<VEC>(st + p * kStep * kStride, base + (size_t)(in ? g : 0) * (is_a ? lda : ldw) + k0 + ld_c, base,
+                     in ? K - k0 - ld_c : 0);
+        }
       }
       if (++ld_sub == kSlice / kBK) { ld_sub = 0; ld_slice += kChains; }
+      ld_stage = ld_stage == T::kStages - 1 ? 0 : ld_stage + 1;
       ++ld_count;
     }
     copy_commit();
@@ -133,17 +171,18 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
 
 #pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) load_next();
+  for (int s = 0; s < T::kStages - 1; ++s) load_next();
 
-  int chain = chain0, count = 0;
+  int chain = chain0, stage = 0;
   bool first = true;
   for (int c = 0; c < n_chains; ++c, ++chain) {
     const int blocks = chain < n_slices ? ((n_slices - 1 - chain) / kChains + 1) * (kSlice / kBK) : 0;
-    for (int b = 0; b < blocks; ++b, ++count) {
-      copy_wait<kStages - 2>();
+    for (int b = 0; b < blocks; ++b) {
+      copy_wait<T::kStages - 2>();
       __syncthreads();
       load_next();
-      const float* st = ring + (count % kStages) * T::kStageFloats;
+      const float* st = ring + stage * T::kStageFloats;
+      stage = stage == T::kStages - 1 ? 0 : stage + 1;
 #pragma unroll
       for (int k4 = 0; k4 < kBK / 4; ++k4) {
         float4 w[8];
@@ -404,10 +443,10 @@ static int dispatch(const float* A, const float* W, float* C, int M, int N, int 
 // Few rows: 8 weight rows a block and six stages where that gives no SM more than two blocks (2,048 x 8,192, 1 / 8 rows:
 // 18 / 35, form 20 26 / 44); 16 weight rows a block above (16,384 x 2,048, 1 / 3 rows: 26 / 30, form 10 29 / 42), and 32
 // from 5 rows on, where a thread's reads of A cost more than its weights (16,384 x 2,048, 8 / 13 rows: 38 / 60, form 20
-// 49 / 76). Tiles: 32 rows high up to 32 rows (2,048 x 2,048, 20 rows: 25, 64 high 34), else 64 x 64 (301 rows: 89, 64 x
-// 128 93). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
-// 317, 4 blocks 364, 1 block 761), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 563, 8
-// 570, 1 589), then each tile has one block (32,000 x 2,048, 512 rows: 1,602, 4 blocks 1,682).
+// 49 / 76). Tiles: 32 rows high up to 32 rows (32,000 x 2,048, 20 rows: 127, 64 high 214), else 64 x 64 (301 rows: 84, 32
+// x 128 90). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
+// 291, 4 blocks 342, 1 block 520), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 529, 8
+// 532, 1 551), then each tile has one block (32,000 x 2,048, 512 rows: 1,504, 4 blocks 1,576).
 static int choose_form(int M, int N) {
   if (M <= kFewRows) {
     const bool narrow = N <= 2 * 8 * 148;
