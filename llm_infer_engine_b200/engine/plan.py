@@ -89,6 +89,13 @@ class KernelPlan:
                                      options.keep_first, options.sink, gate, options.softcap, options.distance_bias,
                                      options.sink_values)
             return True
+        if not ctx.decode and options.plain and ops.attention_prefill_f32_supported(head_dim, kv.page_size, q, kv.k, kv.v):
+            # prompts of the float32 path
+            ops.attention_prefill_f32(q, kv.k, kv.v, out, ctx.cu_q, ctx.seq_slot, ctx.seq_start, kv.block_table,
+                                      kv.page_size, ctx.n_seqs, ctx.max_q_len, n_q, n_kv, head_dim, scale, window)
+            if gate is not None:
+                ops.sigmoid_gate(out, gate)
+            return True
         if options.scored:
             # a cap, a bias by distance or a learned sink: the split-KV kernel below does not know them
             return self._attention_by_rows(ctx, q, kv, out, n_q, n_kv, head_dim, options, gate)

@@ -40,6 +40,7 @@ FAMILIES: Dict[str, tuple] = {
     "moe": ("moe.cu", [], []),
     "latent": ("latent.cu", [], []),
     "attention_simt": ("attention_simt.cu", [], []),
+    "attention_prefill_f32": ("attention_prefill_f32.cu", [], []),
     "attention_decode": ("attention_decode.cu", [], []),
     "attention_decode_mma": ("attention_decode_mma.cu", [], []),
     "attention_prefill_tc": ("attention_prefill_tc.cu", [], []),

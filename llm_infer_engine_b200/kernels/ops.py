@@ -316,6 +316,37 @@ def attention_paged(q, k_cache, v_cache, out, tok_pos, tok_seq, seq_slot, block_
     return out
 
 
+def attention_prefill_f32_supported(head_dim: int, page_size: int, q, k_cache, v_cache) -> bool:
+    """Whether attention_prefill_f32.cu takes a prompt step (answered without loading the library): float32, head size 64
+    or 128 of keys and values alike, pages of 64, 16-byte aligned."""
+    return (q.dtype is torch.float32 and k_cache.dtype is torch.float32 and head_dim in (64, 128) and page_size == 64
+            and v_cache.shape == k_cache.shape and v_cache.is_contiguous()
+            and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) & 15)
+
+
+def attention_prefill_f32(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, block_table, page_size: int, n_seqs: int,
+                          max_q_len: int, n_q: int, n_kv: int, head_dim: int, scale: float, window: int = 0):
+    """Prompts of the float32 path, tiles of query rows over whole cache pages: q, out [T, n_q head_dim], caches [pages,
+    n_kv, 64, head_dim]; scale and window as in attention_paged. A row's bits do not depend on what else is in the step."""
+    T = q.shape[0]
+    _need(q, "q", torch.float32, (T, n_q * head_dim))
+    _need(out, "out", torch.float32, (T, n_q * head_dim))
+    _need(k_cache, "k_cache", torch.float32, (None, n_kv, page_size, head_dim))
+    _need(v_cache, "v_cache", torch.float32, tuple(k_cache.shape))
+    if page_size != 64:
+        raise KernelError(f"attention_prefill_f32: pages of {page_size} are not supported")
+    for name, t in (("cu_q", cu_q), ("seq_slot", seq_slot), ("seq_start", seq_start), ("block_table", block_table)):
+        _need(t, name, torch.int32)
+    _work(_nbytes(q, out) + 1.0 * STEP_HINT["kv_total"] * n_kv * 2 * head_dim * 4,
+          4.0 * n_q * head_dim * STEP_HINT["pairs"])
+    f = _fn("attention_prefill_f32", "llmie_attention_prefill_f32",
+            [_c_void_p] * 8 + [_c_int] * 6 + [_c_float, _c_int, _c_void_p])
+    _check(f(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), cu_q.data_ptr(), seq_slot.data_ptr(),
+             seq_start.data_ptr(), block_table.data_ptr(), block_table.shape[1], n_seqs, max_q_len, n_q, n_kv, head_dim,
+             float(scale), int(window), _stream()), "attention_prefill_f32")
+    return out
+
+
 def _row_slice(t: torch.Tensor, what: str, dtype, rows: int, cols: int) -> int:
     """Checks a [rows, cols] tensor that may be a column slice of a wider contiguous one; returns its row stride."""
     if not t.is_cuda:
