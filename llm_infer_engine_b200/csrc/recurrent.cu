@@ -184,6 +184,175 @@ matrix_scan_kernel(const float* __restrict__ qa, const float* __restrict__ fg, c
   }
 }
 
+// The same recurrences where a head's rows are eight times a power of two and its columns a multiple of four (nearly every
+// model): a thread owns 8 rows x 4 columns, S = D / 8 neighbouring lanes share its columns. Gates (or keys) and queries
+// come 16 bytes at a time, the arithmetic is packed over pairs of rows (fma.rn.f32x2), what is read of four tokens is in
+// flight in a ring of registers, and the lanes' sums meet by an exchange that leaves each lane one column. The state's
+// bits are those of the kernel above (the same products and sums in the same order); only the order in which a read-out's
+// D terms are added differs. What bounds it: instructions issued, about 90 a token for 32 state entries where the kernel
+// above needs 200 for 16. Three prompts, 2,150 tokens, 32 heads of 32 x 64: 158 us for the three
+// kernels with the one above, 84 us so (four tokens in flight and four blocks of 128 threads an SM: two tokens 98 us, no
+// bound on the registers 116 us). Short pieces keep one token in flight and seven blocks: a one-token step is the state's
+// way in and out (64 sequences of 32 x 64: 8.4 -> 6.7 us; of 64 x 128, 134 MB: 37.8 -> 39.2 us; with four tokens 55 us).
+__device__ __forceinline__ float2 scan_fma2(const float2& a, const float2& b, const float2& c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+        "l"(reinterpret_cast<const unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 scan_mul2(const float2& a, const float2& b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ void scan_load4(const float* p, float (&v)[4]) {
+  const float4 r = *reinterpret_cast<const float4*>(p);
+  v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+}
+__device__ __forceinline__ void scan_load4(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+template <typename T, int MODE, int FORM>
+__global__ void __launch_bounds__(kScanThreads, MODE == 0 ? 7 : 4)
+matrix_scan_wide_kernel(const float* __restrict__ qa, const float* __restrict__ fg, const T* __restrict__ v, int v_ld,
+                        float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
+                        float* __restrict__ o, int H, int D, int Dv, int S, int write_state, float* __restrict__ ws,
+                        float* __restrict__ decay, int L, int NC, const float* __restrict__ head_decay,
+                        const float* __restrict__ key_factor, int G) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr bool keyed = FORM != 0, stepped = FORM == 2;
+  constexpr int kAhead = MODE == 0 ? 1 : 4;
+  const int s = threadIdx.x & (S - 1);
+  const int j = (blockIdx.x * (blockDim.x / S) + threadIdx.x / S) * 4;
+  const int h = blockIdx.y;
+  const int seq = MODE == 0 ? blockIdx.z : blockIdx.z / NC;
+  const int chunk = MODE == 0 ? 0 : blockIdx.z - seq * NC;
+  const bool live = j < Dv;
+  const int jj = live ? j : Dv - 4, i0 = s * 8;
+  const int slot = seq_slot[seq], seq_end = cu_q[seq + 1];      // asked for together
+  const int t0 = MODE == 0 ? cu_q[seq] : cu_q[seq] + chunk * L;
+  const int t1 = MODE == 0 ? seq_end : min(t0 + L, seq_end);
+  if (MODE == 1 && t1 >= seq_end) return;          // the last chunk (or none at all): nobody needs its end state
+  if (MODE != 1 && t0 >= seq_end) return;          // no token: nothing is read out, and the state stays as it is
+  float* st = state + (((size_t)slot * H + h) * D + i0) * Dv + jj;
+  const size_t HDDv = (size_t)H * D * Dv;
+  const float* start = MODE == 2 ? ws + ((size_t)seq * NC + chunk) * HDDv + ((size_t)h * D + i0) * Dv + jj : st;
+  float2 St[4][4];                                 // [pair of rows][column]
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+    if (MODE != 1) {
+      scan_load4(start + (size_t)(2 * r) * Dv, lo);
+      scan_load4(start + (size_t)(2 * r + 1) * Dv, hi);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) St[r][c] = make_float2(lo[c], hi[c]);
+  }
+  const size_t GD = (size_t)G * D;
+  const float* f_row = fg + (size_t)(stepped ? h / (H / G) : h) * D + i0;
+  const float* q_row = qa + (size_t)(stepped ? h / (H / G) : h) * D + i0;
+  const T* v_row = v + (size_t)h * Dv + jj;
+  const float dh = FORM == 1 ? head_decay[h] : 0.f;
+  float2 f[kAhead][4], q[kAhead][4];
+  float vv[kAhead][4], tg[kAhead], tf[kAhead];
+  auto fetch = [&](int u, int t) {
+    const float4 a = *reinterpret_cast<const float4*>(f_row + t * GD), b = *reinterpret_cast<const float4*>(f_row + t * GD + 4);
+    f[u][0] = make_float2(a.x, a.y); f[u][1] = make_float2(a.z, a.w);
+    f[u][2] = make_float2(b.x, b.y); f[u][3] = make_float2(b.z, b.w);
+    if (MODE != 1) {
+      const float4 c = *reinterpret_cast<const float4*>(q_row + t * GD), d = *reinterpret_cast<const float4*>(q_row + t * GD + 4);
+      q[u][0] = make_float2(c.x, c.y); q[u][1] = make_float2(c.z, c.w);
+      q[u][2] = make_float2(d.x, d.y); q[u][3] = make_float2(d.z, d.w);
+    }
+    scan_load4(v_row + (size_t)t * v_ld, vv[u]);
+    if (stepped) {
+      tg[u] = head_decay[(size_t)t * H + h];
+      tf[u] = key_factor[(size_t)t * H + h];
+    }
+  };
+  float2 prod[4];                                  // MODE 1: the product of the chunk's gates
+#pragma unroll
+  for (int r = 0; r < 4; ++r) prod[r] = make_float2(1.f, 1.f);
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) fetch(u, min(t0 + u, t1 - 1));
+  for (int tb = t0; tb < t1; tb += kAhead) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int t = tb + u;
+      if (t < t1) {
+        float2 acc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] = make_float2(0.f, 0.f);
+        const float g1 = stepped ? tg[u] : dh;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float2 gate = keyed ? make_float2(g1, g1) : f[u][r];
+          const float2 write = stepped ? scan_mul2(make_float2(tf[u], tf[u]), f[u][r])
+                               : keyed ? f[u][r] : make_float2(1.f - f[u][r].x, 1.f - f[u][r].y);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            St[r][c] = scan_fma2(gate, St[r][c], scan_mul2(write, make_float2(vv[u][c], vv[u][c])));
+            if (MODE != 1) acc[c] = scan_fma2(St[r][c], q[u][r], acc[c]);
+          }
+          if (MODE == 1) prod[r] = scan_mul2(prod[r], gate);
+        }
+        if (MODE != 1) {
+          float a0 = acc[0].x + acc[0].y, a1 = acc[1].x + acc[1].y, a2 = acc[2].x + acc[2].y, a3 = acc[3].x + acc[3].y;
+          float* dst = o + (size_t)t * H * Dv + (size_t)h * Dv + j;
+          if (S == 1) {
+            if (live) *reinterpret_cast<float4*>(dst) = make_float4(a0, a1, a2, a3);
+          } else {
+            // the first two exchanges halve the columns a lane keeps, the others add up the rest of the lanes
+            const bool hi = s & 1;
+            const float x0 = __shfl_xor_sync(0xffffffffu, hi ? a0 : a2, 1), x1 = __shfl_xor_sync(0xffffffffu, hi ? a1 : a3, 1);
+            a0 = (hi ? a2 : a0) + x0;
+            a1 = (hi ? a3 : a1) + x1;
+            if (S == 2) {
+              if (live) *reinterpret_cast<float2*>(dst + 2 * s) = make_float2(a0, a1);
+            } else {
+              const bool hj = s & 2;
+              const float y = __shfl_xor_sync(0xffffffffu, hj ? a0 : a1, 2);
+              a0 = (hj ? a1 : a0) + y;
+              for (int off = 4; off < S; off <<= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+              if (live && s < 4) dst[2 * (s & 1) + (s >> 1)] = a0;
+            }
+          }
+        }
+      }
+      fetch(u, min(t + kAhead, t1 - 1));
+    }
+  }
+  if (MODE == 1) {
+    float* end = ws + ((size_t)seq * NC + chunk + 1) * HDDv + ((size_t)h * D + i0) * Dv + jj;
+    float* dec = decay + (((size_t)seq * NC + chunk + 1) * H + h) * D + i0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (live) {
+        *reinterpret_cast<float4*>(end + (size_t)(2 * r) * Dv) = make_float4(St[r][0].x, St[r][1].x, St[r][2].x, St[r][3].x);
+        *reinterpret_cast<float4*>(end + (size_t)(2 * r + 1) * Dv) = make_float4(St[r][0].y, St[r][1].y, St[r][2].y, St[r][3].y);
+      }
+      if (blockIdx.x == 0 && threadIdx.x < S) *reinterpret_cast<float2*>(dec + 2 * r) = prod[r];
+    }
+    return;
+  }
+  if (write_state && live && t1 >= seq_end) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      *reinterpret_cast<float4*>(st + (size_t)(2 * r) * Dv) = make_float4(St[r][0].x, St[r][1].x, St[r][2].x, St[r][3].x);
+      *reinterpret_cast<float4*>(st + (size_t)(2 * r + 1) * Dv) = make_float4(St[r][0].y, St[r][1].y, St[r][2].y, St[r][3].y);
+    }
+  }
+}
+
 // How a head's state is cut among threads: C columns a thread, S slices of R rows.
 struct ScanShape { int C, S, R; };
 static inline ScanShape scan_shape(int D, int Dv) {
@@ -761,6 +930,35 @@ static void matrix_scan_launch(const ScanArgs& a, const ScanShape& g, cudaStream
 #undef LLMIE_SCAN_ARGS
 }
 
+template <typename T, int FORM>
+static void matrix_scan_wide_launch(const ScanArgs& a, cudaStream_t stream) {
+  const int S = a.D / 8, all = S * (a.Dv / 4), threads = all >= kScanThreads ? kScanThreads : (all + 31) / 32 * 32;
+  const int cols = threads / S * 4;
+  const bool chunked = a.ws != nullptr;
+  const dim3 grid((a.Dv + cols - 1) / cols, a.H, a.n_seqs * (chunked ? a.n_chunks : 1)), block(threads);
+#define LLMIE_SCAN_ARGS                                                                                                 \
+  grid, block, 0, stream, a.qa, a.fg, (const T*)a.v, a.v_ld, a.state, a.cu_q, a.seq_slot, a.o, a.H, a.D, a.Dv, S,       \
+      a.write_state, a.ws, a.decay, a.chunk, a.n_chunks, a.head_decay, a.key_factor, a.G
+  if (!chunked) {
+    launch_k(matrix_scan_wide_kernel<T, 0, FORM>, LLMIE_SCAN_ARGS);
+    return;
+  }
+  launch_k(matrix_scan_wide_kernel<T, 1, FORM>, LLMIE_SCAN_ARGS);
+  const size_t HDDv = (size_t)a.H * a.D * a.Dv;
+  launch_k(matrix_scan_chain_kernel, dim3((unsigned)((HDDv + 255) / 256), a.n_seqs), dim3(256), 0, stream,
+           (const float*)a.state, a.cu_q, a.seq_slot, a.ws, (const float*)a.decay, a.H, a.D, a.Dv, a.chunk, a.n_chunks);
+  launch_k(matrix_scan_wide_kernel<T, 2, FORM>, LLMIE_SCAN_ARGS);
+#undef LLMIE_SCAN_ARGS
+}
+
+// Whether the kernel with 8 rows and 4 columns a thread takes these sizes and places (see there).
+static bool matrix_scan_wide_ok(const ScanArgs& a, int dtype) {
+  const int S = a.D / 8;
+  return a.D % 8 == 0 && (S & (S - 1)) == 0 && S <= 32 && a.Dv % 4 == 0 && a.v_ld % 4 == 0 && aligned16(a.qa) &&
+         aligned16(a.fg) && aligned16(a.state) && aligned16(a.o) && (!a.ws || (aligned16(a.ws) && aligned16(a.decay))) &&
+         (reinterpret_cast<uintptr_t>(a.v) & (dtype == LLMIE_F32 ? 15u : 7u)) == 0;
+}
+
 template <int FORM>
 static int matrix_scan_entry(const ScanArgs& a, int dtype, cudaStream_t stream) {
   if (a.n_seqs < 0 || a.H <= 0 || a.D <= 0 || a.Dv <= 0 || a.v_ld < a.H * a.Dv || a.G <= 0 || a.H % a.G)
@@ -769,6 +967,13 @@ static int matrix_scan_entry(const ScanArgs& a, int dtype, cudaStream_t stream) 
   if (a.D > 32 * kScanR) return LLMIE_ERR_UNSUPPORTED_SIZE;
   if (a.n_seqs == 0) return LLMIE_OK;
   if (a.H > 65535 || a.n_seqs > 65535 || (a.ws && (long long)a.n_seqs * a.n_chunks > 65535)) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (dtype != LLMIE_F32 && dtype != LLMIE_BF16) return LLMIE_ERR_DTYPE;
+  if (matrix_scan_wide_ok(a, dtype)) {
+    if (dtype == LLMIE_F32) matrix_scan_wide_launch<float, FORM>(a, stream);
+    else matrix_scan_wide_launch<__nv_bfloat16, FORM>(a, stream);
+    LLMIE_LAUNCH_CHECK();
+    return LLMIE_OK;
+  }
   const ScanShape g = scan_shape(a.D, a.Dv);
   if (dtype == LLMIE_F32) {
     if (g.C == 4) matrix_scan_launch<float, 4, kScanRWide, FORM>(a, g, stream);
