@@ -1,8 +1,8 @@
 // Plain attention over the paged KV cache, for any number of new tokens per sequence.
 //
-// One warp per (token, query head). It is the float32 path's attention for prefill and
-// decode alike, and the plain twin that the tensor-core and split-KV kernels are checked
-// against. The math is that of the reference's prefill and decode kernels
+// One warp per (token, query head). It is the float32 path's attention for prompts with options
+// or sizes that attention_prefill_f32.cu does not take, and the plain twin that the tensor-core,
+// tiled and split-KV kernels are checked against. The math is that of the reference's prefill and decode kernels
 // (src/flash_attn.py:42-82, src/flash_decode.py:73-113): scores q.k / sqrt(hd) over the keys
 // a token may see, online softmax with float32 running max / sum / accumulator, query head
 // h reading key/value head h / (Hq / Hkv).

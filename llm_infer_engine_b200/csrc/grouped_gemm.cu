@@ -157,7 +157,12 @@ struct MmaTile {
   static constexpr int kStages = BM == 16 && !DUAL ? 5 : 3;
   static constexpr int kOutPitch = kMmaBN + 4;                          // floats between two rows on their way out
   static constexpr int kOutBytes = BM * kOutPitch * 4;
-  static constexpr int smem_bytes() { return kStages * kStageBytes > kOutBytes ? kStages * kStageBytes : kOutBytes; }
+  // a K of fewer steps leaves the ring's other stages out: 2,100 rows of 32 heads, 64 -> 256 (one step): six blocks an SM
+  // instead of four, 22.7 us instead of 26.7
+  static int smem_bytes(int steps) {
+    const int ring = (steps < kStages ? steps : kStages) * kStageBytes;
+    return ring > kOutBytes ? ring : kOutBytes;
+  }
 };
 
 template <typename TC, int BM, bool DUAL>
@@ -317,9 +322,10 @@ template <typename TC, int BM, bool DUAL>
 static int launch_mma_tile(const GroupedArgs& p, dim3 grid, int vec, int cvec, cudaStream_t stream) {
   using T = MmaTile<BM, DUAL>;
   auto kernel = grouped_gemm_mma_kernel<TC, BM, DUAL>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::smem_bytes());
+  const int smem = T::smem_bytes((p.K + kMmaBK - 1) / kMmaBK);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  launch_k(kernel, grid, dim3(128), T::smem_bytes(), stream, p, vec, cvec);
+  launch_k(kernel, grid, dim3(128), smem, stream, p, vec, cvec);
   return LLMIE_OK;
 }
 

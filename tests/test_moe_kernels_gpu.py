@@ -84,3 +84,17 @@ def test_head_norm(Dv, items, per_row, dtype, gated):
         ref = ref * torch.sigmoid(gate.double())
     rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18
     assert bool(((y.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("T,n,q_off,f_off,pad", [(1, 8, 0, 8, 0), (70, 1032, 8, 1048, 8), (3, 100, 0, 100, 0), (2, 64, 4, 72, 4)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gates_of_a_recurrence(T, n, q_off, f_off, pad, dtype):
+    g = torch.Generator().manual_seed(T + n)
+    proj = (torch.randn(T, f_off + n + pad, generator=g) * 3).to(dtype).to(DEV)
+    bias, lower = torch.randn(n, generator=g).to(DEV), (torch.rand(n, generator=g) * 0.9).to(DEV)
+    q, f = torch.empty(T, n, device=DEV), torch.empty(T, n, device=DEV)
+    ops().matrix_gates(proj, q_off, f_off, bias, lower, q, f)
+    x, z = proj[:, q_off:q_off + n].double(), proj[:, f_off:f_off + n].double() + bias.double()
+    want_q, want_f = x * torch.sigmoid(x), lower.double() + (1 - lower.double()) * torch.sigmoid(z)
+    assert bool(((q.double() - want_q).abs() <= 2.0 ** -19 * want_q.abs() + 1e-30).all())
+    assert bool(((f.double() - want_f).abs() <= 2.0 ** -19 * (want_f.abs() + z.abs())).all())
