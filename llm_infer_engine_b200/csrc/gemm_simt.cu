@@ -7,8 +7,8 @@
 // result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
 //
 // What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
-// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 46 TFLOP/s of
-// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 830 us so; a
+// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 48 TFLOP/s of
+// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 785 us so; a
 // one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
 // (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 //
@@ -63,17 +63,18 @@ __device__ __forceinline__ float4 read_peer(const float4* p, unsigned rank) {
 
 // ---------------------------------------------------------------------------------------------------------------
 // Tiles for more than kFewRows rows: WM x WN warps, each 32 x 64 outputs, a thread 8 x 8 of them (rows lane / 8 + 4 i,
-// columns lane % 8 + 8 j), all 16 k of a stage read as four 16-byte pieces a row: rows lie 20 floats apart in shared
+// columns lane % 8 + 8 j), all 32 k of a stage read as eight 16-byte pieces a row: rows lie 36 floats apart in shared
 // memory, so the eight rows a 16-byte access touches fall on different banks. The 8 x 8 packed sums are 128 registers;
 // at a chain's end they are added up into shared memory, a slot per thread. `split` blocks of a cluster share a tile's
 // chains (8 / split chains each, rank 0 the first ones); their sums meet in distributed shared memory in chain order.
-constexpr int kBK = 16, kStride = 20;
+constexpr int kBK = 32, kStride = 36;
 
 template <int WM, int WN>
 struct Tile {
   static constexpr int BM = 32 * WM, BN = 64 * WN, kThreads = 32 * WM * WN;
-  // 32 x 128: three stages, so that four blocks share an SM (32,000 x 2,048, 20 rows: 127 us, 143 with four stages)
-  static constexpr int kStages = WM == 1 ? 3 : 4;
+  // two stages of 32 k: four blocks share an SM, a barrier for every 1,024 packed FMAs a thread (2,048 x 8,192, 301 rows: 275
+  // us; four stages of 16 k 292, three of 32 k, three blocks an SM, 294)
+  static constexpr int kStages = 2;
   static constexpr int kStageFloats = (BM + BN) * kStride;
   static constexpr int kSumFloats = BM * BN;
   // the sums of the last chain of a rank > 0 lie where the stages were
@@ -97,17 +98,17 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
 
   const int n_chains = kChains / split, chain0 = rank * n_chains;
   const int n_slices = (K + kSlice - 1) / kSlice;
-  // the blocks of 16 k that this block works on, chain by chain (each a whole slice: k >= K reads zeros)
+  // the blocks of 32 k that this block works on, chain by chain (each a whole slice: k >= K reads zeros)
   int total_blocks = 0;
   for (int j = chain0; j < chain0 + n_chains; ++j)
     if (j < n_slices) total_blocks += ((n_slices - 1 - j) / kChains + 1) * (kSlice / kBK);
 
-  // ---- loading, T::kStages - 1 blocks early. A thread brings piece tid % 4 of the rows tid / 4 + kStep p: rows of A first,
+  // ---- loading, T::kStages - 1 blocks early. A thread brings piece tid % 8 of the rows tid / 8 + kStep p: rows of A first,
   // then of W. What is left of each piece is an address and a copy, in tiles whose rows are all there; looking at every
   // piece's row and k took two instructions for every three of the products.
-  constexpr int kStep = T::kThreads / 4, kPiecesA = T::BM / kStep, kPiecesW = T::BN / kStep;
+  constexpr int kStep = T::kThreads / (kBK / 4), kPiecesA = T::BM / kStep, kPiecesW = T::BN / kStep;
   static_assert(T::BM % kStep == 0 && T::BN % kStep == 0, "a piece's row is one of A's or one of W's for all threads");
-  const int ld_row = tid >> 2, ld_c = (tid & 3) * 4;
+  const int ld_row = tid / (kBK / 4), ld_c = tid % (kBK / 4) * 4;
   const bool rows_there = m0 + T::BM <= M && n0 + T::BN <= N;
   // how many of this thread's rows there are (they come in order), and its first ones
   const int a_there = M - m0 - ld_row, w_there = N - n0 - ld_row;        // row p is there if p * kStep is below
@@ -443,10 +444,10 @@ static int dispatch(const float* A, const float* W, float* C, int M, int N, int 
 // Few rows: 8 weight rows a block and six stages where that gives no SM more than two blocks (2,048 x 8,192, 1 / 8 rows:
 // 18 / 35, form 20 26 / 44); 16 weight rows a block above (16,384 x 2,048, 1 / 3 rows: 26 / 30, form 10 29 / 42), and 32
 // from 5 rows on, where a thread's reads of A cost more than its weights (16,384 x 2,048, 8 / 13 rows: 38 / 60, form 20
-// 49 / 76). Tiles: 32 rows high up to 32 rows (32,000 x 2,048, 20 rows: 127, 64 high 214), else 64 x 64 (301 rows: 84, 32
-// x 128 90). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
-// 291, 4 blocks 342, 1 block 520), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 529, 8
-// 532, 1 551), then each tile has one block (32,000 x 2,048, 512 rows: 1,504, 4 blocks 1,576).
+// 49 / 76). Tiles: 32 rows high up to 32 rows (16,384 x 2,048, 20 rows: 74, 64 high 115), else 64 x 64 (301 rows: 79, 32
+// x 128 89). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
+// 275, 4 blocks 320, 1 block 463), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 499, 8
+// 507, 1 516), then each tile has one block (16,384 x 2,048, 512 rows: 723, 4 blocks 776).
 static int choose_form(int M, int N) {
   if (M <= kFewRows) {
     const bool narrow = N <= 2 * 8 * 148;
