@@ -165,8 +165,11 @@ struct MmaTile {
   }
 };
 
+// Short products of full tiles wait for their loads, and registers set how many blocks wait at once: eight blocks an SM
+// (64 registers, nothing spilled) instead of six (78) take a latent-attention layer over 2,100 rows, with two products a
+// head, from 163.9 to 162.0 us. Longer rings and pairs of weights are held by shared memory instead.
 template <typename TC, int BM, bool DUAL>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, BM == 64 && !DUAL ? 8 : 1)
 grouped_gemm_mma_kernel(const GroupedArgs p, const int vec, const int cvec) {
   using T = MmaTile<BM, DUAL>;
   constexpr int NW = DUAL ? 2 : 1, kSlices = BM / 16, BK = kMmaBK, BN = kMmaBN;
