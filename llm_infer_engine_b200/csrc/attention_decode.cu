@@ -47,11 +47,11 @@ __device__ __forceinline__ int first_visible(int len, int window) {
 // per block instead of one per key. run_len must be 64.
 template <typename T, int HD, int GMAX>
 __global__ void __launch_bounds__(kDecThreads)
-decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
-                    float* __restrict__ part_m, float* __restrict__ part_l, float* __restrict__ part_acc,
-                    const int* __restrict__ seq_slot, const int* __restrict__ seq_kvlen,
-                    const int* __restrict__ block_table, int max_pages, int page_size, int n_q, int n_kv,
-                    float scale, int window, int run_len, int n_runs, int* __restrict__ counters,
+decode_split_kernel(const T* q, const T* k_cache, const T* v_cache,
+                    float* part_m, float* part_l, float* part_acc,
+                    const int* seq_slot, const int* seq_kvlen,
+                    const int* block_table, int max_pages, int page_size, int n_q, int n_kv,
+                    float scale, int window, int run_len, int n_runs, int* counters,
                     T* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -285,9 +285,9 @@ decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, cons
 // Merge of the runs (src/flash_decode.py:182-205): M = max m_r, w_r = exp(m_r - M),
 // out = sum w_r acc_r / sum w_r l_r, over the runs that hold a visible key, in run order.
 template <typename T>
-__global__ void decode_merge_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
-                                    const float* __restrict__ part_acc, T* __restrict__ out,
-                                    const int* __restrict__ seq_kvlen, int n_q, int hd, int window, int run_len,
+__global__ void decode_merge_kernel(const float* part_m, const float* part_l,
+                                    const float* part_acc, T* __restrict__ out,
+                                    const int* seq_kvlen, int n_q, int hd, int window, int run_len,
                                     int n_runs) {
   pdl_launch_dependents();
   pdl_wait();

@@ -148,12 +148,12 @@ __device__ __forceinline__ void md_merge_head(const float* part_m, const float* 
 // and (with write_kv) into the cache. Rotation in float32, one rounding to bfloat16, as the separate kernel.
 template <int HD, int WARPS, bool ROPE>
 __global__ void __launch_bounds__(WARPS * 32, (HD == 64 && WARPS <= 4) ? 16 / WARPS : 1)
-decode_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* k_cache,
-                  const __nv_bfloat16* v_cache, float* __restrict__ part_m, float* __restrict__ part_l,
-                  float* __restrict__ part_acc, const int* __restrict__ seq_slot, const int* __restrict__ seq_kvlen,
-                  const int* __restrict__ block_table, int max_pages, int n_q, int n_kv, float scale, int window,
-                  int pages_per_run, int n_runs, int* __restrict__ counters, __nv_bfloat16* __restrict__ out,
-                  const float2* __restrict__ rope, int table_len, int q_ld, int write_kv, MdOptions opt) {
+decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
+                  const __nv_bfloat16* v_cache, float* part_m, float* part_l,
+                  float* part_acc, const int* seq_slot, const int* seq_kvlen,
+                  const int* block_table, int max_pages, int n_q, int n_kv, float scale, int window,
+                  int pages_per_run, int n_runs, int* counters, __nv_bfloat16* __restrict__ out,
+                  const float2* LLMIE_WEIGHT rope, int table_len, int q_ld, int write_kv, MdOptions opt) {
   pdl_launch_dependents();
   constexpr int PITCH = HD + 8;                         // elements; rows 16 bytes apart in the banks
   constexpr int KS = HD / 16;                           // k-steps of Q K^T

@@ -18,9 +18,9 @@ static inline int row_threads(int d) {
 // Embedding stage: x = h[t] * scale + pos_table[tok_pos[t]];  h[t] = norm_w ? x * rsqrt(mean(x^2) + eps) * norm_w : x;
 // act[t] = h[t] rounded to A (optional). pos_table and norm_w are optional. One block per token.
 template <typename P, typename A>
-__global__ void scale_pos_norm_kernel(float* __restrict__ h, float scale, const P* __restrict__ pos_table,
-                                      int table_len, const int* __restrict__ tok_pos,
-                                      const float* __restrict__ norm_w, float eps, A* __restrict__ act, int d) {
+__global__ void scale_pos_norm_kernel(float* h, float scale, const P* LLMIE_WEIGHT pos_table,
+                                      int table_len, const int* tok_pos,
+                                      const float* LLMIE_WEIGHT norm_w, float eps, A* __restrict__ act, int d) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float row_buf[];
@@ -57,8 +57,8 @@ __global__ void scale_pos_norm_kernel(float* __restrict__ h, float scale, const 
 //   x = y[t] (+ bias);  h[t] += x * rsqrt(mean(x^2) + eps) * w;  act[t] = h[t] rounded to A (optional)
 // One block per row.
 template <typename Y, typename A>
-__global__ void branch_norm_add_kernel(float* __restrict__ h, const Y* __restrict__ y, const float* __restrict__ bias,
-                                       const float* __restrict__ w, float eps, A* __restrict__ act, int d) {
+__global__ void branch_norm_add_kernel(float* h, const Y* y, const float* LLMIE_WEIGHT bias,
+                                       const float* LLMIE_WEIGHT w, float eps, A* __restrict__ act, int d) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float row_buf[];
@@ -85,8 +85,8 @@ __global__ void branch_norm_add_kernel(float* __restrict__ h, const Y* __restric
 // The same for rows of at most 8 * 1024 elements with d % 8 == 0: a thread owns one run of 8 elements, kept in
 // registers between the two passes, with 16-byte loads and stores.
 template <typename Y, typename A>
-__global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const Y* __restrict__ y,
-                                           const float* __restrict__ bias, const float* __restrict__ w, float eps,
+__global__ void branch_norm_add_vec_kernel(float* h, const Y* y,
+                                           const float* LLMIE_WEIGHT bias, const float* LLMIE_WEIGHT w, float eps,
                                            A* __restrict__ act, int d) {
   pdl_launch_dependents();
   pdl_wait();
@@ -128,8 +128,8 @@ __global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const Y* __res
 //   x = alpha * h[t] + s (.) y[t];  h[t] = x * rsqrt(mean(x^2) + eps) * w;  act[t] = h[t] rounded to A (optional)
 // s is optional (null = ones). The stream stays float32. One block per row.
 template <typename Y, typename A>
-__global__ void scaled_sum_norm_kernel(float* __restrict__ h, const Y* __restrict__ y, const float* __restrict__ s,
-                                       float alpha, const float* __restrict__ w, float eps, A* __restrict__ act,
+__global__ void scaled_sum_norm_kernel(float* h, const Y* y, const float* LLMIE_WEIGHT s,
+                                       float alpha, const float* LLMIE_WEIGHT w, float eps, A* __restrict__ act,
                                        int d) {
   pdl_launch_dependents();
   pdl_wait();
@@ -157,8 +157,8 @@ __global__ void scaled_sum_norm_kernel(float* __restrict__ h, const Y* __restric
 // The same for rows of at most 8 * 1024 elements with d % 8 == 0: a thread owns one run of 8 elements, kept in
 // registers between the two passes, with 16-byte loads and stores.
 template <typename Y, typename A>
-__global__ void scaled_sum_norm_vec_kernel(float* __restrict__ h, const Y* __restrict__ y,
-                                           const float* __restrict__ s, float alpha, const float* __restrict__ w,
+__global__ void scaled_sum_norm_vec_kernel(float* h, const Y* y,
+                                           const float* LLMIE_WEIGHT s, float alpha, const float* LLMIE_WEIGHT w,
                                            float eps, A* __restrict__ act, int d) {
   pdl_launch_dependents();
   __shared__ float red[32];
@@ -197,7 +197,7 @@ __global__ void scaled_sum_norm_vec_kernel(float* __restrict__ h, const Y* __res
 // RMS norm of a run of columns of wider rows: out[t, i] = x * rsqrt(mean(x^2) + eps) * w[i], x = src[t * ld + off + i],
 // i < n (the latent that queries pass through). float32 arithmetic, one rounding at the store. One block per row.
 template <typename T>
-__global__ void rmsnorm_cols_kernel(const T* __restrict__ src, int ld, int off, const float* __restrict__ w, float eps,
+__global__ void rmsnorm_cols_kernel(const T* src, int ld, int off, const float* LLMIE_WEIGHT w, float eps,
                                     T* __restrict__ out, int n) {
   pdl_launch_dependents();
   pdl_wait();
@@ -216,7 +216,7 @@ __global__ void rmsnorm_cols_kernel(const T* __restrict__ src, int ld, int off, 
 // out[t, j] = act(u[t, j] + bias[j]); bias optional. Activations: 0 none, 1 relu, 2 relu squared, 3 gelu (tanh
 // form), 4 silu.
 template <typename T, typename O>
-__global__ void bias_act_kernel(const T* __restrict__ u, const float* __restrict__ bias, O* __restrict__ out, int n,
+__global__ void bias_act_kernel(const T* u, const float* LLMIE_WEIGHT bias, O* __restrict__ out, int n,
                                 size_t total, int act) {
   pdl_launch_dependents();
   pdl_wait();
@@ -231,7 +231,7 @@ __global__ void bias_act_kernel(const T* __restrict__ u, const float* __restrict
 
 // The same, eight outputs a thread with 16-byte loads (n % 8 == 0): grid (column blocks, rows), no index division.
 template <typename T, typename O>
-__global__ void bias_act_vec_kernel(const T* __restrict__ u, const float* __restrict__ bias, O* __restrict__ out, int n8,
+__global__ void bias_act_vec_kernel(const T* u, const float* LLMIE_WEIGHT bias, O* __restrict__ out, int n8,
                                     int n_tokens, int act) {
   pdl_launch_dependents();
   pdl_wait();
@@ -267,7 +267,7 @@ __global__ void bias_act_vec_kernel(const T* __restrict__ u, const float* __rest
 
 // out = float32 -> A, element by element
 template <typename A>
-__global__ void cast_rows_kernel(const float* __restrict__ x, A* __restrict__ out, size_t total) {
+__global__ void cast_rows_kernel(const float* x, A* __restrict__ out, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -278,7 +278,7 @@ __global__ void cast_rows_kernel(const float* __restrict__ x, A* __restrict__ ou
 // out[t, j] *= sigmoid(gate[t * ld + j / group]): group 1 = a gate per element, group = a head's value size = one
 // gate per head
 template <typename T>
-__global__ void sigmoid_gate_kernel(T* __restrict__ out, const T* __restrict__ gate, int ld, int n, int group,
+__global__ void sigmoid_gate_kernel(T* out, const T* gate, int ld, int n, int group,
                                     size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -296,7 +296,7 @@ __global__ void sigmoid_gate_kernel(T* __restrict__ out, const T* __restrict__ g
 // of 2,048 behind a projection of 5,408 columns took 13.6 us element by element, 5.9 us so.
 template <typename T>
 __global__ void __launch_bounds__(256)
-sigmoid_gate_vec_kernel(T* __restrict__ out, const T* __restrict__ gate, int ld, int n) {
+sigmoid_gate_vec_kernel(T* out, const T* gate, int ld, int n) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.y;
@@ -324,12 +324,12 @@ __device__ __forceinline__ float query_temperature(int pos, float coef, int ever
 //   k_cache[page(t), hk, pos % P, :] = k'   v_cache[...] = v'   (only with write_kv)
 // lam is read from device memory (a checkpoint scalar). One block per token.
 template <typename T>
-__global__ void qk_norm_store_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_out, T* __restrict__ k_cache,
-                                     T* __restrict__ v_cache, const float* __restrict__ q_w,
-                                     const float* __restrict__ k_w, float eps, const float* __restrict__ lam_ptr,
-                                     const T* __restrict__ v_first, int v_first_ld, const int* __restrict__ tok_pos,
-                                     const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
-                                     const int* __restrict__ block_table, int max_pages, int page_size, int n_q,
+__global__ void qk_norm_store_kernel(const T* proj, int ld, T* __restrict__ q_out, T* __restrict__ k_cache,
+                                     T* __restrict__ v_cache, const float* LLMIE_WEIGHT q_w,
+                                     const float* LLMIE_WEIGHT k_w, float eps, const float* LLMIE_WEIGHT lam_ptr,
+                                     const T* v_first, int v_first_ld, const int* tok_pos,
+                                     const int* tok_seq, const int* seq_slot,
+                                     const int* block_table, int max_pages, int page_size, int n_q,
                                      int n_kv, int hd, int hdv, int write_kv, float temp_coef, int temp_every) {
   pdl_launch_dependents();
   pdl_wait();
@@ -385,13 +385,13 @@ __global__ void qk_norm_store_kernel(const T* __restrict__ proj, int ld, T* __re
 // and the store. Keys are read again for the store (from L1), values once. The lookups of the token's cache page,
 // a chain of three dependent loads, are placed so that no data load waits behind them.
 template <typename T, int R>
-__global__ void qk_norm_store_vec_kernel(const T* __restrict__ proj, int ld, T* __restrict__ q_out,
+__global__ void qk_norm_store_vec_kernel(const T* proj, int ld, T* __restrict__ q_out,
                                          T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                         const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
-                                         const float* __restrict__ lam_ptr, const T* __restrict__ v_first,
-                                         int v_first_ld, const int* __restrict__ tok_pos,
-                                         const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
-                                         const int* __restrict__ block_table, int max_pages, int page_size, int n_q,
+                                         const float* LLMIE_WEIGHT q_w, const float* LLMIE_WEIGHT k_w, float eps,
+                                         const float* LLMIE_WEIGHT lam_ptr, const T* v_first,
+                                         int v_first_ld, const int* tok_pos,
+                                         const int* tok_seq, const int* seq_slot,
+                                         const int* block_table, int max_pages, int page_size, int n_q,
                                          int n_kv, int hd, int hdv, int write_kv, float temp_coef, int temp_every) {
   pdl_launch_dependents();
   pdl_wait();

@@ -137,6 +137,14 @@ static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t
 // weights that no kernel writes - overlaps the previous kernel's tail. Both calls are no-ops
 // in a kernel launched the ordinary way. llmie_set_pdl(0) turns the attribute off for this library's launches
 // (each kernel library has its own copy of the switch).
+//
+// Pointers of such a kernel. What a kernel in front of it may write (activations, states, caches, index arrays) comes
+// through plain pointers. `const T* __restrict__` says that nothing changes the data while this kernel runs, and it runs
+// from before the wait on: the compiler may then read it by the read-only path, which is not ordered behind pdl_wait(), and
+// gather such reads with those in front of the wait. Kernels that read weights before their wait and a projection so marked
+// behind it returned wrong rows now and then as soon as the kernel in front let them start early. LLMIE_WEIGHT marks what is
+// fixed while kernels run (weights, tables of angles); __restrict__ stays on what a kernel only writes.
+#define LLMIE_WEIGHT __restrict__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

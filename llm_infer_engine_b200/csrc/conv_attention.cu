@@ -79,7 +79,7 @@ __device__ __forceinline__ void ca_store2(__nv_bfloat16* p, bool pair, bool seco
 // next goes token by token, with all K inputs of each.
 template <typename TP, typename TO, int NP, int KM, int TILE>
 __global__ void __launch_bounds__(kCaWarps * 32)
-conv_qk_store_kernel(const TP* __restrict__ proj, TO* __restrict__ q_out, TO* __restrict__ k_cache,
+conv_qk_store_kernel(const TP* proj, TO* __restrict__ q_out, TO* __restrict__ k_cache,
                      TO* __restrict__ v_cache, const ConvQkArgs p) {
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
@@ -200,7 +200,7 @@ conv_qk_store_kernel(const TP* __restrict__ proj, TO* __restrict__ q_out, TO* __
 // square) is shared by the heads of a warp.
 template <typename TP, typename TO, int LPH, int TILE>
 __global__ void __launch_bounds__(kCaWarps * 32, 8)
-conv_qk_store8_kernel(const TP* __restrict__ proj, TO* __restrict__ q_out, TO* __restrict__ k_cache,
+conv_qk_store8_kernel(const TP* proj, TO* __restrict__ q_out, TO* __restrict__ k_cache,
                       TO* __restrict__ v_cache, const ConvQkArgs p, int page_shift) {
   constexpr int KM = 4, W = KM - 1, kHeads = 32 / LPH;
   pdl_launch_dependents();

@@ -9,7 +9,7 @@ namespace llmie {
 // ------------------------------------------------------------------------------------------
 // h[t, :] = table[token[t], :]         (src/model.py:157 of the reference: a plain row gather)
 template <typename W>
-__global__ void embedding_kernel(const int* __restrict__ tokens, const W* __restrict__ table,
+__global__ void embedding_kernel(const int* tokens, const W* LLMIE_WEIGHT table,
                                  float* __restrict__ h, int d, int vocab) {
   // The step's index arrays (positions, lengths, slots) come from the kernel before this one. Later
   // kernels read them ahead of their own waits, so nothing after this kernel may be scheduled before
@@ -32,9 +32,9 @@ __global__ void embedding_kernel(const int* __restrict__ tokens, const W* __rest
 //   y[b] = x * rsqrt(mean(x^2) + eps) * w     one rounding, at the store
 // One block per output row; the row is held in shared memory between the two passes.
 template <typename T>
-__global__ void add_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ delta,
-                                   const float* __restrict__ w, T* __restrict__ y,
-                                   const int* __restrict__ rows, int d, float eps) {
+__global__ void add_rmsnorm_kernel(float* h, const T* delta,
+                                   const float* LLMIE_WEIGHT w, T* __restrict__ y,
+                                   const int* rows, int d, float eps) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float row_buf[];
@@ -62,9 +62,9 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ 
 // The same for rows of at most 8 * 1024 elements with d % 8 == 0: each thread owns one run of 8
 // elements, kept in registers, so the row is read once.
 template <typename T>
-__global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const T* __restrict__ delta,
-                                       const float* __restrict__ w, T* __restrict__ y,
-                                       const int* __restrict__ rows, int d, float eps) {
+__global__ void add_rmsnorm_vec_kernel(float* h, const T* delta,
+                                       const float* LLMIE_WEIGHT w, T* __restrict__ y,
+                                       const int* rows, int d, float eps) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[32];
@@ -102,7 +102,7 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ h, const T* __restric
 
 // h += delta, no norm (used when a block arrangement needs the bare sum)
 template <typename T>
-__global__ void residual_add_kernel(float* __restrict__ h, const T* __restrict__ delta, size_t n) {
+__global__ void residual_add_kernel(float* h, const T* delta, size_t n) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -113,7 +113,7 @@ __global__ void residual_add_kernel(float* __restrict__ h, const T* __restrict__
 // ------------------------------------------------------------------------------------------
 // out[t, j] = silu(gate_up[t, j]) * gate_up[t, ff + j]      (src/model.py:23 of the reference)
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int ff, size_t total) {
+__global__ void swiglu_kernel(const T* gate_up, T* __restrict__ out, int ff, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,7 +141,7 @@ __device__ __forceinline__ float silu_for<__nv_bfloat16>(float g) {
 }
 
 template <typename T>
-__global__ void swiglu_vec_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int ff8, int n_tokens) {
+__global__ void swiglu_vec_kernel(const T* gate_up, T* __restrict__ out, int ff8, int n_tokens) {
   pdl_launch_dependents();
   pdl_wait();
   const int j8 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -166,11 +166,11 @@ __global__ void swiglu_vec_kernel(const T* __restrict__ gate_up, T* __restrict__
 // elements >= rot_dim pass through. table == nullptr means no rotation at all.
 // With write_kv == 0 only q is produced (a layer that reads another layer's cache).
 template <typename T>
-__global__ void rope_store_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
+__global__ void rope_store_kernel(const T* qkv, T* __restrict__ q_out,
                                   T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                  const float2* __restrict__ table, const int* __restrict__ tok_pos,
-                                  const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
-                                  const int* __restrict__ block_table, int max_pages, int page_size,
+                                  const float2* LLMIE_WEIGHT table, const int* tok_pos,
+                                  const int* tok_seq, const int* seq_slot,
+                                  const int* block_table, int max_pages, int page_size,
                                   int n_q, int n_kv, int hd, int hdv, int rot_dim, int table_len, int write_kv) {
   pdl_launch_dependents();
   pdl_wait();
@@ -234,11 +234,11 @@ __global__ void rope_store_kernel(const T* __restrict__ qkv, T* __restrict__ q_o
 // time with 16-byte loads and stores. Items per token: query heads, then key heads (rotated,
 // to the cache), then value heads (copied to the cache).
 template <typename T>
-__global__ void rope_store_vec_kernel(const T* __restrict__ qkv, T* __restrict__ q_out,
+__global__ void rope_store_vec_kernel(const T* qkv, T* __restrict__ q_out,
                                       T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                      const float2* __restrict__ table, const int* __restrict__ tok_pos,
-                                      const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
-                                      const int* __restrict__ block_table, int max_pages, int page_size,
+                                      const float2* LLMIE_WEIGHT table, const int* tok_pos,
+                                      const int* tok_seq, const int* seq_slot,
+                                      const int* block_table, int max_pages, int page_size,
                                       int n_q, int n_kv, int hd, int table_len, int write_kv) {
   pdl_launch_dependents();
   pdl_wait();
@@ -289,7 +289,7 @@ __global__ void rope_store_vec_kernel(const T* __restrict__ qkv, T* __restrict__
 // ------------------------------------------------------------------------------------------
 // Decode-step metadata from the device-resident lengths, so that a captured step needs no
 // host rewrites: lane i continues sequence slots[i] by one token at position len[slot].
-__global__ void prepare_decode_kernel(const int* __restrict__ slots, const int* __restrict__ seq_lens,
+__global__ void prepare_decode_kernel(const int* slots, const int* seq_lens,
                                       int* __restrict__ tok_pos, int* __restrict__ tok_seq,
                                       int* __restrict__ cu_q, int* __restrict__ seq_start,
                                       int* __restrict__ seq_kvlen, int n) {
@@ -308,7 +308,7 @@ __global__ void prepare_decode_kernel(const int* __restrict__ slots, const int* 
 }
 
 // seq_lens[slot] = kv length after the step, except for the scratch slot that padding lanes use.
-__global__ void advance_lengths_kernel(const int* __restrict__ slots, const int* __restrict__ seq_kvlen,
+__global__ void advance_lengths_kernel(const int* slots, const int* seq_kvlen,
                                        int* __restrict__ seq_lens, int n, int scratch_slot) {
   pdl_launch_dependents();
   pdl_wait();

@@ -202,8 +202,8 @@ __device__ __forceinline__ void fd_team_sync(int team, int threads) {
 // warp streams whole rows and nothing is exchanged at all.
 template <int VAR, int WARPS, bool BRANCH>
 __global__ void __launch_bounds__(WARPS * 32)
-norm_gemm_kernel(const float* __restrict__ h, const float* __restrict__ norm_w, float eps,
-                 const __nv_bfloat16* __restrict__ W, void* __restrict__ out, int batch, int K, int ldo, int tiles,
+norm_gemm_kernel(const float* h, const float* LLMIE_WEIGHT norm_w, float eps,
+                 const __nv_bfloat16* LLMIE_WEIGHT W, void* __restrict__ out, int batch, int K, int ldo, int tiles,
                  int half_n, int S, RopeStoreArgs rope, BranchArgs br) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) unsigned char fd_smem[];

@@ -12,10 +12,8 @@
 // one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
 // (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 //
-// These kernels wait for the one before them, but do not let the next one start early: when they did, rows behind a state
-// space or short-convolution layer's projection came out wrong now and then (one prompt in four of the 128-wide test model),
-// never with the next kernel held back. Kernels that follow a float32 product read it through read-only pointers behind work
-// of their own in front of their wait, and were written for a product that ends first.
+// These kernels wait for the one before them and let the next one start when they are done: letting it start early left the
+// time of a step as it was.
 #include "common.cuh"
 
 namespace llmie {
@@ -84,13 +82,13 @@ struct Tile {
 
 template <int WM, int WN, bool VEC>
 __global__ void __launch_bounds__(32 * WM * WN)
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
+gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N,
                      int K, int lda, int ldw, int ldc, int split) {
   using T = Tile<WM, WN>;
   extern __shared__ float4 smem4[];
   float* ring = reinterpret_cast<float*>(smem4);
   float4* held = smem4 + T::kRing / 4;                    // [16][kThreads]: a thread's 64 sums of earlier chains
-  pdl_wait();       // the next kernel starts when this one is done: see the top of the file
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x % split;
   const int m0 = blockIdx.y * T::BM, n0 = (blockIdx.x / split) * T::BN;
@@ -294,13 +292,13 @@ template <int MT, int WARPS, int RW, int STAGES, int RUN> struct Few {
 
 template <int MT, int WARPS, int RW, int STAGES, int RUN, bool VEC>
 __global__ void __launch_bounds__(32 * WARPS)
-gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N,
+gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N,
                     int K, int lda, int ldw, int ldc) {
   using F = Few<MT, WARPS, RW, STAGES, RUN>;
   constexpr int kRunStride = F::kRunStride;
   extern __shared__ float4 smem4[];
   float* ring = reinterpret_cast<float*>(smem4);
-  pdl_wait();       // the next kernel starts when this one is done: see the top of the file
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chain = lane & 7, row = warp * 4 * RW + (lane >> 3);
   const int n0 = blockIdx.x * F::kRows;

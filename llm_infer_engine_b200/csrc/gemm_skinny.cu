@@ -33,7 +33,8 @@ __device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], unsigned a0, uns
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+// 16 bytes of the activations, which the kernel before this one wrote: an ordinary load, not the read-only path
+__device__ __forceinline__ uint4 load_x16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 // 16 bytes of a weight row: read-only path, not kept in L1 (every byte is used once), and L2 is asked to
 // fetch 256 bytes around a miss (the rest of the run is about to be asked for)
 __device__ __forceinline__ uint4 ldg16_stream(const void* p) {
@@ -49,8 +50,8 @@ __device__ __forceinline__ uint4 ldg16_stream(const void* p) {
 // NB: batch blocks of 8 (batch <= 8 * NB). EPI: what happens to the 16 x batch results.
 template <int NB, int EPI, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ W, void* __restrict__ out,
-                   int batch, int K, int ldo, int tile_stride, int hi_delta, const float* __restrict__ bias, GateForm act) {
+skinny_gemm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* LLMIE_WEIGHT W, void* out,
+                   int batch, int K, int ldo, int tile_stride, int hi_delta, const float* LLMIE_WEIGHT bias, GateForm act) {
   pdl_launch_dependents();
   __shared__ float red[WARPS][NB][16][8 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -104,7 +105,7 @@ skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
         xcur[u][nb] = make_uint4(0u, 0u, 0u, 0u);
-        if (c < c_end && xok[nb]) xcur[u][nb] = ldg16(xr[nb] + c * 4);
+        if (c < c_end && xok[nb]) xcur[u][nb] = load_x16(xr[nb] + c * 4);
       }
     }
   }
@@ -120,7 +121,7 @@ skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
           xnext[u][nb] = make_uint4(0u, 0u, 0u, 0u);
-          if (c < c_end && xok[nb]) xnext[u][nb] = ldg16(xr[nb] + c * 4);
+          if (c < c_end && xok[nb]) xnext[u][nb] = load_x16(xr[nb] + c * 4);
         }
       }
     }
@@ -131,7 +132,7 @@ skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
           xcur[u][nb] = make_uint4(0u, 0u, 0u, 0u);
-          if (c < c_end && xok[nb]) xcur[u][nb] = ldg16(xr[nb] + c * 4);
+          if (c < c_end && xok[nb]) xcur[u][nb] = load_x16(xr[nb] + c * 4);
         }
       }
     }

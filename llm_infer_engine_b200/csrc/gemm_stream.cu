@@ -57,7 +57,7 @@ __device__ __forceinline__ void final_store(void* out, int mode, size_t idx, flo
 template <int MPAD>
 __global__ void __launch_bounds__(kSThreads, 1)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                   void* __restrict__ out, int M, int N, int K, int n_splits, int chunks_per_split, int n_tiles,
+                   void* out, int M, int N, int K, int n_splits, int chunks_per_split, int n_tiles,
                    int n_clusters, int n_stages, int mode, int* __restrict__ status) {
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];

@@ -18,12 +18,12 @@ namespace llmie {
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_prepare_kernel(const T* __restrict__ proj, int ld, const T* __restrict__ q_src, int q_ld, int q_off, int dkv_off,
+latent_prepare_kernel(const T* proj, int ld, const T* q_src, int q_ld, int q_off, int dkv_off,
                       T* __restrict__ q_out,
-                      T* __restrict__ cache, const float* __restrict__ norm_w, float eps,
-                      const float* __restrict__ table, int table_len, int rot_dims, const int* __restrict__ tok_pos,
-                      const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
-                      const int* __restrict__ block_table, int max_pages, int page_size, int n_heads, int dim, int rot,
+                      T* __restrict__ cache, const float* LLMIE_WEIGHT norm_w, float eps,
+                      const float* LLMIE_WEIGHT table, int table_len, int rot_dims, const int* tok_pos,
+                      const int* tok_seq, const int* seq_slot,
+                      const int* block_table, int max_pages, int page_size, int n_heads, int dim, int rot,
                       int rank, int write) {
   __shared__ float red[32];
   pdl_launch_dependents();

@@ -38,7 +38,7 @@ constexpr int kGateTokens = 16;
 // grid (channel tiles of 128, token tiles of kGateTokens); x rows of R numbers, ld apart; Bt float32 [R, N].
 template <typename T>
 __global__ void __launch_bounds__(128)
-low_rank_gate_kernel(const T* __restrict__ x, int ld, const float* __restrict__ Bt, const float* __restrict__ bias,
+low_rank_gate_kernel(const T* x, int ld, const float* LLMIE_WEIGHT Bt, const float* LLMIE_WEIGHT bias,
                      float* __restrict__ out, int R, int N, int n_tokens, int mode, float inv_tau) {
   extern __shared__ float gate_smem[];                          // [R][kGateTokens]
   pdl_launch_dependents();
@@ -78,8 +78,8 @@ low_rank_gate_kernel(const T* __restrict__ x, int ld, const float* __restrict__ 
 // qn, kn float32 [T, G D]; scal float32 [T, H, 2] = (beta, g); qk float32 [T, G] = q . k of the results.
 template <typename TC, typename TP>
 __global__ void __launch_bounds__(128)
-delta_prepare_kernel(const TC* __restrict__ qkv, int ld, const TP* __restrict__ ba, int ba_ld, int b_off, int a_off,
-                     const float* __restrict__ A, const float* __restrict__ dt_bias, float eps, float q_scale,
+delta_prepare_kernel(const TC* qkv, int ld, const TP* ba, int ba_ld, int b_off, int a_off,
+                     const float* LLMIE_WEIGHT A, const float* LLMIE_WEIGHT dt_bias, float eps, float q_scale,
                      float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ scal, float* __restrict__ qk,
                      int H, int G, int D) {
   pdl_launch_dependents();
@@ -118,9 +118,9 @@ delta_prepare_kernel(const TC* __restrict__ qkv, int ld, const TP* __restrict__ 
 // out[s][t][c] = x + (x_prev - x) mu[s][c], s < n_mix; x_prev of a piece's first token is prev[slot][c]. grid (column
 // blocks, tokens). `single`: one token per sequence, and prev receives it (in other steps the caller stores it afterwards).
 template <typename T>
-__global__ void shift_mix_kernel(const T* __restrict__ x, float* prev, const float* __restrict__ mu,
-                                 const int* __restrict__ cu_q, const int* __restrict__ tok_seq,
-                                 const int* __restrict__ seq_slot, T* __restrict__ out, int n_mix, int d, int n_tokens,
+__global__ void shift_mix_kernel(const T* x, float* prev, const float* LLMIE_WEIGHT mu,
+                                 const int* cu_q, const int* tok_seq,
+                                 const int* seq_slot, T* __restrict__ out, int n_mix, int d, int n_tokens,
                                  int single) {
   pdl_launch_dependents();
   pdl_wait();
@@ -140,9 +140,9 @@ __global__ void shift_mix_kernel(const T* __restrict__ x, float* prev, const flo
 
 // The same, eight channels a thread (d % 8 == 0, 16-byte aligned rows).
 template <typename T>
-__global__ void shift_mix8_kernel(const T* __restrict__ x, float* prev, const float* __restrict__ mu,
-                                  const int* __restrict__ cu_q, const int* __restrict__ tok_seq,
-                                  const int* __restrict__ seq_slot, T* __restrict__ out, int n_mix, int d, int n_tokens,
+__global__ void shift_mix8_kernel(const T* x, float* prev, const float* LLMIE_WEIGHT mu,
+                                  const int* cu_q, const int* tok_seq,
+                                  const int* seq_slot, T* __restrict__ out, int n_mix, int d, int n_tokens,
                                   int single) {
   pdl_launch_dependents();
   pdl_wait();

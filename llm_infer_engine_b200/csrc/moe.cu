@@ -31,9 +31,9 @@ constexpr int kRouteWarps = 8;
 // 16.9 us; 20 x 4,096, 40 tokens 15.9 -> 10.3 us (with a token a block and an expert a warp at a time before).
 template <typename T, int TB>
 __global__ void __launch_bounds__(kRouteWarps * 32)
-moe_route_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+moe_route_kernel(const T* x, const float* LLMIE_WEIGHT w, const float* LLMIE_WEIGHT bias,
                  int* __restrict__ ids, float* __restrict__ weights, int n_tokens, int d, int n_experts, int top,
-                 int mode, const float* __restrict__ correction, float out_scale, int n_groups, int keep, int pitch) {
+                 int mode, const float* LLMIE_WEIGHT correction, float out_scale, int n_groups, int keep, int pitch) {
   extern __shared__ __align__(16) float route_smem[];            // [TB][pitch] rows | per token logits, scores, groups
   float* xs = route_smem;
   const int per_token = 2 * n_experts + (mode == 3 ? n_groups : 0);
@@ -190,7 +190,7 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ w, const flo
 }
 
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int n_experts, int tile, int max_tiles,
+moe_sort_kernel(const int* ids, int n_pairs, int top, int n_experts, int tile, int max_tiles,
                 int* __restrict__ sorted_token, int* __restrict__ sorted_pair, int* __restrict__ tile_group,
                 int* __restrict__ group_end, int* __restrict__ pair_pos) {
   extern __shared__ int sm[];                      // counts | offsets | cursor, n_experts each
@@ -234,7 +234,7 @@ moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int top, int n_experts
 
 // out[p] = x[rows[p]] (zeros where rows[p] < 0): the tokens in the order of their experts, for a library product that
 // wants each expert's rows side by side. d % 8 == 0, 16-byte aligned.
-__global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ rows,
+__global__ void moe_gather_rows_kernel(const __nv_bfloat16* x, const int* rows,
                                        __nv_bfloat16* __restrict__ out, int d8, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -253,8 +253,8 @@ __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, cons
 // out[p, :] = weights[sorted_pair[p]] * x[sorted_token[p], :] (zeros where sorted_token[p] < 0); the product is formed
 // in float32 and rounded once to the output type.
 template <typename TI, typename TO>
-__global__ void moe_gather_scaled_kernel(const TI* __restrict__ x, const int* __restrict__ sorted_token,
-                                         const int* __restrict__ sorted_pair, const float* __restrict__ weights,
+__global__ void moe_gather_scaled_kernel(const TI* x, const int* sorted_token,
+                                         const int* sorted_pair, const float* weights,
                                          TO* __restrict__ out, int d, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -271,8 +271,8 @@ __global__ void moe_gather_scaled_kernel(const TI* __restrict__ x, const int* __
 }
 
 // 8 elements a thread (16-byte loads and stores), bfloat16 in and out, d % 8 == 0.
-__global__ void moe_gather_scaled_vec_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted_token,
-                                             const int* __restrict__ sorted_pair, const float* __restrict__ weights,
+__global__ void moe_gather_scaled_vec_kernel(const __nv_bfloat16* x, const int* sorted_token,
+                                             const int* sorted_pair, const float* weights,
                                              __nv_bfloat16* __restrict__ out, int d8, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -301,9 +301,9 @@ __global__ void moe_gather_scaled_vec_kernel(const __nv_bfloat16* __restrict__ x
 // 10.2 us so (5 TB/s).
 template <typename TS, typename TY, typename TX>
 __global__ void __launch_bounds__(256)
-moe_combine_vec_kernel(const TY* __restrict__ y, const int* __restrict__ pair_pos, const float* __restrict__ weights,
-                       const TS* __restrict__ shared_out, const int* __restrict__ ids, int n_real,
-                       const TX* __restrict__ x, float* __restrict__ out, int d, int top) {
+moe_combine_vec_kernel(const TY* y, const int* pair_pos, const float* weights,
+                       const TS* shared_out, const int* ids, int n_real,
+                       const TX* x, float* __restrict__ out, int d, int top) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.y;
@@ -332,8 +332,8 @@ moe_combine_vec_kernel(const TY* __restrict__ y, const int* __restrict__ pair_po
 }
 
 template <typename TS, typename TY>
-__global__ void moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ pair_pos,
-                                   const float* __restrict__ weights, const TS* __restrict__ shared_out,
+__global__ void moe_combine_kernel(const TY* y, const int* pair_pos,
+                                   const float* weights, const TS* shared_out,
                                    float* __restrict__ out, int d, int top, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -357,9 +357,9 @@ __device__ __forceinline__ float load_any(const void* p, int dtype, size_t i) {
 }
 
 // The combine with experts that return their input: a choice whose id is n_real or more adds weight * x[t].
-__global__ void moe_combine_identity_kernel(const void* __restrict__ y, int y_dtype, const int* __restrict__ pair_pos,
-                                            const float* __restrict__ weights, const int* __restrict__ ids, int n_real,
-                                            const void* __restrict__ x, int x_dtype, float* __restrict__ out, int d,
+__global__ void moe_combine_identity_kernel(const void* y, int y_dtype, const int* pair_pos,
+                                            const float* weights, const int* ids, int n_real,
+                                            const void* x, int x_dtype, float* __restrict__ out, int d,
                                             int top, size_t total) {
   pdl_launch_dependents();
   pdl_wait();

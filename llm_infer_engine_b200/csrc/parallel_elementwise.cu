@@ -20,10 +20,10 @@ __device__ __forceinline__ float load_as_f32(const void* p, int dtype, size_t i)
 // One thread per element of the produced rows. rows == nullptr: every row of h, and h is updated in place;
 // otherwise only the listed rows are produced and h stays as it is.
 template <typename TY>
-__global__ void add_dyt_kernel(float* __restrict__ h, const void* __restrict__ d1, int d1_dtype,
-                               const void* __restrict__ d2, int d2_dtype, const float* __restrict__ alpha,
-                               const float* __restrict__ w, const float* __restrict__ b, TY* __restrict__ y,
-                               const int* __restrict__ rows, int d, size_t total) {
+__global__ void add_dyt_kernel(float* h, const void* d1, int d1_dtype,
+                               const void* d2, int d2_dtype, const float* LLMIE_WEIGHT alpha,
+                               const float* LLMIE_WEIGHT w, const float* LLMIE_WEIGHT b, TY* __restrict__ y,
+                               const int* rows, int d, size_t total) {
   pdl_launch_dependents();
   const float a = alpha[0];          // a weight: no kernel writes it
   pdl_wait();
@@ -43,9 +43,9 @@ __global__ void add_dyt_kernel(float* __restrict__ h, const void* __restrict__ d
 
 // The same, eight elements a thread with 16-byte accesses: d % 8 == 0 and all pointers 16-byte aligned.
 template <typename TY, typename TD>
-__global__ void add_dyt_vec_kernel(float* __restrict__ h, const TD* __restrict__ d1, const TD* __restrict__ d2,
-                                   const float* __restrict__ alpha, const float* __restrict__ w,
-                                   const float* __restrict__ b, TY* __restrict__ y, const int* __restrict__ rows,
+__global__ void add_dyt_vec_kernel(float* h, const TD* d1, const TD* d2,
+                                   const float* LLMIE_WEIGHT alpha, const float* LLMIE_WEIGHT w,
+                                   const float* LLMIE_WEIGHT b, TY* __restrict__ y, const int* rows,
                                    int d, size_t total8) {
   pdl_launch_dependents();
   const float a = alpha[0];
@@ -80,7 +80,7 @@ __global__ void add_dyt_vec_kernel(float* __restrict__ h, const TD* __restrict__
 }
 
 template <typename T>
-__global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int ff, GateForm form, size_t total) {
+__global__ void gated_act_kernel(const T* gate_up, T* __restrict__ out, int ff, GateForm form, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,7 +96,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ 
 
 // ff % 8 == 0, 16-byte aligned: eight outputs a thread, a row of blocks per token (no index is divided)
 template <typename T>
-__global__ void gated_act_vec_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int ff, GateForm form) {
+__global__ void gated_act_vec_kernel(const T* gate_up, T* __restrict__ out, int ff, GateForm form) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.y;
@@ -111,7 +111,7 @@ __global__ void gated_act_vec_kernel(const T* __restrict__ gate_up, T* __restric
   }
 }
 
-__global__ void scale_rows_kernel(float* __restrict__ x, float s, size_t n) {
+__global__ void scale_rows_kernel(float* x, float s, size_t n) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,7 +119,7 @@ __global__ void scale_rows_kernel(float* __restrict__ x, float s, size_t n) {
   for (; i < n; i += stride) x[i] *= s;
 }
 
-__global__ void cap_rows_kernel(float* __restrict__ x, float c, size_t n) {
+__global__ void cap_rows_kernel(float* x, float c, size_t n) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -37,8 +37,8 @@ __device__ __forceinline__ float softplusf_(float z) { return fmaxf(z, 0.f) + lo
 
 // ------------------------------------------------------------------------------------------ matrix state
 template <typename T>
-__global__ void matrix_gates_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off,
-                                    const float* __restrict__ f_bias, const float* __restrict__ lower,
+__global__ void matrix_gates_kernel(const T* proj, int ld, int q_off, int f_off,
+                                    const float* LLMIE_WEIGHT f_bias, const float* LLMIE_WEIGHT lower,
                                     float* __restrict__ q_out, float* __restrict__ f_out, int n, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -60,8 +60,8 @@ __global__ void matrix_gates_kernel(const T* __restrict__ proj, int ld, int q_of
 // 2,150 tokens of 2 x 1,024: 10.9 us element by element with an index divided for each, 8.4 us so.
 template <typename T>
 __global__ void __launch_bounds__(128)
-matrix_gates_vec_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, const float* __restrict__ f_bias,
-                        const float* __restrict__ lower, float* __restrict__ q_out, float* __restrict__ f_out, int n) {
+matrix_gates_vec_kernel(const T* proj, int ld, int q_off, int f_off, const float* LLMIE_WEIGHT f_bias,
+                        const float* LLMIE_WEIGHT lower, float* __restrict__ q_out, float* __restrict__ f_out, int n) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.y;
@@ -100,11 +100,11 @@ constexpr int kScanRWide = 8;       // ... when it owns four columns
 // and the last one writes the slot's state.
 template <typename T, int MODE, int C, int RMAX, int FORM>
 __global__ void __launch_bounds__(kScanThreads)
-matrix_scan_kernel(const float* __restrict__ qa, const float* __restrict__ fg, const T* __restrict__ v, int v_ld,
-                   float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
+matrix_scan_kernel(const float* qa, const float* fg, const T* v, int v_ld,
+                   float* state, const int* cu_q, const int* seq_slot,
                    float* __restrict__ o, int H, int D, int Dv, int S, int R, int write_state,
-                   float* __restrict__ ws, float* __restrict__ decay, int L, int NC,
-                   const float* __restrict__ head_decay, const float* __restrict__ key_factor, int G) {
+                   float* ws, float* decay, int L, int NC,
+                   const float* head_decay, const float* key_factor, int G) {
   pdl_launch_dependents();
   // keyed forms: fg holds keys k_t instead of gates, and every row of head h has the same gate
   constexpr bool keyed = FORM != 0, stepped = FORM == 2;
@@ -247,11 +247,11 @@ __device__ __forceinline__ void scan_load4(const __nv_bfloat16* p, float (&v)[4]
 
 template <typename T, int MODE, int FORM>
 __global__ void __launch_bounds__(kScanThreads, MODE == 0 ? 7 : 4)
-matrix_scan_wide_kernel(const float* __restrict__ qa, const float* __restrict__ fg, const T* __restrict__ v, int v_ld,
-                        float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
-                        float* __restrict__ o, int H, int D, int Dv, int S, int write_state, float* __restrict__ ws,
-                        float* __restrict__ decay, int L, int NC, const float* __restrict__ head_decay,
-                        const float* __restrict__ key_factor, int G) {
+matrix_scan_wide_kernel(const float* qa, const float* fg, const T* v, int v_ld,
+                        float* state, const int* cu_q, const int* seq_slot,
+                        float* __restrict__ o, int H, int D, int Dv, int S, int write_state, float* ws,
+                        float* decay, int L, int NC, const float* head_decay,
+                        const float* key_factor, int G) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr bool keyed = FORM != 0, stepped = FORM == 2;
@@ -396,9 +396,9 @@ static inline ScanShape scan_shape(int D, int Dv) {
 
 // The chain over a sequence's chunks, a thread per element of the state: ws[0] = the slot's state and
 // ws[c] = decay[c] (.) ws[c - 1] + ws[c] for the chunks the sequence has, so that ws[c] is where chunk c starts.
-__global__ void matrix_scan_chain_kernel(const float* __restrict__ state, const int* __restrict__ cu_q,
-                                         const int* __restrict__ seq_slot, float* __restrict__ ws,
-                                         const float* __restrict__ decay, int H, int D, int Dv, int L, int NC) {
+__global__ void matrix_scan_chain_kernel(const float* state, const int* cu_q,
+                                         const int* seq_slot, float* ws,
+                                         const float* decay, int H, int D, int Dv, int L, int NC) {
   pdl_launch_dependents();
   pdl_wait();
   const int seq = blockIdx.y;
@@ -426,8 +426,8 @@ __device__ __forceinline__ float gate_factor(float z, int silu) { return (silu ?
 // the result is multiplied by sigmoid(gate) (or silu) of the same place. An item may also be a token's whole row (Dv = the
 // row). The weights repeat every w_items items (1: all heads share them).
 template <typename T>
-__global__ void head_rmsnorm_kernel(const float* __restrict__ o, const float* __restrict__ w, float eps,
-                                    T* __restrict__ y, int Dv, size_t n_items, const T* __restrict__ gate, int gate_ld,
+__global__ void head_rmsnorm_kernel(const float* o, const float* LLMIE_WEIGHT w, float eps,
+                                    T* __restrict__ y, int Dv, size_t n_items, const T* gate, int gate_ld,
                                     int items_per_row, int silu, int w_items) {
   pdl_launch_dependents();
   pdl_wait();
@@ -455,8 +455,8 @@ __global__ void head_rmsnorm_kernel(const float* __restrict__ o, const float* __
 // pass, 6.3 us so.
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256)
-head_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, float eps, T* __restrict__ y,
-                        size_t n_items, const T* __restrict__ gate, int gate_ld, int items_per_row, int silu,
+head_rmsnorm_vec_kernel(const float* o, const float* LLMIE_WEIGHT w, float eps, T* __restrict__ y,
+                        size_t n_items, const T* gate, int gate_ld, int items_per_row, int silu,
                         int w_items) {
   pdl_launch_dependents();
   pdl_wait();
@@ -487,8 +487,8 @@ head_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w
 // rows are not each one warp's work. Dv % 4 == 0 and 16-byte aligned rows: four elements a thread and access.
 template <typename T>
 __global__ void __launch_bounds__(256)
-row_rmsnorm_kernel(const float* __restrict__ o, const float* __restrict__ w, float eps, T* __restrict__ y, int Dv,
-                   const T* __restrict__ gate, int gate_ld, int items_per_row, int silu, int w_items) {
+row_rmsnorm_kernel(const float* o, const float* LLMIE_WEIGHT w, float eps, T* __restrict__ y, int Dv,
+                   const T* gate, int gate_ld, int items_per_row, int silu, int w_items) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[32];
@@ -522,7 +522,7 @@ row_rmsnorm_kernel(const float* __restrict__ o, const float* __restrict__ w, flo
 // Float32 copies of up to three runs of columns of proj [T, ld], each through the activation `act`:
 // out_k[t, c] = act(proj[t, off_k + c]), c < n_k. (What a linear-attention layer reads of its projections.)
 template <typename T>
-__global__ void act_columns_kernel(const T* __restrict__ proj, int ld, int off0, int n0, float* __restrict__ out0,
+__global__ void act_columns_kernel(const T* proj, int ld, int off0, int n0, float* __restrict__ out0,
                                    int off1, int n1, float* __restrict__ out1, int off2, int n2,
                                    float* __restrict__ out2, int act, size_t total) {
   pdl_launch_dependents();
@@ -587,10 +587,10 @@ __device__ __forceinline__ void conv_output(TO* dst, const float (&a)[V]) {
 // TILE: tokens a thread works on. A tile that lies within one sequence (nearly all do) asks for its TILE + K - 1 inputs at
 // once; one that crosses from a sequence into the next goes token by token, with all K inputs of each.
 template <typename TP, typename TO, int KM, int V, int TILE>
-__global__ void causal_conv_kernel(const TP* __restrict__ proj, int ld, int x_off, const float* __restrict__ x_bias,
-                                   const float* __restrict__ taps, const float* __restrict__ conv_bias,
-                                   float* conv_state, const int* __restrict__ cu_q,
-                                   const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
+__global__ void causal_conv_kernel(const TP* proj, int ld, int x_off, const float* LLMIE_WEIGHT x_bias,
+                                   const float* LLMIE_WEIGHT taps, const float* LLMIE_WEIGHT conv_bias,
+                                   float* conv_state, const int* cu_q,
+                                   const int* tok_seq, const int* seq_slot,
                                    TO* __restrict__ u, int C, int K, int n_tokens, int act, int single) {
   pdl_launch_dependents();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
@@ -679,9 +679,9 @@ __global__ void causal_conv_kernel(const TP* __restrict__ proj, int ld, int x_of
 // The convolution's new state: a thread per (sequence, channel) leaves the last K-1 inputs of the sequence, this step's
 // and before them what the state held.
 template <typename T>
-__global__ void conv_state_store_kernel(const T* __restrict__ proj, int ld, int x_off, const float* __restrict__ x_bias,
-                                        float* __restrict__ conv_state, const int* __restrict__ cu_q,
-                                        const int* __restrict__ seq_slot, int C, int K) {
+__global__ void conv_state_store_kernel(const T* proj, int ld, int x_off, const float* LLMIE_WEIGHT x_bias,
+                                        float* conv_state, const int* cu_q,
+                                        const int* seq_slot, int C, int K) {
   pdl_launch_dependents();
   pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -705,9 +705,9 @@ __global__ void conv_state_store_kernel(const T* __restrict__ proj, int ld, int 
 
 // gates [T, groups * 2 * bw]: per group the pre-activations of r (bw) and then of i (bw). In place: r's place receives
 // a = exp(-c r softplus(lam)), i's place the drive sqrt(1 - a^2) * i * u.
-__global__ void unit_gate_values_kernel(float* __restrict__ gates, const float* __restrict__ u,
-                                        const float* __restrict__ r_bias, const float* __restrict__ i_bias,
-                                        const float* __restrict__ lam, float c_decay, int C, int bw, size_t total) {
+__global__ void unit_gate_values_kernel(float* gates, const float* u,
+                                        const float* LLMIE_WEIGHT r_bias, const float* LLMIE_WEIGHT i_bias,
+                                        const float* LLMIE_WEIGHT lam, float c_decay, int C, int bw, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -729,10 +729,10 @@ __global__ void unit_gate_values_kernel(float* __restrict__ gates, const float* 
 // a thread per (sequence, channel): the recurrence over the step's tokens, the output gate act(y_raw + y_bias), and
 // the new state of the recurrence and of the convolution.
 template <typename T>
-__global__ void unit_scan_kernel(const float* __restrict__ gates, const T* __restrict__ proj, int ld, int y_off,
-                                 int x_off, const float* __restrict__ y_bias, const float* __restrict__ x_bias,
-                                 int act, float* __restrict__ state, float* __restrict__ conv_state,
-                                 const int* __restrict__ cu_q, const int* __restrict__ seq_slot, T* __restrict__ out,
+__global__ void unit_scan_kernel(const float* gates, const T* proj, int ld, int y_off,
+                                 int x_off, const float* LLMIE_WEIGHT y_bias, const float* LLMIE_WEIGHT x_bias,
+                                 int act, float* state, float* conv_state,
+                                 const int* cu_q, const int* seq_slot, T* __restrict__ out,
                                  int C, int bw, int K, int write_state) {
   pdl_launch_dependents();
   pdl_wait();
@@ -791,10 +791,10 @@ constexpr int kUnitChunks = 32;
 
 template <typename T>
 __global__ void __launch_bounds__(32 * kUnitChunks)
-unit_scan_chunked_kernel(const float* __restrict__ gates, const T* __restrict__ proj, int ld, int y_off, int x_off,
-                         const float* __restrict__ y_bias, const float* __restrict__ x_bias, int act,
-                         float* __restrict__ state, float* __restrict__ conv_state, const int* __restrict__ cu_q,
-                         const int* __restrict__ seq_slot, T* __restrict__ out, int C, int bw, int K, int write_state) {
+unit_scan_chunked_kernel(const float* gates, const T* proj, int ld, int y_off, int x_off,
+                         const float* LLMIE_WEIGHT y_bias, const float* LLMIE_WEIGHT x_bias, int act,
+                         float* state, float* conv_state, const int* cu_q,
+                         const int* seq_slot, T* __restrict__ out, int C, int bw, int K, int write_state) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float sA[kUnitChunks][33], sB[kUnitChunks][33];

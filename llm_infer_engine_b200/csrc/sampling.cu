@@ -58,9 +58,9 @@ __device__ MaxIdx block_argmax(const float* row, int V, MaxIdx* scratch) {
 }
 
 __global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature, float top_p,
-              unsigned long long seed, const unsigned* __restrict__ dev_params, const int* __restrict__ seq_ids,
-              int* __restrict__ counters, int* __restrict__ out) {
+sample_kernel(const float* logits, int ld, int V, float temperature, float top_p,
+              unsigned long long seed, const unsigned* dev_params, const int* seq_ids,
+              int* counters, int* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
   if (dev_params) {
@@ -157,7 +157,7 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
 // Greedy choice with many blocks per row, for large vocabularies: block (s, r) scans one slice
 // of row r, a second kernel merges the slices. Ties go to the lowest index in both stages.
 __global__ void __launch_bounds__(256)
-argmax_partial_kernel(const float* __restrict__ logits, int ld, int V, int slices, float* __restrict__ part_val,
+argmax_partial_kernel(const float* logits, int ld, int V, int slices, float* __restrict__ part_val,
                       int* __restrict__ part_idx) {
   pdl_launch_dependents();
   pdl_wait();
@@ -203,7 +203,7 @@ argmax_partial_kernel(const float* __restrict__ logits, int ld, int V, int slice
   }
 }
 
-__global__ void argmax_merge_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx, int slices,
+__global__ void argmax_merge_kernel(const float* part_val, const int* part_idx, int slices,
                                     int* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -219,7 +219,7 @@ __global__ void argmax_merge_kernel(const float* __restrict__ part_val, const in
 }
 
 // tokens[i] = sampled[i] for the lanes of a decode step (feeds the next step on the device)
-__global__ void copy_int_kernel(const int* __restrict__ src, int* __restrict__ dst, int n) {
+__global__ void copy_int_kernel(const int* src, int* __restrict__ dst, int n) {
   pdl_launch_dependents();
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -41,11 +41,11 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 // The same kernel four channels a thread (d a multiple of 4, every row 16-byte aligned): the element's arithmetic is
 // the scalar kernel's, only who sums which squares differs.
 template <typename TY>
-__global__ void scaled_add_rmsnorm4_kernel(float* __restrict__ h, const void* __restrict__ d1, int d1_dtype, float c1,
-                                           const void* __restrict__ d2, int d2_dtype, float c2,
-                                           const float* __restrict__ s, const float* __restrict__ bias,
-                                           const float* __restrict__ w, float eps, TY* __restrict__ y, int y_ld,
-                                           const int* __restrict__ rows, int d) {
+__global__ void scaled_add_rmsnorm4_kernel(float* h, const void* d1, int d1_dtype, float c1,
+                                           const void* d2, int d2_dtype, float c2,
+                                           const float* LLMIE_WEIGHT s, const float* LLMIE_WEIGHT bias,
+                                           const float* LLMIE_WEIGHT w, float eps, TY* __restrict__ y, int y_ld,
+                                           const int* rows, int d) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];
   pdl_launch_dependents();
@@ -95,11 +95,11 @@ __global__ void scaled_add_rmsnorm4_kernel(float* __restrict__ h, const void* __
 }
 
 template <typename TY>
-__global__ void scaled_add_rmsnorm_kernel(float* __restrict__ h, const void* __restrict__ d1, int d1_dtype, float c1,
-                                          const void* __restrict__ d2, int d2_dtype, float c2,
-                                          const float* __restrict__ s, const float* __restrict__ bias,
-                                          const float* __restrict__ w, float eps, TY* __restrict__ y, int y_ld,
-                                          const int* __restrict__ rows, int d) {
+__global__ void scaled_add_rmsnorm_kernel(float* h, const void* d1, int d1_dtype, float c1,
+                                          const void* d2, int d2_dtype, float c2,
+                                          const float* LLMIE_WEIGHT s, const float* LLMIE_WEIGHT bias,
+                                          const float* LLMIE_WEIGHT w, float eps, TY* __restrict__ y, int y_ld,
+                                          const int* rows, int d) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];
   pdl_launch_dependents();
@@ -133,11 +133,11 @@ __global__ void scaled_add_rmsnorm_kernel(float* __restrict__ h, const void* __r
 // NR runs of four channels and keeps them in registers from the branch outputs to the last store; weights are asked for
 // before the wait on the kernel that makes the branch outputs. d a multiple of 4 with d / 4 <= NR * blockDim.x.
 template <typename TY, int NR>
-__global__ void sandwich_add_norm4_kernel(float* __restrict__ h, const void* __restrict__ d1, int d1_dtype, float c1,
-                                          const float* __restrict__ w1, const void* __restrict__ d2, int d2_dtype,
-                                          float c2, const float* __restrict__ w2, float eps_in,
-                                          const float* __restrict__ w_out, float eps_out, const float* __restrict__ w,
-                                          float eps, TY* __restrict__ y, int y_ld, const int* __restrict__ rows, int d) {
+__global__ void sandwich_add_norm4_kernel(float* h, const void* d1, int d1_dtype, float c1,
+                                          const float* LLMIE_WEIGHT w1, const void* d2, int d2_dtype,
+                                          float c2, const float* LLMIE_WEIGHT w2, float eps_in,
+                                          const float* LLMIE_WEIGHT w_out, float eps_out, const float* LLMIE_WEIGHT w,
+                                          float eps, TY* __restrict__ y, int y_ld, const int* rows, int d) {
   __shared__ float red[32];
   pdl_launch_dependents();
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -220,11 +220,11 @@ __global__ void sandwich_add_norm4_kernel(float* __restrict__ h, const void* __r
 
 // The same for every width that fits shared memory, element by element.
 template <typename TY>
-__global__ void sandwich_add_norm_kernel(float* __restrict__ h, const void* __restrict__ d1, int d1_dtype, float c1,
-                                         const float* __restrict__ w1, const void* __restrict__ d2, int d2_dtype,
-                                         float c2, const float* __restrict__ w2, float eps_in,
-                                         const float* __restrict__ w_out, float eps_out, const float* __restrict__ w,
-                                         float eps, TY* __restrict__ y, int y_ld, const int* __restrict__ rows, int d) {
+__global__ void sandwich_add_norm_kernel(float* h, const void* d1, int d1_dtype, float c1,
+                                         const float* LLMIE_WEIGHT w1, const void* d2, int d2_dtype,
+                                         float c2, const float* LLMIE_WEIGHT w2, float eps_in,
+                                         const float* LLMIE_WEIGHT w_out, float eps_out, const float* LLMIE_WEIGHT w,
+                                         float eps, TY* __restrict__ y, int y_ld, const int* rows, int d) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];
   pdl_launch_dependents();
@@ -269,7 +269,7 @@ __global__ void sandwich_add_norm_kernel(float* __restrict__ h, const void* __re
 }
 
 template <typename T>
-__global__ void poly_norm_kernel(const T* __restrict__ z, const float* __restrict__ coef, float eps, T* __restrict__ y,
+__global__ void poly_norm_kernel(const T* z, const float* LLMIE_WEIGHT coef, float eps, T* __restrict__ y,
                                  int n) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];
@@ -300,7 +300,7 @@ __global__ void poly_norm_kernel(const T* __restrict__ z, const float* __restric
 
 // Eight values a thread (n a multiple of 8, rows 16-byte aligned); the element's arithmetic is the scalar kernel's.
 template <typename T>
-__global__ void poly_norm8_kernel(const T* __restrict__ z, const float* __restrict__ coef, float eps, T* __restrict__ y,
+__global__ void poly_norm8_kernel(const T* z, const float* LLMIE_WEIGHT coef, float eps, T* __restrict__ y,
                                   int n) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];

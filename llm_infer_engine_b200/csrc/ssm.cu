@@ -28,8 +28,8 @@ namespace llmie {
 __device__ __forceinline__ float ssm_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 template <typename T>
-__global__ void ssm_steps_kernel(const T* __restrict__ proj, int ld, int dt_off, const float* __restrict__ dt_bias,
-                                 const float* __restrict__ A, float* __restrict__ dt, float* __restrict__ decay, int H,
+__global__ void ssm_steps_kernel(const T* proj, int ld, int dt_off, const float* LLMIE_WEIGHT dt_bias,
+                                 const float* LLMIE_WEIGHT A, float* __restrict__ dt, float* __restrict__ decay, int H,
                                  int total) {
   pdl_launch_dependents();
   pdl_wait();
@@ -62,7 +62,7 @@ struct SsmArgs {
 // wait for the previous kernel: the state was last written a whole step ago.
 template <typename TP, int V>
 __global__ void __launch_bounds__(kStepThreads)
-ssm_step_kernel(const SsmArgs p, const float* __restrict__ xbc, float* __restrict__ y, int CT, int RT, int ctiles) {
+ssm_step_kernel(const SsmArgs p, const float* xbc, float* __restrict__ y, int CT, int RT, int ctiles) {
   extern __shared__ float st_smem[];                // B [N], C [N], then RT x CT partial sums of V
   __shared__ float step_dt, step_decay;
   pdl_launch_dependents();
@@ -198,7 +198,7 @@ struct SsmTile {
 // grid (value tiles, H, sequences). NT: rows of the state, N rounded up; PS: value columns a block.
 template <typename TP, typename TO, int NT, int PS>
 __global__ void __launch_bounds__(kSsmThreads)
-ssm_scan_kernel(const SsmArgs p, const __nv_bfloat16* __restrict__ xbc, TO* __restrict__ y) {
+ssm_scan_kernel(const SsmArgs p, const __nv_bfloat16* xbc, TO* __restrict__ y) {
   using Tile = SsmTile<NT, PS>;
   constexpr int NP = Tile::NP, XP = Tile::XP;
   constexpr int MT = (NT + 63) / 64;                        // 16-row tiles of the state a warp owns
@@ -497,9 +497,9 @@ ssm_scan_kernel(const SsmArgs p, const __nv_bfloat16* __restrict__ xbc, TO* __re
 // A block per (token, run of columns). y float32 [T, n]; z rows of n elements, z_ld apart. With `skip_d` the row is
 // y + skip_d[c / P] * x[c] first (x float32, rows x_ld apart: for a scan that leaves the skip term out).
 template <typename TZ, typename TO, int V>
-__global__ void gated_group_norm_kernel(const float* __restrict__ y, const TZ* __restrict__ z, int z_ld,
-                                        const float* __restrict__ w, float eps, TO* __restrict__ out, int n, int size,
-                                        const float* __restrict__ skip_x, int x_ld, const float* __restrict__ skip_d,
+__global__ void gated_group_norm_kernel(const float* y, const TZ* z, int z_ld,
+                                        const float* LLMIE_WEIGHT w, float eps, TO* __restrict__ out, int n, int size,
+                                        const float* skip_x, int x_ld, const float* LLMIE_WEIGHT skip_d,
                                         int P) {
   extern __shared__ float row_smem[];
   __shared__ float red[32];
