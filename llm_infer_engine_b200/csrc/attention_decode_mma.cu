@@ -515,13 +515,13 @@ static int launch_mma(const void* q, const void* k_cache, const void* v_cache, f
                       MdOptions opt, cudaStream_t stream) {
   const int G = n_q / n_kv;
   const int chunks = (G + 15) / 16;
-  const size_t smem = (size_t)WARPS * 2 * kMdPage * (HD + 8) * sizeof(__nv_bfloat16);
-  if (smem > 48 * 1024) {
+  constexpr size_t kSmem = (size_t)WARPS * 2 * kMdPage * (HD + 8) * sizeof(__nv_bfloat16);
+  if (kSmem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(decode_mma_kernel<HD, WARPS, ROPE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return (int)e;
   }
-  launch_k(decode_mma_kernel<HD, WARPS, ROPE>, dim3(n_runs, n_kv * chunks, n_seqs), dim3(WARPS * 32), smem, stream,
+  launch_k(decode_mma_kernel<HD, WARPS, ROPE>, dim3(n_runs, n_kv * chunks, n_seqs), dim3(WARPS * 32), kSmem, stream,
            (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, part_m, part_l,
            part_acc, seq_slot, seq_kvlen, block_table, max_pages, n_q, n_kv, scale, window, pages_per_run, n_runs,
            counters, (__nv_bfloat16*)out, rope, table_len, q_ld, write_kv, opt);

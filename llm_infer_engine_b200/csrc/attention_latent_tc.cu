@@ -30,6 +30,8 @@ constexpr int kLtMaxSubs = 5;                                         // head si
 constexpr int kLtScoreCol = 256;                                      // TMEM columns: output 0.., scores 256 and 320
 constexpr float kLtSlack = 8.f;                                       // log2: how far a maximum may run ahead
 
+constexpr int lt_smem_bytes(int subs) { return subs * kLtQSub + kLtQSub + kLtStages * subs * kLtKSub + 1024; }
+
 struct LatentArgs {
   __nv_bfloat16* out;            // [T * heads, hdv]
   const int* cu_q;
@@ -321,8 +323,9 @@ extern "C" int llmie_attention_latent_tc(const void* q, const void* cache, void*
   if (rc != LLMIE_OK) return rc;
   rc = tc::make_tmap_bf16_2d(&map_k, cache, (uint64_t)n_pages * kLtKeys, hd, hd, kLtKeys);
   if (rc != LLMIE_OK) return rc;
-  const int subs = (hd + 63) / 64, smem = subs * kLtQSub + kLtQSub + kLtStages * subs * kLtKSub + 1024;
-  const cudaError_t e = cudaFuncSetAttribute(attention_latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int smem = lt_smem_bytes((hd + 63) / 64);
+  const cudaError_t e = cudaFuncSetAttribute(attention_latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             lt_smem_bytes(kLtMaxSubs));
   if (e != cudaSuccess) return (int)e;
   const LatentArgs a{(__nv_bfloat16*)out, cu_q, seq_slot, seq_start, block_table, max_pages, heads, hd, hdv, window,
                      sink ? 1 : 0, scale, sink_vals, status};

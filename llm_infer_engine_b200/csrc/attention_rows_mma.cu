@@ -322,7 +322,7 @@ using namespace llmie;
 extern "C" int llmie_attention_rows_mma_supported(int hd, int hdv, int page_size, int shared_rows) {
   if (hd <= 0 || hd % 16 || hd > 1024 || hdv <= 0 || hdv % 8 || hdv > 512 || page_size % kRmKeys) return 0;
   if (shared_rows && hdv > hd) return 0;
-  return rows_smem_bytes(hd, hdv, shared_rows != 0) <= 200 * 1024 ? 1 : 0;
+  return rows_smem_bytes(hd, hdv, shared_rows != 0) <= kMostRowSmem ? 1 : 0;
 }
 
 // q [T, n_q hd], out [T, n_q hdv], caches as in llmie_attention_paged_ex (v_cache rows v_ld apart; shared_rows != 0: the
@@ -354,7 +354,7 @@ extern "C" int llmie_attention_rows_mma(const void* q, const void* k_cache, cons
   const int ntw = (hdv / 8 + kRmWarps - 1) / kRmWarps;
 #define LLMIE_ROWS_LAUNCH(N)                                                                                     \
   do {                                                                                                           \
-    cudaFuncSetAttribute(attention_rows_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+    cudaFuncSetAttribute(attention_rows_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostRowSmem); \
     launch_k(attention_rows_mma_kernel<N>, grid, dim3(kRmWarps * 32), smem, stream, a);                          \
   } while (0)
   if (ntw <= 1) LLMIE_ROWS_LAUNCH(1);

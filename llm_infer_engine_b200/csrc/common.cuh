@@ -148,6 +148,12 @@ static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Dynamic shared memory beyond 48 KB is allowed per kernel, by an attribute that stays with the kernel, not with a launch;
+// and launches come from several host threads at once. So each kernel is allowed one size, the largest it is ever launched
+// with: were it a call's own size, a smaller call could lower it between another's setting it and launching. kMostRowSmem is
+// the largest for kernels whose size follows a row's width.
+constexpr int kMostRowSmem = 200 * 1024;
+
 // Asks the memory system to bring `bytes` (a multiple of 16, from a 16-byte aligned address) into
 // L2. No register, no shared memory and no waiting on the issuing thread: a block can ask for all
 // the weights it is going to stream, long before its loads of them, even before pdl_wait().

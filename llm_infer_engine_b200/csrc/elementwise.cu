@@ -354,9 +354,9 @@ static int add_rmsnorm_launch(float* h, const void* delta, const float* w, void*
     return LLMIE_OK;
   }
   const size_t smem = (size_t)d * sizeof(float);
-  if (smem > 200 * 1024) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (smem > kMostRowSmem) return LLMIE_ERR_UNSUPPORTED_SIZE;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostRowSmem);
     if (e != cudaSuccess) return (int)e;
   }
   launch_k(add_rmsnorm_kernel<T>, dim3(n_out), dim3(norm_threads(d)), smem, stream, h, (const T*)delta, w, (T*)y, rows, d, eps);

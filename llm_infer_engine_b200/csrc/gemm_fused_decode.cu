@@ -439,9 +439,9 @@ static int fused_blocks_per_sm(int K) {
   if (cached_k != K) {
     const size_t smem = fused_smem<VAR, WARPS>(K);
     int n = 0;
-    if (smem <= 200 * 1024) {
+    if (smem <= kMostRowSmem) {
       if (smem > 48 * 1024)
-        cudaFuncSetAttribute(norm_gemm_kernel<VAR, WARPS, BRANCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(norm_gemm_kernel<VAR, WARPS, BRANCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostRowSmem);
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, norm_gemm_kernel<VAR, WARPS, BRANCH>, WARPS * 32, smem) != cudaSuccess)
         n = 0;
     }

@@ -269,6 +269,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (n_splits > 1) cluster_sync_all();           // shared memory of a block outlives its peers' accesses to it
 }
 
+constexpr int kSMostSmem = kSSmemBudget + 1024;       // of every plan below
+
 struct StreamPlan {
   int mpad, n_tiles, n_splits, chunks_per_split, n_clusters, n_stages, smem;
 };
@@ -318,13 +320,13 @@ extern "C" int llmie_gemm_stream_active_clusters(int rows, int N, int K, int n_s
   int n = 0;
   cudaError_t e;
   if (p.mpad == 16) {
-    cudaFuncSetAttribute(gemm_stream_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem);
+    cudaFuncSetAttribute(gemm_stream_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSMostSmem);
     e = cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel<16>, &cfg);
   } else if (p.mpad == 32) {
-    cudaFuncSetAttribute(gemm_stream_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem);
+    cudaFuncSetAttribute(gemm_stream_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSMostSmem);
     e = cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel<32>, &cfg);
   } else {
-    cudaFuncSetAttribute(gemm_stream_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem);
+    cudaFuncSetAttribute(gemm_stream_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSMostSmem);
     e = cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel<64>, &cfg);
   }
   return e == cudaSuccess ? n : 0;
@@ -349,7 +351,7 @@ extern "C" int llmie_gemm_stream(const void* X, const void* W, void* out, int M,
   cudaError_t e;
 #define LLMIE_STREAM_CASE(MP)                                                                                       \
   case MP:                                                                                                          \
-    e = cudaFuncSetAttribute(gemm_stream_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem);          \
+    e = cudaFuncSetAttribute(gemm_stream_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSMostSmem);          \
     if (e != cudaSuccess) return (int)e;                                                                            \
     if (p.n_splits > 1)                                                                                             \
       launch_k_cluster(gemm_stream_kernel<MP>, grid, dim3(kSThreads), (size_t)p.smem, stream, (unsigned)p.n_splits, \

@@ -326,7 +326,7 @@ static int launch_mma_tile(const GroupedArgs& p, dim3 grid, int vec, int cvec, c
   using T = MmaTile<BM, DUAL>;
   auto kernel = grouped_gemm_mma_kernel<TC, BM, DUAL>;
   const int smem = T::smem_bytes((p.K + kMmaBK - 1) / kMmaBK);
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::smem_bytes(T::kStages));
   if (e != cudaSuccess) return (int)e;
   launch_k(kernel, grid, dim3(128), smem, stream, p, vec, cvec);
   return LLMIE_OK;

@@ -386,6 +386,10 @@ __global__ void moe_combine_identity_kernel(const void* y, int y_dtype, const in
 
 using namespace llmie;
 
+// a token's part of a block's shared memory: 48 KB at most, and the row's end filled up to whole 16 bytes; two tokens are
+// taken up to 100 KB
+constexpr int kRouteMostSmem = 50 * 1024 + 16;
+
 template <typename T, int TB>
 static int launch_route(const T* x, const float* w, const float* bias, int* ids, float* weights, int n_tokens, int d,
                         int n_experts, int top, int mode, const float* correction, float out_scale, int n_groups, int keep,
@@ -393,7 +397,8 @@ static int launch_route(const T* x, const float* w, const float* bias, int* ids,
   const int pitch = (d + 3) / 4 * 4;
   const size_t smem = TB * ((size_t)pitch + 2 * (size_t)n_experts + (mode == 3 ? (size_t)n_groups : 0)) * sizeof(float);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(moe_route_kernel<T, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(moe_route_kernel<T, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               TB * kRouteMostSmem);
     if (e != cudaSuccess) return (int)e;
   }
   launch_k(moe_route_kernel<T, TB>, dim3((n_tokens + TB - 1) / TB), dim3(kRouteWarps * 32), smem, stream, x, w, bias, ids,

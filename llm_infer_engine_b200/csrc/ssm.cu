@@ -572,7 +572,7 @@ static int gated_group_norm_launch(const float* y, const void* z, int z_ld, cons
   const dim3 grid(n_tokens, groups), block(threads);
   auto kernel = by4 ? gated_group_norm_kernel<TZ, TO, 4> : gated_group_norm_kernel<TZ, TO, 1>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostRowSmem);
     if (e != cudaSuccess) return (int)e;
   }
   launch_k(kernel, grid, block, smem, stream, y, (const TZ*)z, z_ld, w, eps, (TO*)out, n, size, skip_x, x_ld, skip_d, P);
@@ -690,7 +690,7 @@ extern "C" int llmie_gated_group_norm(const float* y, const void* z, int z_ld, i
   if (n_tokens < 0 || n <= 0 || groups <= 0 || n % groups || z_ld < n || !w || (!skip_x) != (!skip_d) ||
       (skip_d && (P <= 0 || n % P || x_ld < n)))
     return LLMIE_ERR_BAD_ARG;
-  if ((size_t)(n / groups) * sizeof(float) > 200 * 1024 || groups > 65535) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if ((size_t)(n / groups) * sizeof(float) > kMostRowSmem || groups > 65535) return LLMIE_ERR_UNSUPPORTED_SIZE;
   if (n_tokens == 0) return LLMIE_OK;
 #define LLMIE_GGN(TZ, TO) \
   gated_group_norm_launch<TZ, TO>(y, z, z_ld, w, eps, out, n_tokens, n, groups, skip_x, x_ld, skip_d, P, stream)
