@@ -12,7 +12,8 @@
 //               registers, mask, running maximum and sum, P as bfloat16 into shared memory
 // The output stays in tensor memory. A row's reference maximum moves only when a page's maximum lies more than 2^8 above
 // it (its probabilities are then at most 2^8 and keep their relative precision in bfloat16 as in the float32 sums); the
-// warp then multiplies its rows' output by the change before it lets the next product go. Every wait is bounded.
+// warp then multiplies its rows' output by the change before it lets the next product go. Every wait is bounded; a block
+// that gives up waits for its copies and products (again bounded), leaves NaN in its rows and a code in the status word.
 //
 // What bounds it: a page of 64 keys is 544 (hd + hdv) x 128 x 64 products, 544 tensor cycles at hd 288, hdv 256, and as
 // many cycles of exponentials; Q and the ring take 216 KB, one block an SM. Two prompts, 2,100 tokens, 32 heads of 288 /
@@ -45,7 +46,7 @@ struct LatentArgs {
 };
 
 struct LatentShared {
-  uint64_t q_full, k_full[kLtStages], k_empty[kLtStages], s_full[2], s_free[2], p_ready, pv_full, pair_bar[4];
+  uint64_t q_full, k_full[kLtStages], k_empty[kLtStages], s_full[2], s_free[2], p_ready, pv_full, pair_bar[4], drained;
   uint32_t tmem_base;
   int abort;
   float row_val[2][2][kLtRows];
@@ -57,7 +58,9 @@ __device__ __forceinline__ float lt_exp2(float x) {
   return y;
 }
 
-__global__ void __launch_bounds__(kLtThreads)
+// LIMIT: polls before a wait gives up (a constant: read from the arguments it cost 5 % of the time).
+template <unsigned LIMIT>
+__global__ void __launch_bounds__(kLtThreads, 1)
 attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const LatentArgs p) {
   extern __shared__ uint8_t lt_smem[];
@@ -93,6 +96,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     mbar_init(&sh.p_ready, kLtSoftmax);
     mbar_init(&sh.pv_full, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&sh.pair_bar[i], 64);
+    mbar_init(&sh.drained, 1);
     sh.abort = 0;
     fence_mbar_init();
     tma_prefetch_desc(&map_q);
@@ -111,25 +115,20 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   tc_fence_after_sync();
   const uint32_t tmem = sh.tmem_base;
   volatile int* abort = &sh.abort;
+  int issued = 1;                                             // pages asked for (thread 0)
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait(bar, parity, abort, LIMIT); };
 #define LLMIE_FAIL(code) do { if (!*abort) { *abort = 1; atomicExch(p.status, (code)); } } while (0)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (page 0 is on its way)
     if (lane == 0) {
-      int issued = 1;
       for (int jt = 1; jt < n_tiles; ++jt) {
-        if (jt >= kLtStages && !mbar_wait(&sh.k_empty[jt % kLtStages], ((jt / kLtStages) - 1) & 1, abort)) {
+        if (jt >= kLtStages && !wait(&sh.k_empty[jt % kLtStages], ((jt / kLtStages) - 1) & 1)) {
           LLMIE_FAIL(kStatusTimeoutEmpty);
           break;
         }
         load_page(jt);
         issued = jt + 1;
-      }
-      if (*abort) {   // let copies that are still in flight land before the block gives its memory up
-        for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.q_full, 0); ++spin) __nanosleep(64);
-        for (int jt = max(0, issued - kLtStages); jt < issued; ++jt)
-          for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.k_full[jt % kLtStages], (jt / kLtStages) & 1); ++spin)
-            __nanosleep(64);
       }
     }
   } else if (warp == 1) {
@@ -139,12 +138,12 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       const uint32_t idesc_pv = make_instr_desc_bf16(kLtRows, p.hdv, 0, 1);      // V is MN-major
       const uint32_t q_addr = smem_u32(q_smem), p_addr = smem_u32(p_smem);
       const int k_steps = p.hd / 16;
-      bool ok = mbar_wait(&sh.q_full, 0, abort);
+      bool ok = wait(&sh.q_full, 0);
       if (!ok) LLMIE_FAIL(kStatusTimeoutFull);
       auto issue_scores = [&](int jt) -> bool {
         const int st = jt % kLtStages, b = jt & 1, use = jt >> 1;
-        if (!mbar_wait(&sh.k_full[st], (jt / kLtStages) & 1, abort)) { LLMIE_FAIL(kStatusTimeoutFull); return false; }
-        if (use >= 1 && !mbar_wait(&sh.s_free[b], (use - 1) & 1, abort)) { LLMIE_FAIL(kStatusTimeoutMma); return false; }
+        if (!wait(&sh.k_full[st], (jt / kLtStages) & 1)) { LLMIE_FAIL(kStatusTimeoutFull); return false; }
+        if (use >= 1 && !wait(&sh.s_free[b], (use - 1) & 1)) { LLMIE_FAIL(kStatusTimeoutMma); return false; }
         tc_fence_after_sync();
         const uint32_t k_addr = smem_u32(k_smem + st * stage_bytes);
         for (int kk = 0; kk < k_steps; ++kk)
@@ -157,7 +156,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       if (ok) ok = issue_scores(0);
       if (ok && n_tiles > 1) ok = issue_scores(1);
       for (int jt = 0; ok && jt < n_tiles; ++jt) {
-        if (!mbar_wait(&sh.p_ready, jt & 1, abort)) { LLMIE_FAIL(kStatusTimeoutMma); break; }
+        if (!wait(&sh.p_ready, jt & 1)) { LLMIE_FAIL(kStatusTimeoutMma); break; }
         tc_fence_after_sync();
         const uint32_t v_addr = smem_u32(k_smem + (jt % kLtStages) * stage_bytes);
 #pragma unroll
@@ -189,7 +188,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       const int buf = n_exchanges & 1;
       sh.row_val[buf][half][r] = mine;
       mbar_arrive(&sh.pair_bar[quarter]);
-      const bool ok_ = mbar_wait(&sh.pair_bar[quarter], n_exchanges & 1, abort);
+      const bool ok_ = wait(&sh.pair_bar[quarter], n_exchanges & 1);
       theirs = sh.row_val[buf][half ^ 1][r];
       ++n_exchanges;
       return ok_;
@@ -197,7 +196,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     for (int jt = 0; jt < n_tiles; ++jt) {
       const int b = jt & 1;
       // every decision to give up is the whole warp's: the tensor-memory accesses are warp-wide instructions
-      if (!__all_sync(0xffffffffu, mbar_wait(&sh.s_full[b], (jt >> 1) & 1, abort))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; break; }
+      if (!__all_sync(0xffffffffu, wait(&sh.s_full[b], (jt >> 1) & 1))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; break; }
       tc_fence_after_sync();
       uint32_t v[32];
       tmem_ld_32x32(lane_addr + kLtScoreCol + b * kLtKeys + half * 32, v);
@@ -235,7 +234,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         w[i >> 1] = *reinterpret_cast<const uint32_t*>(&pr);
       }
       // the product before this one is done with P, and with the output where that has to be brought to a new reference
-      if (jt > 0 && !__all_sync(0xffffffffu, mbar_wait(&sh.pv_full, (jt - 1) & 1, abort))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; break; }
+      if (jt > 0 && !__all_sync(0xffffffffu, wait(&sh.pv_full, (jt - 1) & 1))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; break; }
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch)
         *reinterpret_cast<uint4*>(p_smem + swizzle128_offset(r, half * 4 + ch)) =
@@ -258,7 +257,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       l_run = fmaf(l_run, alpha, (ls[0] + ls[1]) + (ls[2] + ls[3]));
       m_ref = m_new;
     }
-    if (ok && !__all_sync(0xffffffffu, mbar_wait(&sh.pv_full, (n_tiles - 1) & 1, abort))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; }
+    if (ok && !__all_sync(0xffffffffu, wait(&sh.pv_full, (n_tiles - 1) & 1))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; }
     float other = 0.f;
     if (ok && !__all_sync(0xffffffffu, exchange(l_run, other))) { LLMIE_FAIL(kStatusTimeoutMma); ok = false; }
     if (ok) {
@@ -287,10 +286,25 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #undef LLMIE_FAIL
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem, 512);
+  tc_fence_after_sync();
+  if (*abort) {
+    // copies and products still in flight land before the block gives its memory up; the rows are no result
+    if (threadIdx.x == 0) {
+      for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.q_full, 0); ++spin) __nanosleep(64);
+      for (int jt = max(0, issued - kLtStages); jt < issued; ++jt)
+        for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.k_full[jt % kLtStages], (jt / kLtStages) & 1); ++spin)
+          __nanosleep(64);
+    }
+    if (warp == 1 && elect_one()) {                            // the lane that issued the products
+      mma_commit(&sh.drained);
+      for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.drained, 0); ++spin) __nanosleep(64);
+    }
+    uint4* rows = reinterpret_cast<uint4*>(p.out + ((size_t)q_begin * p.heads + r0) * p.hdv);
+    const uint4 nan8 = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+    for (int i = threadIdx.x; i < rows_here * p.hdv / 8; i += kLtThreads) rows[i] = nan8;
+    __syncthreads();
   }
+  if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace llmie
@@ -306,10 +320,12 @@ extern "C" int llmie_attention_latent_tc_supported(int hd, int hdv, int page_siz
 // q bfloat16 [n_tokens, heads hd], out [n_tokens, heads hdv]; cache bfloat16 [n_pages, 1, 64, hd], the values its rows'
 // first hdv columns. cu_q, seq_slot, seq_start, block_table, window as in llmie_attention_prefill_tc; scale > 0. sink != 0:
 // one more softmax term without a value, of score 0 or sink_vals float32 [heads].
-extern "C" int llmie_attention_latent_tc(const void* q, const void* cache, void* out, const int* cu_q, const int* seq_slot,
+// no_wait != 0: every wait gives up at once (for tests of that path).
+extern "C" int llmie_attention_latent_tc_form(const void* q, const void* cache, void* out, const int* cu_q, const int* seq_slot,
                                          const int* seq_start, const int* block_table, int max_pages, int n_pages,
                                          int n_tokens, int n_seqs, int max_q_len, int heads, int hd, int hdv, float scale,
-                                         int window, const float* sink_vals, int sink, int* status, cudaStream_t stream) {
+                                         int window, const float* sink_vals, int sink, int* status, int no_wait,
+                                         cudaStream_t stream) {
   if (n_tokens < 0 || n_seqs < 0 || heads <= 0 || max_pages <= 0 || n_pages <= 0 || !(scale > 0.f) || !status ||
       (sink_vals && !sink))
     return LLMIE_ERR_BAD_ARG;
@@ -324,12 +340,21 @@ extern "C" int llmie_attention_latent_tc(const void* q, const void* cache, void*
   rc = tc::make_tmap_bf16_2d(&map_k, cache, (uint64_t)n_pages * kLtKeys, hd, hd, kLtKeys);
   if (rc != LLMIE_OK) return rc;
   const int smem = lt_smem_bytes((hd + 63) / 64);
-  const cudaError_t e = cudaFuncSetAttribute(attention_latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             lt_smem_bytes(kLtMaxSubs));
+  auto kernel = no_wait ? attention_latent_tc_kernel<0> : attention_latent_tc_kernel<kSpinLimit>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lt_smem_bytes(kLtMaxSubs));
   if (e != cudaSuccess) return (int)e;
   const LatentArgs a{(__nv_bfloat16*)out, cu_q, seq_slot, seq_start, block_table, max_pages, heads, hd, hdv, window,
                      sink ? 1 : 0, scale, sink_vals, status};
-  attention_latent_tc_kernel<<<dim3(n_seqs, (unsigned)row_blocks), kLtThreads, smem, stream>>>(map_q, map_k, a);
+  kernel<<<dim3(n_seqs, (unsigned)row_blocks), kLtThreads, smem, stream>>>(map_q, map_k, a);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
+}
+
+extern "C" int llmie_attention_latent_tc(const void* q, const void* cache, void* out, const int* cu_q, const int* seq_slot,
+                                         const int* seq_start, const int* block_table, int max_pages, int n_pages,
+                                         int n_tokens, int n_seqs, int max_q_len, int heads, int hd, int hdv, float scale,
+                                         int window, const float* sink_vals, int sink, int* status, cudaStream_t stream) {
+  return llmie_attention_latent_tc_form(q, cache, out, cu_q, seq_slot, seq_start, block_table, max_pages, n_pages, n_tokens,
+                                         n_seqs, max_q_len, heads, hd, hdv, scale, window, sink_vals, sink, status, 0,
+                                         stream);
 }

@@ -84,6 +84,28 @@ def test_prompts(heads, hd, hdv, window, sink, growth):
     assert torch.equal(one, out[a:a + 200])
 
 
+def test_a_block_that_gives_up_leaves_no_numbers():
+    """A wait that runs out (no polls at all here): NaN in every row and an error for whoever asks, not what was there."""
+    from llm_infer_engine_b200.kernels import ops
+    lens, held, heads, hd, hdv = [130, 40], [0, 300], 5, 144, 128
+    q, cache, rows, cu, slot, start, table = _case(lens, held, heads, hd, hdv)
+    out = torch.full((sum(lens), heads * hdv), 3.0, dtype=torch.bfloat16, device=DEV)
+    status = ops.tc_status_word(torch.device(DEV, 0))
+    p = [t.data_ptr() for t in (q, cache, out, cu, slot, start, table)]
+    f = ops._fn("attention_latent_tc", "llmie_attention_latent_tc_form",
+                [ops._c_void_p] * 7 + [ops._c_int] * 8 + [ops._c_float, ops._c_int, ops._c_void_p, ops._c_int, ops._c_void_p,
+                                                          ops._c_int, ops._c_void_p])
+    assert f(*p, table.shape[1], cache.shape[0], sum(lens), 2, 130, heads, hd, hdv, 0.1, 0, None, 0, status.data_ptr(), 1,
+             ops._stream()) == 0
+    torch.cuda.synchronize()
+    assert bool(out.isnan().all())
+    with pytest.raises(ops.KernelError):
+        ops.check_tc_status(torch.device(DEV, 0))
+    ops.check_tc_status(torch.device(DEV, 0))                            # raised once
+    ops.attention_latent_tc(q, cache, cache[..., :hdv], out, cu, slot, start, table, 64, 2, 130, heads, hd, 0.1)
+    assert bool(out.isfinite().all())
+
+
 def test_both_kernels_agree():
     """The kernel of 32 rows takes the same calls (and all that this one refuses)."""
     from llm_infer_engine_b200.kernels import ops
