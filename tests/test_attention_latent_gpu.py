@@ -84,6 +84,48 @@ def test_prompts(heads, hd, hdv, window, sink, growth):
     assert torch.equal(one, out[a:a + 200])
 
 
+@pytest.mark.parametrize("heads,hd,hdv", [(32, 288, 256), (3, 80, 64), (1, 144, 128)])
+@pytest.mark.parametrize("window", [0, 70, -96])
+@pytest.mark.parametrize("value", [math.nan, math.inf, -math.inf])
+def test_values_that_are_not_finite_stay_with_the_rows_that_see_them(heads, hd, hdv, window, value):
+    """A key that went wrong, at places where a page's first tokens do not see it yet or its last no longer do, in a first and
+    in a later page; and whatever the last page holds behind the sequence, and pages of nobody."""
+    from llm_infer_engine_b200.kernels import ops
+    lens, held = [65, 1, 200, 9], [0, 63, 130, 700]
+    wrong = [20, None, 200, 650]
+    q, cache, rows, cu, slot, start, table = _case(lens, held, heads, hd, hdv, seed=7)
+    used = torch.zeros(cache.shape[0], 64, dtype=torch.bool)
+    for i, k in enumerate(rows):
+        for t in range(len(k)):
+            used[table[i, t // 64], t % 64] = True
+    cache[~used[:, None].to(DEV)] = value
+    for i, t in enumerate(wrong):
+        if t is not None:
+            cache[table[i, t // 64], 0, t % 64, ::5] = value
+    values, scale = cache[..., :hdv], 1.7 * hd ** -0.5
+    out = torch.full((sum(lens), heads * hdv), 3.0, dtype=torch.bfloat16, device=DEV)
+    ops.attention_latent_tc(q, cache, values, out, cu, slot, start, table, 64, len(lens), max(lens), heads, hd, scale, window)
+    ops.check_tc_status(torch.device(DEV, 0))
+    want = _reference(q, rows, lens, held, heads, hd, hdv, scale, window, None)
+    at = 0
+    for i, (l, h) in enumerate(zip(lens, held)):
+        pos = torch.arange(h, h + l)
+        sees = torch.zeros(l, dtype=torch.bool)
+        if wrong[i] is not None:
+            sees = pos >= wrong[i]
+            if window > 0:
+                sees &= wrong[i] > pos - window
+            if window < 0:
+                sees &= wrong[i] >= pos - pos % -window
+        sees, got, ref = sees.to(DEV), out[at:at + l].double(), want[at:at + l]
+        at += l
+        bound = 2.0 ** -7 * rows[i].abs().max().double().to(DEV)             # as in test_prompts
+        diff = (got - ref)[~sees].abs()
+        assert bool((diff <= bound).all()), (i, float(diff.max()), int((~(diff <= bound)).any(1).sum()))
+        if value != value and bool(sees.any()):
+            assert bool(got[sees].isnan().all())
+
+
 def test_a_block_that_gives_up_leaves_no_numbers():
     """A wait that runs out (no polls at all here): NaN in every row and an error for whoever asks, not what was there."""
     from llm_infer_engine_b200.kernels import ops
