@@ -141,12 +141,13 @@ class KernelPlan:
 
     def _attention_by_rows(self, ctx, q, kv, out, n_q, n_kv, head_dim, options, gate) -> bool:
         """The tensor-core kernel whose rows are the (token, head) pairs of a key/value head: prompts and one-token
-        steps of the shapes and options the kernels above do not take. It knows no kept first keys."""
+        steps of the shapes and options the kernels above do not take. It knows no kept first keys. Latent attention has
+        one of its own where its sizes allow, whatever the step is: a token's bits do not depend on what else is in it."""
         shared_rows = not kv.v.is_contiguous()
-        if not ctx.decode and shared_rows and options.keep_first == 0 and not options.softcap \
+        if shared_rows and options.keep_first == 0 and not options.softcap \
                 and options.distance_bias is None and options.sigmoid_bias is None and ops.attention_latent_tc_supported(
                     q, kv.k, kv.v, kv.page_size, n_q, n_kv, head_dim, ctx.max_q_len, options.scale):
-            # latent attention over prompts: the tcgen05 kernel whose pages are key and value at once
+            # latent attention: the tcgen05 kernel whose pages are key and value at once
             ops.attention_latent_tc(q, kv.k, kv.v, out, ctx.cu_q, ctx.seq_slot, ctx.seq_start, kv.block_table,
                                     kv.page_size, ctx.n_seqs, ctx.max_q_len, n_q, head_dim, options.scale,
                                     options.reach, options.sink_values, options.sink)

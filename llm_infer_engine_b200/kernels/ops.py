@@ -1628,28 +1628,30 @@ def attention_rows_mma(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, bloc
 
 def attention_latent_tc_supported(q, k_cache, v_cache, page_size: int, n_q: int, n_kv: int, head_dim: int, max_q_len: int,
                                   scale: float) -> bool:
-    """Whether attention_latent_tc.cu takes a prompt step (answered without loading the library): bfloat16, one key head
+    """Whether attention_latent_tc.cu takes a step (answered without loading the library): bfloat16, one key head
     whose rows' first columns are the values, head size a multiple of 16 up to 320, value size a multiple of 64 up to 256,
-    pages of 64. From one whole tile of 128 (token, head) rows on: shorter pieces leave most of a tile empty, and the kernel
-    of 32 rows a block has more blocks for them."""
+    pages of 64. Pieces of any length, one token included, so that a sequence's bits do not depend on how long the others of
+    its step are; a tile that is mostly empty still costs less than the kernel of 32 rows a block behind any held tokens (32 heads of 288 / 256,
+    one to three new tokens behind 0 / 300 / 2,000 / 8,000: 7 to 9 / 11 to 13 / 41 / 140 us, the other kernel 6 / 23 / 125 /
+    488 us)."""
     hdv = v_cache.shape[-1]
     return (q.dtype is torch.bfloat16 and k_cache.dtype is torch.bfloat16 and n_kv == 1 and page_size == 64
             and v_cache.data_ptr() == k_cache.data_ptr() and v_cache.stride(-2) == head_dim and k_cache.is_contiguous()
             and head_dim % 16 == 0 and head_dim <= 320 and hdv % 64 == 0 and 0 < hdv <= min(256, head_dim) and scale > 0
-            and 128 <= max_q_len * n_q <= 128 * 65535 and not (q.data_ptr() | k_cache.data_ptr()) & 15)
+            and max_q_len * n_q <= 128 * 65535 and not (q.data_ptr() | k_cache.data_ptr()) & 15)
 
 
 def attention_latent_tc(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, block_table, page_size: int, n_seqs: int,
                         max_q_len: int, n_q: int, head_dim: int, scale: float, window: int = 0,
                         sink_values: Optional[torch.Tensor] = None, sink: bool = False):
-    """Prompts of latent attention on the tensor cores: q [T, n_q head_dim], out [T, n_q hdv], k_cache [pages, 1, 64,
+    """Latent attention on the tensor cores: q [T, n_q head_dim], out [T, n_q hdv], k_cache [pages, 1, 64,
     head_dim] whose rows' first hdv columns are the values (v_cache: the view of them); scale > 0, window and sink as in
-    attention_paged."""
+    attention_paged. A block whose waits run out leaves NaN in its rows, and check_tc_status raises."""
     T, hdv = q.shape[0], v_cache.shape[-1]
     _need(q, "q", torch.bfloat16, (T, n_q * head_dim))
     _need(out, "out", torch.bfloat16, (T, n_q * hdv))
     _need(k_cache, "k_cache", torch.bfloat16, (None, 1, page_size, head_dim))
-    if not attention_latent_tc_supported(q, k_cache, v_cache, page_size, n_q, 1, head_dim, max(max_q_len, 128), scale):
+    if not attention_latent_tc_supported(q, k_cache, v_cache, page_size, n_q, 1, head_dim, max_q_len, scale):
         raise KernelError(f"attention_latent_tc: sizes {head_dim} / {hdv}, page {page_size} are not supported")
     for name, t in (("cu_q", cu_q), ("seq_slot", seq_slot), ("seq_start", seq_start), ("block_table", block_table)):
         _need(t, name, torch.int32)

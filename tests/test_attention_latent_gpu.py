@@ -148,6 +148,31 @@ def test_a_block_that_gives_up_leaves_no_numbers():
     assert bool(out.isfinite().all())
 
 
+@pytest.mark.parametrize("heads,hd,hdv", [(32, 288, 256), (2, 80, 64)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_a_piece_gets_the_same_bits_beside_others(heads, hd, hdv, gated):
+    """Pieces of one to five tokens, alone (a step of one token, a short prompt) and beside a long one, as a layer calls it."""
+    import types
+    from llm_infer_engine_b200.parts.base import AttentionOptions
+    from test_parts_gpu import kernel_plan, make_ctx
+    lens, held = [1, 2, 5, 300], [90, 0, 700, 20]
+    q, cache, rows, cu, slot, start, table = _case(lens, held, heads, hd, hdv, seed=11)
+    kv = types.SimpleNamespace(k=cache, v=cache[..., :hdv], page_size=64, block_table=table)
+    gate = torch.randn(sum(lens), heads * hdv, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    plan, options = kernel_plan("bfloat16"), AttentionOptions(scale=hd ** -0.5)
+
+    def run(which):
+        at = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in which]).to(DEV)
+        out = torch.empty(len(at), heads * hdv, dtype=torch.bfloat16, device=DEV)
+        ctx = make_ctx([lens[i] for i in which], [held[i] for i in which], which, "bfloat16")
+        assert plan.attention(ctx, q[at].contiguous(), kv, out, heads, 1, hd, options, gate[at].contiguous() if gated else None)
+        return list(out.split([lens[i] for i in which]))
+
+    whole = run([0, 1, 2, 3])
+    for which in ([0], [1], [2], [0, 1], [1, 2]):
+        assert all(torch.equal(a, whole[i]) for i, a in zip(which, run(which))), which
+
+
 def test_both_kernels_agree():
     """The kernel of 32 rows takes the same calls (and all that this one refuses)."""
     from llm_infer_engine_b200.kernels import ops
@@ -169,5 +194,6 @@ def test_what_it_refuses():
     ok = lambda **kw: ops.attention_latent_tc_supported(**{**dict(q=q, k_cache=cache, v_cache=cache[..., :64], page_size=64,  # noqa: E731
                                                                   n_q=4, n_kv=1, head_dim=96, max_q_len=130, scale=1.0), **kw})
     assert ok()
-    assert not ok(v_cache=cache[..., :48]) and not ok(v_cache=cache[..., 32:]) and not ok(max_q_len=31)
+    assert not ok(v_cache=cache[..., :48]) and not ok(v_cache=cache[..., 32:])
+    assert ok(max_q_len=1) and not ok(max_q_len=1 << 30)
     assert not ok(scale=0.0) and not ok(page_size=32) and not ok(n_kv=2) and not ok(q=q.float())
