@@ -7,10 +7,10 @@
 // result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
 //
 // What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
-// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory, 48 TFLOP/s of
-// it. A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 785 us so; a
-// one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also halve the error against 64-bit sums several times
-// (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
+// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory (16,384 x 2,048,
+// 512 rows: 48 TFLOP/s). A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 785
+// us so (39 TFLOP/s; the 301 rows fill tiles of 320); a one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also
+// halve the error against 64-bit sums several times (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 //
 // These kernels wait for the one before them and let the next one start when they are done: letting it start early left the
 // time of a step as it was.
@@ -96,13 +96,17 @@ gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int 
 
   const int n_chains = kChains / split, chain0 = rank * n_chains;
   const int n_slices = (K + kSlice - 1) / kSlice;
-  // the blocks of 32 k that this block works on, chain by chain (each a whole slice: k >= K reads zeros)
+  // the blocks of 32 k that this block works on, chain by chain: whole slices, and of the last one the blocks that hold a k
+  const int last_blocks = (K - (n_slices - 1) * kSlice + kBK - 1) / kBK;
+  auto chain_blocks = [&](int j) {
+    return j >= n_slices ? 0 : ((n_slices - 1 - j) / kChains + 1) * (kSlice / kBK) -
+                                   (j == (n_slices - 1) % kChains ? kSlice / kBK - last_blocks : 0);
+  };
   int total_blocks = 0;
-  for (int j = chain0; j < chain0 + n_chains; ++j)
-    if (j < n_slices) total_blocks += ((n_slices - 1 - j) / kChains + 1) * (kSlice / kBK);
+  for (int j = chain0; j < chain0 + n_chains; ++j) total_blocks += chain_blocks(j);
 
   // ---- loading, T::kStages - 1 blocks early. A thread brings piece tid % 8 of the rows tid / 8 + kStep p: rows of A first,
-  // then of W. What is left of each piece is an address and a copy, in tiles whose rows are all there; looking at every
+  // then of W. What is left of each piece is an address and a copy, where its rows and its 32 k are all there; looking at every
   // piece's row and k took two instructions for every three of the products.
   constexpr int kStep = T::kThreads / (kBK / 4), kPiecesA = T::BM / kStep, kPiecesW = T::BN / kStep;
   static_assert(T::BM % kStep == 0 && T::BN % kStep == 0, "a piece's row is one of A's or one of W's for all threads");
@@ -119,10 +123,11 @@ gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int 
       const int k0 = ld_slice * kSlice + ld_sub * kBK;
       float* st = ring + ld_stage * T::kStageFloats + ld_row * kStride + ld_c;
       const unsigned dst = (unsigned)__cvta_generic_to_shared(st);
-      if (VEC && k0 + kBK <= K) {
+      if (VEC) {
+        const int bytes = min(max(K - k0 - ld_c, 0), 4) * 4;       // of each piece; the rest reads zeros
         const float* a = a_src + k0;
         const float* w = w_src + k0;
-        if (rows_there) {
+        if (rows_there && k0 + kBK <= K) {
 #pragma unroll
           for (int p = 0; p < kPiecesA; ++p)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + p * kStep * kStride * 4),
@@ -134,15 +139,15 @@ gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int 
         } else {
 #pragma unroll
           for (int p = 0; p < kPiecesA; ++p) {
-            const bool in = p * kStep < a_there;
+            const bool in = bytes && p * kStep < a_there;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + p * kStep * kStride * 4),
-                         "l"(in ? a + (size_t)p * kStep * lda : a), "r"(in ? 16 : 0) : "memory");
+                         "l"(in ? a + (size_t)p * kStep * lda : A), "r"(in ? bytes : 0) : "memory");
           }
 #pragma unroll
           for (int p = 0; p < kPiecesW; ++p) {
-            const bool in = p * kStep < w_there;
+            const bool in = bytes && p * kStep < w_there;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (T::BM + p * kStep) * kStride * 4),
-                         "l"(in ? w + (size_t)p * kStep * ldw : w), "r"(in ? 16 : 0) : "memory");
+                         "l"(in ? w + (size_t)p * kStep * ldw : W), "r"(in ? bytes : 0) : "memory");
           }
         }
       } else {
@@ -156,7 +161,7 @@ gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int 
                      in ? K - k0 - ld_c : 0);
         }
       }
-      if (++ld_sub == kSlice / kBK) { ld_sub = 0; ld_slice += kChains; }
+      if (++ld_sub == (ld_slice == n_slices - 1 ? last_blocks : kSlice / kBK)) { ld_sub = 0; ld_slice += kChains; }
       ld_stage = ld_stage == T::kStages - 1 ? 0 : ld_stage + 1;
       ++ld_count;
     }
@@ -175,7 +180,7 @@ gemm_f32_tile_kernel(const float* A, const float* W, float* __restrict__ C, int 
   int chain = chain0, stage = 0;
   bool first = true;
   for (int c = 0; c < n_chains; ++c, ++chain) {
-    const int blocks = chain < n_slices ? ((n_slices - 1 - chain) / kChains + 1) * (kSlice / kBK) : 0;
+    const int blocks = chain_blocks(chain);
     for (int b = 0; b < blocks; ++b) {
       copy_wait<T::kStages - 2>();
       __syncthreads();
@@ -304,7 +309,9 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
   const int n0 = blockIdx.x * F::kRows;
   const int n_slices = (K + kSlice - 1) / kSlice;
   constexpr int kPerSlice = kSlice / RUN;
-  const int steps = (n_slices + kChains - 1) / kChains * kPerSlice;
+  // rounds of a slice a chain; of the last round the runs that hold a k
+  const int rounds = (n_slices + kChains - 1) / kChains;
+  const int steps = (rounds - 1) * kPerSlice + (min(K - (rounds - 1) * kChains * kSlice, kSlice) + RUN - 1) / RUN;
 
   auto load = [&](int t) {
     if (t < steps) {
@@ -442,19 +449,41 @@ static int dispatch(const float* A, const float* W, float* C, int M, int N, int 
 // Few rows: 8 weight rows a block and six stages where that gives no SM more than two blocks (2,048 x 8,192, 1 / 8 rows:
 // 18 / 35, form 20 26 / 44); 16 weight rows a block above (16,384 x 2,048, 1 / 3 rows: 26 / 30, form 10 29 / 42), and 32
 // from 5 rows on, where a thread's reads of A cost more than its weights (16,384 x 2,048, 8 / 13 rows: 38 / 60, form 20
-// 49 / 76). Tiles: 32 rows high up to 32 rows (16,384 x 2,048, 20 rows: 74, 64 high 115), else 64 x 64 (301 rows: 79, 32
-// x 128 89). The chains are shared among 8 blocks until the tiles alone fill the GPU's 592 places (2,048 x 8,192, 301 rows:
-// 275, 4 blocks 320, 1 block 463), among 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 499, 8
-// 507, 1 516), then each tile has one block (16,384 x 2,048, 512 rows: 723, 4 blocks 776).
-static int choose_form(int M, int N) {
-  if (M <= kFewRows) {
+// 49 / 76) or all lanes have little to do (2,048 x 48, 16 rows: 5.0, form 20 6.5). A K of little more than a slice leaves
+// most lanes idle there, and from 9 rows on wide outputs take tiles instead (8,192 x 64 / 128 / 160, 16 rows: 8.3 / 11.5 /
+// 13.3, form 30 9.6 / 16.2 / 16.2).
+// Tiles: 32 rows high up to 32 rows (16,384 x 2,048, 20 rows: 74, 64 high 115), else 64 x 64 (301 rows: 79, 32 x 128 89).
+//
+// How many blocks share a tile's chains follows from what a slice costs a block: 7 us while an SM holds one or two blocks (a
+// warp on each quarter), 10.5 with three, 14 with four, which is all that fit; clusters do not spread as evenly (14 with
+// three), ranks without a chain hold their places all the same, and every round of clusters costs 2 us. The sum below picks
+// within 20 % of the best of the three forms at 1 to 64 slices and 1 to 4,000 tiles (2,048 x 8,192, 301 rows: 8 blocks 275, 4
+// 320, 1 463; 16,384 x 2,048, 301 rows: 507, 499, 516; 2,048 x 256, 2,100 rows: 209, 208, 64; 2,048 x 512, 128 rows: 18, 21,
+// 32; one plain 64 x 64 tile a block: 122 us at the third, 78 at the last).
+static float tile_time(long long tiles, int slices, int split) {
+  constexpr int kSms = 148, kPlaces = 4 * kSms;
+  const long long blocks = tiles * split, full = blocks / kPlaces, rest = blocks % kPlaces;
+  const int on_sm = (int)((rest + kSms - 1) / kSms);                          // blocks an SM holds in the last round
+  const float last = rest == 0 ? 0.f : (on_sm <= 2 ? 7.f : (split > 1 ? 14.f : 3.5f * on_sm));
+  // slices of the busiest rank: it has the first 8 / split chains
+  int busiest = 0;
+  for (int j = 0; j < kChains / split; ++j) busiest += slices > j ? (slices - 1 - j) / kChains + 1 : 0;
+  return (full * 14.f + last) * busiest + (split > 1 ? 2.f * (full + (rest != 0)) : 0.f);
+}
+
+static int choose_form(int M, int N, int K) {
+  const int slices = (K + kSlice - 1) / kSlice;
+  if (M <= kFewRows && !(M > 8 && K > 32 && K <= 192 && N > 2 * 16 * 148)) {
     const bool narrow = N <= 2 * 8 * 148;
-    if (narrow) return M <= 8 ? 10 : 20;
+    if (narrow) return M <= 8 ? 10 : (K <= 64 ? 30 : 20);
     return M <= 4 ? 20 : 30;
   }
-  if (M <= 32) return 58;
-  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64);
-  return tiles < 640 ? 68 : (tiles < 1900 ? 64 : 61);
+  const bool low = M > kFewRows && M <= 32;
+  const long long tiles = low ? (N + 127) / 128 : (long long)((M + 63) / 64) * ((N + 63) / 64);
+  int best = 1;
+  for (int split = 4; split <= kChains; split *= 2)
+    if (tile_time(tiles, slices, split) < tile_time(tiles, slices, best)) best = split;
+  return (low ? 50 : 60) + best;
 }
 
 }  // namespace llmie
@@ -466,7 +495,7 @@ extern "C" int llmie_gemm_f32_nt_form(const float* A, const float* W, float* C, 
                                       int ldc, int form, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N) return LLMIE_ERR_BAD_ARG;
   if (M == 0) return LLMIE_OK;
-  if (form == 0) form = choose_form(M, N);
+  if (form == 0) form = choose_form(M, N, K);
   const bool vec = aligned16(A) && aligned16(W) && lda % 4 == 0 && ldw % 4 == 0;
   return vec ? dispatch<true>(A, W, C, M, N, K, lda, ldw, ldc, form, stream)
              : dispatch<false>(A, W, C, M, N, K, lda, ldw, ldc, form, stream);

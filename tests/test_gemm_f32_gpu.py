@@ -23,7 +23,8 @@ def _form(a, w, form, ld_extra=0):
 
 @pytest.mark.parametrize("M,N,K", [(1, 2500, 96), (2, 33, 130), (4, 130, 1031), (8, 2369, 128), (9, 100, 1152),
                                    (16, 70, 2052), (17, 129, 4097), (33, 64, 1), (64, 65, 1024), (130, 999, 777),
-                                   (301, 640, 2048)])
+                                   (301, 640, 2048), (64, 130, 16), (13, 4800, 40), (9, 5000, 160), (70, 200, 33),
+                                   (700, 900, 250), (301, 1000, 513), (24, 2100, 384)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_every_form_gives_the_same_bits(M, N, K, offset):
     g = torch.Generator().manual_seed(M * 1000 + K)
