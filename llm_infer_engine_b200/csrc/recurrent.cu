@@ -159,9 +159,9 @@ matrix_scan_kernel(const float* qa, const float* fg, const T* v, int v_ld,
   for (int r = 0; r < RMAX; ++r) prod[r] = 1.f;
   if (t0 < t1) fetch(t0);
   for (int t = t0; t < t1; ++t) {
-    float cf[RMAX], cq[RMAX], cv[C], acc[C];
+    float cf[RMAX], cq[RMAX], cv[C], acc[C], part[C][2];
 #pragma unroll
-    for (int c = 0; c < C; ++c) { cv[c] = vj[c]; acc[c] = 0.f; }
+    for (int c = 0; c < C; ++c) { cv[c] = vj[c]; acc[c] = part[c][0] = part[c][1] = 0.f; }
 #pragma unroll
     for (int r = 0; r < RMAX; ++r) { cf[r] = f[r]; cq[r] = MODE != 1 ? q[r] : 0.f; }
     const float tg = dt_gate, tf = dt_factor;
@@ -173,7 +173,14 @@ matrix_scan_kernel(const float* qa, const float* fg, const T* v, int v_ld,
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         St[r][c] = fmaf(gate, St[r][c], write * cv[c]);
-        if (MODE != 1) acc[c] = fmaf(St[r][c], cq[r], acc[c]);
+        if (MODE != 1) {                           // eight rows' even and odd ones apart, as the kernel below adds them up
+          part[c][r & 1] = fmaf(St[r][c], cq[r], part[c][r & 1]);
+          if (r % 8 == 7) {
+            const float eight = part[c][0] + part[c][1];
+            acc[c] = r < 8 ? eight : acc[c] + eight;
+            part[c][0] = part[c][1] = 0.f;
+          }
+        }
       }
       if (MODE == 1) prod[r] *= gate;
     }
@@ -212,13 +219,12 @@ matrix_scan_kernel(const float* qa, const float* fg, const T* v, int v_ld,
 // The same recurrences where a head's rows are eight times a power of two and its columns a multiple of four (nearly every
 // model): a thread owns 8 rows x 4 columns, S = D / 8 neighbouring lanes share its columns. Gates (or keys) and queries
 // come 16 bytes at a time, the arithmetic is packed over pairs of rows (fma.rn.f32x2), what is read of four tokens is in
-// flight in a ring of registers, and the lanes' sums meet by an exchange that leaves each lane one column. The state's
-// bits are those of the kernel above (the same products and sums in the same order); only the order in which a read-out's
-// D terms are added differs. What bounds it: instructions issued, about 90 a token for 32 state entries where the kernel
-// above needs 200 for 16. Three prompts, 2,150 tokens, 32 heads of 32 x 64: 158 us for the three
-// kernels with the one above, 84 us so (four tokens in flight and four blocks of 128 threads an SM: two tokens 98 us, no
-// bound on the registers 116 us). Short pieces keep one token in flight and seven blocks: a one-token step is the state's
-// way in and out (64 sequences of 32 x 64: 8.4 -> 6.7 us; of 64 x 128, 134 MB: 37.8 -> 39.2 us; with four tokens 55 us).
+// flight in a ring of registers, and the lanes' sums meet by an exchange that leaves each lane one column. The bits are
+// those of the kernel above (the same products and sums in the same order). What bounds it: instructions issued, about 90 a
+// token for 32 state entries where the kernel above needs 200 for 16. Three prompts, 2,150 tokens, 32 heads of 32 x 64: 158
+// us for the three kernels with the one above, 84 us so (four tokens in flight and four blocks of 128 threads an SM: two
+// tokens 98 us, no bound on the registers 116 us). Short pieces keep one token in flight and seven blocks: a one-token step
+// is the state's way in and out (64 sequences of 64 x 128: with four tokens 55 us, so 39).
 __device__ __forceinline__ float2 scan_fma2(const float2& a, const float2& b, const float2& c) {
   float2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -945,6 +951,7 @@ struct ScanArgs {
   float* ws;                   // chunked: scratch, else null
   float* decay;
   int chunk, n_chunks;
+  int one_token;                 // every sequence of the step brings one token (unchunked calls)
 };
 
 template <typename T, int C, int RM, int FORM>
@@ -988,8 +995,17 @@ static void matrix_scan_wide_launch(const ScanArgs& a, cudaStream_t stream) {
 #undef LLMIE_SCAN_ARGS
 }
 
-// Whether the kernel with 8 rows and 4 columns a thread takes these sizes and places (see there).
+// Whether the kernel with 8 rows and 4 columns a thread takes these sizes and places (see there). One-token steps are the
+// state's way in and out, and up to 64 rows the first kernel has an edge in two places (the bits are the same): narrow heads
+// (its one column a thread) while a step's states are below 12 MB (16 heads of 64 x 32, 32 / 64 sequences: 4.1 / 6.3 us, with
+// this one 8.4 / 8.6; 32 of 32 x 64, 16 / 32: 3.8 / 5.8 and 5.5 / 6.0, but 64: 10.0 and 7.8), and wide heads from 24 MB on (64
+// of 64 x 128, 16 / 64: 20.7 / 72.9 and 21.5 / 76.3, but 32 of 64 x 128, 1 / 16: 3.8 / 12.1 and 3.2 / 11.4). From 128 rows on
+// the first has one column a thread and is slower throughout (16 of 128 x 128, 16: 20.7 and 11.3).
 static bool matrix_scan_wide_ok(const ScanArgs& a, int dtype) {
+  if (a.one_token && a.D <= 64) {
+    const long long bytes = 4LL * a.n_seqs * a.H * a.D * a.Dv;
+    if (scan_shape(a.D, a.Dv).C == 1 ? bytes < 12 << 20 : bytes >= 24 << 20) return false;
+  }
   const int S = a.D / 8;
   return a.D % 8 == 0 && (S & (S - 1)) == 0 && S <= 32 && a.Dv % 4 == 0 && a.v_ld % 4 == 0 && aligned16(a.qa) &&
          aligned16(a.fg) && aligned16(a.state) && aligned16(a.o) && (!a.ws || (aligned16(a.ws) && aligned16(a.decay))) &&
@@ -1027,12 +1043,14 @@ static int matrix_scan_entry(const ScanArgs& a, int dtype, cudaStream_t stream) 
 
 // qa, fg float32 [T, H * D]; v rows of H * Dv elements of `dtype`, v_ld apart; state float32 [slots, H, D, Dv];
 // o float32 [T, H * Dv]. D up to 512.
-// head_decay float32 [H] or null: with it, fg holds keys and S <- head_decay[h] S + k_t v_t^T.
+// head_decay float32 [H] or null: with it, fg holds keys and S <- head_decay[h] S + k_t v_t^T. one_token: 1 if every
+// sequence of the step brings one token (it chooses the kernel; both do the same).
 extern "C" int llmie_matrix_scan_ex(const float* qa, const float* fg, const void* v, int v_ld, float* state,
                                     const int* cu_q, const int* seq_slot, float* o, int n_seqs, int H, int D, int Dv,
-                                    int write_state, int dtype, const float* head_decay, cudaStream_t stream) {
+                                    int write_state, int dtype, const float* head_decay, int one_token,
+                                    cudaStream_t stream) {
   const ScanArgs a{qa, fg, v, v_ld, state, cu_q, seq_slot, o, n_seqs, H, D, Dv, write_state, head_decay, nullptr, H,
-                   nullptr, nullptr, 0, 1};
+                   nullptr, nullptr, 0, 1, one_token};
   return head_decay ? matrix_scan_entry<1>(a, dtype, stream) : matrix_scan_entry<0>(a, dtype, stream);
 }
 
@@ -1044,7 +1062,7 @@ extern "C" int llmie_matrix_scan_chunked_ex(const float* qa, const float* fg, co
                                             int dtype, const float* head_decay, cudaStream_t stream) {
   if (!ws || !decay) return LLMIE_ERR_BAD_ARG;
   const ScanArgs a{qa, fg, v, v_ld, state, cu_q, seq_slot, o, n_seqs, H, D, Dv, write_state, head_decay, nullptr, H,
-                   ws, decay, chunk, n_chunks};
+                   ws, decay, chunk, n_chunks, 0};
   return head_decay ? matrix_scan_entry<1>(a, dtype, stream) : matrix_scan_entry<0>(a, dtype, stream);
 }
 
@@ -1054,10 +1072,10 @@ extern "C" int llmie_matrix_scan_stepped(const float* qa, const float* fg, const
                                          const int* cu_q, const int* seq_slot, float* o, float* ws, float* decay,
                                          int n_seqs, int H, int G, int D, int Dv, int chunk, int n_chunks,
                                          int write_state, int dtype, const float* token_decay, const float* key_factor,
-                                         cudaStream_t stream) {
+                                         int one_token, cudaStream_t stream) {
   if (!token_decay || !key_factor) return LLMIE_ERR_BAD_ARG;
   const ScanArgs a{qa, fg, v, v_ld, state, cu_q, seq_slot, o, n_seqs, H, D, Dv, write_state, token_decay, key_factor, G,
-                   ws, decay, chunk, n_chunks};
+                   ws, decay, chunk, n_chunks, ws ? 0 : one_token};
   return matrix_scan_entry<2>(a, dtype, stream);
 }
 

@@ -1631,9 +1631,9 @@ def attention_latent_tc_supported(q, k_cache, v_cache, page_size: int, n_q: int,
     """Whether attention_latent_tc.cu takes a step (answered without loading the library): bfloat16, one key head
     whose rows' first columns are the values, head size a multiple of 16 up to 320, value size a multiple of 64 up to 256,
     pages of 64. Pieces of any length, one token included, so that a sequence's bits do not depend on how long the others of
-    its step are; a tile that is mostly empty still costs less than the kernel of 32 rows a block behind any held tokens (32 heads of 288 / 256,
-    one to three new tokens behind 0 / 300 / 2,000 / 8,000: 7 to 9 / 11 to 13 / 41 / 140 us, the other kernel 6 / 23 / 125 /
-    488 us)."""
+    its step are; a tile that is mostly empty still costs less than the kernel of 32 rows a block behind any held tokens (32
+    heads of 288 / 256, one to three new tokens behind 0 / 300 / 2,000 / 8,000: 7 to 9 / 11 to 13 / 41 / 140 us, the other
+    kernel 6 / 23 / 125 / 488 us)."""
     hdv = v_cache.shape[-1]
     return (q.dtype is torch.bfloat16 and k_cache.dtype is torch.bfloat16 and n_kv == 1 and page_size == 64
             and v_cache.data_ptr() == k_cache.data_ptr() and v_cache.stride(-2) == head_dim and k_cache.is_contiguous()
@@ -1843,23 +1843,24 @@ def matrix_scan(q, f, v, state, cu_q, seq_slot, out, n_seqs: int, heads: int, di
             return out
     if stepped:
         _matrix_scan_stepped(q, f, v, v_ld, state, cu_q, seq_slot, out, None, None, n_seqs, heads, n_qk, dim, vdim, 0, 1,
-                             write_state, head_decay, key_factor)
+                             write_state, head_decay, key_factor, max_len == 1)
         return out
     f_ = _fn("recurrent", "llmie_matrix_scan_ex", [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p,
-                                                   _c_void_p, _c_void_p] + [_c_int] * 6 + [_c_void_p, _c_void_p])
+                                                   _c_void_p, _c_void_p] + [_c_int] * 6 + [_c_void_p, _c_int, _c_void_p])
     _check(f_(q.data_ptr(), f.data_ptr(), v.data_ptr(), v_ld, state.data_ptr(), cu_q.data_ptr(), seq_slot.data_ptr(),
               out.data_ptr(), n_seqs, heads, dim, vdim, 1 if write_state else 0, _dt(v, "v"), _ptr(head_decay),
-              _stream()), "matrix_scan")
+              1 if max_len == 1 else 0, _stream()), "matrix_scan")
     return out
 
 
 def _matrix_scan_stepped(q, f, v, v_ld, state, cu_q, seq_slot, out, ws, decay, n_seqs, heads, groups, dim, vdim, chunk,
-                         n_chunks, write_state, token_decay, key_factor):
+                         n_chunks, write_state, token_decay, key_factor, one_token=False):
     f_ = _fn("recurrent", "llmie_matrix_scan_stepped",
-             [_c_void_p, _c_void_p, _c_void_p, _c_int] + [_c_void_p] * 6 + [_c_int] * 9 + [_c_void_p] * 3)
+             [_c_void_p, _c_void_p, _c_void_p, _c_int] + [_c_void_p] * 6 + [_c_int] * 9 + [_c_void_p] * 2 + [_c_int, _c_void_p])
     _check(f_(q.data_ptr(), f.data_ptr(), v.data_ptr(), v_ld, state.data_ptr(), cu_q.data_ptr(), seq_slot.data_ptr(),
               out.data_ptr(), _ptr(ws), _ptr(decay), n_seqs, heads, groups, dim, vdim, chunk, n_chunks,
-              1 if write_state else 0, _dt(v, "v"), token_decay.data_ptr(), key_factor.data_ptr(), _stream()),
+              1 if write_state else 0, _dt(v, "v"), token_decay.data_ptr(), key_factor.data_ptr(), 1 if one_token else 0,
+              _stream()),
            "matrix_scan_stepped")
 
 

@@ -10,7 +10,7 @@ DEV = "cuda"
 
 @pytest.mark.parametrize("D,Dv", [(8, 4), (16, 12), (32, 64), (64, 36), (128, 8), (256, 68), (24, 20), (32, 30)])
 @pytest.mark.parametrize("form", ["gates", "decay", "stepped"])
-@pytest.mark.parametrize("lens", [[1, 1, 1], [3, 0, 70, 200]])
+@pytest.mark.parametrize("lens", [[1, 1, 1], [5, 1, 40], [3, 0, 70, 200]])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_scan(D, Dv, form, lens, dtype):
     from llm_infer_engine_b200.kernels import ops
@@ -61,3 +61,33 @@ def test_scan(D, Dv, form, lens, dtype):
     one = run(alone, q[a:b].contiguous(), f[a:b].contiguous(), v[a:b], [0, b - a], slots[i:i + 1].contiguous(),
               decay if form != "stepped" else decay[a:b].contiguous(), factor[a:b].contiguous() if form == "stepped" else None)
     assert torch.equal(one, out[a:b]) and torch.equal(alone[int(slots[i])], got_state[int(slots[i])])
+
+
+@pytest.mark.parametrize("H,D,Dv,n", [(4, 8, 4, 3), (2, 16, 16, 2), (16, 64, 32, 5), (32, 32, 64, 60), (32, 64, 128, 3), (32, 64, 128, 40),
+                                      (2, 128, 64, 2)])
+@pytest.mark.parametrize("form", ["gates", "decay", "stepped"])
+def test_both_kernels_give_the_same_bits(H, D, Dv, n, form):
+    """One-token steps go to either kernel by their size and pieces beside a long one to the chunked one: the same bits, values
+    that do not start on 16 bytes (never the kernel with 16-byte loads) included."""
+    from llm_infer_engine_b200.kernels import ops
+    g = torch.Generator().manual_seed(D + Dv)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)                              # noqa: E731
+    T = n + 90                                                     # the last piece is long where it is there
+    q, f = torch.randn(T, H * D, generator=g).to(DEV), torch.rand(T, H * D, generator=g).to(DEV)
+    wide = torch.randn(T, H * Dv + 9, generator=g).to(torch.bfloat16).to(DEV)
+    odd, even = wide[:, 9:], torch.cat([wide[:, 9:]], 1).contiguous()
+    decay = None if form == "gates" else (torch.rand(H, generator=g) if form == "decay" else torch.rand(T, H, generator=g)).to(DEV)
+    factor = torch.rand(T, H, generator=g).to(DEV) if form == "stepped" else None
+    first = torch.randn(n + 1, H, D, Dv, generator=g).to(DEV)
+
+    def run(v, lens):
+        t, state = sum(lens), first.clone()
+        cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        out = torch.empty(t, H * Dv, device=DEV)
+        ops.matrix_scan(q[:t], f[:t], v[:t], state, i32(cu), i32(list(range(len(lens)))), out, len(lens), H, D, Dv,
+                        max_len=max(lens), head_decay=decay if form != "stepped" else decay[:t],
+                        key_factor=factor[:t] if form == "stepped" else None)
+        return out[:n], state[:n]
+
+    a, b, c = run(even, [1] * n), run(odd, [1] * n), run(even, [1] * n + [90])
+    assert all(torch.equal(a[k], b[k]) and torch.equal(a[k], c[k]) for k in (0, 1))
