@@ -454,12 +454,15 @@ static int dispatch(const float* A, const float* W, float* C, int M, int N, int 
 // 13.3, form 30 9.6 / 16.2 / 16.2).
 // Tiles: 32 rows high up to 32 rows (16,384 x 2,048, 20 rows: 74, 64 high 115), else 64 x 64 (301 rows: 79, 32 x 128 89).
 //
-// How many blocks share a tile's chains follows from what a slice costs a block: 7 us while an SM holds one or two blocks (a
-// warp on each quarter), 10.5 with three, 14 with four, which is all that fit; clusters do not spread as evenly (14 with
-// three), ranks without a chain hold their places all the same, and every round of clusters costs 2 us. The sum below picks
-// within 20 % of the best of the three forms at 1 to 64 slices and 1 to 4,000 tiles (2,048 x 8,192, 301 rows: 8 blocks 275, 4
-// 320, 1 463; 16,384 x 2,048, 301 rows: 507, 499, 516; 2,048 x 256, 2,100 rows: 209, 208, 64; 2,048 x 512, 128 rows: 18, 21,
-// 32; one plain 64 x 64 tile a block: 122 us at the third, 78 at the last).
+// How many blocks share a tile's chains: from 16 slices on, 8 until the tiles alone fill the GPU's 592 places (2,048 x 8,192,
+// 301 rows: 275, 4 blocks 320, 1 block 463), 4 until they fill them three times and more (16,384 x 2,048, 301 rows: 499, 8
+// 507, 1 516), then one (16,384 x 2,048, 512 rows: 723, 4 blocks 776). Up to 32 rows 8.
+// With fewer slices some ranks would have one chain or none, and it follows from what a slice costs a block: 7 us while an SM
+// holds one or two blocks (a warp on each quarter), 10.5 with three, 14 with four, which is all that fit; clusters do not
+// spread as evenly (14 with three), ranks without a chain hold their places all the same, and every round of clusters costs 2
+// us. That sum picks within 20 % of the best of the three forms at 1 to 12 slices and 1 to 4,000 tiles (2,048 x 256, 2,100
+// rows: 8 blocks 209, 4 208, 1 64; 2,048 x 512, 128 rows: 18, 21, 32; one plain 64 x 64 tile a block: 122 and 78; from 16
+// slices on it is up to 10 % off the rule above).
 static float tile_time(long long tiles, int slices, int split) {
   constexpr int kSms = 148, kPlaces = 4 * kSms;
   const long long blocks = tiles * split, full = blocks / kPlaces, rest = blocks % kPlaces;
@@ -480,6 +483,7 @@ static int choose_form(int M, int N, int K) {
   }
   const bool low = M > kFewRows && M <= 32;
   const long long tiles = low ? (N + 127) / 128 : (long long)((M + 63) / 64) * ((N + 63) / 64);
+  if (slices >= 2 * kChains) return low ? 58 : (tiles < 640 ? 68 : (tiles < 1900 ? 64 : 61));
   int best = 1;
   for (int split = 4; split <= kChains; split *= 2)
     if (tile_time(tiles, slices, split) < tile_time(tiles, slices, best)) best = split;
