@@ -89,7 +89,7 @@ class KernelPlan:
                                      options.keep_first, options.sink, gate, options.softcap, options.distance_bias,
                                      options.sink_values)
             return True
-        if not ctx.decode and options.plain and ops.attention_prefill_f32_supported(head_dim, kv.page_size, q, kv.k, kv.v):
+        if not ctx.decode and options.plain and ops.attention_prefill_f32_supported(head_dim, kv.page_size, q, kv.k, kv.v, out):
             # prompts of the float32 path
             ops.attention_prefill_f32(q, kv.k, kv.v, out, ctx.cu_q, ctx.seq_slot, ctx.seq_start, kv.block_table,
                                       kv.page_size, ctx.n_seqs, ctx.max_q_len, n_q, n_kv, head_dim, scale, window)
@@ -146,7 +146,7 @@ class KernelPlan:
         shared_rows = not kv.v.is_contiguous()
         if shared_rows and options.keep_first == 0 and not options.softcap \
                 and options.distance_bias is None and options.sigmoid_bias is None and ops.attention_latent_tc_supported(
-                    q, kv.k, kv.v, kv.page_size, n_q, n_kv, head_dim, ctx.max_q_len, options.scale):
+                    q, kv.k, kv.v, kv.page_size, n_q, n_kv, head_dim, ctx.max_q_len, options.scale, out):
             # latent attention: the tcgen05 kernel whose pages are key and value at once
             ops.attention_latent_tc(q, kv.k, kv.v, out, ctx.cu_q, ctx.seq_slot, ctx.seq_start, kv.block_table,
                                     kv.page_size, ctx.n_seqs, ctx.max_q_len, n_q, head_dim, options.scale,

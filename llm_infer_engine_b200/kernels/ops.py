@@ -316,12 +316,12 @@ def attention_paged(q, k_cache, v_cache, out, tok_pos, tok_seq, seq_slot, block_
     return out
 
 
-def attention_prefill_f32_supported(head_dim: int, page_size: int, q, k_cache, v_cache) -> bool:
+def attention_prefill_f32_supported(head_dim: int, page_size: int, q, k_cache, v_cache, out=None) -> bool:
     """Whether attention_prefill_f32.cu takes a prompt step (answered without loading the library): float32, head size 64
-    or 128 of keys and values alike, pages of 64, 16-byte aligned."""
+    or 128 of keys and values alike, pages of 64, everything on 16 bytes."""
     return (q.dtype is torch.float32 and k_cache.dtype is torch.float32 and head_dim in (64, 128) and page_size == 64
             and v_cache.shape == k_cache.shape and v_cache.is_contiguous()
-            and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) & 15)
+            and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | (out.data_ptr() if out is not None else 0)) & 15)
 
 
 def attention_prefill_f32(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, block_table, page_size: int, n_seqs: int,
@@ -1627,10 +1627,10 @@ def attention_rows_mma(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, bloc
 
 
 def attention_latent_tc_supported(q, k_cache, v_cache, page_size: int, n_q: int, n_kv: int, head_dim: int, max_q_len: int,
-                                  scale: float) -> bool:
+                                  scale: float, out=None) -> bool:
     """Whether attention_latent_tc.cu takes a step (answered without loading the library): bfloat16, one key head
     whose rows' first columns are the values, head size a multiple of 16 up to 320, value size a multiple of 64 up to 256,
-    pages of 64. Pieces of any length, one token included, so that a sequence's bits do not depend on how long the others of
+    pages of 64, everything on 16 bytes. Pieces of any length, one token included, so that a sequence's bits do not depend on how long the others of
     its step are; a tile that is mostly empty still costs less than the kernel of 32 rows a block behind any held tokens (32
     heads of 288 / 256, one to three new tokens behind 0 / 300 / 2,000 / 8,000: 7 to 9 / 11 to 13 / 41 / 140 us, the other
     kernel 6 / 23 / 125 / 488 us)."""
@@ -1638,7 +1638,8 @@ def attention_latent_tc_supported(q, k_cache, v_cache, page_size: int, n_q: int,
     return (q.dtype is torch.bfloat16 and k_cache.dtype is torch.bfloat16 and n_kv == 1 and page_size == 64
             and v_cache.data_ptr() == k_cache.data_ptr() and v_cache.stride(-2) == head_dim and k_cache.is_contiguous()
             and head_dim % 16 == 0 and head_dim <= 320 and hdv % 64 == 0 and 0 < hdv <= min(256, head_dim) and scale > 0
-            and max_q_len * n_q <= 128 * 65535 and not (q.data_ptr() | k_cache.data_ptr()) & 15)
+            and max_q_len * n_q <= 128 * 65535
+            and not (q.data_ptr() | k_cache.data_ptr() | (out.data_ptr() if out is not None else 0)) & 15)
 
 
 def attention_latent_tc(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, block_table, page_size: int, n_seqs: int,
@@ -1651,7 +1652,7 @@ def attention_latent_tc(q, k_cache, v_cache, out, cu_q, seq_slot, seq_start, blo
     _need(q, "q", torch.bfloat16, (T, n_q * head_dim))
     _need(out, "out", torch.bfloat16, (T, n_q * hdv))
     _need(k_cache, "k_cache", torch.bfloat16, (None, 1, page_size, head_dim))
-    if not attention_latent_tc_supported(q, k_cache, v_cache, page_size, n_q, 1, head_dim, max_q_len, scale):
+    if not attention_latent_tc_supported(q, k_cache, v_cache, page_size, n_q, 1, head_dim, max_q_len, scale, out):
         raise KernelError(f"attention_latent_tc: sizes {head_dim} / {hdv}, page {page_size} are not supported")
     for name, t in (("cu_q", cu_q), ("seq_slot", seq_slot), ("seq_start", seq_start), ("block_table", block_table)):
         _need(t, name, torch.int32)

@@ -81,3 +81,24 @@ def test_what_is_not_finite_stays_behind(bad):
         a, b = (spoiled, v) if cache is k else (k, spoiled)
         out = _run(q, a, b, table, lens, held, [0], n_q, n_kv, hd, 0.2, 0)
         assert torch.equal(out[:60], want[:60]) and not bool(torch.isfinite(out[60:]).all())
+
+
+@pytest.mark.parametrize("dtype,heads,hd,hdv", [("float32", 4, 64, 64), ("bfloat16", 4, 96, 64)])
+def test_an_output_that_does_not_start_on_16_bytes(dtype, heads, hd, hdv):
+    """As a layer calls it: float32 prompts, and latent rows in bfloat16. The kernels with 16-byte stores refuse such an output
+    and others take it."""
+    import types
+    from llm_infer_engine_b200.parts.base import AttentionOptions
+    from test_parts_gpu import DTYPES, kernel_plan, make_ctx
+    g, dt = torch.Generator().manual_seed(3), DTYPES[dtype]
+    k = torch.randn(4, 1, 64, hd, generator=g).to(dt).to(DEV)
+    v = k[..., :hdv] if hdv != hd else torch.randn(4, 1, 64, hd, generator=g).to(dt).to(DEV)
+    kv = types.SimpleNamespace(k=k, v=v, page_size=64, block_table=torch.tensor([[0, 1, 2]], dtype=torch.int32, device=DEV))
+    q = torch.randn(130, heads * hd, generator=g).to(dt).to(DEV)
+    ctx = make_ctx([130], [0], [0], dtype, kernel_plan(dtype))
+    whole, odd = torch.empty(130, heads * hdv, dtype=dt, device=DEV), torch.empty(130 * heads * hdv + 4, dtype=dt, device=DEV)
+    outs = whole, odd[4 if dtype == "bfloat16" else 1:][:whole.numel()].view_as(whole)
+    for out in outs:
+        ctx.attention(q, kv, out, heads, 1, hd, AttentionOptions(scale=0.1))
+    # two kernels: sums in another order, and in bfloat16 a rounding of the weights and of the result each
+    assert float((outs[0].float() - outs[1].float()).abs().max()) <= (2e-5 if dtype == "float32" else 3e-2)
