@@ -19,7 +19,8 @@ def _close(got, ref, absolute, out_dtype):
 
 
 @pytest.mark.parametrize("T", [1, 16, 17, 64, 65, 200])
-@pytest.mark.parametrize("G,N,K,shift", [(3, 64, 64, 0), (2, 72, 8, 0), (4, 130, 200, 0), (2, 33, 65, 0), (3, 64, 128, 1)])
+@pytest.mark.parametrize("G,N,K,shift", [(3, 64, 64, 0), (2, 72, 8, 0), (4, 130, 200, 0), (2, 33, 65, 0), (3, 64, 128, 1),
+                                         (2, 70, 712, 0)])                   # rings that come round more than once
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_batched(T, G, N, K, shift, out_dtype):
     g = torch.Generator().manual_seed(T + N + K)
@@ -35,7 +36,7 @@ def test_batched(T, G, N, K, shift, out_dtype):
 
 
 @pytest.mark.parametrize("pairs", [5, 63, 150])
-@pytest.mark.parametrize("N,K", [(64, 64), (100, 72), (40, 37)])
+@pytest.mark.parametrize("N,K", [(64, 64), (100, 72), (40, 37), (70, 712)])
 @pytest.mark.parametrize("dual", [False, True])
 def test_routed_tiles_of_both_heights(pairs, N, K, dual):
     E, o = 5, ops()

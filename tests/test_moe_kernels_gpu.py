@@ -33,6 +33,41 @@ def test_route(T, d, E, top, dtype):
     assert torch.equal(one[0], ids[T // 2]) and torch.equal(one_w[0], wt[T // 2])
 
 
+@pytest.mark.parametrize("T", [3, 297])
+@pytest.mark.parametrize("rule", ["all", "sigmoid", "groups"])
+@pytest.mark.parametrize("d,E,top", [(64, 16, 3), (100, 8, 2), (136, 40, 5)])
+def test_route_rules(T, rule, d, E, top):
+    """The other choices and weights, a token and two tokens a block: scores that each token's own part of shared memory holds."""
+    g = torch.Generator().manual_seed(T + E)
+    x, w = torch.randn(T, d, generator=g).to(torch.bfloat16).to(DEV), (torch.randn(E, d, generator=g) / d ** 0.5).to(DEV)
+    correction = None if rule == "sigmoid" else (torch.randn(E, generator=g) * 0.1).to(DEV)
+    mode = {"all": True, "sigmoid": ops().ROUTE_SIGMOID, "groups": ops().ROUTE_SIGMOID_GROUPS}[rule]
+    groups = (4, 2) if rule == "groups" else (1, 1)
+
+    def route(rows):
+        ids = torch.empty(len(rows), top, dtype=torch.int32, device=DEV)
+        wt = torch.empty(len(rows), top, device=DEV)
+        ops().moe_route(rows, w, None, ids, wt, mode, correction, 1.7, groups)
+        return ids, wt
+
+    ids, wt = route(x)
+    z = x.double() @ w.double().T
+    score = z.softmax(1) if rule == "all" else torch.sigmoid(z)
+    choice = z.clone() if rule == "sigmoid" else score + correction.double()
+    if rule == "groups":
+        best = choice.view(T, 4, -1).topk(2, dim=2).values.sum(2).topk(2, dim=1).indices
+        kept = torch.zeros(T, 4, dtype=torch.bool, device=DEV).scatter(1, best, True)
+        choice = choice.masked_fill(~kept.repeat_interleave(E // 4, 1), -1e9)
+    bound = d * 2.0 ** -23 * float((x.double().abs() @ w.double().abs().T).max()) + 1e-6     # sums of d products in float32
+    assert bool(((choice.gather(1, ids.long()) - choice.topk(top, dim=1).values).abs() <= bound).all())
+    picked = score.gather(1, ids.long())
+    want = picked / picked.sum(1, keepdim=True) * 1.7 if rule == "all" else picked * 1.7
+    assert bool(((wt.double() - want).abs() <= 4 * bound).all())
+    for t in (0, T // 2, T - 1):                                             # a token alone: the same bits
+        one, one_w = route(x[t:t + 1].contiguous())
+        assert torch.equal(one[0], ids[t]) and torch.equal(one_w[0], wt[t])
+
+
 @pytest.mark.parametrize("T,d,top", [(1, 8, 1), (5, 2056, 3), (3, 100, 9), (70, 264, 2)])
 @pytest.mark.parametrize("y_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("identity", [False, True])
@@ -71,17 +106,20 @@ def test_gate_per_element(T, n, extra, dtype):
 @pytest.mark.parametrize("Dv", [32, 64, 128, 48, 256])
 @pytest.mark.parametrize("items,per_row", [(1, 1), (7, 7), (66, 3)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("gated", [False, True])
-def test_head_norm(Dv, items, per_row, dtype, gated):
+@pytest.mark.parametrize("gated", [False, "sigmoid", "silu"])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_head_norm(Dv, items, per_row, dtype, gated, per_head):
     g = torch.Generator().manual_seed(Dv + items)
     rows = items // per_row
-    o, w = torch.randn(rows, per_row * Dv, generator=g).to(DEV), (torch.rand(Dv, generator=g) + 0.5).to(DEV)
+    o = torch.randn(rows, per_row * Dv, generator=g).to(DEV)
+    w = (torch.rand(Dv * (per_row if per_head else 1), generator=g) + 0.5).to(DEV)      # of all heads, or one a head
     gate = torch.randn(rows, per_row * Dv + 5, generator=g).to(dtype).to(DEV)[:, 5:] if gated else None
-    y = ops().head_rmsnorm(o, w, 1e-6, torch.empty(rows, per_row * Dv, dtype=dtype, device=DEV), Dv, gate=gate)
+    y = ops().head_rmsnorm(o, w, 1e-6, torch.empty(rows, per_row * Dv, dtype=dtype, device=DEV), Dv, gate=gate,
+                           gate_silu=gated == "silu")
     x = o.double().view(rows, per_row, Dv)
-    ref = (x / (x.square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()).view(rows, -1)
+    ref = (x / (x.square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double().view(-1, Dv)).view(rows, -1)
     if gated:
-        ref = ref * torch.sigmoid(gate.double())
+        ref = ref * torch.sigmoid(gate.double()) * (gate.double() if gated == "silu" else 1)
     rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -18
     assert bool(((y.double() - ref).abs() <= rel * ref.abs() + 1e-30).all())
 
