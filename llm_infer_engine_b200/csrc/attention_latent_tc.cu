@@ -18,10 +18,10 @@
 // A key that a row may not see has weight 0, and 0 times a value that is not finite is NaN. So pages that the causal line or
 // a window's end crosses (one or two of a block's, with whatever the page held behind the sequence's last key) are looked at
 // for such values first; where there is one, that page's share of the output is added up on the CUDA cores, over the keys that
-// a row sees, and the product is left zeros. Two prompts, 2,100 tokens: 57 us, without the look 55.
+// a row sees, and the product is left zeros. Two prompts, 1,805 tokens: 57 us, without the look 55.
 //
 // What bounds it: a page of 64 keys is 544 (hd + hdv) x 128 x 64 products, 544 tensor cycles at hd 288, hdv 256, and as
-// many cycles of exponentials; Q and the ring take 216 KB, one block an SM. Two prompts, 2,100 tokens, 32 heads of 288 /
+// many cycles of exponentials; Q and the ring take 216 KB, one block an SM. Two prompts, 1,805 tokens, 32 heads of 288 /
 // 256: 323 us with the mma.sync kernel of 32 rows (attention_rows_mma.cu), 57 us so.
 #include "tcgen05.cuh"
 #include <math.h>
@@ -51,7 +51,8 @@ struct LatentArgs {
 };
 
 struct LatentShared {
-  uint64_t q_full, k_full[kLtStages], k_empty[kLtStages], s_full[2], s_free[2], p_ready, pv_full, pair_bar[4], looked[kLtStages], odd_bar, drained;
+  uint64_t q_full, k_full[kLtStages], k_empty[kLtStages], s_full[2], s_free[2], p_ready, pv_full, pair_bar[4];
+  uint64_t looked[kLtStages], odd_bar, drained;
   uint32_t tmem_base;
   int abort;
   int odd[kLtStages];             // 1 + the last of a stage's pages that held a value that is not finite

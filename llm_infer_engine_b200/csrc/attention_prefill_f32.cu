@@ -14,8 +14,9 @@
 // the rows in front of it, pages that the causal line or the window's end crosses are looked at for such values first, and
 // keys beyond the sequence's last are never read.
 //
-// What bounds it: operands out of shared memory (12 16-byte reads for 64 packed FMAs). Three prompts of 100 to 700 tokens,
-// 32 heads of 64: 185 us with the plain kernel, 57 us so.
+// What bounds it: three blocks of four warps an SM (168 registers, 68 KB), which wait for dependent instructions and for one
+// another at the pages' barriers (22 % of the issue rate, 21 % of the FMA pipes, 16 % of shared memory). Prompts of 217, 118
+// and 130 tokens, 32 heads of 64: 185 us with the plain kernel, 57 us so.
 #include "common.cuh"
 #include <math.h>
 

@@ -7,9 +7,10 @@
 // result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
 //
 // What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
-// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) and the way of the operands out of shared memory (16,384 x 2,048,
-// 512 rows: 48 TFLOP/s). A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a block, 785
-// us so (39 TFLOP/s; the 301 rows fill tiles of 320); a one-token step of 3 rows went from 4.4 to 0.3 ms. Eight chains also
+// rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) less what the 128 sums of a thread cost: eight warps an SM, which
+// wait for dependent instructions in between (2,048 x 8,192, 301 rows: FMA pipes 60 %, issue 39 %, shared memory 41 %; 16,384
+// x 2,048, 512 rows: 48 TFLOP/s). A gated feed-forward of 2,048 / 8,192 at 301 rows: 2,820 us with one plain 64 x 64 tile a
+// block, 785 us so (39 TFLOP/s; 301 rows fill tiles of 320); a one-token step of 3 rows 4.4 -> 0.3 ms. Eight chains also
 // halve the error against 64-bit sums several times (2,048 terms: 2.0e-6 with one chain, 5e-7 so, relative).
 //
 // These kernels wait for the one before them and let the next one start when they are done: letting it start early left the

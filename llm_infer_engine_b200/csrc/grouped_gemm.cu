@@ -129,9 +129,10 @@ grouped_gemm_kernel(const GroupedArgs p) {
 //
 // With a few rows a group (the experts of a batched one-token step) the weights' stream is what bounds it, with many rows
 // and a short K (the heads of a latent attention layer) the rows' way in and out. So: K steps of 64 arrive in a ring of
-// asynchronous copies, 16 bytes each, two steps ahead; fragments come by ldmatrix from rows of 128 bytes whose
-// eight pieces are exchanged by the row's number (no two rows of an 8 x 8 block share a bank); only the 16-row slices of a
-// tile that hold rows are multiplied; and results leave through shared memory in whole rows.
+// asynchronous copies, 16 bytes each, kStages - 1 steps ahead (two, or four for 16 rows of one matrix); fragments come by
+// ldmatrix from rows of 128 bytes whose eight pieces are exchanged by the row's number (no two rows of an 8 x 8 block share a
+// bank); only the 16-row slices of a tile that hold rows are multiplied; and results leave through shared memory in whole
+// rows.
 // `vec`: K, the leading dimensions and the group strides are multiples of 8 elements and the bases 16-byte aligned;
 // otherwise the tiles are brought element by element. `cvec`: the same of C, for 16-byte stores.
 __device__ __forceinline__ void gg_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
@@ -157,7 +158,7 @@ struct MmaTile {
   static constexpr int kStages = BM == 16 && !DUAL ? 5 : 3;
   static constexpr int kOutPitch = kMmaBN + 4;                          // floats between two rows on their way out
   static constexpr int kOutBytes = BM * kOutPitch * 4;
-  // a K of fewer steps leaves the ring's other stages out: 2,100 rows of 32 heads, 64 -> 256 (one step): six blocks an SM
+  // a K of fewer steps leaves the ring's other stages out: 1,805 rows of 32 heads, 64 -> 256 (one step): six blocks an SM
   // instead of four, 22.7 us instead of 26.7
   static int smem_bytes(int steps) {
     const int ring = (steps < kStages ? steps : kStages) * kStageBytes;
@@ -166,7 +167,7 @@ struct MmaTile {
 };
 
 // Short products of full tiles wait for their loads, and registers set how many blocks wait at once: eight blocks an SM
-// (64 registers, nothing spilled) instead of six (78) take a latent-attention layer over 2,100 rows, with two products a
+// (64 registers, nothing spilled) instead of six (78) take a latent-attention layer over 1,805 rows, with two products a
 // head, from 163.9 to 162.0 us. Longer rings and pairs of weights are held by shared memory instead.
 template <typename TC, int BM, bool DUAL>
 __global__ void __launch_bounds__(128, BM == 64 && !DUAL ? 8 : 1)

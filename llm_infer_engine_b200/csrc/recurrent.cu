@@ -57,7 +57,7 @@ __global__ void matrix_gates_kernel(const T* proj, int ld, int q_off, int f_off,
 }
 
 // The same, eight elements a thread and a row of blocks per token (n, ld and the offsets multiples of 8, 16-byte aligned):
-// 2,150 tokens of 2 x 1,024: 10.9 us element by element with an index divided for each, 8.4 us so.
+// 2,117 tokens of 2 x 1,024: 10.9 us element by element with an index divided for each, 8.4 us so.
 template <typename T>
 __global__ void __launch_bounds__(128)
 matrix_gates_vec_kernel(const T* proj, int ld, int q_off, int f_off, const float* LLMIE_WEIGHT f_bias,
@@ -220,10 +220,11 @@ matrix_scan_kernel(const float* qa, const float* fg, const T* v, int v_ld,
 // model): a thread owns 8 rows x 4 columns, S = D / 8 neighbouring lanes share its columns. Gates (or keys) and queries
 // come 16 bytes at a time, the arithmetic is packed over pairs of rows (fma.rn.f32x2), what is read of four tokens is in
 // flight in a ring of registers, and the lanes' sums meet by an exchange that leaves each lane one column. The bits are
-// those of the kernel above (the same products and sums in the same order). What bounds it: instructions issued, about 90 a
-// token for 32 state entries where the kernel above needs 200 for 16. Three prompts, 2,150 tokens, 32 heads of 32 x 64: 158
-// us for the three kernels with the one above, 84 us so (four tokens in flight and four blocks of 128 threads an SM: two
-// tokens 98 us, no bound on the registers 116 us). Short pieces keep one token in flight and seven blocks: a one-token step
+// those of the kernel above (the same products and sums in the same order). What bounds it: instructions, about 90 a token
+// for 32 state entries where the kernel above needs 200 for 16, at half of the issue rate: a dozen warps an SM, which wait
+// for a token's operands and for one another's results. Three prompts, 2,117 tokens, 32 heads of 32 x 64: 158 us for the
+// three kernels with the one above, 84 us so, 67 us in a captured launch (four tokens in flight and four blocks of 128
+// threads an SM: two tokens 98 us, no bound on the registers 116 us). Short pieces keep one token in flight and seven blocks: a one-token step
 // is the state's way in and out (64 sequences of 64 x 128: with four tokens 55 us, so 39).
 __device__ __forceinline__ float2 scan_fma2(const float2& a, const float2& b, const float2& c) {
   float2 d;
@@ -457,7 +458,7 @@ __global__ void head_rmsnorm_kernel(const float* o, const float* LLMIE_WEIGHT w,
 }
 
 // Heads of 4 LANES channels (32, 64, 128): LANES lanes hold an item in registers, four channels each, so the row is read
-// once and 16 bytes at a time. 2,150 tokens of 32 heads of 64: 19 us with 4-byte accesses, a warp an item and a second
+// once and 16 bytes at a time. 2,117 tokens of 32 heads of 64: 19 us with 4-byte accesses, a warp an item and a second
 // pass, 6.3 us so.
 template <typename T, int LANES>
 __global__ void __launch_bounds__(256)

@@ -1,7 +1,7 @@
-"""Which kernel serves which call. The float32 engine uses the plain kernels throughout; the
-bfloat16 engine swaps in the fast ones where their size limits are met and says no otherwise,
-in which case the caller falls back to the plain kernel of the same math (never to a CPU or
-library path)."""
+"""Which kernel serves which call. Both engines take a fast kernel where its size limits and
+options are met (the float32 engine: prompts in tiles, one-token steps split over the keys) and
+say no otherwise, in which case the caller falls back to the plain kernel of the same math (never
+to a CPU or library path)."""
 from __future__ import annotations
 
 import torch
