@@ -1,0 +1,675 @@
+// True float32 matrix product on the tensor cores: C[M, N] = A[M, K] * W[N, K]^T for large weights of the 32-bit path.
+//
+// A float32 number is the exact sum of three bfloat16 numbers, x = x1 + x2 + x3: x rounded, what is left rounded, the rest. A
+// product of two bfloat16 numbers is exact in float32. Of the nine products of parts the six with a weight of 2^-16 or more are
+// formed; the three left out are below 2^-25 of the product and of either sign (parts that were cut off instead of rounded
+// would leave out 3e-8 of one sign). w1 x1 has a sum of its own, G1; the other five share G2, which is 2^-8 of it, so that only
+// G1 is subject to the accumulator's rounding (it cuts off what does not fit), and that for 128 k only: then G1 + G2 joins a
+// float32 sum in registers. Relative error against 64-bit sums (2-norm; sums in packed FMAs, gemm_simt.cu, in brackets): 2,048
+// terms 1.3e-7 (2.1e-7), 8,192 terms 1.4e-7 (4.1e-7); an attention layer of 2,048 3.6e-7 (3.9e-7), a feed-forward of 2,048 /
+// 8,192 3.9e-7 (5.2e-7).
+//
+// One summation order for every shape. K is cut into slices of 128; n slices make four chains, chain j the slices
+// [j n / 4, (j + 1) n / 4); a chain's sum P_j adds its slices in order, and the result is (P_0 + P_1) + (P_2 + P_3). A row's
+// result does not depend on which other rows share the launch, on the tile or on how the chains are shared among blocks.
+//
+// Sums that are not finite (an infinity or NaN among the inputs, whose parts are NaN, or an overflow, of a part too) are formed again by plain
+// FMAs over K, which give what IEEE arithmetic gives.
+//
+// A block makes 128 weight rows x NT tokens. The weights are the 128-row operand; per 16 k five tcgen05.mma: w1 by [x1 x2] into
+// [G1 G2], then w1 x3, w2 x1, w2 x2, w3 x1 into G2. Sixteen warps in four groups, a group a stage of 32 k, read the weights as
+// float32, 32 bytes a lane and a round of the groups ahead, split them and store the parts as swizzled operands; the tokens'
+// parts were made by a kernel in front and come by TMA, eight stages deep (NT = 16: the same warps split them); one lane issues
+// the products, two stages a turn; eight warps empty one of two accumulators while the other fills, and keep the sums of
+// finished chains in the tensor memory behind them.
+//
+// What bounds it: 128 x 80 tokens x 32 k are 480 cycles of products, a stage takes about 900: the hand-over from the splitting
+// warps to the issuing lane and back, and the splitting itself (nine instructions for two weights). Products of 2,048 k (FMA in
+// brackets): 301 x 16,384 149 us (498), 465 x 3,072 40 (165), 301 x 2,048 x 8,192 k 75 (275); a gated feed-forward of 2,048 /
+// 8,192 at 301 rows 250 us (784), 72 rows 85 (385).
+#include "tcgen05.cuh"
+
+namespace llmie {
+namespace {
+using namespace tc;
+
+constexpr int kMt = 128;                  // weight rows of a block
+constexpr int kStageK = 32;              // 64 bytes of a part's row, 64-byte swizzle
+constexpr int kPerSlice = 128 / kStageK;  // stages of a slice
+constexpr int kSliceK = 128;
+constexpr int kChains = 4;
+constexpr int kSumWarps = 8, kSplitWarps = 16;
+constexpr int kStages = 4;                // four warps split for each
+constexpr int kPieces = kMt * (kStageK / 8) / 128;        // pieces of 8 weights a thread and stage
+static_assert(kSplitWarps == 4 * kStages && kStages == kPerSlice, "the stages of a slice go round four groups of warps");
+constexpr int kTcThreads = 32 * (kSumWarps + kSplitWarps + 4);        // the last four: one issues products, one copies
+
+template <int NT>
+struct Shape {
+  static constexpr bool kSplitsX = NT == 16;                 // else the tokens' parts come by TMA
+  static constexpr int kWPart = kMt * 64, kXPart = NT * 64;  // bytes of one part of a stage
+  static constexpr int kWStage = 3 * kWPart, kXStage = 3 * kXPart;
+  static constexpr int kXStages = kSplitsX ? kStages : 8;    // copies run further ahead: a copy takes two stages' time
+  static constexpr int kSmem = kStages * kWStage + kXStages * kXStage + 1024;
+  static constexpr int kHold0 = 4 * NT, kHold1 = 5 * NT;     // columns behind the two accumulators: sums of finished chains
+  static constexpr int kAccCols = 2 * NT, kTmemCols = NT == 16 ? 128 : 512;
+  static constexpr int kCols = NT / 2;                       // of a sum warp
+  static_assert(6 * NT <= kTmemCols && NT * kMt * 4 <= kStages * kWStage, "");
+};
+
+// Byte offset of piece `piece` (16 bytes) of row `row` in 64-byte rows with the 64-byte swizzle, and its operand descriptor.
+__device__ __forceinline__ uint32_t swizzle64_offset(int row, int piece) {
+  return (uint32_t)row * 64u + (uint32_t)((piece ^ ((row >> 1) & 3)) << 4);
+}
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr >> 4) & 0x3FFF) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)4 << 61;
+}
+
+struct TcShared {
+  uint64_t full[kStages], empty[kStages], x_full[8], x_empty[8], acc_full[2], acc_empty[2];
+  uint32_t tmem;
+  int abort;
+};
+
+// 8 neighbouring floats; WIDE: from a 32-byte aligned address. No condition around it: the values of a load that is skipped
+// would have to be merged with what it brings, and that waits for it.
+template <bool WIDE>
+__device__ __forceinline__ void load_8(const float* p, float (&v)[8]) {
+  if (WIDE) {
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v[e]) : "l"(p + e));
+  }
+}
+
+__device__ __forceinline__ unsigned pack_rn(float a, float b) {
+  unsigned v;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(b), "f"(a));
+  return v;
+}
+// The three parts of 8 floats, 16 bytes each.
+__device__ __forceinline__ void split_8(const float (&v)[8], uint4 (&parts)[3]) {
+  unsigned h[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = v[2 * i], b = v[2 * i + 1];
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      h[part][i] = pack_rn(a, b);
+      if (part < 2) {
+        a -= __uint_as_float(h[part][i] << 16);
+        b -= __uint_as_float(h[part][i] & 0xffff0000u);
+      }
+    }
+  }
+#pragma unroll
+  for (int part = 0; part < 3; ++part) parts[part] = make_uint4(h[part][0], h[part][1], h[part][2], h[part][3]);
+}
+__device__ __forceinline__ void split_store(const float (&v)[8], unsigned char* dst, int part_bytes) {
+  uint4 parts[3];
+  split_8(v, parts);
+#pragma unroll
+  for (int part = 0; part < 3; ++part) *reinterpret_cast<uint4*>(dst + part * part_bytes) = parts[part];
+}
+
+// parts[p][t][k]: part p of A[t][k], K a multiple of 8.
+template <bool WIDE>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* A, __nv_bfloat16* __restrict__ out, int M, int K, int lda) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int per_row = K >> 3;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= (long long)M * per_row) return;
+  const int t = (int)(i / per_row), k = (int)(i - (long long)t * per_row) << 3;
+  float v[8];
+  uint4 parts[3];
+  load_8<WIDE>(A + (size_t)t * lda + k, v);
+  split_8(v, parts);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(out + ((size_t)p * M + t) * K + k) = parts[p];
+}
+
+__device__ __forceinline__ float plain_dot(const float* x, const float* w, int K) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
+  return s;
+}
+
+// N consecutive columns of 32 lanes, N a multiple of 8; tmem_ld_wait() before they are used.
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+// run (+)= G1 + G2, 24 columns at a time.
+template <int C0, int N>
+__device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)[N], bool fresh) {
+  constexpr int n = N - C0 < 24 ? N - C0 : 24;
+  uint32_t a[n], b[n];
+#pragma unroll
+  for (int c = 0; c < n; c += 8) tmem_ld_32x8(g1 + C0 + c, a + c);
+#pragma unroll
+  for (int c = 0; c < n; c += 8) tmem_ld_32x8(g1 + to_g2 + C0 + c, b + c);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < n; ++c) {
+    const float v = __uint_as_float(a[c]) + __uint_as_float(b[c]);
+    run[C0 + c] = fresh ? v : run[C0 + c] + v;
+  }
+  if constexpr (C0 + n < N) sum_columns<C0 + n, N>(g1, to_g2, run, fresh);
+}
+
+// The held sums of a warp's columns: `run` becomes held + run, or what is held.
+template <int N>
+__device__ __forceinline__ void add_held(uint32_t taddr, float (&run)[N]) {
+#pragma unroll
+  for (int c = 0; c < N; c += 8) {
+    uint32_t a[8];
+    tmem_ld_32x8(taddr + c, a);
+    tmem_ld_wait();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) run[c + e] = __uint_as_float(a[e]) + run[c + e];
+  }
+}
+template <int N>
+__device__ __forceinline__ void put_held(uint32_t taddr, const float (&run)[N]) {
+#pragma unroll
+  for (int c = 0; c < N; c += 8)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr + c), "f"(run[c]), "f"(run[c + 1]), "f"(run[c + 2]), "f"(run[c + 3]), "f"(run[c + 4]),
+                 "f"(run[c + 5]), "f"(run[c + 6]), "f"(run[c + 7]) : "memory");
+  tmem_st_wait();
+}
+
+template <int NT, bool WIDE>
+__global__ void __launch_bounds__(kTcThreads, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, const float* LLMIE_WEIGHT W, float* C, int M, int N,
+                   int K, int lda, int ldw, int ldc, int split, int* __restrict__ status) {
+  using S = Shape<NT>;
+  extern __shared__ __align__(1024) unsigned char tc_smem[];
+  __shared__ TcShared sh;
+  unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~(uintptr_t)1023);
+  unsigned char* x_stages = stages + kStages * S::kWStage;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x % split;
+  const int tiles_m = (M + NT - 1) / NT, tile = blockIdx.x / split;
+  const int m0 = (tile % tiles_m) * NT, n0 = (tile / tiles_m) * kMt;
+  const int slices = K / kSliceK;
+  const int chain0 = rank * (kChains / split);
+  const int slice0 = chain0 * slices / kChains, slice1 = (chain0 + kChains / split) * slices / kChains;
+  const int n_stages = kPerSlice * (slice1 - slice0);
+  volatile int* abort = &sh.abort;
+
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&sh.full[i], 4);
+      mbar_init(&sh.empty[i], 1);
+    }
+    for (int i = 0; i < 8; ++i) {
+      mbar_init(&sh.x_full[i], 1);
+      mbar_init(&sh.x_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh.acc_full[i], 1);
+      mbar_init(&sh.acc_empty[i], kSumWarps);
+    }
+    sh.abort = 0;
+    fence_mbar_init();
+  }
+  if (warp == kSumWarps + kSplitWarps) {
+    tmem_alloc(&sh.tmem, S::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = sh.tmem;
+
+  if (warp < kSumWarps) {
+    // ---------------------------------------------------------------- sums: half of the tokens each four warps
+    if (!S::kSplitsX) asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+    pdl_wait();
+    const int quarter = warp & 3, col0 = (warp >> 2) * S::kCols, row = quarter * 32 + lane;
+    const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
+    const bool row_there = n0 + row < N;
+    float* out = C + (size_t)(m0 + col0) * ldc + n0 + row;
+    const int n_cols = row_there ? min(S::kCols, M - m0 - col0) : 0;       // of the result
+    float run[S::kCols] = {};
+    int chain = 0, chain_end = (chain0 + 1) * slices / kChains;
+    bool fresh = true, ok = true;
+#pragma unroll 1
+    for (int slice = slice0; slice < slice1; ++slice) {
+      const int i = slice - slice0, ab = i & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[ab], (i >> 1) & 1, abort));
+      if (!ok) {
+        if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutMma); }
+        break;
+      }
+      tc_fence_after_sync();
+      sum_columns<0, S::kCols>(acc + ab * S::kAccCols, NT, run, fresh);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
+      fresh = slice + 1 == chain_end;
+      if (fresh) {                        // the chain is done: ((P_0 + P_1) + (P_2 + P_3)) as far as this block has them
+        if (chain & 1) add_held<S::kCols>(acc + (chain == 3 ? S::kHold1 : S::kHold0), run);
+        if (chain == 3) add_held<S::kCols>(acc + S::kHold0, run);
+        if (chain < kChains / split - 1) put_held<S::kCols>(acc + (chain == 2 ? S::kHold1 : S::kHold0), run);
+        ++chain;
+        chain_end = (chain0 + chain + 1) * slices / kChains;
+      }
+    }
+    if (!ok) {                            // (the plain sums below then replace these)
+#pragma unroll
+      for (int c = 0; c < S::kCols; ++c) run[c] = __int_as_float(0x7fc00000);
+    }
+    if (split > 1) {                      // the operands have been read: their place takes the sums
+      float* h = reinterpret_cast<float*>(stages) + (size_t)col0 * kMt + row;
+#pragma unroll
+      for (int c = 0; c < S::kCols; ++c) h[c * kMt] = run[c];
+    } else {
+      bool finite = true;
+#pragma unroll
+      for (int c = 0; c < S::kCols; ++c) {
+        if (c < n_cols) {
+          out[(size_t)c * ldc] = run[c];
+          finite = finite && fabsf(run[c]) <= 3.402823466e38f;
+        }
+      }
+      if (!finite) {
+        for (int c = 0; c < n_cols; ++c)
+          if (!(fabsf(out[(size_t)c * ldc]) <= 3.402823466e38f))
+            out[(size_t)c * ldc] = plain_dot(A + (size_t)(m0 + col0 + c) * lda, W + (size_t)(n0 + row) * ldw, K);
+      }
+    }
+  } else if (warp < kSumWarps + kSplitWarps) {
+    // ---------------------------------------------------------------- float32 in, parts out
+    if (!S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const int group = (warp - kSumWarps) >> 2, gt = tid & 127, r = gt >> 2, piece = gt & 3;
+    // rows behind the last are the last one again, stages behind the last one too: nobody reads what becomes of them
+    const float* w_src[kPieces];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i)
+      w_src[i] = W + (size_t)min(n0 + r + 32 * i, N - 1) * ldw + slice0 * kSliceK + piece * 8;
+    const float* a_src = A + (size_t)min(m0 + r, M - 1) * lda + slice0 * kSliceK + piece * 8;
+    const uint32_t at = swizzle64_offset(r, piece);            // 32 rows on: the same place in its 128 bytes
+    unsigned char* st = stages + group * S::kWStage + at;
+    float w[kPieces][8], x[8];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) load_8<WIDE>(w_src[i] + group * kStageK, w[i]);
+    if (S::kSplitsX) {
+      pdl_wait();                           // weights are written by no kernel
+      load_8<WIDE>(a_src + group * kStageK, x);
+    }
+    uint32_t parity = 1;                    // a fresh barrier counts as released
+    for (int s = group; s < n_stages; s += kStages, parity ^= 1) {
+      if (!mbar_wait(&sh.empty[group], parity, abort)) {
+        if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
+        break;
+      }
+      const int next = min(s + kStages, n_stages - 1) * kStageK;
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        split_store(w[i], st + 32 * 64 * i, S::kWPart);
+        load_8<WIDE>(w_src[i] + next, w[i]);
+      }
+      if (S::kSplitsX) {
+        if (r < NT) split_store(x, x_stages + group * S::kXStage + at, S::kXPart);
+        load_8<WIDE>(a_src + next, x);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.full[group]);
+    }
+  } else {
+    if (!S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == kSumWarps + kSplitWarps) {
+      // -------------------------------------------------------------- products
+      // The whole warp walks the stages, so that addresses and descriptors are the warp's and not a thread's; one lane issues.
+      constexpr uint32_t d2 = make_instr_desc_bf16(kMt, 2 * NT, 0, 0), d1 = make_instr_desc_bf16(kMt, NT, 0, 0);
+      const bool leader = elect_one();
+      const uint64_t first_w = operand_desc(smem_u32(stages)), first_x = operand_desc(smem_u32(x_stages));
+      constexpr uint64_t kWNext = S::kWPart / 16, kXNext = S::kXPart / 16;
+      const int n_slices = slice1 - slice0;
+      bool ok = true;
+      for (int slice = 0; ok && slice < n_slices; ++slice) {
+        const uint32_t g1 = tmem + (slice & 1) * S::kAccCols, g2 = g1 + NT;
+        if (slice >= 2) ok = mbar_wait(&sh.acc_empty[slice & 1], ((slice >> 1) - 1) & 1, abort);
+#pragma unroll
+        for (int pair = 0; pair < kStages; pair += 2) {       // two stages a turn: half as many waits in the way of the products
+          // stage `pair` of an even slice is the tokens' stage `pair`, of an odd one 4 + pair
+          const int xs = S::kSplitsX ? pair : (slice & 1) * kStages + pair;
+          ok = ok && mbar_wait(&sh.full[pair], slice & 1, abort) && mbar_wait(&sh.full[pair + 1], slice & 1, abort);
+          if (!S::kSplitsX)
+            ok = ok && mbar_wait(&sh.x_full[xs], (slice >> 1) & 1, abort) && mbar_wait(&sh.x_full[xs + 1], (slice >> 1) & 1, abort);
+          if (!ok) break;
+          // the parts were written through the generic proxy. The fence stands here and not behind the stores: there it would
+          // also wait for the loads that run ahead
+          fence_proxy_async_smem();
+          tc_fence_after_sync();
+          if (leader) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int stage = pair + e;
+              const uint64_t w1 = first_w + stage * (S::kWStage / 16), w2 = w1 + kWNext, w3 = w2 + kWNext;
+              const uint64_t x1 = first_x + (xs + e) * (S::kXStage / 16), x2 = x1 + kXNext, x3 = x2 + kXNext;
+#pragma unroll
+              for (int kk = 0; kk < 2 * (kStageK / 16); kk += 2) {        // 32 bytes of a row: 2 in a descriptor's units
+                mma_bf16_ss(g1, w1 + kk, x1 + kk, d2, stage > 0 || kk > 0 ? 1u : 0u);
+                mma_bf16_ss(g2, w1 + kk, x3 + kk, d1, 1u);
+                mma_bf16_ss(g2, w2 + kk, x1 + kk, d1, 1u);
+                mma_bf16_ss(g2, w2 + kk, x2 + kk, d1, 1u);
+                mma_bf16_ss(g2, w3 + kk, x1 + kk, d1, 1u);
+              }
+              mma_commit(&sh.empty[stage]);
+              if (!S::kSplitsX) mma_commit(&sh.x_empty[xs + e]);
+            }
+            if (pair + 2 == kStages) mma_commit(&sh.acc_full[slice & 1]);
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok && leader && !*abort) { *abort = 1; atomicExch(status, kStatusTimeoutFull); }
+      __syncwarp();
+    } else if (warp == kSumWarps + kSplitWarps + 1 && !S::kSplitsX) {
+      // -------------------------------------------------------------- the tokens' parts
+      if (elect_one()) {
+        tma_prefetch_desc(&map_x);
+        pdl_wait();
+        int issued = 0;
+        for (int s = 0; s < n_stages; ++s) {
+          const int xs = s & 7;
+          if (!mbar_wait(&sh.x_empty[xs], ((s >> 3) & 1) ^ 1, abort)) {
+            if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
+            break;
+          }
+          mbar_arrive_expect_tx(&sh.x_full[xs], S::kXStage);
+#pragma unroll
+          for (int p = 0; p < 3; ++p)
+            tma_load_2d(x_stages + xs * S::kXStage + p * S::kXPart, &map_x, slice0 * kSliceK + s * kStageK, p * M + m0,
+                        &sh.x_full[xs]);
+          issued = s + 1;
+        }
+        if (*abort) {       // the copies of this thread land, or have had the time to, before their shared memory is given up
+          for (int s = max(0, issued - 8); s < issued; ++s)
+            for (unsigned spin = 0; spin < (1u << 14) && !mbar_test(&sh.x_full[s & 7], (s >> 3) & 1); ++spin) __nanosleep(64);
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (split > 1) {
+    cluster_sync_all();
+    if (warp < kSumWarps) {               // each block of the cluster finishes its share of the tokens
+      const int row = (warp & 3) * 32 + lane;
+      if (n0 + row < N) {
+        for (int c = rank * 2 + (warp >> 2); c < NT && m0 + c < M; c += 2 * split) {
+          const uint32_t a = smem_u32(reinterpret_cast<float*>(stages) + (size_t)c * kMt + row);
+          float v;
+          if (split == 2)
+            v = ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1));
+          else
+            v = (ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1))) +
+                (ld_cluster_f32(map_to_block(a, 2)) + ld_cluster_f32(map_to_block(a, 3)));
+          if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(A + (size_t)(m0 + c) * lda, W + (size_t)(n0 + row) * ldw, K);
+          C[(size_t)(m0 + c) * ldc + n0 + row] = v;
+        }
+      }
+    }
+    cluster_sync_all();                   // nobody leaves while its sums are read
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == kSumWarps + kSplitWarps) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, S::kTmemCols);
+  }
+}
+
+// ------------------------------------------------------------------------------------------ up to 16 tokens
+// What bounds it is the weights' way from memory: 3 tokens, 16,384 x 2,048 27.7 us (4.8 TB/s; FMA from shared memory 29.5),
+// 32,000 x 2,048 47 (5.6 TB/s; 49.7), 2,048 x 8,192 19.7 (22.5), 3,072 x 2,048 9.3 (9.7), 1 token 2,048 x 2,048 7.4 (5.6); 16
+// tokens, 2,048 x 2,048 8.8 (15.5).
+//
+// The same sums by mma.sync, which rounds as tcgen05.mma does, whatever the order of the k inside a product (tests compare the
+// bits): weights go from memory into registers and are split there, so nothing stands between a load and the next one. A block
+// makes 16 weight rows; its warps take slices in turn, and a slice's sums meet in shared memory, where they are added in the
+// order of the chains. A lane's 16 bytes of a row are four neighbouring k of the sixteen of a product.
+constexpr int kFewWarps = 8;
+
+__device__ __forceinline__ void few_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool VEC>
+__device__ __forceinline__ float4 few_load_w(const float* p) {
+  float4 v;
+  if (VEC) {
+    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  } else {
+    v = make_float4(p[0], p[1], p[2], p[3]);
+  }
+  return v;
+}
+// The parts of four neighbours, each part as two packed pairs.
+__device__ __forceinline__ void split_4(const float4& v, unsigned (&h)[3][2]) {
+  float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int part = 0; part < 3; ++part) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      h[part][i] = pack_rn(e[2 * i], e[2 * i + 1]);
+      if (part < 2) {
+        e[2 * i] -= __uint_as_float(h[part][i] << 16);
+        e[2 * i + 1] -= __uint_as_float(h[part][i] & 0xffff0000u);
+      }
+    }
+  }
+}
+
+template <int T8, bool VEC>      // T8: eights of tokens
+__global__ void __launch_bounds__(kFewWarps * 32, 2)
+gemm_f32_few_kernel(const float* A, const float* LLMIE_WEIGHT W, float* __restrict__ C, int M, int N, int K, int lda, int ldw,
+                    int ldc) {
+  extern __shared__ float sums[];         // [slices][T8][4][32]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int tiles = (N + 15) / 16, slices = K / kSliceK;
+  const float* a_src[T8];
+#pragma unroll
+  for (int i = 0; i < T8; ++i) a_src[i] = A + (size_t)min(g + 8 * i, M - 1) * lda + 4 * t;
+  const float *w_lo, *w_hi;               // of the slice that is loaded
+  auto point = [&](int tile, int slice) {
+    const float* w = W + slice * kSliceK + 4 * t;
+    w_lo = w + (size_t)min(tile * 16 + g, N - 1) * ldw;
+    w_hi = w + (size_t)min(tile * 16 + g + 8, N - 1) * ldw;
+  };
+  float4 lo[8], hi[8];                    // a slice of this warp: eight products' worth of k
+  point(blockIdx.x, min(warp, slices - 1));
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    lo[j] = few_load_w<VEC>(w_lo + 16 * j);
+    hi[j] = few_load_w<VEC>(w_hi + 16 * j);
+  }
+  pdl_wait();                             // weights are written by no kernel
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+#pragma unroll 1
+    for (int slice = warp; slice < slices; slice += kFewWarps) {
+      float g1[T8][4], g2[T8][4];
+#pragma unroll
+      for (int i = 0; i < T8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g1[i][e] = g2[i][e] = 0.f;
+      // the next slice of this tile, or this warp's first of the block's next tile
+      if (slice + kFewWarps < slices) point(tile, slice + kFewWarps);
+      else point(min(tile + (int)gridDim.x, tiles - 1), warp);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        unsigned a[2][3][2];
+        split_4(lo[j], a[0]);
+        split_4(hi[j], a[1]);
+        lo[j] = few_load_w<VEC>(w_lo + 16 * j);
+        hi[j] = few_load_w<VEC>(w_hi + 16 * j);
+        unsigned w[3][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          w[p][0] = a[0][p][0];
+          w[p][1] = a[1][p][0];
+          w[p][2] = a[0][p][1];
+          w[p][3] = a[1][p][1];
+        }
+#pragma unroll
+        for (int i = 0; i < T8; ++i) {
+          const float* x_at = a_src[i] + slice * kSliceK + 16 * j;
+          const float4 v = VEC ? *reinterpret_cast<const float4*>(x_at) : make_float4(x_at[0], x_at[1], x_at[2], x_at[3]);
+          unsigned x[3][2];
+          split_4(v, x);
+          few_mma(g1[i], w[0], x[0][0], x[0][1]);
+          few_mma(g2[i], w[0], x[1][0], x[1][1]);
+          few_mma(g2[i], w[0], x[2][0], x[2][1]);
+          few_mma(g2[i], w[1], x[0][0], x[0][1]);
+          few_mma(g2[i], w[1], x[1][0], x[1][1]);
+          few_mma(g2[i], w[2], x[0][0], x[0][1]);
+        }
+      }
+      if (slice == warp) __syncthreads();       // the sums of the tile before have been read
+#pragma unroll
+      for (int i = 0; i < T8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sums[((slice * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
+    }
+    __syncthreads();
+    const int i = threadIdx.x >> 7, e = (threadIdx.x >> 5) & 3;
+    const int row = tile * 16 + g + (e >> 1) * 8, token = i * 8 + 2 * t + (e & 1);
+    if (i < T8 && row < N && token < M) {
+      float P[kChains];
+#pragma unroll
+      for (int j = 0; j < kChains; ++j) {
+        const float* s = sums + ((size_t)(j * slices / kChains) * T8 * 4 + i * 4 + e) * 32 + lane;
+        const int n = (j + 1) * slices / kChains - j * slices / kChains;
+        P[j] = s[0];
+        for (int k = 1; k < n; ++k) P[j] += s[(size_t)k * T8 * 128];
+      }
+      float v = (P[0] + P[1]) + (P[2] + P[3]);
+      if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(A + (size_t)token * lda, W + (size_t)row * ldw, K);
+      C[(size_t)token * ldc + row] = v;
+    }
+  }
+}
+
+constexpr int kFewSmem = 100 * 1024;      // two blocks an SM
+
+template <int T8, bool VEC>
+int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+  const size_t smem = (size_t)(K / kSliceK) * T8 * 128 * 4;
+  if (smem > kFewSmem) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<T8, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+  if (e != cudaSuccess) return (int)e;
+  const int tiles = (N + 15) / 16;
+  launch_k(gemm_f32_few_kernel<T8, VEC>, dim3(tiles < 2 * 148 ? tiles : 2 * 148), dim3(kFewWarps * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
+  LLMIE_LAUNCH_CHECK();
+  return LLMIE_OK;
+}
+
+template <int NT, bool WIDE>
+int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw, int ldc, int split,
+              int* status, cudaStream_t stream) {
+  using S = Shape<NT>;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<NT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+  if (e != cudaSuccess) return (int)e;
+  const long long blocks = (long long)((M + NT - 1) / NT) * ((N + kMt - 1) / kMt) * split;
+  if (blocks > 0x7fffffffLL) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  CUtensorMap map = {};
+  if (!S::kSplitsX) {
+    if (!parts) return LLMIE_ERR_BAD_ARG;
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return LLMIE_ERR_BAD_ARG;
+    if (!aligned16(parts)) return LLMIE_ERR_ALIGNMENT;
+    cuuint64_t dims[2] = {(cuuint64_t)K, 3 * (cuuint64_t)M}, pitch[1] = {(cuuint64_t)K * 2};
+    cuuint32_t box[2] = {kStageK, NT}, one[2] = {1, 1};
+    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, parts, dims, pitch, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return LLMIE_ERR_BAD_ARG;
+    launch_k(split_rows_kernel<WIDE>, dim3((unsigned)(((long long)M * (K / 8) + 255) / 256)), dim3(256), 0, stream, A,
+             (__nv_bfloat16*)parts, M, K, lda);
+    LLMIE_LAUNCH_CHECK();
+  }
+  if (split > 1)
+    launch_k_cluster(gemm_f32_tc_kernel<NT, WIDE>, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, split, map, A, W, C, M, N,
+                     K, lda, ldw, ldc, split, status);
+  else
+    launch_k(gemm_f32_tc_kernel<NT, WIDE>, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, map, A, W, C, M, N, K, lda, ldw,
+             ldc, split, status);
+  LLMIE_LAUNCH_CHECK();
+  return LLMIE_OK;
+}
+
+}  // namespace
+}  // namespace llmie
+
+using namespace llmie;
+
+// 1 when the kernel takes a weight [N, K]. The answer depends on the weight alone: a row's bits are then the same in every step.
+extern "C" int llmie_gemm_f32_tc_takes(int N, int K) { return N >= 128 && K >= 1024 && K % kSliceK == 0; }
+
+// form: tokens a block (8: the kernel for up to 16 tokens; 16, 64, 80) + 1000 * split (blocks of a tile: 1, 2, 4), for tests: every form gives the same bits. 0:
+// chosen by size. `parts`: 3 M K bfloat16 of scratch, not needed for 16 tokens a block.
+extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
+                                      int ldc, int form, int* status, cudaStream_t stream) {
+  if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N || !status) return LLMIE_ERR_BAD_ARG;
+  if (!llmie_gemm_f32_tc_takes(N, K)) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (M == 0) return LLMIE_OK;
+  int nt = form % 1000, split = form / 1000;
+  if (form == 0) {
+    const long long rows = (N + kMt - 1) / kMt;
+    // blocks of a tile: as many as fit the GPU at once, a block a SM (33 clusters of 4, 74 of 2)
+    auto share = [&](int n) {
+      const long long tiles = (M + n - 1) / n * rows;
+      return tiles <= 33 ? 4 : tiles <= 74 ? 2 : 1;
+    };
+    if (M <= 16) {
+      // up to 8 tokens the stream of the weights bounds both; with 16 the splitting of both operands by every warp does, where
+      // there are many rows (16 tokens, microseconds: 2,048 x 2,048 8.8 against 11.6, 16,384 x 2,048 40.8 against 31.9)
+      const bool few = (size_t)(K / kSliceK) * (M <= 8 ? 1 : 2) * 512 <= kFewSmem && (M <= 8 || N < 8192);
+      nt = few ? 8 : 16;
+    } else {
+      // a block's time does not follow its tokens (2,048 k: 35 us with 64, 37 with 80), so what counts is how many rounds of
+      // blocks there are, and how many share a tile
+      auto cost = [&](int n, int us) {
+        const long long blocks = (M + n - 1) / n * rows * share(n);
+        return (double)us * ((blocks + 147) / 148) / share(n);
+      };
+      nt = cost(64, 35) <= cost(80, 37) ? 64 : 80;
+    }
+    split = share(nt);
+  }
+  if (split != 1 && split != 2 && split != 4) return LLMIE_ERR_BAD_ARG;
+  const bool wide = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 31) == 0 && ((lda | ldw) & 7) == 0;
+  if (nt == 8) {
+    if (M > 16) return LLMIE_ERR_UNSUPPORTED_SIZE;
+    const bool vec = aligned16(A) && aligned16(W) && ((lda | ldw) & 3) == 0;
+    if (M <= 8)
+      return vec ? launch_few<1, true>(A, W, C, M, N, K, lda, ldw, ldc, stream) : launch_few<1, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    return vec ? launch_few<2, true>(A, W, C, M, N, K, lda, ldw, ldc, stream) : launch_few<2, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+  }
+#define LLMIE_TC(nt_)                                                                                     \
+  case nt_:                                                                                               \
+    return wide ? launch_tc<nt_, true>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, status, stream)      \
+                : launch_tc<nt_, false>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, status, stream)
+  switch (nt) {
+    LLMIE_TC(16);
+    LLMIE_TC(64);
+    LLMIE_TC(80);
+    default: return LLMIE_ERR_BAD_ARG;
+  }
+#undef LLMIE_TC
+}
+
+extern "C" int llmie_gemm_f32_tc(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
+                                 int ldc, int* status, cudaStream_t stream) {
+  return llmie_gemm_f32_tc_form(A, W, C, parts, M, N, K, lda, ldw, ldc, 0, status, stream);
+}

@@ -1,5 +1,5 @@
 // True float32 matrix product for the 32-bit path: C[M, N] = A[M, K] * W[N, K]^T, FMA on the
-// CUDA cores, no tensor cores and no reduced-precision mode anywhere.
+// CUDA cores, for the weights that gemm_f32_tc.cu does not take (few rows or a short or odd K).
 //
 // One summation order for every shape. K is cut into slices of 128; chain j (j = 0..7) takes the slices j, j + 8, ...
 // in turn and keeps two running sums, of its even and of its odd k (the two halves of a packed fma.rn.f32x2); P_j is

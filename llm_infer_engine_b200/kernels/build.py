@@ -47,6 +47,7 @@ FAMILIES: Dict[str, tuple] = {
     "attention_latent_tc": ("attention_latent_tc.cu", [], []),
     "attention_rows_mma": ("attention_rows_mma.cu", [], []),
     "gemm_simt": ("gemm_simt.cu", [], []),
+    "gemm_f32_tc": ("gemm_f32_tc.cu", [], []),
     "gemm_skinny": ("gemm_skinny.cu", [], []),
     "gemm_tc": ("gemm_tc.cu", [], []),
     "gemm_stream": ("gemm_stream.cu", [], []),

@@ -729,8 +729,15 @@ def attention_decode_mma_rope(qkv, k_cache, v_cache, out, table, seq_slot, seq_k
     return out
 
 
+def gemm_f32_tc_takes(n: int, k: int) -> bool:
+    """Whether a float32 weight [n, k] is multiplied on the tensor cores (the kernel's own rule, without a call)."""
+    return n >= 128 and k >= 1024 and k % 128 == 0
+
+
 def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FMA on CUDA cores, fixed summation order)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32, fixed summation order: a row's bits do not depend on the other rows.
+    Large weights on the tensor cores, every number as the sum of three bfloat16 (csrc/gemm_f32_tc.cu; which weights are
+    large is settled by their size alone), others by FMA on the CUDA cores."""
     M, K = a.shape
     N = w.shape[0]
     _need(a, "a", torch.float32)
@@ -739,6 +746,13 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
         out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     _need(out, "out", torch.float32, (M, N))
     _work(_nbytes(a, w) + a.shape[0] * w.shape[0] * 4, 2.0 * a.shape[0] * w.shape[0] * w.shape[1])
+    if gemm_f32_tc_takes(N, K):
+        # scratch: the parts of `a`, which the kernel for few rows makes itself
+        parts = torch.empty(3 * M * K, dtype=torch.bfloat16, device=a.device) if M > 16 else None
+        f = _fn("gemm_f32_tc", "llmie_gemm_f32_tc", [_c_void_p] * 4 + [_c_int] * 6 + [_c_void_p] * 2)
+        _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(parts), M, N, K, K, K, N,
+                 tc_status_word(a.device).data_ptr(), _stream()), "gemm_f32_tc")
+        return out
     f = _fn("gemm_simt", "llmie_gemm_f32_nt", [_c_void_p] * 3 + [_c_int] * 6 + [_c_void_p])
     _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, _stream()), "gemm_f32_nt")
     return out

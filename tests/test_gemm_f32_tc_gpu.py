@@ -1,0 +1,82 @@
+"""The float32 product on the tensor cores against 64-bit sums and against itself: every form gives the same bits, at the edges
+of tiles, slices and chains, with rows that start on 32 bytes and rows that do not; infinities and overflow."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+FORMS = (1008, 1016, 2016, 4016, 1064, 2064, 4064, 1080, 2080, 4080, 0)
+
+
+def _form(a, w, form, ld_extra=0):
+    from llm_infer_engine_b200.kernels import ops
+    f = ops._fn("gemm_f32_tc", "llmie_gemm_f32_tc_form", [ctypes.c_void_p] * 4 + [ctypes.c_int] * 7 + [ctypes.c_void_p] * 2)
+    (M, K), N = a.shape, w.shape[0]
+    out = torch.full((M, N + ld_extra), float("nan"), device=DEV)
+    parts = torch.empty(3 * M * K, dtype=torch.bfloat16, device=DEV)
+    status = f(a.data_ptr(), w.data_ptr(), out.data_ptr(), parts.data_ptr(), M, N, K, a.stride(0), w.stride(0), N + ld_extra,
+               form, ops.tc_status_word(torch.device(DEV, 0)).data_ptr(), ops._stream())
+    return status, out[:, :N]
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 1024), (3, 2369, 1152), (8, 300, 2048), (9, 129, 1408), (16, 640, 3072), (17, 200, 1024),
+                                   (64, 257, 1280), (65, 1000, 1024), (80, 384, 8192), (81, 130, 1536), (301, 640, 2048)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_every_form_gives_the_same_bits(M, N, K, offset):
+    from llm_infer_engine_b200.kernels import ops
+    g = torch.Generator().manual_seed(M * 1000 + K)
+    a = (torch.randn(M, K + 8 + offset, generator=g) * torch.exp(torch.randn(M, 1, generator=g))).to(DEV)[:, :K]
+    w = torch.randn(N, K + 8 + offset, generator=g).to(DEV)[:, :K]       # offset 1: rows that do not start on 16 bytes
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    status, first = _form(a, w, 1064)
+    assert status == 0
+    # 17 terms a product and 8 products a slice, each cut off at 2^-24 of the largest; the parts left out; the sums behind
+    bound = (17 * 8 + 6 + K / 512 + 4) * 2.0 ** -24 * size
+    assert bool(((first.double() - ref).abs() <= bound).all())
+    # what is seen, beside sums in one float32 chain each
+    assert float((first.double() - ref).norm() / ref.norm()) < 2e-7
+    for form in FORMS:
+        status, out = _form(a, w, form, ld_extra=3)
+        if form == 1008 and M > 16:
+            assert status == -2
+            continue
+        assert status == 0, form
+        assert torch.equal(out, first), form
+    status, some = _form(a[M // 2:M // 2 + 1], w, 0)          # a row alone
+    assert status == 0 and torch.equal(some[0], first[M // 2])
+    if offset:
+        assert torch.equal(ops.gemm_f32_nt(a.contiguous(), w.contiguous()), first)
+    ops.check_tc_status(torch.device(DEV, 0))
+
+
+def test_infinities_nan_overflow_and_nothing():
+    torch.manual_seed(5)
+    a, w = torch.randn(40, 1152, device=DEV), torch.randn(200, 1152, device=DEV)
+    w[7, 1151], w[130, 5] = float("inf"), float("nan")
+    a[3, 600] = float("-inf")
+    a[5, 0] = 3e38                                            # times 100: a product that float32 does not hold
+    w[:, 0] = w[:, 0].clamp(-1, 1)
+    w[9, 0] = 100.0                                           # and the only one (beside an infinity it would make NaN, in float32)
+    want = a.double() @ w.double().T
+    for rows in (6, 14, 40):
+        for form in FORMS[(0 if rows <= 16 else 1):]:
+            out = _form(a[:rows], w, form)[1]
+            nan = torch.isnan(want[:rows])
+            assert torch.equal(torch.isnan(out), nan), form
+            huge = want[:rows].abs() > 3.4e38
+            assert torch.equal(torch.isinf(out), huge & ~nan) and bool((out[huge & ~nan].sign() == want[:rows][huge & ~nan].sign()).all())
+            fine = ~nan & ~huge
+            assert bool(((out.double() - want[:rows])[fine].abs() <= 1e-5 * (want[:rows][fine].abs() + 1e3)).all())
+    assert _form(a[:0], w, 0)[0] == 0
+
+
+def test_what_it_takes():
+    from llm_infer_engine_b200.kernels import build, ops
+    takes = build.load("gemm_f32_tc").llmie_gemm_f32_tc_takes
+    for n in (1, 127, 128, 5000):
+        for k in (128, 896, 1024, 1025, 1152, 8192):
+            assert bool(takes(n, k)) == ops.gemm_f32_tc_takes(n, k)
+    a, w = torch.randn(3, 1024, device=DEV), torch.randn(100, 1024, device=DEV)
+    assert _form(a, w, 0)[0] == -2                            # fewer rows than a tile
