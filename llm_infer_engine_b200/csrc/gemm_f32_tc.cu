@@ -16,17 +16,18 @@
 // Sums that are not finite (an infinity or NaN among the inputs, whose parts are NaN, or an overflow, of a part too) are formed again by plain
 // FMAs over K, which give what IEEE arithmetic gives.
 //
-// A block makes 128 weight rows x NT tokens. The weights are the 128-row operand; per 16 k five tcgen05.mma: w1 by [x1 x2] into
-// [G1 G2], then w1 x3, w2 x1, w2 x2, w3 x1 into G2. Sixteen warps in four groups, a group a stage of 32 k, read the weights as
-// float32, 32 bytes a lane and a round of the groups ahead, split them and store the parts as swizzled operands; the tokens'
-// parts were made by a kernel in front and come by TMA, eight stages deep (NT = 16: the same warps split them); one lane issues
-// the products, two stages a turn; eight warps empty one of two accumulators while the other fills, and keep the sums of
-// finished chains in the tensor memory behind them.
+// A block makes 128 weight rows x NT tokens. The weights are the 128-row operand, in tensor memory; per 16 k five tcgen05.mma: w1
+// by [x1 x2] into [G1 G2], then w1 x3, w2 x1, w2 x2, w3 x1 into G2. Sixteen warps in four groups, a group a stage of 32 k, read
+// the weights as float32, a lane its row, a round of the groups ahead, split them and store the parts; the tokens' parts were
+// made by a kernel in front and come by TMA, eight stages deep (NT = 16: the same warps split them); one lane issues the
+// products, two stages a turn behind one barrier; eight warps empty one of two accumulators while the other fills, and keep the
+// sums of finished chains in shared memory.
 //
-// What bounds it: 128 x 80 tokens x 32 k are 480 cycles of products, a stage takes about 900: the hand-over from the splitting
-// warps to the issuing lane and back, and the splitting itself (nine instructions for two weights). Products of 2,048 k (FMA in
-// brackets): 301 x 16,384 149 us (498), 465 x 3,072 40 (165), 301 x 2,048 x 8,192 k 75 (275); a gated feed-forward of 2,048 /
-// 8,192 at 301 rows 250 us (784), 72 rows 85 (385).
+// What bounds it: the issue of the products, about 80 cycles each with 80 tokens, 56 with 16, of which the tensor cores work 48
+// (80 tokens). With the weights' parts in shared memory it was its bandwidth: 128 x 80 tokens x 32 k wrote and read 110 KB of it,
+// 890 cycles of the 926 they took (now 820). Products of 2,048 k (weights in shared memory; FMA): 301 x 16,384 141 us (149; 498),
+// 465 x 3,072 38 (40; 165), 301 x 2,048 x 8,192 k 70 (76; 275); a gated feed-forward of 2,048 / 8,192 at 301 rows 253 us (260; FMA
+// 784).
 #include "tcgen05.cuh"
 
 namespace llmie {
@@ -40,21 +41,19 @@ constexpr int kSliceK = 128;
 constexpr int kChains = 4;
 constexpr int kSumWarps = 8, kSplitWarps = 16;
 constexpr int kStages = 4;                // four warps split for each
-constexpr int kPieces = kMt * (kStageK / 8) / 128;        // pieces of 8 weights a thread and stage
 static_assert(kSplitWarps == 4 * kStages && kStages == kPerSlice, "the stages of a slice go round four groups of warps");
 constexpr int kTcThreads = 32 * (kSumWarps + kSplitWarps + 4);        // the last four: one issues products, one copies
 
 template <int NT>
 struct Shape {
   static constexpr bool kSplitsX = NT == 16;                 // else the tokens' parts come by TMA
-  static constexpr int kWPart = kMt * 64, kXPart = NT * 64;  // bytes of one part of a stage
-  static constexpr int kWStage = 3 * kWPart, kXStage = 3 * kXPart;
-  static constexpr int kXStages = kSplitsX ? kStages : 8;    // copies run further ahead: a copy takes two stages' time
-  static constexpr int kSmem = kStages * kWStage + kXStages * kXStage + 1024;
-  static constexpr int kHold0 = 4 * NT, kHold1 = 5 * NT;     // columns behind the two accumulators: sums of finished chains
-  static constexpr int kAccCols = 2 * NT, kTmemCols = NT == 16 ? 128 : 512;
+  static constexpr int kXPart = NT * 64, kXStage = 3 * kXPart;        // bytes of one part of a stage, of all
+  static constexpr int kXTurns = kSplitsX ? 2 : 4;           // two stages each: copies run further ahead, they take a turn's time
+  static constexpr int kSmem = kXTurns * 2 * kXStage + 2 * NT * kMt * 4 + 1024;
+  static constexpr int kAccCols = 2 * NT, kWCol = 2 * kAccCols;       // tensor memory: two accumulators, then the weights' parts
+  static constexpr int kWStageCols = 3 * kStageK / 2, kTmemCols = NT == 16 ? 256 : 512;
+  static_assert(kWCol + kStages * kWStageCols <= kTmemCols, "");
   static constexpr int kCols = NT / 2;                       // of a sum warp
-  static_assert(6 * NT <= kTmemCols && NT * kMt * 4 <= kStages * kWStage, "");
 };
 
 // Byte offset of piece `piece` (16 bytes) of row `row` in 64-byte rows with the 64-byte swizzle, and its operand descriptor.
@@ -67,21 +66,21 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
 }
 
 struct TcShared {
-  uint64_t full[kStages], empty[kStages], x_full[8], x_empty[8], acc_full[2], acc_empty[2];
+  uint64_t ready[4], empty[kStages], x_empty[4], acc_full[2];       // ready: all that a turn of two stages needs
   uint32_t tmem;
   int abort;
 };
 
-// 8 neighbouring floats; WIDE: from a 32-byte aligned address. No condition around it: the values of a load that is skipped
-// would have to be merged with what it brings, and that waits for it.
+// 8 neighbouring floats; WIDE: from a 32-byte aligned address. No condition around it, and the registers are named as read too:
+// a value that is merged with another, or moved, waits for its load.
 template <bool WIDE>
 __device__ __forceinline__ void load_8(const float* p, float (&v)[8]) {
   if (WIDE) {
     asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]) : "l"(p));
   } else {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v[e]) : "l"(p + e));
+    for (int e = 0; e < 8; ++e) asm volatile("ld.global.f32 %0, [%1];" : "+f"(v[e]) : "l"(p + e));
   }
 }
 
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* A, __nv_bf
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= (long long)M * per_row) return;
   const int t = (int)(i / per_row), k = (int)(i - (long long)t * per_row) << 3;
-  float v[8];
+  float v[8] = {};
   uint4 parts[3];
   load_8<WIDE>(A + (size_t)t * lda + k, v);
   split_8(v, parts);
@@ -144,10 +143,10 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-// run (+)= G1 + G2, 24 columns at a time.
+// run (+)= G1 + G2, 16 columns at a time.
 template <int C0, int N>
 __device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)[N], bool fresh) {
-  constexpr int n = N - C0 < 24 ? N - C0 : 24;
+  constexpr int n = N - C0 < 16 ? N - C0 : 16;
   uint32_t a[n], b[n];
 #pragma unroll
   for (int c = 0; c < n; c += 8) tmem_ld_32x8(g1 + C0 + c, a + c);
@@ -162,26 +161,18 @@ __device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)
   if constexpr (C0 + n < N) sum_columns<C0 + n, N>(g1, to_g2, run, fresh);
 }
 
-// The held sums of a warp's columns: `run` becomes held + run, or what is held.
-template <int N>
-__device__ __forceinline__ void add_held(uint32_t taddr, float (&run)[N]) {
-#pragma unroll
-  for (int c = 0; c < N; c += 8) {
-    uint32_t a[8];
-    tmem_ld_32x8(taddr + c, a);
-    tmem_ld_wait();
-#pragma unroll
-    for (int e = 0; e < 8; ++e) run[c + e] = __uint_as_float(a[e]) + run[c + e];
-  }
+__device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const uint4& v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
 }
-template <int N>
-__device__ __forceinline__ void put_held(uint32_t taddr, const float (&run)[N]) {
-#pragma unroll
-  for (int c = 0; c < N; c += 8)
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr + c), "f"(run[c]), "f"(run[c + 1]), "f"(run[c + 2]), "f"(run[c + 3]), "f"(run[c + 4]),
-                 "f"(run[c + 5]), "f"(run[c + 6]), "f"(run[c + 7]) : "memory");
-  tmem_st_wait();
+// D[tmem] (+)= A[tmem] * B[smem]; one thread issues.
+__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 
 template <int NT, bool WIDE>
@@ -191,8 +182,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
   using S = Shape<NT>;
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ TcShared sh;
-  unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~(uintptr_t)1023);
-  unsigned char* x_stages = stages + kStages * S::kWStage;
+  unsigned char* x_stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~(uintptr_t)1023);
+  float* hold = reinterpret_cast<float*>(x_stages + S::kXTurns * 2 * S::kXStage);        // [2][NT][kMt]: sums of finished chains
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x % split;
   const int tiles_m = (M + NT - 1) / NT, tile = blockIdx.x / split;
@@ -204,18 +195,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
   volatile int* abort = &sh.abort;
 
   if (tid == 0) {
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&sh.full[i], 4);
+    for (int i = 0; i < 4; ++i) {         // eight splitting warps, the tokens' copy, before a slice the sum warps
+      mbar_init(&sh.ready[i], 8 + (S::kSplitsX ? 0 : 1) + (i & 1 ? 0 : kSumWarps));
       mbar_init(&sh.empty[i], 1);
-    }
-    for (int i = 0; i < 8; ++i) {
-      mbar_init(&sh.x_full[i], 1);
       mbar_init(&sh.x_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&sh.acc_full[i], 1);
-      mbar_init(&sh.acc_empty[i], kSumWarps);
-    }
+    for (int i = 0; i < 2; ++i) mbar_init(&sh.acc_full[i], 1);
     sh.abort = 0;
     fence_mbar_init();
   }
@@ -230,16 +215,19 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
 
   if (warp < kSumWarps) {
     // ---------------------------------------------------------------- sums: half of the tokens each four warps
-    if (!S::kSplitsX) asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+    if (S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     pdl_wait();
     const int quarter = warp & 3, col0 = (warp >> 2) * S::kCols, row = quarter * 32 + lane;
     const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + col0;
     const bool row_there = n0 + row < N;
+    float* h = hold + (size_t)col0 * kMt + row;
     float* out = C + (size_t)(m0 + col0) * ldc + n0 + row;
     const int n_cols = row_there ? min(S::kCols, M - m0 - col0) : 0;       // of the result
     float run[S::kCols] = {};
     int chain = 0, chain_end = (chain0 + 1) * slices / kChains;
     bool fresh = true, ok = true;
+    if (lane < 2) mbar_arrive(&sh.ready[2 * lane]);       // both accumulators are free
 #pragma unroll 1
     for (int slice = slice0; slice < slice1; ++slice) {
       const int i = slice - slice0, ab = i & 1;
@@ -252,25 +240,32 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       sum_columns<0, S::kCols>(acc + ab * S::kAccCols, NT, run, fresh);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.acc_empty[ab]);
+      if (lane == 0) mbar_arrive(&sh.ready[2 * ab]);
       fresh = slice + 1 == chain_end;
       if (fresh) {                        // the chain is done: ((P_0 + P_1) + (P_2 + P_3)) as far as this block has them
-        if (chain & 1) add_held<S::kCols>(acc + (chain == 3 ? S::kHold1 : S::kHold0), run);
-        if (chain == 3) add_held<S::kCols>(acc + S::kHold0, run);
-        if (chain < kChains / split - 1) put_held<S::kCols>(acc + (chain == 2 ? S::kHold1 : S::kHold0), run);
+        if (chain & 1) {
+          const float* from = h + (chain == 3 ? NT * kMt : 0);
+#pragma unroll
+          for (int c = 0; c < S::kCols; ++c) run[c] = from[c * kMt] + run[c];
+        }
+        if (chain == 3) {
+#pragma unroll
+          for (int c = 0; c < S::kCols; ++c) run[c] = h[c * kMt] + run[c];
+        }
+        if (chain < kChains / split - 1 || split > 1) {       // (the last one of a cluster's block: for the others to read)
+          float* to = h + (chain == 2 ? NT * kMt : 0);
+#pragma unroll
+          for (int c = 0; c < S::kCols; ++c) to[c * kMt] = run[c];
+        }
         ++chain;
         chain_end = (chain0 + chain + 1) * slices / kChains;
       }
     }
     if (!ok) {                            // (the plain sums below then replace these)
 #pragma unroll
-      for (int c = 0; c < S::kCols; ++c) run[c] = __int_as_float(0x7fc00000);
+      for (int c = 0; c < S::kCols; ++c) h[c * kMt] = run[c] = __int_as_float(0x7fc00000);
     }
-    if (split > 1) {                      // the operands have been read: their place takes the sums
-      float* h = reinterpret_cast<float*>(stages) + (size_t)col0 * kMt + row;
-#pragma unroll
-      for (int c = 0; c < S::kCols; ++c) h[c * kMt] = run[c];
-    } else {
+    if (split == 1) {
       bool finite = true;
 #pragma unroll
       for (int c = 0; c < S::kCols; ++c) {
@@ -287,89 +282,93 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     }
   } else if (warp < kSumWarps + kSplitWarps) {
     // ---------------------------------------------------------------- float32 in, parts out
-    if (!S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    const int group = (warp - kSumWarps) >> 2, gt = tid & 127, r = gt >> 2, piece = gt & 3;
-    // rows behind the last are the last one again, stages behind the last one too: nobody reads what becomes of them
-    const float* w_src[kPieces];
+    if (S::kSplitsX) asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // a thread a weight row (a lane of the tensor memory) and 32 k of a stage
+    const int group = (warp - kSumWarps) >> 2, quarter = warp & 3;
+    const uint32_t to = tmem + ((uint32_t)(quarter * 32) << 16) + S::kWCol + group * S::kWStageCols;
+    // the row behind the last is the last one again, the stage behind the last one too: nobody reads what becomes of them
+    const float* w_src = W + (size_t)min(n0 + quarter * 32 + lane, N - 1) * ldw + slice0 * kSliceK;
+    float w[4][8] = {}, x[8] = {};
 #pragma unroll
-    for (int i = 0; i < kPieces; ++i)
-      w_src[i] = W + (size_t)min(n0 + r + 32 * i, N - 1) * ldw + slice0 * kSliceK + piece * 8;
-    const float* a_src = A + (size_t)min(m0 + r, M - 1) * lda + slice0 * kSliceK + piece * 8;
-    const uint32_t at = swizzle64_offset(r, piece);            // 32 rows on: the same place in its 128 bytes
-    unsigned char* st = stages + group * S::kWStage + at;
-    float w[kPieces][8], x[8];
-#pragma unroll
-    for (int i = 0; i < kPieces; ++i) load_8<WIDE>(w_src[i] + group * kStageK, w[i]);
+    for (int i = 0; i < 4; ++i) load_8<WIDE>(w_src + group * kStageK + 8 * i, w[i]);
+    // (up to 16 tokens: 64 threads of the group a piece of 8)
+    const int gt = tid & 127, r = gt >> 2;
+    const float* a_src = A + (size_t)min(m0 + r, M - 1) * lda + slice0 * kSliceK + (gt & 3) * 8;
+    unsigned char* x_to = x_stages + group * S::kXStage + swizzle64_offset(r, gt & 3);
     if (S::kSplitsX) {
       pdl_wait();                           // weights are written by no kernel
       load_8<WIDE>(a_src + group * kStageK, x);
     }
+    uint64_t* empty = &sh.empty[group];
     uint32_t parity = 1;                    // a fresh barrier counts as released
     for (int s = group; s < n_stages; s += kStages, parity ^= 1) {
-      if (!mbar_wait(&sh.empty[group], parity, abort)) {
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(empty, parity, abort));
+      if (!ok) {
         if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
         break;
       }
+      tc_fence_after_sync();
       const int next = min(s + kStages, n_stages - 1) * kStageK;
 #pragma unroll
-      for (int i = 0; i < kPieces; ++i) {
-        split_store(w[i], st + 32 * 64 * i, S::kWPart);
-        load_8<WIDE>(w_src[i] + next, w[i]);
+      for (int i = 0; i < 4; ++i) {
+        uint4 parts[3];
+        split_8(w[i], parts);
+        load_8<WIDE>(w_src + next + 8 * i, w[i]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) tmem_st_32x4(to + p * (kStageK / 2) + 4 * i, parts[p]);
       }
       if (S::kSplitsX) {
-        if (r < NT) split_store(x, x_stages + group * S::kXStage + at, S::kXPart);
+        if (r < NT) split_store(x, x_to, S::kXPart);
         load_8<WIDE>(a_src + next, x);
       }
+      tmem_st_wait();
+      tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.full[group]);
+      if (lane == 0) mbar_arrive(&sh.ready[(s >> 1) & 3]);
     }
   } else {
-    if (!S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == kSumWarps + kSplitWarps) {
       // -------------------------------------------------------------- products
       // The whole warp walks the stages, so that addresses and descriptors are the warp's and not a thread's; one lane issues.
       constexpr uint32_t d2 = make_instr_desc_bf16(kMt, 2 * NT, 0, 0), d1 = make_instr_desc_bf16(kMt, NT, 0, 0);
       const bool leader = elect_one();
-      const uint64_t first_w = operand_desc(smem_u32(stages)), first_x = operand_desc(smem_u32(x_stages));
-      constexpr uint64_t kWNext = S::kWPart / 16, kXNext = S::kXPart / 16;
-      const int n_slices = slice1 - slice0;
-      bool ok = true;
-      for (int slice = 0; ok && slice < n_slices; ++slice) {
-        const uint32_t g1 = tmem + (slice & 1) * S::kAccCols, g2 = g1 + NT;
-        if (slice >= 2) ok = mbar_wait(&sh.acc_empty[slice & 1], ((slice >> 1) - 1) & 1, abort);
-#pragma unroll
-        for (int pair = 0; pair < kStages; pair += 2) {       // two stages a turn: half as many waits in the way of the products
-          // stage `pair` of an even slice is the tokens' stage `pair`, of an odd one 4 + pair
-          const int xs = S::kSplitsX ? pair : (slice & 1) * kStages + pair;
-          ok = ok && mbar_wait(&sh.full[pair], slice & 1, abort) && mbar_wait(&sh.full[pair + 1], slice & 1, abort);
-          if (!S::kSplitsX)
-            ok = ok && mbar_wait(&sh.x_full[xs], (slice >> 1) & 1, abort) && mbar_wait(&sh.x_full[xs + 1], (slice >> 1) & 1, abort);
-          if (!ok) break;
-          // the parts were written through the generic proxy. The fence stands here and not behind the stores: there it would
-          // also wait for the loads that run ahead
-          fence_proxy_async_smem();
-          tc_fence_after_sync();
-          if (leader) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int stage = pair + e;
-              const uint64_t w1 = first_w + stage * (S::kWStage / 16), w2 = w1 + kWNext, w3 = w2 + kWNext;
-              const uint64_t x1 = first_x + (xs + e) * (S::kXStage / 16), x2 = x1 + kXNext, x3 = x2 + kXNext;
-#pragma unroll
-              for (int kk = 0; kk < 2 * (kStageK / 16); kk += 2) {        // 32 bytes of a row: 2 in a descriptor's units
-                mma_bf16_ss(g1, w1 + kk, x1 + kk, d2, stage > 0 || kk > 0 ? 1u : 0u);
-                mma_bf16_ss(g2, w1 + kk, x3 + kk, d1, 1u);
-                mma_bf16_ss(g2, w2 + kk, x1 + kk, d1, 1u);
-                mma_bf16_ss(g2, w2 + kk, x2 + kk, d1, 1u);
-                mma_bf16_ss(g2, w3 + kk, x1 + kk, d1, 1u);
-              }
-              mma_commit(&sh.empty[stage]);
-              if (!S::kSplitsX) mma_commit(&sh.x_empty[xs + e]);
-            }
-            if (pair + 2 == kStages) mma_commit(&sh.acc_full[slice & 1]);
-          }
-          __syncwarp();
+      const uint64_t first_x = operand_desc(smem_u32(x_stages));
+      constexpr uint64_t kXNext = S::kXPart / 16;
+      constexpr uint32_t kWNext = kStageK / 2;
+      const int n_turns = 2 * (slice1 - slice0);
+      bool ok = mbar_wait(&sh.ready[0], 0, abort);
+      for (int turn = 0; ok && turn < n_turns; ++turn) {
+        const int ws = turn & 1, xs = S::kSplitsX ? ws : turn & 3, ab = (turn >> 1) & 1;
+        const uint32_t g1 = tmem + ab * S::kAccCols, g2 = g1 + NT;
+        if (S::kSplitsX) fence_proxy_async_smem();     // these parts were written through the generic proxy
+        tc_fence_after_sync();
+        auto products = [&](int e, int kk) {           // 32 bytes of a token's row: 2 in a descriptor's units; 8 columns
+          const uint32_t w1 = tmem + S::kWCol + (2 * ws + e) * S::kWStageCols + 8 * kk, w2 = w1 + kWNext, w3 = w2 + kWNext;
+          const uint64_t x1 = first_x + (2 * xs + e) * (S::kXStage / 16) + 2 * kk, x2 = x1 + kXNext, x3 = x2 + kXNext;
+          mma_bf16_ts(g1, w1, x1, d2, ws > 0 || e > 0 || kk > 0 ? 1u : 0u);
+          mma_bf16_ts(g2, w1, x3, d1, 1u);
+          mma_bf16_ts(g2, w2, x1, d1, 1u);
+          mma_bf16_ts(g2, w2, x2, d1, 1u);
+          mma_bf16_ts(g2, w3, x1, d1, 1u);
+        };
+        if (leader) {
+          products(0, 0);
+          products(0, 1);
+          mma_commit(&sh.empty[2 * ws]);
+          products(1, 0);
         }
+        __syncwarp();
+        // the wait for the next turn stands in front of this one's last products: they are worked on meanwhile
+        if (turn + 1 < n_turns) ok = mbar_wait(&sh.ready[(turn + 1) & 3], ((turn + 1) >> 2) & 1, abort);
+        if (leader) {
+          products(1, 1);
+          mma_commit(&sh.empty[2 * ws + 1]);
+          if (!S::kSplitsX) mma_commit(&sh.x_empty[xs]);
+          if (ws) mma_commit(&sh.acc_full[ab]);
+        }
+        __syncwarp();
       }
       if (!ok && leader && !*abort) { *abort = 1; atomicExch(status, kStatusTimeoutFull); }
       __syncwarp();
@@ -379,22 +378,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
         tma_prefetch_desc(&map_x);
         pdl_wait();
         int issued = 0;
-        for (int s = 0; s < n_stages; ++s) {
-          const int xs = s & 7;
-          if (!mbar_wait(&sh.x_empty[xs], ((s >> 3) & 1) ^ 1, abort)) {
+        for (int turn = 0; turn < n_stages / 2; ++turn) {
+          const int xs = turn & 3;
+          if (!mbar_wait(&sh.x_empty[xs], ((turn >> 2) & 1) ^ 1, abort)) {
             if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
             break;
           }
-          mbar_arrive_expect_tx(&sh.x_full[xs], S::kXStage);
+          mbar_arrive_expect_tx(&sh.ready[xs], 2 * S::kXStage);
 #pragma unroll
-          for (int p = 0; p < 3; ++p)
-            tma_load_2d(x_stages + xs * S::kXStage + p * S::kXPart, &map_x, slice0 * kSliceK + s * kStageK, p * M + m0,
-                        &sh.x_full[xs]);
-          issued = s + 1;
+          for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+              tma_load_2d(x_stages + (2 * xs + e) * S::kXStage + p * S::kXPart, &map_x,
+                          slice0 * kSliceK + (2 * turn + e) * kStageK, p * M + m0, &sh.ready[xs]);
+          issued = turn + 1;
         }
         if (*abort) {       // the copies of this thread land, or have had the time to, before their shared memory is given up
-          for (int s = max(0, issued - 8); s < issued; ++s)
-            for (unsigned spin = 0; spin < (1u << 14) && !mbar_test(&sh.x_full[s & 7], (s >> 3) & 1); ++spin) __nanosleep(64);
+          for (int turn = max(0, issued - 4); turn < issued; ++turn)
+            for (unsigned spin = 0; spin < (1u << 14) && !mbar_test(&sh.ready[turn & 3], (turn >> 2) & 1); ++spin) __nanosleep(64);
         }
       }
       __syncwarp();
@@ -406,7 +407,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       const int row = (warp & 3) * 32 + lane;
       if (n0 + row < N) {
         for (int c = rank * 2 + (warp >> 2); c < NT && m0 + c < M; c += 2 * split) {
-          const uint32_t a = smem_u32(reinterpret_cast<float*>(stages) + (size_t)c * kMt + row);
+          const uint32_t a = smem_u32(hold + (size_t)c * kMt + row);
           float v;
           if (split == 2)
             v = ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1));
