@@ -75,6 +75,7 @@ struct MdOptions {
   int bias_len;
   const float* sink_vals;
   const float* sigmoid_bias;
+  int longest_first;       // set by the launcher
 };
 
 __device__ __forceinline__ float md_tanh(float x) {
@@ -139,6 +140,24 @@ __device__ __forceinline__ void md_merge_head(const float* part_m, const float* 
         md_gated(unnormalised ? num[k] : md_finish(num[k], denom, M, sink, sv), gate_row, lane + 32 * k));
 }
 
+// The sequence that the blocks with z = `turn` serve: the longest sequences first, so that what is left for the end of a launch is
+// short (64 sequences of 700 to 3,900 keys, 6 warps a block: 46.2 us in the order they come, 41.2 so). For up to 64 sequences.
+__device__ __forceinline__ int md_sequence(const int* seq_kvlen, int n_seqs, int turn) {
+  const int lane = threadIdx.x & 31;
+  // length and number in one word: a longer sequence, or an earlier one of the same length, is the larger word
+  const int a = lane < n_seqs ? max(seq_kvlen[lane], 0) * 64 + 63 - lane : -1;
+  const int b = lane + 32 < n_seqs ? max(seq_kvlen[lane + 32], 0) * 64 + 31 - lane : -1;
+  int rank_a = 0, rank_b = 0;
+  for (int i = 0; i < n_seqs; ++i) {
+    const int v = __shfl_sync(0xffffffffu, i < 32 ? a : b, i & 31);
+    rank_a += v > a;
+    rank_b += v > b;
+  }
+  const unsigned in_a = __ballot_sync(0xffffffffu, a >= 0 && rank_a == turn);
+  const unsigned in_b = __ballot_sync(0xffffffffu, b >= 0 && rank_b == turn);
+  return in_a ? __ffs(in_a) - 1 : in_b ? __ffs(in_b) + 31 : turn;
+}
+
 // grid (n_runs, n_kv * chunks, n_seqs), chunks = ceil(G / 16); WARPS warps per block.
 // With ROPE the kernel takes the step's raw projections instead of finished queries: `q` is then the packed
 // [n_seqs, (n_q + 2 n_kv) * HD] rows of q, k and v heads (row pitch q_ld), `rope` the float32 (cos, sin) table
@@ -147,7 +166,7 @@ __device__ __forceinline__ void md_merge_head(const float* part_m, const float* 
 // half page holds the sequence's newest position rotates the new key, puts key and value into its staged tile
 // and (with write_kv) into the cache. Rotation in float32, one rounding to bfloat16, as the separate kernel.
 template <int HD, int WARPS, bool ROPE>
-__global__ void __launch_bounds__(WARPS * 32, (HD == 64 && WARPS <= 4) ? 16 / WARPS : 1)
+__global__ void __launch_bounds__(WARPS * 32, HD != 64 ? 1 : WARPS <= 4 ? 16 / WARPS : WARPS <= 6 ? 2 : 1)
 decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
                   const __nv_bfloat16* v_cache, float* part_m, float* part_l,
                   float* part_acc, const int* seq_slot, const int* seq_kvlen,
@@ -164,7 +183,7 @@ decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
   extern __shared__ __align__(16) unsigned char md_smem[];
   __shared__ int is_last;
 
-  const int run = blockIdx.x, seq = blockIdx.z;
+  const int run = blockIdx.x, seq = opt.longest_first ? md_sequence(seq_kvlen, gridDim.z, blockIdx.z) : blockIdx.z;
   const int G = n_q / n_kv;
   const int chunks = (G + 15) / 16;
   const int hk = blockIdx.y / chunks;
@@ -585,16 +604,19 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
   // takes two. Estimate: waves x (pages a warp takes in turn + a fixed part), smallest wins.
   const long long blocks = (long long)n_seqs * n_kv * chunks * n_runs;
   const int tile_bytes = 2 * kMdPage * (hd + 8) * (int)sizeof(__nv_bfloat16);
-  const int options[4] = {8, 4, 3, 2};
+  const int options[5] = {8, 4, 3, 2, 6};
   int best_w = 4;
   double best_cost = 1e30;
-  for (int i = 0; i < 4; ++i) {
-    const int w = options[i];
-    if (w * tile_bytes > 200 * 1024) continue;
+  auto slots_of = [&](int w) {
     int per_sm = (227 * 1024) / (w * tile_bytes + 1024);                      // 1 KB of every block is the system's
     if (hd == 64 && per_sm > 16 / w) per_sm = 16 / w > 0 ? 16 / w : 1;       // registers
-    if (per_sm < 1) continue;
-    const long long slots = 148LL * per_sm;
+    return 148LL * per_sm;
+  };
+  for (int i = 0; i < 5; ++i) {
+    const int w = options[i];
+    if (w * tile_bytes > 210 * 1024 || (w == 6 && window != 0)) continue;
+    const long long slots = slots_of(w);
+    if (slots < 1) continue;
     const double waves = (double)((blocks + slots - 1) / slots);
     const double cost = waves * ((pages_per_run + w - 1) / w + 1.5);
     if (cost < best_cost) {
@@ -602,6 +624,19 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
       best_w = w;
     }
   }
+  // That is right for sequences of one length. Lengths differ where batches are served, and then a long sequence's block with few
+  // warps is what a launch ends with, however many others run beside it. Where some sequence is longer than 2,048 keys (a captured
+  // step of shorter ones is sized for 2,048 at most): six warps a block (two blocks an SM; head size 128, one, up to 50
+  // sequences), served longest first where blocks have to queue. Measured, us, the choice above / this one: head size 64, 64
+  // sequences of 700 to 3,900 keys 56.0 / 41.2, 64 of 200 to 4,000 54.6 / 32.9, 48 of 200 to 4,000 42.2 / 31.8, 24 of 200 to
+  // 4,000 37.4 / 29.5, 64 of 3,000 70.0 / 65.3, 48 of 3,000 53.3 / 59.0; head size 128, 64 of 200 to 4,000 (three warps,
+  // queueing) 86.6 / 69.8, 48 of 200 to 4,000 77.9 / 48.8, 24 of 200 to 4,000 53.5 / 34.0, 32 of 3,000 70.6 / 67.6, 24 of 3,000
+  // 57.2 / 63.7, but 64 of 3,000 124 / 134. With shorter ones six warps cost more where lengths are equal (64 of 512, 14.2 /
+  // 19.4) than they give where not. A window or a chunk makes the work of long sequences alike.
+  const bool long_ones = window == 0 && pages_per_run > 32;
+  if (long_ones && blocks > 148 && (hd == 64 || blocks <= 400)) best_w = 6;
+  // (finding the order takes a block about half a microsecond; blocks that are all there at once gain nothing by it)
+  opt.longest_first = long_ones && n_seqs <= 64 && blocks > slots_of(best_w) ? 1 : 0;
 #define LLMIE_MMA(HD, W)                                                                                             \
   return rope ? launch_mma<HD, W, true>(q, k_cache, v_cache, part_m, part_l, part_acc, seq_slot, seq_kvlen,          \
                                         block_table, max_pages, n_seqs, n_q, n_kv, scale, window, pages_per_run,     \
@@ -611,10 +646,12 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
                                          n_runs, counters, out, nullptr, 0, 0, 0, opt, stream)
   if (hd == 64) {
     if (best_w == 8) LLMIE_MMA(64, 8);
+    if (best_w == 6) LLMIE_MMA(64, 6);
     if (best_w == 4) LLMIE_MMA(64, 4);
     if (best_w == 3) LLMIE_MMA(64, 3);
     LLMIE_MMA(64, 2);
   }
+  if (best_w == 6) LLMIE_MMA(128, 6);
   if (best_w >= 4) LLMIE_MMA(128, 4);
   if (best_w == 3) LLMIE_MMA(128, 3);
   LLMIE_MMA(128, 2);
