@@ -1,0 +1,304 @@
+// Many matrix products of one shape in one launch, C_g = A_g W_g^T, bfloat16 in and out, on the 5th-generation tensor cores
+// (tcgen05.mma, float32 accumulators in tensor memory): what prompts give to the products of grouped_gemm.cu. Two forms:
+//
+//   batched   every group has the same M rows; group g reads columns [g * a_gcs, + K) of A and writes columns
+//             [g * c_gcs, + N) of C (the heads of an attention layer, each with a matrix of its own)
+//   routed    group g has rows [group_end[g - 1], group_end[g]) of A and C (the experts of a routed feed-forward, rows
+//             sorted by expert); rows behind the last group's are neither read for a result nor written
+//
+// W is [groups][N (or 2 N), K]. With DUAL it is [gate rows | up rows] and the result is act(A gate^T) * (A up^T), both
+// products rounded to bfloat16 first, as two launches would leave them; otherwise act(A W^T).
+//
+// One block per SM walks over the tiles (128 rows x BN weight rows; the row tiles of one slice of weights follow one another,
+// so the slice comes from memory once). Warp 0 loads (TMA, 128-byte swizzle, a ring of stages of 64 k), warp 1 multiplies,
+// warps 2 to 9 take the sums out of tensor memory, two tiles of sums in turn, while the next tile is multiplied. Every wait is
+// bounded; one that gives up records a status, and the block frees its tensor memory and returns.
+//
+// What bounds it: many rows, shared memory (a stage of 48 KB is written and read once for 512 cycles of products); few, the
+// weights' way from memory; one short K (attention heads), the way of the results out of tensor memory, hence eight warps for
+// it (four: 15.5 us where eight take 13.4) and stores of 64 bytes a row (a thread storing its own row: 17.5). Measured, us, the
+// vendor's grouped products with the activation by itself / this: 16 experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, 600 pairs 75.4 +
+// 38.3 / 50.8 + 27.3, 5,331 pairs 117 + 56.1 / 97.7 + 51.1, 16,384 pairs 260 + 115 / 226 + 120; 8 of 2 x 1,408 x 4,096, 5,331 pairs
+// 118 + 57.1 / 117 + 63.4, 16,384 pairs 304 + 137 / 279 + 157; 128 of 2 x 768 x 2,048, 3,000 pairs 188 + 93.3 / 142 + 71.1. Heads, the
+// mma.sync kernel / this: 32 of 256 x 64, 2,130 rows 22.8 / 13.4; of 64 x 256, 19.9 / 9.3.
+#include "tcgen05.cuh"
+
+namespace llmie {
+using namespace tc;
+
+namespace {
+
+constexpr int kRows = 128, kK = 64;
+constexpr int kRing = 192 * 1024;                 // bytes of the ring of stages
+constexpr int kMostGroups = 1024;
+constexpr int kThreads = 320;
+constexpr int kStaged = 8 * 32 * 64;              // 32 rows x 32 columns of results for each epilogue warp, on their way to memory
+constexpr int kSmem = kRing + kStaged + 1024 + 2 * (kMostGroups + 1) * 4;
+
+struct Args {
+  __nv_bfloat16* C;
+  long long ldc, c_gcs;
+  const int* group_end;
+  int groups, M, N, K, a_gcs, act;
+  int* status;
+};
+
+struct Shared {
+  uint64_t full[8], empty[8], acc_full[2], acc_empty[2], drained;
+  uint32_t tmem;
+  int abort;
+};
+
+__device__ __forceinline__ void give_up(volatile int* abort, int* status, int code) {
+  if (!*abort) { *abort = 1; atomicExch(status, code); }
+}
+
+template <int BN, bool DUAL>
+__global__ void __launch_bounds__(kThreads, 1)
+grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Args p) {
+  constexpr int kStageBytes = (kRows + BN) * kK * 2;
+  constexpr int kStages = kRing / kStageBytes;            // 4 at BN 256, 6 at 128, 8 at 64
+  constexpr int kCols = DUAL ? BN / 2 : BN;               // columns of C a tile covers
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Shared sh;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  int* tile0 = reinterpret_cast<int*>(ring + kRing + kStaged);      // first tile of each group, groups + 1 of them
+  int* row0 = tile0 + p.groups + 1;                       // first row of each group, groups + 1
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k_tiles = (p.K + kK - 1) / kK, n_tiles = (p.N + kCols - 1) / kCols;
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&sh.full[s], 1);
+      mbar_init(&sh.empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sh.acc_full[b], 1);
+      mbar_init(&sh.acc_empty[b], 8);
+    }
+    mbar_init(&sh.drained, 1);
+    sh.abort = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&map_a);
+    tma_prefetch_desc(&map_w);
+  }
+  if (warp == 1) {
+    tmem_alloc(&sh.tmem, 2 * BN);
+    tmem_relinquish();
+  }
+  pdl_wait();
+  if (warp == 0) {                                        // where the groups' tiles and rows begin
+    int before = 0;
+    for (int e0 = 0; e0 < p.groups; e0 += 32) {
+      const int e = e0 + lane;
+      int rows = 0, first = 0;
+      if (e < p.groups) {
+        if (p.group_end) {
+          first = e ? min(max(p.group_end[e - 1], 0), p.M) : 0;
+          rows = max(min(p.group_end[e], p.M) - first, 0);
+        } else {
+          rows = p.M;
+        }
+        row0[e] = first;
+      }
+      const int tiles = (rows + kRows - 1) / kRows * n_tiles;
+      int sum = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      if (e < p.groups) tile0[e] = before + sum - tiles;
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) {
+      tile0[p.groups] = before;
+      row0[p.groups] = p.group_end ? min(max(p.group_end[p.groups - 1], 0), p.M) : p.M;
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = sh.tmem;
+  volatile int* abort = &sh.abort;
+  const int n_all = tile0[p.groups];
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int it = 0, e = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < n_all && ok; t += gridDim.x) {
+        while (t >= tile0[e + 1]) ++e;
+        const int r = t - tile0[e], m_tiles = (tile0[e + 1] - tile0[e]) / n_tiles;
+        const int m0 = row0[e] + r % m_tiles * kRows, n0 = r / m_tiles * kCols;
+        const int w0 = e * (DUAL ? 2 * p.N : p.N) + n0;
+        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
+          const int s = it % kStages;
+          if (it >= kStages && !mbar_wait(&sh.empty[s], ((it / kStages) - 1) & 1, abort)) {
+            give_up(abort, p.status, kStatusTimeoutEmpty);
+            ok = false;
+            break;
+          }
+          uint8_t* a = ring + s * kStageBytes;
+          uint8_t* w = a + kRows * kK * 2;
+          mbar_arrive_expect_tx(&sh.full[s], kStageBytes);
+          tma_load_2d(a, &map_a, (p.group_end ? 0 : e * p.a_gcs) + kt * kK, m0, &sh.full[s]);
+          tma_load_2d(w, &map_w, kt * kK, w0, &sh.full[s]);
+          if (DUAL) tma_load_2d(w + BN / 2 * kK * 2, &map_w, kt * kK, w0 + p.N, &sh.full[s]);
+        }
+      }
+      if (*abort) {        // the copies on their way land (bounded) before their shared memory is given up
+        for (int i = max(0, it - kStages); i < it; ++i)
+          for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.full[i % kStages], (i / kStages) & 1); ++spin)
+            __nanosleep(64);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_instr_desc_bf16(kRows, BN, 0, 0);
+      int it = 0, i = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < n_all && ok; t += gridDim.x, ++i) {
+        const int buf = i & 1;
+        if (i >= 2 && !mbar_wait(&sh.acc_empty[buf], ((i >> 1) - 1) & 1, abort)) {
+          give_up(abort, p.status, kStatusTimeoutMma);
+          break;
+        }
+        tc_fence_after_sync();
+        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
+          const int s = it % kStages;
+          if (!mbar_wait(&sh.full[s], (it / kStages) & 1, abort)) {
+            give_up(abort, p.status, kStatusTimeoutFull);
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t a = smem_u32(ring + s * kStageBytes), w = a + kRows * kK * 2;
+#pragma unroll
+          for (int kk = 0; kk < kK / 16; ++kk)
+            mma_bf16_ss(tmem + buf * BN, make_smem_desc(a + kk * 32, 16, 1024), make_smem_desc(w + kk * 32, 16, 1024), idesc,
+                        (kt > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(&sh.empty[s]);
+        }
+        if (ok) mma_commit(&sh.acc_full[buf]);
+      }
+      if (*abort) {        // no product may still run when the tensor memory is freed
+        mma_commit(&sh.drained);
+        for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.drained, 0); ++spin) __nanosleep(64);
+      }
+    }
+  } else {
+    const int quarter = warp & 3;                          // the tensor memory lanes this warp may read
+    const int c_first = warp < 6 ? 0 : kCols / 2;          // and its half of the columns
+    int e = 0, i = 0;
+    for (int t = blockIdx.x; t < n_all; t += gridDim.x, ++i) {
+      while (t >= tile0[e + 1]) ++e;
+      const int r = t - tile0[e], m_tiles = (tile0[e + 1] - tile0[e]) / n_tiles;
+      const int end = p.group_end ? row0[e + 1] : p.M;
+      const int row = row0[e] + r % m_tiles * kRows + quarter * 32, n0 = r / m_tiles * kCols;
+      const int buf = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sh.acc_full[buf], (i >> 1) & 1, abort))) {
+        give_up(abort, p.status, kStatusTimeoutMma);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + buf * BN;
+      __nv_bfloat16* dst = p.C + (size_t)row * p.ldc + (p.group_end ? 0 : (size_t)e * p.c_gcs) + n0;
+      uint8_t* staged = ring + kRing + (warp - 2) * (32 * 64);
+#pragma unroll 1
+      for (int c = c_first; c < c_first + kCols / 2; c += 32) {
+        float v[4][8];
+        uint32_t g[32];
+        tmem_ld_32x32(acc + c, g);
+        if (DUAL) {
+          uint32_t u[32];
+          tmem_ld_32x32(acc + BN / 2 + c, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            v[j >> 3][j & 7] = apply_act(__bfloat162float(__float2bfloat16(__uint_as_float(g[j]))), p.act) *
+                               __bfloat162float(__float2bfloat16(__uint_as_float(u[j])));
+        } else {
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j >> 3][j & 7] = __uint_as_float(g[j]);
+          if (p.act) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              v[j >> 3][j & 7] = apply_act(__bfloat162float(__float2bfloat16(v[j >> 3][j & 7])), p.act);
+          }
+        }
+        // a thread has a row: through shared memory (the four 16-byte pieces of a row in swizzled order) to stores in which
+        // neighbours write neighbouring pieces
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          store8(reinterpret_cast<__nv_bfloat16*>(staged + lane * 64 + ((j ^ (lane >> 1 & 3)) << 4)), v[j]);
+        __syncwarp();
+        const int piece = lane & 3, col = c + piece * 8;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int rr = j * 8 + (lane >> 2);
+          const uint4 x = *reinterpret_cast<const uint4*>(staged + rr * 64 + ((piece ^ (rr >> 1 & 3)) << 4));
+          if (row + rr < end && n0 + col < p.N) *reinterpret_cast<uint4*>(dst + (size_t)rr * p.ldc + col) = x;
+        }
+        __syncwarp();
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 2 * BN);
+  }
+}
+
+template <int BN, bool DUAL>
+int launch(const CUtensorMap& map_a, const void* W, const Args& p, cudaStream_t stream) {
+  CUtensorMap map_w;
+  const int rc = make_tmap_bf16_2d(&map_w, W, (uint64_t)p.groups * p.N * (DUAL ? 2 : 1), (uint64_t)p.K, (uint64_t)p.K,
+                                   DUAL ? BN / 2 : BN);
+  if (rc != LLMIE_OK) return rc;
+  const cudaError_t e = cudaFuncSetAttribute(grouped_tc_kernel<BN, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (e != cudaSuccess) return (int)e;
+  const int kCols = DUAL ? BN / 2 : BN;
+  const long long n_tiles = (p.N + kCols - 1) / kCols, m_tiles = (p.M + kRows - 1) / kRows;
+  const long long most = n_tiles * (p.group_end ? m_tiles + p.groups : m_tiles * p.groups);
+  if (most > 0x3fffffff) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  launch_k(grouped_tc_kernel<BN, DUAL>, dim3((unsigned)(most < 148 ? most : 148)), dim3(kThreads), kSmem, stream, map_a, map_w, p);
+  LLMIE_LAUNCH_CHECK();
+  return LLMIE_OK;
+}
+
+}  // namespace
+}  // namespace llmie
+
+using namespace llmie;
+
+// A [M, lda], W [groups, N or 2 N (dual), K] contiguous, C [M, ldc], all bfloat16 and on 16 bytes. group_end (int32 [groups],
+// rising) = the routed form, null = the batched one. Strides, group columns, N and K in multiples of 8 elements; K of the
+// batched form a multiple of 64 (a stage of 64 k of A would reach into the next group's columns). At most 1,024 groups.
+extern "C" int llmie_grouped_gemm_tc(const void* A, long long lda, long long a_gcs, const void* W, void* C, long long ldc,
+                                     long long c_gcs, const int* group_end, int groups, int M, int N, int K, int dual, int act,
+                                     int* status, cudaStream_t stream) {
+  if (M < 0 || N <= 0 || K <= 0 || groups <= 0 || a_gcs < 0 || c_gcs < 0 || !status) return LLMIE_ERR_BAD_ARG;
+  if (groups > kMostGroups || K % 8 || N % 8 || lda % 8 || ldc % 8 || a_gcs % 8 || c_gcs % 8 || (!group_end && K % 64) ||
+      (dual && !group_end) || (group_end && (lda < K || ldc < N)) || (!group_end && (lda < (groups - 1) * a_gcs + K || ldc < (groups - 1) * c_gcs + N)) ||
+      (long long)groups * N * 2 > 0x7fffffff || lda > 0x7fffffff)
+    return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (!aligned16(A) || !aligned16(W) || !aligned16(C)) return LLMIE_ERR_ALIGNMENT;
+  if (M == 0) return LLMIE_OK;
+  CUtensorMap map_a;
+  const int rc = tc::make_tmap_bf16_2d(&map_a, A, (uint64_t)M, group_end ? (uint64_t)K : (uint64_t)((groups - 1) * a_gcs + K),
+                                       (uint64_t)lda, kRows);
+  if (rc != LLMIE_OK) return rc;
+  const Args p = {(__nv_bfloat16*)C, ldc, c_gcs, group_end, groups, M, N, K, (int)a_gcs, act, status};
+  if (dual) return launch<256, true>(map_a, W, p, stream);
+  if (N <= 64) return launch<64, false>(map_a, W, p, stream);
+  if (N <= 128) return launch<128, false>(map_a, W, p, stream);
+  return launch<256, false>(map_a, W, p, stream);
+}

@@ -48,6 +48,7 @@ FAMILIES: Dict[str, tuple] = {
     "attention_rows_mma": ("attention_rows_mma.cu", [], []),
     "gemm_simt": ("gemm_simt.cu", [], []),
     "gemm_f32_tc": ("gemm_f32_tc.cu", [], []),
+    "grouped_gemm_tc": ("grouped_gemm_tc.cu", [], []),
     "gemm_skinny": ("gemm_skinny.cu", [], []),
     "gemm_tc": ("gemm_tc.cu", [], []),
     "gemm_stream": ("gemm_stream.cu", [], []),

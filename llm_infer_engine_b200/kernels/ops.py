@@ -1306,6 +1306,7 @@ def cap_rows(x: torch.Tensor, cap: float) -> torch.Tensor:
 _c_ll = ctypes.c_longlong
 _GROUPED_ARGS = [_c_void_p, _c_ll, _c_ll, _c_void_p, _c_void_p, _c_ll, _c_ll, _c_void_p, _c_ll, _c_ll, _c_void_p,
                  _c_void_p] + [_c_int] * 10 + [_c_void_p]
+_GROUPED_TC_ARGS = [_c_void_p, _c_ll, _c_ll, _c_void_p, _c_void_p, _c_ll, _c_ll, _c_void_p] + [_c_int] * 6 + [_c_void_p] * 2
 GROUPED_SMALL_ROWS = 64        # up to this many rows the tiles of 16 rows are used
 
 
@@ -1328,6 +1329,11 @@ def _cols(t: torch.Tensor, what: str) -> int:
     return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
 
 
+# From here on a batched bfloat16 product of whole 64 k on 16 bytes takes the tcgen05 kernel (us, mma.sync / this: 32 groups of
+# 256 x 64, 65 rows 5.9 / 8.0, 128 rows 6.8 / 6.5, 1,000 rows 12.6 / 8.8; of 64 x 256, 128 rows 7.5 / 5.2, 1,000 rows 10.8 / 6.4).
+BATCHED_TC_FROM = 128
+
+
 def batched_gemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, a_group_cols: int, out_group_cols: int,
                     k: int) -> torch.Tensor:
     """For every group g < G: out[:, g * out_group_cols : + N] = a[:, g * a_group_cols : + k] @ w[g]^T.
@@ -1343,6 +1349,13 @@ def batched_gemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, a_group
     _need(w, "w", a.dtype)
     lda, ldc = _cols(a, "a"), _cols(out, "out")
     _work(_nbytes(w) + T * G * (K * a.element_size() + N * out.element_size()), 2.0 * T * G * N * K)
+    if (T >= BATCHED_TC_FROM and a.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and K % 64 == 0 and G <= 1024
+            and not (N | lda | ldc | a_group_cols | out_group_cols) & 7
+            and not (a.data_ptr() | w.data_ptr() | out.data_ptr()) & 15):
+        f = _fn("grouped_gemm_tc", "llmie_grouped_gemm_tc", _GROUPED_TC_ARGS)
+        _check(f(a.data_ptr(), lda, a_group_cols, w.data_ptr(), out.data_ptr(), ldc, out_group_cols, None, G, T, N, K, 0, 0,
+                 tc_status_word(a.device).data_ptr(), _stream()), "batched_gemm_nt")
+        return out
     f = _fn("grouped_gemm", "llmie_grouped_gemm_nt", _GROUPED_ARGS)
     _check(f(a.data_ptr(), lda, a_group_cols, None, w.data_ptr(), N * K, K, out.data_ptr(), ldc, out_group_cols, None,
              None, 0, G, T, N, K, 0, 0, 1 if T <= GROUPED_SMALL_ROWS else 0, _dt(a, "a"), _dt(out, "out"), _stream()),
@@ -1522,25 +1535,34 @@ def moe_gather_scaled(x, sorted_token, sorted_pair, weights, out):
     return out
 
 
-def library_grouped_mm(x: torch.Tensor, w: torch.Tensor, group_end: torch.Tensor) -> torch.Tensor:
-    """Rows [group_end[e-1], group_end[e]) of x [P, K] times w[e]^T (w [E, N, K]) through the library's grouped GEMM
-    (bfloat16 in and out, float32 accumulation); rows beyond group_end[-1] are left as they are. Like `library_mm`
-    this is the product that prompts leave to the vendor library; the offsets stay on the device."""
-    def run():
-        return torch._grouped_mm(x, w.transpose(-2, -1), offs=group_end)
-    t = trace.timer
-    if t is None:
-        return run()
-    P, K = x.shape
-    t.note(_nbytes(x, w) + P * w.shape[1] * 2, 2.0 * P * w.shape[1] * K)
-    return t.run("library_grouped_mm", run, ())
-
-
-def library_grouped_mm_ok(n_pairs: int, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
-    """Whether the routed products of a prompt go to the library: bfloat16, enough pairs for tiles of 64 to fill, and
-    rows that start on 16 bytes."""
-    return (hasattr(torch, "_grouped_mm") and w_gate_up.dtype == torch.bfloat16 and n_pairs > GROUPED_SMALL_ROWS * 4
+def grouped_tc_takes(n_pairs: int, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
+    """Whether the routed products of a prompt go to the tcgen05 kernel (csrc/grouped_gemm_tc.cu): bfloat16, rows that start on
+    16 bytes, and more than 16 rows an expert on average. Below, tiles of 16 rows without the gather cost less or as much
+    (sort to combine, tiles of 16 / this, us: 16 experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, 7.5 rows each 88 / 96, 16 rows 114 /
+    96, 48 rows 179 / 99; 128 of 2 x 768 x 2,048, 8 rows 223 / 252, 16 rows 259 / 256; 64 of 2 x 1,408 x 2,048, 12 rows 201 / 215, 19
+    rows 254 / 217)."""
+    E = w_gate_up.shape[0]
+    return (w_gate_up.dtype == torch.bfloat16 and not routed_tiles_small(n_pairs, E, w_gate_up.dtype) and E <= 1024
             and w_gate_up.shape[2] % 8 == 0 and w_down.shape[2] % 8 == 0 and w_down.shape[1] % 8 == 0)
+
+
+def routed_gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, group_end: torch.Tensor, dual: bool = False,
+                   act: int = ACT_NONE) -> torch.Tensor:
+    """Rows [group_end[e-1], group_end[e]) of a [P, K] times w[e]^T (w [E, N or 2 N, K]) into the same rows of out [P, N], all
+    bfloat16; dual: w holds [gate | up] rows and the result is act(gate) * up, otherwise act(product). Rows beyond
+    group_end[-1] are left as they are; the offsets stay on the device."""
+    E, rows_w, K = w.shape
+    N = rows_w // 2 if dual else rows_w
+    P = a.shape[0]
+    _need(a, "a", torch.bfloat16, (P, K))
+    _need(w, "w", torch.bfloat16)
+    _need(out, "out", torch.bfloat16, (P, N))
+    _need(group_end, "group_end", torch.int32, (E,))
+    _work(_nbytes(a, w, out), 2.0 * P * rows_w * K)
+    f = _fn("grouped_gemm_tc", "llmie_grouped_gemm_tc", _GROUPED_TC_ARGS)
+    _check(f(a.data_ptr(), K, 0, w.data_ptr(), out.data_ptr(), N, 0, group_end.data_ptr(), E, P, N, K, 1 if dual else 0, int(act),
+             tc_status_word(a.device).data_ptr(), _stream()), "routed_gemm_tc")
+    return out
 
 
 # ------------------------------------------------------------------------------------------ latent attention

@@ -22,9 +22,8 @@ sum of its two largest s + c. `weight_on` "input" (default "output"): the weight
 expert_e(a_t,e u_t), which is not the same thing under a non-linear expert; the rows are scaled while they are gathered
 into the order of their experts, and the combine adds with weight one.
 `identity_experts` n: the router has n more outputs than there are experts; the last n stand for experts that return
-their input (their share is weight * u_t), and they hold no tensors. Prompts of a bfloat16 engine
-hand the two products to the vendor library's grouped GEMM instead (as the dense layers hand theirs to its plain one):
-the tokens are gathered into the order of their experts first, the offsets stay on the device.
+their input (their share is weight * u_t), and they hold no tensors. Prompts of a bfloat16 engine take the two products to
+the tcgen05 kernel: the tokens are gathered into the order of their experts first, the offsets stay on the device.
 """
 from __future__ import annotations
 
@@ -91,7 +90,6 @@ class RoutedExperts(FeedForward):
                 "activation": str(p.get("shared_activation", name)), "out_float32": True,
                 "names": {"gate": n["gate"], "up": n["up"], "down": n["down"]}}), runtime)
         self.w_router = self.b_router = self.correction = self.w_gate_up = self.w_down = None
-        self._library = True          # prompts may use the vendor's grouped GEMM until it refuses a shape
 
     def _expert_name(self, e: int, which: str) -> str:
         return f"{self.names['expert'].format(e=e)}.{self.names[which]}"
@@ -148,16 +146,15 @@ class RoutedExperts(FeedForward):
             ops.moe_route(x, self.w_router, self.b_router, ids, weights, self.route_mode, self.correction,
                           self.weight_scale, self.groups)
             n_pairs = T * top
-            library = self._library and ops.library_grouped_mm_ok(n_pairs, w, self.w_down)
-            small = not library and ops.routed_tiles_small(n_pairs, E, w.dtype)
+            prompt = ops.grouped_tc_takes(n_pairs, w, self.w_down)
+            small = ops.routed_tiles_small(n_pairs, E, w.dtype)
             tile = ops.grouped_tile_rows(small)
             n_tiles = ops.moe_max_tiles(n_pairs, E, tile)
             index = torch.empty(2 * n_tiles * tile + n_tiles, dtype=torch.int32, device=dev)
             sorted_token, sorted_pair = index[:n_tiles * tile], index[n_tiles * tile:2 * n_tiles * tile]
             tile_group = index[2 * n_tiles * tile:]
-            shared = None
-            if library:
-                # prompts: each expert's rows side by side, the two products by the library's grouped GEMM
+            if prompt:
+                # each expert's rows side by side; gate, up and the activation one launch, down the next
                 extra = torch.empty(E + n_pairs, dtype=torch.int32, device=dev)
                 group_end, pair_pos = extra[:E], extra[E:]
                 ops.moe_sort(ids, E, tile, sorted_token, sorted_pair, tile_group, group_end, pair_pos)
@@ -166,23 +163,10 @@ class RoutedExperts(FeedForward):
                     ops.moe_gather_scaled(x, sorted_token, sorted_pair, weights, xs)
                 else:
                     ops.moe_gather_rows(xin, sorted_token, xs)
-                try:
-                    gu = ops.library_grouped_mm(xs, w, group_end)
-                except RuntimeError as exc:
-                    # the library refuses these sizes (it checks before it launches): this library's own routed
-                    # products take them, from now on without asking again
-                    if "CUDA error" in str(exc):
-                        raise
-                    self._library = False
-                    gu = None
-                if gu is not None:
-                    act = torch.empty((n_tiles * tile, self.expert_ff), dtype=w.dtype, device=dev)
-                    if self.gated:
-                        ops.gated_act(gu, act, self.activation)
-                    else:
-                        ops.bias_act(gu, None, act, self.activation)
-                    y = ops.library_grouped_mm(act, self.w_down, group_end)
-                    return self._combine(y, weights, ids, x, ctx, pair_pos)
+                act = ops.routed_gemm_tc(xs, w, torch.empty((n_tiles * tile, self.expert_ff), dtype=w.dtype, device=dev),
+                                         group_end, self.gated, self.activation)
+                y = ops.routed_gemm_tc(act, self.w_down, xs, group_end)          # the rows read are not needed any more
+                return self._combine(y, weights, ids, x, ctx, pair_pos)
             ops.moe_sort(ids, E, tile, sorted_token, sorted_pair, tile_group)
             # gate and up of every pair's expert with the activation; rows stay in sorted order
             act = torch.empty((n_tiles * tile, self.expert_ff), dtype=w.dtype, device=dev)

@@ -1,0 +1,84 @@
+"""The prompts' grouped bfloat16 products on tcgen05 at the edges of their tiles (128 rows, 64 to 256 weight rows, 64 k): groups
+without rows, remainders of rows, N and K, more tiles than blocks; against float64 sums, and against the kernel of fewer rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+U = 2.0 ** -8          # unit roundoff of bfloat16: 8 significant bits, round to nearest
+
+
+def ops():
+    from llm_infer_engine_b200.kernels import ops as o
+    return o
+
+
+def _sum_bound(x, w):
+    """float32 sums of K products: relative to the sum of the products' magnitudes, as for the other grouped products."""
+    return 2.0 ** -16 * (x.abs() @ w.abs().T) + 1e-6
+
+
+@pytest.mark.parametrize("rows", [(64, 0, 128, 1, 0), (0, 0, 0, 300, 257), (1, 1, 1, 1, 1), (0, 0, 0, 0, 0), (640, 0, 64, 129, 127)])
+@pytest.mark.parametrize("N,K", [(8, 8), (256, 64), (120, 200), (264, 72), (2048, 320)])
+@pytest.mark.parametrize("form", ["plain", "relu", "dual"])
+def test_routed(rows, N, K, form):
+    o, E, P = ops(), len(rows), sum(rows) + 70
+    g = torch.Generator().manual_seed(P + N + K)
+    a = torch.randn(P, K, generator=g).to(torch.bfloat16)
+    w = torch.randn(E, (2 if form == "dual" else 1) * N, K, generator=g).to(torch.bfloat16)
+    end = torch.tensor(rows).cumsum(0)
+    out = torch.full((P, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.routed_gemm_tc(a.to(DEV), w.to(DEV), out, end.int().to(DEV), form == "dual",
+                     o.ACT_NONE if form == "plain" else o.ACTIVATIONS["relu"])
+    got = out.cpu().double()
+    assert bool((got[int(end[-1]):] == 7.0).all())                     # nothing behind the last group's rows
+    for e in range(E):
+        x, y = a[int(end[e]) - rows[e]:int(end[e])].double(), w[e].double()
+        s, b = x @ y.T, _sum_bound(x, y)
+        mine = got[int(end[e]) - rows[e]:int(end[e])]
+        if form == "dual":
+            # both products rounded to bfloat16 (U each, and the sums' own error), their product rounded again
+            (gate, up), (bg, bu) = s.split(N, 1), b.split(N, 1)
+            eg, eu = bg + U * (gate.abs() + bg), bu + U * (up.abs() + bu)
+            s, b = gate.clamp(min=0) * up, eg * up.abs() + eu * gate.abs() + eg * eu
+        elif form == "relu":
+            b, s = b + U * (s.abs() + b), s.clamp(min=0)
+        assert bool(((mine - s).abs() <= b + U * (s.abs() + b)).all()), float((mine - s).abs().max())
+
+
+@pytest.mark.parametrize("T", [128, 129, 255, 1000])
+@pytest.mark.parametrize("G,N,K", [(3, 64, 64), (2, 72, 128), (5, 8, 64), (2, 264, 192), (32, 256, 64), (40, 64, 256)])
+def test_batched(T, G, N, K):
+    o = ops()
+    assert T >= o.BATCHED_TC_FROM
+    g = torch.Generator().manual_seed(T + N + K)
+    a = torch.randn(T, G * (K + 8) + 8, generator=g).to(torch.bfloat16)
+    w = torch.randn(G, N, K, generator=g).to(torch.bfloat16)
+    out = torch.zeros(T, G * (N + 8) + 8, dtype=torch.bfloat16, device=DEV)
+    few = torch.zeros(64, G * (N + 8) + 8, dtype=torch.bfloat16, device=DEV)
+    o.batched_gemm_nt(a.to(DEV)[:, 8:], w.to(DEV), out[:, 8:], K + 8, N + 8, K)
+    o.batched_gemm_nt(a.to(DEV)[:64, 8:], w.to(DEV), few[:, 8:], K + 8, N + 8, K)          # the kernel of fewer rows
+    assert not bool(out[:, :8].any())
+    for i in range(G):
+        x, y = a[:, 8 + i * (K + 8):8 + i * (K + 8) + K].double(), w[i].double()
+        mine = out[:, 8 + i * (N + 8):8 + (i + 1) * (N + 8)].cpu().double()
+        s, b = x @ y.T, _sum_bound(x, y)
+        assert bool(((mine[:, :N] - s).abs() <= b + U * (s.abs() + b)).all())
+        assert not bool(mine[:, N:].any())                            # nothing beside the columns
+        f = few[:, 8 + i * (N + 8):8 + i * (N + 8) + N].cpu().double()
+        assert bool(((mine[:64, :N] - f).abs() <= 2 * b[:64] + 2 * U * (s[:64].abs() + b[:64])).all())
+
+
+def test_no_finite_value_crosses_rows_or_groups():
+    o = ops()
+    a = torch.ones(256, 72, dtype=torch.bfloat16, device=DEV)
+    a[130] = float("nan")
+    w = torch.ones(2, 64, 72, dtype=torch.bfloat16, device=DEV)
+    w[1, 5] = float("inf")
+    out = torch.zeros(256, 64, dtype=torch.bfloat16, device=DEV)
+    o.routed_gemm_tc(a, w, out, torch.tensor([100, 256], dtype=torch.int32, device=DEV))
+    bad = ~torch.isfinite(out)
+    want = torch.zeros_like(bad)
+    want[130] = True
+    want[100:, 5] = True
+    assert torch.equal(bad, want)
