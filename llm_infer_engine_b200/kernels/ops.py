@@ -970,7 +970,7 @@ _TC_STATUS_TEXT = {1: "a TMA load did not arrive", 2: "the tensor cores did not 
 
 def tc_status_word(device) -> torch.Tensor:
     """One int32 per device that the tensor-core kernels set when a bounded wait gives up."""
-    key = torch.device(device).index or 0
+    key = (device if type(device) is torch.device else torch.device(device)).index or 0
     t = _tc_status.get(key)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=device)
@@ -1341,23 +1341,23 @@ def batched_gemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, a_group
     w [G, N, k] contiguous, of a's dtype (float32, or bfloat16 with bfloat16 or float32 out). float32 accumulation in
     the order of k."""
     G, N, K = w.shape
-    T = a.shape[0]
-    if K != k or a.shape[1] < (G - 1) * a_group_cols + k or out.shape[1] < (G - 1) * out_group_cols + N \
-            or out.shape[0] != T:
+    (T, a_cols), (out_rows, out_cols) = a.shape, out.shape
+    if K != k or a_cols < (G - 1) * a_group_cols + k or out_cols < (G - 1) * out_group_cols + N or out_rows != T:
         raise KernelError(f"batched_gemm_nt: shapes a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} "
                           f"do not fit (group columns {a_group_cols} / {out_group_cols})")
     _need(w, "w", a.dtype)
     lda, ldc = _cols(a, "a"), _cols(out, "out")
-    _work(_nbytes(w) + T * G * (K * a.element_size() + N * out.element_size()), 2.0 * T * G * N * K)
-    if (T >= BATCHED_TC_FROM and a.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and K % 64 == 0 and G <= 1024
-            and not (N | lda | ldc | a_group_cols | out_group_cols) & 7
-            and not (a.data_ptr() | w.data_ptr() | out.data_ptr()) & 15):
+    if trace.timer is not None:
+        _work(_nbytes(w) + T * G * (K * a.element_size() + N * out.element_size()), 2.0 * T * G * N * K)
+    pa, pw, po = a.data_ptr(), w.data_ptr(), out.data_ptr()
+    if (T >= BATCHED_TC_FROM and a.dtype is torch.bfloat16 and out.dtype is torch.bfloat16 and G <= 1024
+            and not (K & 63 or (N | lda | ldc | a_group_cols | out_group_cols) & 7 or (pa | pw | po) & 15)):
         f = _fn("grouped_gemm_tc", "llmie_grouped_gemm_tc", _GROUPED_TC_ARGS)
-        _check(f(a.data_ptr(), lda, a_group_cols, w.data_ptr(), out.data_ptr(), ldc, out_group_cols, None, G, T, N, K, 0, 0,
+        _check(f(pa, lda, a_group_cols, pw, po, ldc, out_group_cols, None, G, T, N, K, 0, 0,
                  tc_status_word(a.device).data_ptr(), _stream()), "batched_gemm_nt")
         return out
     f = _fn("grouped_gemm", "llmie_grouped_gemm_nt", _GROUPED_ARGS)
-    _check(f(a.data_ptr(), lda, a_group_cols, None, w.data_ptr(), N * K, K, out.data_ptr(), ldc, out_group_cols, None,
+    _check(f(pa, lda, a_group_cols, None, pw, N * K, K, po, ldc, out_group_cols, None,
              None, 0, G, T, N, K, 0, 0, 1 if T <= GROUPED_SMALL_ROWS else 0, _dt(a, "a"), _dt(out, "out"), _stream()),
            "batched_gemm_nt")
     return out
