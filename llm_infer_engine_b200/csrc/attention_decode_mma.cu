@@ -626,15 +626,19 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
   }
   // That is right for sequences of one length. Lengths differ where batches are served, and then a long sequence's block with few
   // warps is what a launch ends with, however many others run beside it. Where some sequence is longer than 2,048 keys (a captured
-  // step of shorter ones is sized for 2,048 at most): six warps a block (two blocks an SM; head size 128, one, up to 50
-  // sequences), served longest first where blocks have to queue. Measured, us, the choice above / this one: head size 64, 64
-  // sequences of 700 to 3,900 keys 56.0 / 41.2, 64 of 200 to 4,000 54.6 / 32.9, 48 of 200 to 4,000 42.2 / 31.8, 24 of 200 to
-  // 4,000 37.4 / 29.5, 64 of 3,000 70.0 / 65.3, 48 of 3,000 53.3 / 59.0; head size 128, 64 of 200 to 4,000 (three warps,
-  // queueing) 86.6 / 69.8, 48 of 200 to 4,000 77.9 / 48.8, 24 of 200 to 4,000 53.5 / 34.0, 32 of 3,000 70.6 / 67.6, 24 of 3,000
-  // 57.2 / 63.7, but 64 of 3,000 124 / 134. With shorter ones six warps cost more where lengths are equal (64 of 512, 14.2 /
-  // 19.4) than they give where not. A window or a chunk makes the work of long sequences alike.
+  // step of shorter ones is sized for 2,048 at most): six warps a block (two blocks an SM; head size 128, one), served longest
+  // first where blocks have to queue, as long as equal lengths do not pay for it, which they do where the last round of such
+  // blocks fills the SMs badly. Measured, us, the choice above / this one, head size 64: 64 sequences of 700 to 3,900 keys 56.0 /
+  // 41.2, of 200 to 4,000 54.6 / 32.9, of 3,000 70.0 / 65.3; 24 of 200 to 4,000 37.4 / 29.5, of 3,000 38.1 / 29.4; 48 (left as they
+  // were) of 200 to 4,000 42.2 / 31.8, of 3,000 53.3 / 59.0. Head size 128: 48 of 200 to 4,000 77.9 / 48.8, of 3,000 104 / 101, 50 of
+  // 2,000 to 2,400 about 76 / 80; 32 of 200 to 4,000 58.5 / 36.1, of 3,000 70.6 / 67.6; 24 (left) 53.5 / 34.0 and 57.2 / 63.7; 64
+  // (three warps, longest first) of 200 to 4,000 86.6 / 69.8, of 3,000 124 / 124, with six warps 66.6 and 134. With shorter ones six
+  // warps cost more where lengths are equal (64 of 512, 14.2 / 19.4) than they give where not. A window or a chunk makes the work
+  // of long sequences alike.
   const bool long_ones = window == 0 && pages_per_run > 32;
-  if (long_ones && blocks > 148 && (hd == 64 || blocks <= 400)) best_w = 6;
+  const long long slots_6 = slots_of(6), rounds_6 = (blocks + slots_6 - 1) / slots_6;
+  const bool fill = 100 * blocks >= 85 * rounds_6 * slots_6;
+  if (long_ones && blocks > 148 && (hd == 64 ? rounds_6 == 1 || (rounds_6 == 2 && fill) : fill && blocks <= 400)) best_w = 6;
   // (finding the order takes a block about half a microsecond; blocks that are all there at once gain nothing by it)
   opt.longest_first = long_ones && n_seqs <= 64 && blocks > slots_of(best_w) ? 1 : 0;
 #define LLMIE_MMA(HD, W)                                                                                             \

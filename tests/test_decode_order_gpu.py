@@ -8,7 +8,7 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("n,longest", [(19, 2100), (40, 2113), (64, 2300), (65, 2200), (33, 1100)])
+@pytest.mark.parametrize("n,longest", [(19, 2100), (36, 2113), (40, 2113), (49, 2100), (64, 2300), (65, 2200), (33, 1100)])
 def test_every_sequence_is_served(hd, n, longest):
     from llm_infer_engine_b200.kernels import ops
     n_q, n_kv = 32, 8
