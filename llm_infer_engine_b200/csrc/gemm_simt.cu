@@ -6,6 +6,7 @@
 // their sum, and the result is ((P_0 + P_1) + P_2) + ... + P_7. Both kernels below compute exactly this, so a row's
 // result does not depend on which other rows share the launch, on the tile or on how K was split among blocks.
 //
+// (Sizes below from before gemm_f32_tc.cu took them; the bounds hold for what is left, weights whose K is short or not whole 128s.)
 // What bounds it: up to 16 rows the weights' way from memory (32,000 x 2,048, one row: 45 us, 5.8 TB/s); above, the FMA
 // rate (148 SMs x 128 lanes x 2 x 1.965 GHz = 74 TFLOP/s) less what the 128 sums of a thread cost: eight warps an SM, which
 // wait for dependent instructions in between (2,048 x 8,192, 301 rows: FMA pipes 60 %, issue 39 %, shared memory 41 %; 16,384

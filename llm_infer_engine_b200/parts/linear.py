@@ -4,9 +4,9 @@ bfloat16 weights: up to 8 rows this library's skinny kernel (up to 16 with the a
 blocks an SM); above that the library GEMM (cuBLAS through torch.mm), as the reference does with nn.Linear (src/model.py:17-19,34-37,137),
 accumulating in float32, except where this library's weight-streaming tcgen05 kernel measured faster
 (`ops.gemm_stream_wins`: a vocabulary-sized head at 33 to 64 rows). float32 weights: this
-library's own FMA kernel, true 32-bit with a fixed summation order; that is the whole of
-the 32-bit path, and also what a bfloat16 engine does with a tensor that its checkpoint
-stores in 32-bit.
+library's own kernels, true 32-bit with a fixed summation order (large weights on the tensor cores
+with every number as three bfloat16, others by FMA); that is the whole of the 32-bit path, and also
+what a bfloat16 engine does with a tensor that its checkpoint stores in 32-bit.
 """
 from __future__ import annotations
 
