@@ -12,7 +12,9 @@
 // One block per SM walks over the tiles (128 rows x BN weight rows; the row tiles of one slice of weights follow one another,
 // so the slice comes from memory once). Warp 0 loads (TMA, 128-byte swizzle, a ring of stages of 64 k), warp 1 multiplies,
 // warps 2 to 9 take the sums out of tensor memory, two tiles of sums in turn, while the next tile is multiplied. Every wait is
-// bounded; one that gives up records a status, and the block frees its tensor memory and returns.
+// bounded; one that gives up records a status, what the block has not finished becomes NaN (C may hold something else that
+// looks like a result: the routed experts' second product writes over their gathered inputs), and the block waits for its copies
+// and products, frees its tensor memory and returns.
 //
 // What bounds it: many rows, shared memory (a stage of 48 KB is written and read once for 512 cycles of products); few, the
 // weights' way from memory; one short K (attention heads), the way of the results out of tensor memory, hence eight warps for
@@ -46,14 +48,15 @@ struct Args {
 struct Shared {
   uint64_t full[8], empty[8], acc_full[2], acc_empty[2], drained;
   uint32_t tmem;
-  int abort;
+  int abort, loaded;       // loaded: stages that warp 0 has asked for
 };
 
 __device__ __forceinline__ void give_up(volatile int* abort, int* status, int code) {
   if (!*abort) { *abort = 1; atomicExch(status, code); }
 }
 
-template <int BN, bool DUAL>
+// LIMIT: polls before a wait gives up, a constant as in attention_latent_tc.cu.
+template <int BN, bool DUAL, unsigned LIMIT>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Args p) {
   constexpr int kStageBytes = (kRows + BN) * kK * 2;
@@ -78,7 +81,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       mbar_init(&sh.acc_empty[b], 8);
     }
     mbar_init(&sh.drained, 1);
-    sh.abort = 0;
+    sh.abort = sh.loaded = 0;
     fence_mbar_init();
     tma_prefetch_desc(&map_a);
     tma_prefetch_desc(&map_w);
@@ -135,7 +138,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int w0 = e * (DUAL ? 2 * p.N : p.N) + n0;
         for (int kt = 0; kt < k_tiles; ++kt, ++it) {
           const int s = it % kStages;
-          if (it >= kStages && !mbar_wait(&sh.empty[s], ((it / kStages) - 1) & 1, abort)) {
+          if (it >= kStages && !mbar_wait(&sh.empty[s], ((it / kStages) - 1) & 1, abort, LIMIT)) {
             give_up(abort, p.status, kStatusTimeoutEmpty);
             ok = false;
             break;
@@ -148,11 +151,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (DUAL) tma_load_2d(w + BN / 2 * kK * 2, &map_w, kt * kK, w0 + p.N, &sh.full[s]);
         }
       }
-      if (*abort) {        // the copies on their way land (bounded) before their shared memory is given up
-        for (int i = max(0, it - kStages); i < it; ++i)
-          for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.full[i % kStages], (i / kStages) & 1); ++spin)
-            __nanosleep(64);
-      }
+      sh.loaded = it;
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -161,14 +160,14 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       bool ok = true;
       for (int t = blockIdx.x; t < n_all && ok; t += gridDim.x, ++i) {
         const int buf = i & 1;
-        if (i >= 2 && !mbar_wait(&sh.acc_empty[buf], ((i >> 1) - 1) & 1, abort)) {
+        if (i >= 2 && !mbar_wait(&sh.acc_empty[buf], ((i >> 1) - 1) & 1, abort, LIMIT)) {
           give_up(abort, p.status, kStatusTimeoutMma);
           break;
         }
         tc_fence_after_sync();
         for (int kt = 0; kt < k_tiles; ++kt, ++it) {
           const int s = it % kStages;
-          if (!mbar_wait(&sh.full[s], (it / kStages) & 1, abort)) {
+          if (!mbar_wait(&sh.full[s], (it / kStages) & 1, abort, LIMIT)) {
             give_up(abort, p.status, kStatusTimeoutFull);
             ok = false;
             break;
@@ -183,28 +182,31 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
         if (ok) mma_commit(&sh.acc_full[buf]);
       }
-      if (*abort) {        // no product may still run when the tensor memory is freed
-        mma_commit(&sh.drained);
-        for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.drained, 0); ++spin) __nanosleep(64);
-      }
     }
   } else {
     const int quarter = warp & 3;                          // the tensor memory lanes this warp may read
     const int c_first = warp < 6 ? 0 : kCols / 2;          // and its half of the columns
     int e = 0, i = 0;
+    bool ok = true;
     for (int t = blockIdx.x; t < n_all; t += gridDim.x, ++i) {
       while (t >= tile0[e + 1]) ++e;
       const int r = t - tile0[e], m_tiles = (tile0[e + 1] - tile0[e]) / n_tiles;
       const int end = p.group_end ? row0[e + 1] : p.M;
       const int row = row0[e] + r % m_tiles * kRows + quarter * 32, n0 = r / m_tiles * kCols;
       const int buf = i & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(&sh.acc_full[buf], (i >> 1) & 1, abort))) {
+      __nv_bfloat16* dst = p.C + (size_t)row * p.ldc + (p.group_end ? 0 : (size_t)e * p.c_gcs) + n0;
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[buf], (i >> 1) & 1, abort, LIMIT));
+      if (!ok) {                                           // neither this tile nor those behind it have a result
         give_up(abort, p.status, kStatusTimeoutMma);
-        break;
+        const uint4 nan8 = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+        for (int at = lane; at < 32 * (kCols / 16); at += 32) {
+          const int rr = at / (kCols / 16), col = c_first + at % (kCols / 16) * 8;
+          if (row + rr < end && n0 + col < p.N) *reinterpret_cast<uint4*>(dst + (size_t)rr * p.ldc + col) = nan8;
+        }
+        continue;
       }
       tc_fence_after_sync();
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + buf * BN;
-      __nv_bfloat16* dst = p.C + (size_t)row * p.ldc + (p.group_end ? 0 : (size_t)e * p.c_gcs) + n0;
       uint8_t* staged = ring + kRing + (warp - 2) * (32 * 64);
 #pragma unroll 1
       for (int c = c_first; c < c_first + kCols / 2; c += 32) {
@@ -251,25 +253,37 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem, 2 * BN);
+  tc_fence_after_sync();
+  if (*abort) {
+    // whichever role gave up: copies and products still in flight end (bounded) before the block gives its memory up
+    if (threadIdx.x == 0) {
+      for (int i = max(0, sh.loaded - kStages); i < sh.loaded; ++i)
+        for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.full[i % kStages], (i / kStages) & 1); ++spin)
+          __nanosleep(64);
+    }
+    if (warp == 1 && elect_one()) {                        // the lane that issued the products
+      mma_commit(&sh.drained);
+      for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.drained, 0); ++spin) __nanosleep(64);
+    }
+    __syncthreads();
   }
+  if (warp == 1) tmem_dealloc(tmem, 2 * BN);
 }
 
 template <int BN, bool DUAL>
-int launch(const CUtensorMap& map_a, const void* W, const Args& p, cudaStream_t stream) {
+int launch(const CUtensorMap& map_a, const void* W, const Args& p, bool no_wait, cudaStream_t stream) {
   CUtensorMap map_w;
   const int rc = make_tmap_bf16_2d(&map_w, W, (uint64_t)p.groups * p.N * (DUAL ? 2 : 1), (uint64_t)p.K, (uint64_t)p.K,
                                    DUAL ? BN / 2 : BN);
   if (rc != LLMIE_OK) return rc;
-  const cudaError_t e = cudaFuncSetAttribute(grouped_tc_kernel<BN, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  auto kernel = no_wait ? grouped_tc_kernel<BN, DUAL, 0> : grouped_tc_kernel<BN, DUAL, kSpinLimit>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return (int)e;
   const int kCols = DUAL ? BN / 2 : BN;
   const long long n_tiles = (p.N + kCols - 1) / kCols, m_tiles = (p.M + kRows - 1) / kRows;
   const long long most = n_tiles * (p.group_end ? m_tiles + p.groups : m_tiles * p.groups);
   if (most > 0x3fffffff) return LLMIE_ERR_UNSUPPORTED_SIZE;
-  launch_k(grouped_tc_kernel<BN, DUAL>, dim3((unsigned)(most < 148 ? most : 148)), dim3(kThreads), kSmem, stream, map_a, map_w, p);
+  launch_k(kernel, dim3((unsigned)(most < 148 ? most : 148)), dim3(kThreads), kSmem, stream, map_a, map_w, p);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
@@ -282,9 +296,10 @@ using namespace llmie;
 // A [M, lda], W [groups, N or 2 N (dual), K] contiguous, C [M, ldc], all bfloat16 and on 16 bytes. group_end (int32 [groups],
 // rising) = the routed form, null = the batched one. Strides, group columns, N and K in multiples of 8 elements; K of the
 // batched form a multiple of 64 (a stage of 64 k of A would reach into the next group's columns). At most 1,024 groups.
-extern "C" int llmie_grouped_gemm_tc(const void* A, long long lda, long long a_gcs, const void* W, void* C, long long ldc,
-                                     long long c_gcs, const int* group_end, int groups, int M, int N, int K, int dual, int act,
-                                     int* status, cudaStream_t stream) {
+// no_wait != 0: every wait gives up at once (for tests of that path).
+extern "C" int llmie_grouped_gemm_tc_form(const void* A, long long lda, long long a_gcs, const void* W, void* C, long long ldc,
+                                          long long c_gcs, const int* group_end, int groups, int M, int N, int K, int dual, int act,
+                                          int* status, int no_wait, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || groups <= 0 || a_gcs < 0 || c_gcs < 0 || !status) return LLMIE_ERR_BAD_ARG;
   if (groups > kMostGroups || K % 8 || N % 8 || lda % 8 || ldc % 8 || a_gcs % 8 || c_gcs % 8 || (!group_end && K % 64) ||
       (dual && !group_end) || (group_end && (lda < K || ldc < N)) || (!group_end && (lda < (groups - 1) * a_gcs + K || ldc < (groups - 1) * c_gcs + N)) ||
@@ -297,8 +312,14 @@ extern "C" int llmie_grouped_gemm_tc(const void* A, long long lda, long long a_g
                                        (uint64_t)lda, kRows);
   if (rc != LLMIE_OK) return rc;
   const Args p = {(__nv_bfloat16*)C, ldc, c_gcs, group_end, groups, M, N, K, (int)a_gcs, act, status};
-  if (dual) return launch<256, true>(map_a, W, p, stream);
-  if (N <= 64) return launch<64, false>(map_a, W, p, stream);
-  if (N <= 128) return launch<128, false>(map_a, W, p, stream);
-  return launch<256, false>(map_a, W, p, stream);
+  if (dual) return launch<256, true>(map_a, W, p, no_wait, stream);
+  if (N <= 64) return launch<64, false>(map_a, W, p, no_wait, stream);
+  if (N <= 128) return launch<128, false>(map_a, W, p, no_wait, stream);
+  return launch<256, false>(map_a, W, p, no_wait, stream);
+}
+
+extern "C" int llmie_grouped_gemm_tc(const void* A, long long lda, long long a_gcs, const void* W, void* C, long long ldc,
+                                     long long c_gcs, const int* group_end, int groups, int M, int N, int K, int dual, int act,
+                                     int* status, cudaStream_t stream) {
+  return llmie_grouped_gemm_tc_form(A, lda, a_gcs, W, C, ldc, c_gcs, group_end, groups, M, N, K, dual, act, status, 0, stream);
 }

@@ -82,3 +82,36 @@ def test_no_finite_value_crosses_rows_or_groups():
     want[130] = True
     want[100:, 5] = True
     assert torch.equal(bad, want)
+
+
+@pytest.mark.parametrize("form", ["routed", "dual", "batched"])
+def test_a_block_that_gives_up_leaves_no_numbers(form):
+    """Waits that run out (no polls at all here): NaN in every row that has a group, also in tiles that a block never came to, an
+    error for whoever asks, and the next call is none the worse."""
+    o = ops()
+    E, K = 5, 128
+    N = 4104 if form == "routed" else 2056 if form == "dual" else 64        # more tiles than blocks; the batched form has fewer
+    rows = torch.tensor([640, 0, 64, 129, 127])
+    end = rows.cumsum(0).int().to(DEV)
+    P = int(rows.sum()) + 30
+    a = torch.randn(P, E * K if form == "batched" else K, device=DEV).to(torch.bfloat16)
+    w = torch.randn(E, 2 * N if form == "dual" else N, K, device=DEV).to(torch.bfloat16)
+    out = torch.full((P, E * N if form == "batched" else N), 3.0, dtype=torch.bfloat16, device=DEV)
+    status = o.tc_status_word(torch.device(DEV, 0))
+    groups = (None, E, P, N, K, 0, 0) if form == "batched" else (end.data_ptr(), E, P, N, K, int(form == "dual"), 0)
+    cols = (K, N) if form == "batched" else (0, 0)
+    f = o._fn("grouped_gemm_tc", "llmie_grouped_gemm_tc_form",
+              [o._c_void_p, o._c_ll, o._c_ll, o._c_void_p, o._c_void_p, o._c_ll, o._c_ll, o._c_void_p] + [o._c_int] * 6
+              + [o._c_void_p, o._c_int, o._c_void_p])
+
+    def call(no_wait):
+        assert f(a.data_ptr(), a.shape[1], cols[0], w.data_ptr(), out.data_ptr(), out.shape[1], cols[1], *groups, status.data_ptr(),
+                 no_wait, o._stream()) == 0
+        torch.cuda.synchronize()
+        return out[:P if form == "batched" else int(rows.sum())]
+
+    assert bool(call(1).isnan().all())
+    with pytest.raises(o.KernelError):
+        o.check_tc_status(torch.device(DEV, 0))
+    assert bool(call(0).isfinite().all()) and (form == "batched" or bool((out[int(rows.sum()):] == 3.0).all()))
+    o.check_tc_status(torch.device(DEV, 0))
