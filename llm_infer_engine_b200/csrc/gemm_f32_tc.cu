@@ -66,9 +66,9 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
 }
 
 struct TcShared {
-  uint64_t ready[4], empty[kStages], x_empty[4], acc_full[2];       // ready: all that a turn of two stages needs
+  uint64_t ready[4], empty[kStages], x_empty[4], acc_full[2], drained;       // ready: all that a turn of two stages needs
   uint32_t tmem;
-  int abort;
+  int abort, copied;                        // copied: turns whose tokens' parts have been asked for
 };
 
 // 8 neighbouring floats; WIDE: from a 32-byte aligned address. No condition around it, and the registers are named as read too:
@@ -175,7 +175,8 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       : "memory");
 }
 
-template <int NT, bool WIDE>
+// LIMIT: polls before a wait gives up, a constant as in attention_latent_tc.cu.
+template <int NT, bool WIDE, unsigned LIMIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, const float* LLMIE_WEIGHT W, float* C, int M, int N,
                    int K, int lda, int ldw, int ldc, int split, int* __restrict__ status) {
@@ -201,7 +202,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       mbar_init(&sh.x_empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) mbar_init(&sh.acc_full[i], 1);
-    sh.abort = 0;
+    mbar_init(&sh.drained, 1);
+    sh.abort = sh.copied = 0;
     fence_mbar_init();
   }
   if (warp == kSumWarps + kSplitWarps) {
@@ -231,7 +233,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
 #pragma unroll 1
     for (int slice = slice0; slice < slice1; ++slice) {
       const int i = slice - slice0, ab = i & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[ab], (i >> 1) & 1, abort));
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[ab], (i >> 1) & 1, abort, LIMIT));
       if (!ok) {
         if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutMma); }
         break;
@@ -303,7 +305,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     uint64_t* empty = &sh.empty[group];
     uint32_t parity = 1;                    // a fresh barrier counts as released
     for (int s = group; s < n_stages; s += kStages, parity ^= 1) {
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(empty, parity, abort));
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(empty, parity, abort, LIMIT));
       if (!ok) {
         if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
         break;
@@ -338,7 +340,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       constexpr uint64_t kXNext = S::kXPart / 16;
       constexpr uint32_t kWNext = kStageK / 2;
       const int n_turns = 2 * (slice1 - slice0);
-      bool ok = mbar_wait(&sh.ready[0], 0, abort);
+      bool ok = mbar_wait(&sh.ready[0], 0, abort, LIMIT);
       for (int turn = 0; ok && turn < n_turns; ++turn) {
         const int ws = turn & 1, xs = S::kSplitsX ? ws : turn & 3, ab = (turn >> 1) & 1;
         const uint32_t g1 = tmem + ab * S::kAccCols, g2 = g1 + NT;
@@ -361,7 +363,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
         }
         __syncwarp();
         // the wait for the next turn stands in front of this one's last products: they are worked on meanwhile
-        if (turn + 1 < n_turns) ok = mbar_wait(&sh.ready[(turn + 1) & 3], ((turn + 1) >> 2) & 1, abort);
+        if (turn + 1 < n_turns) ok = mbar_wait(&sh.ready[(turn + 1) & 3], ((turn + 1) >> 2) & 1, abort, LIMIT);
         if (leader) {
           products(1, 1);
           mma_commit(&sh.empty[2 * ws + 1]);
@@ -377,10 +379,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       if (elect_one()) {
         tma_prefetch_desc(&map_x);
         pdl_wait();
-        int issued = 0;
-        for (int turn = 0; turn < n_stages / 2; ++turn) {
+        int turn = 0;
+        for (; turn < n_stages / 2; ++turn) {
           const int xs = turn & 3;
-          if (!mbar_wait(&sh.x_empty[xs], ((turn >> 2) & 1) ^ 1, abort)) {
+          if (!mbar_wait(&sh.x_empty[xs], ((turn >> 2) & 1) ^ 1, abort, LIMIT)) {
             if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
             break;
           }
@@ -391,12 +393,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
             for (int p = 0; p < 3; ++p)
               tma_load_2d(x_stages + (2 * xs + e) * S::kXStage + p * S::kXPart, &map_x,
                           slice0 * kSliceK + (2 * turn + e) * kStageK, p * M + m0, &sh.ready[xs]);
-          issued = turn + 1;
         }
-        if (*abort) {       // the copies of this thread land, or have had the time to, before their shared memory is given up
-          for (int turn = max(0, issued - 4); turn < issued; ++turn)
-            for (unsigned spin = 0; spin < (1u << 14) && !mbar_test(&sh.ready[turn & 3], (turn >> 2) & 1); ++spin) __nanosleep(64);
-        }
+        sh.copied = turn;
       }
       __syncwarp();
     }
@@ -423,10 +421,21 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kSumWarps + kSplitWarps) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem, S::kTmemCols);
+  tc_fence_after_sync();
+  if (*abort) {
+    // whichever role gave up: copies and products still in flight end, or have had the time to, before the block gives its memory up
+    // (a turn's barrier is also short of the splitting warps that gave up: its copies then have the whole of the wait)
+    if (tid == 0) {
+      for (int turn = max(0, sh.copied - 4); turn < sh.copied; ++turn)
+        for (unsigned spin = 0; spin < (1u << 14) && !mbar_test(&sh.ready[turn & 3], (turn >> 2) & 1); ++spin) __nanosleep(64);
+    }
+    if (warp == kSumWarps + kSplitWarps && elect_one()) {       // the lane that issued the products
+      mma_commit(&sh.drained);
+      for (unsigned spin = 0; spin < (1u << 16) && !mbar_test(&sh.drained, 0); ++spin) __nanosleep(64);
+    }
+    __syncthreads();
   }
+  if (warp == kSumWarps + kSplitWarps) tmem_dealloc(tmem, S::kTmemCols);
 }
 
 // ------------------------------------------------------------------------------------------ up to 16 tokens
@@ -578,9 +587,10 @@ int launch_few(const float* A, const float* W, float* C, int M, int N, int K, in
 
 template <int NT, bool WIDE>
 int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw, int ldc, int split,
-              int* status, cudaStream_t stream) {
+              bool no_wait, int* status, cudaStream_t stream) {
   using S = Shape<NT>;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel<NT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
+  auto kernel = no_wait ? gemm_f32_tc_kernel<NT, WIDE, 0> : gemm_f32_tc_kernel<NT, WIDE, kSpinLimit>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
   if (e != cudaSuccess) return (int)e;
   const long long blocks = (long long)((M + NT - 1) / NT) * ((N + kMt - 1) / kMt) * split;
   if (blocks > 0x7fffffffLL) return LLMIE_ERR_UNSUPPORTED_SIZE;
@@ -600,11 +610,10 @@ int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int 
     LLMIE_LAUNCH_CHECK();
   }
   if (split > 1)
-    launch_k_cluster(gemm_f32_tc_kernel<NT, WIDE>, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, split, map, A, W, C, M, N,
-                     K, lda, ldw, ldc, split, status);
+    launch_k_cluster(kernel, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, split, map, A, W, C, M, N, K, lda, ldw, ldc,
+                     split, status);
   else
-    launch_k(gemm_f32_tc_kernel<NT, WIDE>, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, map, A, W, C, M, N, K, lda, ldw,
-             ldc, split, status);
+    launch_k(kernel, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, map, A, W, C, M, N, K, lda, ldw, ldc, split, status);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
@@ -618,12 +627,14 @@ using namespace llmie;
 extern "C" int llmie_gemm_f32_tc_takes(int N, int K) { return N >= 128 && K >= 1024 && K % kSliceK == 0; }
 
 // form: tokens a block (8: the kernel for up to 16 tokens; 16, 64, 80) + 1000 * split (blocks of a tile: 1, 2, 4), for tests: every form gives the same bits. 0:
-// chosen by size. `parts`: 3 M K bfloat16 of scratch, not needed for 16 tokens a block.
+// chosen by size. + 10000: every wait gives up at once (for tests of that path; the sums are then made by plain FMAs). `parts`: 3 M K bfloat16 of scratch, not needed for 16 tokens a block.
 extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
                                       int ldc, int form, int* status, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N || !status) return LLMIE_ERR_BAD_ARG;
   if (!llmie_gemm_f32_tc_takes(N, K)) return LLMIE_ERR_UNSUPPORTED_SIZE;
   if (M == 0) return LLMIE_OK;
+  const bool no_wait = form >= 10000;
+  form %= 10000;
   int nt = form % 1000, split = form / 1000;
   if (form == 0) {
     const long long rows = (N + kMt - 1) / kMt;
@@ -659,8 +670,8 @@ extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, 
   }
 #define LLMIE_TC(nt_)                                                                                     \
   case nt_:                                                                                               \
-    return wide ? launch_tc<nt_, true>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, status, stream)      \
-                : launch_tc<nt_, false>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, status, stream)
+    return wide ? launch_tc<nt_, true>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, no_wait, status, stream)      \
+                : launch_tc<nt_, false>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, no_wait, status, stream)
   switch (nt) {
     LLMIE_TC(16);
     LLMIE_TC(64);

@@ -80,3 +80,20 @@ def test_what_it_takes():
             assert bool(takes(n, k)) == ops.gemm_f32_tc_takes(n, k)
     a, w = torch.randn(3, 1024, device=DEV), torch.randn(100, 1024, device=DEV)
     assert _form(a, w, 0)[0] == -2                            # fewer rows than a tile
+
+
+@pytest.mark.parametrize("form", [1016, 4016, 1064, 1080, 2080, 4080])
+def test_waits_that_run_out(form):
+    """No polls at all: an error for whoever asks, plain sums in place of those that did not come, and the next call is none the worse."""
+    from llm_infer_engine_b200.kernels import ops
+    M, N, K = 16 if form % 1000 == 16 else 90, 300, 1152
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    status, out = _form(a, w, 10000 + form)
+    torch.cuda.synchronize()
+    assert status == 0 and bool(((out.double() - ref).abs() <= K * 2.0 ** -24 * size).all())
+    with pytest.raises(ops.KernelError):
+        ops.check_tc_status(torch.device(DEV, 0))
+    status, out = _form(a, w, form)
+    assert status == 0 and torch.equal(out, ops.gemm_f32_nt(a, w))
+    ops.check_tc_status(torch.device(DEV, 0))
