@@ -178,8 +178,8 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 // LIMIT: polls before a wait gives up, a constant as in attention_latent_tc.cu.
 template <int NT, bool WIDE, unsigned LIMIT>
 __global__ void __launch_bounds__(kTcThreads, 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, const float* LLMIE_WEIGHT W, float* C, int M, int N,
-                   int K, int lda, int ldw, int ldc, int split, int* __restrict__ status) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, const float* W, float* C, int M, int N, int K, int lda,
+                   int ldw, int ldc, int split, int w_written, int* __restrict__ status) {
   using S = Shape<NT>;
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ TcShared sh;
@@ -292,6 +292,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     // the row behind the last is the last one again, the stage behind the last one too: nobody reads what becomes of them
     const float* w_src = W + (size_t)min(n0 + quarter * 32 + lane, N - 1) * ldw + slice0 * kSliceK;
     float w[4][8] = {}, x[8] = {};
+    if (w_written) pdl_wait();
 #pragma unroll
     for (int i = 0; i < 4; ++i) load_8<WIDE>(w_src + group * kStageK + 8 * i, w[i]);
     // (up to 16 tokens: 64 threads of the group a piece of 8)
@@ -299,7 +300,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     const float* a_src = A + (size_t)min(m0 + r, M - 1) * lda + slice0 * kSliceK + (gt & 3) * 8;
     unsigned char* x_to = x_stages + group * S::kXStage + swizzle64_offset(r, gt & 3);
     if (S::kSplitsX) {
-      pdl_wait();                           // weights are written by no kernel
+      pdl_wait();
       load_8<WIDE>(a_src + group * kStageK, x);
     }
     uint64_t* empty = &sh.empty[group];
@@ -458,10 +459,11 @@ template <bool VEC>
 __device__ __forceinline__ float4 few_load_w(const float* p) {
   float4 v;
   if (VEC) {
-    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.L2::256B.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
   } else {
-    v = make_float4(p[0], p[1], p[2], p[3]);
+    asm volatile("ld.global.f32 %0, [%4];\n\tld.global.f32 %1, [%4 + 4];\n\tld.global.f32 %2, [%4 + 8];\n\tld.global.f32 %3, [%4 + 12];"
+                 : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w) : "l"(p));
   }
   return v;
 }
@@ -483,8 +485,8 @@ __device__ __forceinline__ void split_4(const float4& v, unsigned (&h)[3][2]) {
 
 template <int T8, bool VEC>      // T8: eights of tokens
 __global__ void __launch_bounds__(kFewWarps * 32, 2)
-gemm_f32_few_kernel(const float* A, const float* LLMIE_WEIGHT W, float* __restrict__ C, int M, int N, int K, int lda, int ldw,
-                    int ldc) {
+gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
+                    int w_written) {
   extern __shared__ float sums[];         // [slices][T8][4][32]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tiles = (N + 15) / 16, slices = K / kSliceK;
@@ -499,12 +501,13 @@ gemm_f32_few_kernel(const float* A, const float* LLMIE_WEIGHT W, float* __restri
   };
   float4 lo[8], hi[8];                    // a slice of this warp: eight products' worth of k
   point(blockIdx.x, min(warp, slices - 1));
+  if (w_written) pdl_wait();
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     lo[j] = few_load_w<VEC>(w_lo + 16 * j);
     hi[j] = few_load_w<VEC>(w_hi + 16 * j);
   }
-  pdl_wait();                             // weights are written by no kernel
+  pdl_wait();
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
 #pragma unroll 1
@@ -574,20 +577,22 @@ gemm_f32_few_kernel(const float* A, const float* LLMIE_WEIGHT W, float* __restri
 constexpr int kFewSmem = 100 * 1024;      // two blocks an SM
 
 template <int T8, bool VEC>
-int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
+int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
+               cudaStream_t stream) {
   const size_t smem = (size_t)(K / kSliceK) * T8 * 128 * 4;
   if (smem > kFewSmem) return LLMIE_ERR_UNSUPPORTED_SIZE;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<T8, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = (N + 15) / 16;
-  launch_k(gemm_f32_few_kernel<T8, VEC>, dim3(tiles < 2 * 148 ? tiles : 2 * 148), dim3(kFewWarps * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
+  launch_k(gemm_f32_few_kernel<T8, VEC>, dim3(tiles < 2 * 148 ? tiles : 2 * 148), dim3(kFewWarps * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc,
+           w_written);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
 
 template <int NT, bool WIDE>
 int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw, int ldc, int split,
-              bool no_wait, int* status, cudaStream_t stream) {
+              int w_written, bool no_wait, int* status, cudaStream_t stream) {
   using S = Shape<NT>;
   auto kernel = no_wait ? gemm_f32_tc_kernel<NT, WIDE, 0> : gemm_f32_tc_kernel<NT, WIDE, kSpinLimit>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem);
@@ -611,27 +616,31 @@ int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int 
   }
   if (split > 1)
     launch_k_cluster(kernel, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, split, map, A, W, C, M, N, K, lda, ldw, ldc,
-                     split, status);
+                     split, w_written, status);
   else
-    launch_k(kernel, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, map, A, W, C, M, N, K, lda, ldw, ldc, split, status);
+    launch_k(kernel, dim3((unsigned)blocks), dim3(kTcThreads), S::kSmem, stream, map, A, W, C, M, N, K, lda, ldw, ldc, split, w_written,
+             status);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
 
-}  // namespace
-}  // namespace llmie
-
-using namespace llmie;
+template <int T8>
+int few_form(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
+             cudaStream_t stream) {
+  const bool vec = aligned16(A) && aligned16(W) && ((lda | ldw) & 3) == 0;
+  return vec ? launch_few<T8, true>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream)
+             : launch_few<T8, false>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream);
+}
 
 // 1 when the kernel takes a weight [N, K]. The answer depends on the weight alone: a row's bits are then the same in every step.
-extern "C" int llmie_gemm_f32_tc_takes(int N, int K) { return N >= 128 && K >= 1024 && K % kSliceK == 0; }
+bool takes(int N, int K) { return N >= 128 && K >= 1024 && K % kSliceK == 0; }
 
 // form: tokens a block (8: the kernel for up to 16 tokens; 16, 64, 80) + 1000 * split (blocks of a tile: 1, 2, 4), for tests: every form gives the same bits. 0:
 // chosen by size. + 10000: every wait gives up at once (for tests of that path; the sums are then made by plain FMAs). `parts`: 3 M K bfloat16 of scratch, not needed for 16 tokens a block.
-extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
-                                      int ldc, int form, int* status, cudaStream_t stream) {
+int product(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw, int ldc, int form,
+            int w_written, int* status, cudaStream_t stream) {
   if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N || !status) return LLMIE_ERR_BAD_ARG;
-  if (!llmie_gemm_f32_tc_takes(N, K)) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (!takes(N, K)) return LLMIE_ERR_UNSUPPORTED_SIZE;
   if (M == 0) return LLMIE_OK;
   const bool no_wait = form >= 10000;
   form %= 10000;
@@ -663,15 +672,13 @@ extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, 
   const bool wide = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 31) == 0 && ((lda | ldw) & 7) == 0;
   if (nt == 8) {
     if (M > 16) return LLMIE_ERR_UNSUPPORTED_SIZE;
-    const bool vec = aligned16(A) && aligned16(W) && ((lda | ldw) & 3) == 0;
-    if (M <= 8)
-      return vec ? launch_few<1, true>(A, W, C, M, N, K, lda, ldw, ldc, stream) : launch_few<1, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    return vec ? launch_few<2, true>(A, W, C, M, N, K, lda, ldw, ldc, stream) : launch_few<2, false>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    return M <= 8 ? few_form<1>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream)
+                  : few_form<2>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream);
   }
 #define LLMIE_TC(nt_)                                                                                     \
   case nt_:                                                                                               \
-    return wide ? launch_tc<nt_, true>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, no_wait, status, stream)      \
-                : launch_tc<nt_, false>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, no_wait, status, stream)
+    return wide ? launch_tc<nt_, true>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, w_written, no_wait, status, stream)      \
+                : launch_tc<nt_, false>(A, W, C, parts, M, N, K, lda, ldw, ldc, split, w_written, no_wait, status, stream)
   switch (nt) {
     LLMIE_TC(16);
     LLMIE_TC(64);
@@ -681,7 +688,20 @@ extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, 
 #undef LLMIE_TC
 }
 
+}  // namespace
+}  // namespace llmie
+
+using namespace llmie;
+
+extern "C" int llmie_gemm_f32_tc_takes(int N, int K) { return takes(N, K) ? 1 : 0; }
+
+extern "C" int llmie_gemm_f32_tc_form(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
+                                      int ldc, int form, int* status, cudaStream_t stream) {
+  return product(A, W, C, parts, M, N, K, lda, ldw, ldc, form, 1, status, stream);
+}
+
+// w_written: whether a kernel in front may have written W, which is then read behind the wait for it.
 extern "C" int llmie_gemm_f32_tc(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw,
-                                 int ldc, int* status, cudaStream_t stream) {
-  return llmie_gemm_f32_tc_form(A, W, C, parts, M, N, K, lda, ldw, ldc, 0, status, stream);
+                                 int ldc, int w_written, int* status, cudaStream_t stream) {
+  return product(A, W, C, parts, M, N, K, lda, ldw, ldc, 0, w_written, status, stream);
 }

@@ -734,10 +734,11 @@ def gemm_f32_tc_takes(n: int, k: int) -> bool:
     return n >= 128 and k >= 1024 and k % 128 == 0
 
 
-def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, stored: bool = False) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T in true float32, fixed summation order: a row's bits do not depend on the other rows.
     Large weights on the tensor cores, every number as the sum of three bfloat16 (csrc/gemm_f32_tc.cu; which weights are
-    large is settled by their size alone), others by FMA on the CUDA cores."""
+    large is settled by their size alone), others by FMA on the CUDA cores. stored: no kernel writes `w` (a model's weight),
+    so that it may be read while the kernels in front still run."""
     M, K = a.shape
     N = w.shape[0]
     _need(a, "a", torch.float32)
@@ -749,8 +750,8 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     if gemm_f32_tc_takes(N, K):
         # scratch: the parts of `a`, which the kernel for few rows makes itself
         parts = torch.empty(3 * M * K, dtype=torch.bfloat16, device=a.device) if M > 16 else None
-        f = _fn("gemm_f32_tc", "llmie_gemm_f32_tc", [_c_void_p] * 4 + [_c_int] * 6 + [_c_void_p] * 2)
-        _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(parts), M, N, K, K, K, N,
+        f = _fn("gemm_f32_tc", "llmie_gemm_f32_tc", [_c_void_p] * 4 + [_c_int] * 7 + [_c_void_p] * 2)
+        _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(parts), M, N, K, K, K, N, 0 if stored else 1,
                  tc_status_word(a.device).data_ptr(), _stream()), "gemm_f32_tc")
         return out
     f = _fn("gemm_simt", "llmie_gemm_f32_nt", [_c_void_p] * 3 + [_c_int] * 6 + [_c_void_p])

@@ -44,7 +44,7 @@ class Linear:
         out_dtype = out_dtype or x.dtype
         w = self.weight
         if w.dtype == torch.float32:
-            y = ops.gemm_f32_nt(x if x.dtype == torch.float32 else x.float(), w)
+            y = ops.gemm_f32_nt(x if x.dtype == torch.float32 else x.float(), w, stored=True)
             return y if out_dtype == torch.float32 else y.to(out_dtype)
         xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
         T = xb.shape[0]

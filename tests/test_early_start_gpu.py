@@ -61,7 +61,7 @@ def _consumer(kind, rows, n, g, dtype):
 
 @pytest.mark.parametrize("product", ["skinny", "float32"])
 @pytest.mark.parametrize("kind", ["conv", "conv_prompt", "conv_qk", "conv_qk_odd", "steps"])
-@pytest.mark.parametrize("rows,k,n", [(1, 128, 512), (3, 2048, 2816), (8, 96, 448), (40, 128, 640)])
+@pytest.mark.parametrize("rows,k,n", [(1, 128, 512), (3, 2048, 2816), (8, 96, 448), (40, 128, 640), (17, 1024, 512), (301, 2048, 2816)])
 def test_rows_behind_a_product_are_that_products(product, kind, rows, k, n):
     from llm_infer_engine_b200.kernels import ops
     if product == "skinny" and rows > 8:
@@ -81,6 +81,35 @@ def test_rows_behind_a_product_are_that_products(product, kind, rows, k, n):
             else:
                 ops.gemm_f32_nt(x, w, out=proj)
             got.append(call(proj))
+        torch.cuda.synchronize()
+        return torch.stack(got)
+
+    was = ops.PDL
+    try:
+        ops.set_pdl(False)
+        want = rounds()
+        ops.set_pdl(True)
+        for _ in range(3):
+            assert torch.equal(rounds(), want)
+    finally:
+        ops.set_pdl(was)
+
+
+@pytest.mark.parametrize("rows,k,n", [(3, 2048, 2816), (16, 1024, 256), (16, 1024, 8192), (17, 1024, 512), (90, 1152, 300), (301, 2048, 2816),
+                                      (3, 96, 448)])
+def test_a_matrix_that_a_kernel_in_front_writes(rows, k, n):
+    """A float32 product reads ahead only what its caller calls a stored weight: here its matrix is scaled by the kernel in front,
+    which lets it start early."""
+    from llm_infer_engine_b200.kernels import ops
+    g = torch.Generator().manual_seed(rows + n)
+    w = torch.randn(n, k, generator=g).to(DEV)
+    xs = [torch.randn(rows, k, generator=g).to(DEV) for _ in range(ROUNDS)]
+
+    def rounds():
+        got = []
+        for i, x in enumerate(xs):
+            ops.scale_rows(w, 0.5 if i % 2 else 2.0)            # exact, and back where it was after two rounds
+            got.append(ops.gemm_f32_nt(x, w))
         torch.cuda.synchronize()
         return torch.stack(got)
 
