@@ -39,6 +39,7 @@ constexpr int kStageK = 32;              // 64 bytes of a part's row, 64-byte sw
 constexpr int kPerSlice = 128 / kStageK;  // stages of a slice
 constexpr int kSliceK = 128;
 constexpr int kChains = 4;
+constexpr uint32_t kNegateA = 1u << 13;   // of an instruction descriptor: the products' signs
 constexpr int kSumWarps = 8, kSplitWarps = 16;
 constexpr int kStages = 4;                // four warps split for each
 static_assert(kSplitWarps == 4 * kStages && kStages == kPerSlice, "the stages of a slice go round four groups of warps");
@@ -143,9 +144,9 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-// run (+)= G1 + G2, 16 columns at a time.
+// run (+)= times (G1 + G2), 16 columns at a time.
 template <int C0, int N>
-__device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)[N], bool fresh) {
+__device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)[N], bool fresh, float times) {
   constexpr int n = N - C0 < 16 ? N - C0 : 16;
   uint32_t a[n], b[n];
 #pragma unroll
@@ -156,9 +157,9 @@ __device__ __forceinline__ void sum_columns(uint32_t g1, int to_g2, float (&run)
 #pragma unroll
   for (int c = 0; c < n; ++c) {
     const float v = __uint_as_float(a[c]) + __uint_as_float(b[c]);
-    run[C0 + c] = fresh ? v : run[C0 + c] + v;
+    run[C0 + c] = fmaf(times, v, fresh ? 0.f : run[C0 + c]);
   }
-  if constexpr (C0 + n < N) sum_columns<C0 + n, N>(g1, to_g2, run, fresh);
+  if constexpr (C0 + n < N) sum_columns<C0 + n, N>(g1, to_g2, run, fresh, times);
 }
 
 __device__ __forceinline__ void tmem_st_32x4(uint32_t taddr, const uint4& v) {
@@ -192,12 +193,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
   const int slices = K / kSliceK;
   const int chain0 = rank * (kChains / split);
   const int slice0 = chain0 * slices / kChains, slice1 = (chain0 + kChains / split) * slices / kChains;
-  const int n_stages = kPerSlice * (slice1 - slice0);
+  const int n_stages = kPerSlice * (slice1 - slice0), n_turns = n_stages / 2;
   volatile int* abort = &sh.abort;
 
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) {         // eight splitting warps, the tokens' copy, before a slice the sum warps
-      mbar_init(&sh.ready[i], 8 + (S::kSplitsX ? 0 : 1) + (i & 1 ? 0 : kSumWarps));
+    for (int i = 0; i < 4; ++i) {         // eight splitting warps, the tokens' copy, the sum warps
+      mbar_init(&sh.ready[i], 8 + (S::kSplitsX ? 0 : 1) + kSumWarps);
       mbar_init(&sh.empty[i], 1);
       mbar_init(&sh.x_empty[i], 1);
     }
@@ -228,22 +229,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     const int n_cols = row_there ? min(S::kCols, M - m0 - col0) : 0;       // of the result
     float run[S::kCols] = {};
     int chain = 0, chain_end = (chain0 + 1) * slices / kChains;
-    bool fresh = true, ok = true;
-    if (lane < 2) mbar_arrive(&sh.ready[2 * lane]);       // both accumulators are free
+    bool fresh = true, second = false, ok = true;
+    if (lane < 2) mbar_arrive(&sh.ready[lane]);           // both accumulators are free
 #pragma unroll 1
-    for (int slice = slice0; slice < slice1; ++slice) {
-      const int i = slice - slice0, ab = i & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[ab], (i >> 1) & 1, abort, LIMIT));
+    for (int turn = 0; turn < n_turns; ++turn) {
+      const int ab = turn & 1, slice = slice0 + (turn >> 1);
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_full[ab], (turn >> 1) & 1, abort, LIMIT));
       if (!ok) {
         if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutMma); }
         break;
       }
       tc_fence_after_sync();
-      sum_columns<0, S::kCols>(acc + ab * S::kAccCols, NT, run, fresh);
+      sum_columns<0, S::kCols>(acc + ab * S::kAccCols, NT, run, fresh, second ? -1.f : slice + 1 < chain_end ? 2.f : 1.f);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.ready[2 * ab]);
-      fresh = slice + 1 == chain_end;
+      if (lane == 0) mbar_arrive(&sh.ready[(turn + 2) & 3]);
+      fresh = ab && slice + 1 == chain_end;
+      second = second != (ab != 0) && !fresh;
       if (fresh) {                        // the chain is done: ((P_0 + P_1) + (P_2 + P_3)) as far as this block has them
         if (chain & 1) {
           const float* from = h + (chain == 3 ? NT * kMt : 0);
@@ -340,21 +342,22 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       const uint64_t first_x = operand_desc(smem_u32(x_stages));
       constexpr uint64_t kXNext = S::kXPart / 16;
       constexpr uint32_t kWNext = kStageK / 2;
-      const int n_turns = 2 * (slice1 - slice0);
+      int chain = chain0, chain_end = (chain0 + 1) * slices / kChains;
+      uint32_t second = 0;                             // a pair's second slice: its products are subtracted from the first one's sums
       bool ok = mbar_wait(&sh.ready[0], 0, abort, LIMIT);
       for (int turn = 0; ok && turn < n_turns; ++turn) {
-        const int ws = turn & 1, xs = S::kSplitsX ? ws : turn & 3, ab = (turn >> 1) & 1;
-        const uint32_t g1 = tmem + ab * S::kAccCols, g2 = g1 + NT;
+        const int ws = turn & 1, xs = S::kSplitsX ? ws : turn & 3;
+        const uint32_t g1 = tmem + ws * S::kAccCols, g2 = g1 + NT, minus = second * kNegateA;
         if (S::kSplitsX) fence_proxy_async_smem();     // these parts were written through the generic proxy
         tc_fence_after_sync();
         auto products = [&](int e, int kk) {           // 32 bytes of a token's row: 2 in a descriptor's units; 8 columns
           const uint32_t w1 = tmem + S::kWCol + (2 * ws + e) * S::kWStageCols + 8 * kk, w2 = w1 + kWNext, w3 = w2 + kWNext;
           const uint64_t x1 = first_x + (2 * xs + e) * (S::kXStage / 16) + 2 * kk, x2 = x1 + kXNext, x3 = x2 + kXNext;
-          mma_bf16_ts(g1, w1, x1, d2, ws > 0 || e > 0 || kk > 0 ? 1u : 0u);
-          mma_bf16_ts(g2, w1, x3, d1, 1u);
-          mma_bf16_ts(g2, w2, x1, d1, 1u);
-          mma_bf16_ts(g2, w2, x2, d1, 1u);
-          mma_bf16_ts(g2, w3, x1, d1, 1u);
+          mma_bf16_ts(g1, w1, x1, d2 | minus, e > 0 || kk > 0 ? 1u : second);
+          mma_bf16_ts(g2, w1, x3, d1 | minus, 1u);
+          mma_bf16_ts(g2, w2, x1, d1 | minus, 1u);
+          mma_bf16_ts(g2, w2, x2, d1 | minus, 1u);
+          mma_bf16_ts(g2, w3, x1, d1 | minus, 1u);
         };
         if (leader) {
           products(0, 0);
@@ -369,9 +372,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
           products(1, 1);
           mma_commit(&sh.empty[2 * ws + 1]);
           if (!S::kSplitsX) mma_commit(&sh.x_empty[xs]);
-          if (ws) mma_commit(&sh.acc_full[ab]);
+          mma_commit(&sh.acc_full[ws]);
         }
         __syncwarp();
+        if (ws) {
+          second ^= 1;
+          if (slice0 + (turn >> 1) + 1 == chain_end) {
+            second = 0;
+            chain_end = (++chain + 1) * slices / kChains;
+          }
+        }
       }
       if (!ok && leader && !*abort) { *abort = 1; atomicExch(status, kStatusTimeoutFull); }
       __syncwarp();
@@ -381,7 +391,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
         tma_prefetch_desc(&map_x);
         pdl_wait();
         int turn = 0;
-        for (; turn < n_stages / 2; ++turn) {
+        for (; turn < n_turns; ++turn) {
           const int xs = turn & 3;
           if (!mbar_wait(&sh.x_empty[xs], ((turn >> 2) & 1) ^ 1, abort, LIMIT)) {
             if (!*abort) { *abort = 1; atomicExch(status, kStatusTimeoutEmpty); }
@@ -483,50 +493,73 @@ __device__ __forceinline__ void split_4(const float4& v, unsigned (&h)[3][2]) {
   }
 }
 
+// What a warp takes at a time: 64 k of each slice of a pair, or the two halves of a slice that has no partner; as many items as
+// slices. Halves are counted over all slices: the item is half `a` = few_item >> 1 and half a + 1 + (few_item & 1).
+__device__ __forceinline__ int few_item(int item, int slices) {
+  int chain = 0;
+  while (item >= (chain + 1) * slices / kChains) ++chain;
+  const int c0 = chain * slices / kChains, n = (chain + 1) * slices / kChains - c0, at = item - c0;
+  return at + 1 == n && (n & 1) ? 4 * item : 4 * item - 2 * (at & 1) + 1;
+}
+
 template <int T8, bool VEC>      // T8: eights of tokens
 __global__ void __launch_bounds__(kFewWarps * 32, 2)
 gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
                     int w_written) {
-  extern __shared__ float sums[];         // [slices][T8][4][32]
+  extern __shared__ float sums[];         // [halves of slices][T8][4][32]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int tiles = (N + 15) / 16, slices = K / kSliceK;
   const float* a_src[T8];
 #pragma unroll
   for (int i = 0; i < T8; ++i) a_src[i] = A + (size_t)min(g + 8 * i, M - 1) * lda + 4 * t;
-  const float *w_lo, *w_hi;               // of the slice that is loaded
-  auto point = [&](int tile, int slice) {
-    const float* w = W + slice * kSliceK + 4 * t;
+  const float *w_lo, *w_hi;               // of the item that is loaded
+  int w_to_b;                             // from where half `a` ends to half `b`
+  auto point = [&](int tile, int f) {
+    const float* w = W + (f >> 1) * (kSliceK / 2) + 4 * t;
     w_lo = w + (size_t)min(tile * 16 + g, N - 1) * ldw;
     w_hi = w + (size_t)min(tile * 16 + g + 8, N - 1) * ldw;
+    w_to_b = (f & 1) * (kSliceK / 2);
   };
-  float4 lo[8], hi[8];                    // a slice of this warp: eight products' worth of k
-  point(blockIdx.x, min(warp, slices - 1));
+  float4 lo[8], hi[8];                    // an item of this warp: eight products' worth of k
+  auto load = [&](int j) {
+    const int k = 16 * j + (j < 4 ? 0 : w_to_b);
+    lo[j] = few_load_w<VEC>(w_lo + k);
+    hi[j] = few_load_w<VEC>(w_hi + k);
+  };
+  const int first = few_item(min(warp, slices - 1), slices);
+  point(blockIdx.x, first);
   if (w_written) pdl_wait();
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    lo[j] = few_load_w<VEC>(w_lo + 16 * j);
-    hi[j] = few_load_w<VEC>(w_hi + 16 * j);
-  }
+  for (int j = 0; j < 8; ++j) load(j);
   pdl_wait();
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    int now = first;
 #pragma unroll 1
-    for (int slice = warp; slice < slices; slice += kFewWarps) {
+    for (int item = warp; item < slices; item += kFewWarps) {
       float g1[T8][4], g2[T8][4];
-#pragma unroll
-      for (int i = 0; i < T8; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) g1[i][e] = g2[i][e] = 0.f;
-      // the next slice of this tile, or this warp's first of the block's next tile
-      if (slice + kFewWarps < slices) point(tile, slice + kFewWarps);
-      else point(min(tile + (int)gridDim.x, tiles - 1), warp);
+      // the next item of this tile, or this warp's first of the block's next tile
+      const bool more = item + kFewWarps < slices;
+      const int next = more ? few_item(item + kFewWarps, slices) : first;
+      point(more ? tile : min(tile + (int)gridDim.x, tiles - 1), next);
+      if (item == warp) __syncthreads();        // the sums of the tile before have been read
+      const unsigned minus = (unsigned)now << 31;
+      const int half = now >> 1;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
+        if (j % 4 == 0) {
+#pragma unroll
+          for (int i = 0; i < T8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (j == 4) sums[((half * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
+              if (j == 0 || !minus) g1[i][e] = g2[i][e] = 0.f;
+            }
+        }
         unsigned a[2][3][2];
         split_4(lo[j], a[0]);
         split_4(hi[j], a[1]);
-        lo[j] = few_load_w<VEC>(w_lo + 16 * j);
-        hi[j] = few_load_w<VEC>(w_hi + 16 * j);
+        load(j);
         unsigned w[3][4];
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
@@ -537,8 +570,14 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
         }
 #pragma unroll
         for (int i = 0; i < T8; ++i) {
-          const float* x_at = a_src[i] + slice * kSliceK + 16 * j;
-          const float4 v = VEC ? *reinterpret_cast<const float4*>(x_at) : make_float4(x_at[0], x_at[1], x_at[2], x_at[3]);
+          const float* x_at = a_src[i] + half * (kSliceK / 2) + 16 * j + (j < 4 ? 0 : (now & 1) * (kSliceK / 2));
+          float4 v = VEC ? *reinterpret_cast<const float4*>(x_at) : make_float4(x_at[0], x_at[1], x_at[2], x_at[3]);
+          if (j >= 4) {                   // subtracted from the pair's first slice
+            v.x = __uint_as_float(__float_as_uint(v.x) ^ minus);
+            v.y = __uint_as_float(__float_as_uint(v.y) ^ minus);
+            v.z = __uint_as_float(__float_as_uint(v.z) ^ minus);
+            v.w = __uint_as_float(__float_as_uint(v.w) ^ minus);
+          }
           unsigned x[3][2];
           split_4(v, x);
           few_mma(g1[i], w[0], x[0][0], x[0][1]);
@@ -549,11 +588,11 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
           few_mma(g2[i], w[2], x[0][0], x[0][1]);
         }
       }
-      if (slice == warp) __syncthreads();       // the sums of the tile before have been read
 #pragma unroll
       for (int i = 0; i < T8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sums[((slice * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
+        for (int e = 0; e < 4; ++e) sums[(((half + 1 + (now & 1)) * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
+      now = next;
     }
     __syncthreads();
     const int i = threadIdx.x >> 7, e = (threadIdx.x >> 5) & 3;
@@ -562,10 +601,13 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
       float P[kChains];
 #pragma unroll
       for (int j = 0; j < kChains; ++j) {
-        const float* s = sums + ((size_t)(j * slices / kChains) * T8 * 4 + i * 4 + e) * 32 + lane;
-        const int n = (j + 1) * slices / kChains - j * slices / kChains;
-        P[j] = s[0];
-        for (int k = 1; k < n; ++k) P[j] += s[(size_t)k * T8 * 128];
+        const int c0 = j * slices / kChains, n = (j + 1) * slices / kChains - c0;
+        const float* s = sums + ((size_t)2 * c0 * T8 * 4 + i * 4 + e) * 32 + lane;
+        P[j] = 0.f;
+        for (int k = 0; k < n; ++k, s += 2 * T8 * 128) {
+          const float times = k & 1 ? -1.f : k + 1 < n ? 2.f : 1.f;
+          P[j] = fmaf(times, s[T8 * 128], fmaf(times, s[0], P[j]));
+        }
       }
       float v = (P[0] + P[1]) + (P[2] + P[3]);
       if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(A + (size_t)token * lda, W + (size_t)row * ldw, K);
@@ -574,12 +616,14 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
   }
 }
 
-constexpr int kFewSmem = 100 * 1024;      // two blocks an SM
+constexpr int kFewSmem = 200 * 1024;
+
+size_t few_smem(int K, int t8) { return (size_t)(K / kSliceK) * 2 * t8 * 128 * 4; }
 
 template <int T8, bool VEC>
 int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
                cudaStream_t stream) {
-  const size_t smem = (size_t)(K / kSliceK) * T8 * 128 * 4;
+  const size_t smem = few_smem(K, T8);
   if (smem > kFewSmem) return LLMIE_ERR_UNSUPPORTED_SIZE;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<T8, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
   if (e != cudaSuccess) return (int)e;
@@ -655,7 +699,8 @@ int product(const float* A, const float* W, float* C, void* parts, int M, int N,
     if (M <= 16) {
       // up to 8 tokens the stream of the weights bounds both; with 16 the splitting of both operands by every warp does, where
       // there are many rows (16 tokens, microseconds: 2,048 x 2,048 8.8 against 11.6, 16,384 x 2,048 40.8 against 31.9)
-      const bool few = (size_t)(K / kSliceK) * (M <= 8 ? 1 : 2) * 512 <= kFewSmem && (M <= 8 || N < 8192);
+      // (two blocks an SM, or one where there are no more)
+      const bool few = few_smem(K, M <= 8 ? 1 : 2) <= (N <= 148 * 16 ? kFewSmem : kFewSmem / 2) && (M <= 8 || N < 8192);
       nt = few ? 8 : 16;
     } else {
       // a block's time does not follow its tokens (2,048 k: 35 us with 64, 37 with 80), so what counts is how many rounds of
