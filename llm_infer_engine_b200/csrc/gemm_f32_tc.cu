@@ -132,11 +132,66 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* A, __nv_bf
   for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(out + ((size_t)p * M + t) * K + k) = parts[p];
 }
 
-__device__ __forceinline__ float plain_dot(const float* x, const float* w, int K) {
-  float s = 0.f;
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+template <bool VEC>
+__device__ __forceinline__ float4 load_4(const float* p) {
+  return VEC ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ float dot_4(const float4& x, const float4& w, float s) {
+  return fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, s))));
+}
+
+// Sums that are not finite are formed again by FMAs: a warp a sum, lane l the k of 4 l to 4 l + 3 of every 128, in turn; then the lanes'
+// sums in pairs. R weight rows at a time.
+template <int R, bool VEC>
+__device__ __forceinline__ void warp_dots(const float* x, const float* const (&w)[R], int K, float (&s)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) s[r] = 0.f;
+#pragma unroll 2
+  for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+    const float4 a = load_4<VEC>(x + k);
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = dot_4(a, load_4<VEC>(w[r] + k), s[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+}
+// Those of the n results out[i * out_step] of rows x + i * x_step and this lane's weight row (w of lane 0) that are not finite; whole warps.
+template <int R, bool VEC>
+__device__ __forceinline__ void plain_sums(const float* x, size_t x_step, const float* w, int ldw, float* out, size_t out_step, int n,
+                                           bool there, int K) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-  return s;
+  for (int i = 0; i < n; ++i, x += x_step, out += out_step) {
+    unsigned again = __ballot_sync(0xffffffffu, there && !is_finite(*out));
+    if (!again) continue;
+    bool nan = false;                     // then so are all results of this row, and they are already
+#pragma unroll 2
+    for (int k = 4 * lane; k < K; k += 128) {
+      const float4 v = load_4<VEC>(x + k);
+      nan = nan || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+    }
+    if (__any_sync(0xffffffffu, nan)) continue;
+#pragma unroll 1
+    while (again) {
+      const float* rows[R];
+      float s[R];
+      int at[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        at[r] = again ? __ffs(again) - 1 : at[0];
+        again &= again - 1;
+        rows[r] = w + (size_t)at[r] * ldw;
+      }
+      warp_dots<R, VEC>(x, rows, K, s);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (lane == at[r]) *out = s[r];
+    }
+  }
 }
 
 // N consecutive columns of 32 lanes, N a multiple of 8; tmem_ld_wait() before they are used.
@@ -218,7 +273,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
 
   if (warp < kSumWarps) {
     // ---------------------------------------------------------------- sums: half of the tokens each four warps
-    if (S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    if (S::kSplitsX) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     pdl_wait();
     const int quarter = warp & 3, col0 = (warp >> 2) * S::kCols, row = quarter * 32 + lane;
@@ -226,7 +281,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
     const bool row_there = n0 + row < N;
     float* h = hold + (size_t)col0 * kMt + row;
     float* out = C + (size_t)(m0 + col0) * ldc + n0 + row;
-    const int n_cols = row_there ? min(S::kCols, M - m0 - col0) : 0;       // of the result
+    const int n_cols = min(S::kCols, M - m0 - col0);       // of the result
     float run[S::kCols] = {};
     int chain = 0, chain_end = (chain0 + 1) * slices / kChains;
     bool fresh = true, second = false, ok = true;
@@ -273,16 +328,34 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       bool finite = true;
 #pragma unroll
       for (int c = 0; c < S::kCols; ++c) {
-        if (c < n_cols) {
+        if (row_there && c < n_cols) {
           out[(size_t)c * ldc] = run[c];
-          finite = finite && fabsf(run[c]) <= 3.402823466e38f;
+          finite = finite && is_finite(run[c]);
         }
       }
-      if (!finite) {
-        for (int c = 0; c < n_cols; ++c)
-          if (!(fabsf(out[(size_t)c * ldc]) <= 3.402823466e38f))
-            out[(size_t)c * ldc] = plain_dot(A + (size_t)(m0 + col0 + c) * lda, W + (size_t)(n0 + row) * ldw, K);
+      if (!__all_sync(0xffffffffu, finite))
+        plain_sums<NT == 16 ? 1 : 4, WIDE>(A + (size_t)(m0 + col0) * lda, lda, W + (size_t)(n0 + quarter * 32) * ldw, ldw, out, ldc, n_cols, row_there, K);
+    } else {                              // each block of the cluster finishes its share of the tokens
+      cluster_sync_all();
+      const int first = rank * 2 + (warp >> 2), step = 2 * split;
+      float* out = C + (size_t)(m0 + first) * ldc + n0 + row;
+      bool finite = true;
+      const int n = (min(NT, M - m0) - first + step - 1) / step;
+      for (int i = 0; row_there && i < n; ++i) {
+        const uint32_t a = smem_u32(hold + (size_t)(first + i * step) * kMt + row);
+        float v;
+        if (split == 2)
+          v = ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1));
+        else
+          v = (ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1))) +
+              (ld_cluster_f32(map_to_block(a, 2)) + ld_cluster_f32(map_to_block(a, 3)));
+        out[(size_t)i * step * ldc] = v;
+        finite = finite && is_finite(v);
       }
+      if (!__all_sync(0xffffffffu, finite))
+        plain_sums<1, WIDE>(A + (size_t)(m0 + first) * lda, (size_t)step * lda, W + (size_t)(n0 + quarter * 32) * ldw, ldw, out,
+                         (size_t)step * ldc, n, row_there, K);
+      cluster_sync_all();                 // nobody leaves while its sums are read
     }
   } else if (warp < kSumWarps + kSplitWarps) {
     // ---------------------------------------------------------------- float32 in, parts out
@@ -410,25 +483,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
       __syncwarp();
     }
   }
-  if (split > 1) {
+  if (split > 1 && warp >= kSumWarps) {
     cluster_sync_all();
-    if (warp < kSumWarps) {               // each block of the cluster finishes its share of the tokens
-      const int row = (warp & 3) * 32 + lane;
-      if (n0 + row < N) {
-        for (int c = rank * 2 + (warp >> 2); c < NT && m0 + c < M; c += 2 * split) {
-          const uint32_t a = smem_u32(hold + (size_t)c * kMt + row);
-          float v;
-          if (split == 2)
-            v = ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1));
-          else
-            v = (ld_cluster_f32(map_to_block(a, 0)) + ld_cluster_f32(map_to_block(a, 1))) +
-                (ld_cluster_f32(map_to_block(a, 2)) + ld_cluster_f32(map_to_block(a, 3)));
-          if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(A + (size_t)(m0 + c) * lda, W + (size_t)(n0 + row) * ldw, K);
-          C[(size_t)(m0 + c) * ldc + n0 + row] = v;
-        }
-      }
-    }
-    cluster_sync_all();                   // nobody leaves while its sums are read
+    cluster_sync_all();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -597,7 +654,9 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
     __syncthreads();
     const int i = threadIdx.x >> 7, e = (threadIdx.x >> 5) & 3;
     const int row = tile * 16 + g + (e >> 1) * 8, token = i * 8 + 2 * t + (e & 1);
-    if (i < T8 && row < N && token < M) {
+    const bool there = i < T8 && row < N && token < M;
+    float v = 0.f;
+    if (there) {
       float P[kChains];
 #pragma unroll
       for (int j = 0; j < kChains; ++j) {
@@ -609,10 +668,16 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
           P[j] = fmaf(times, s[T8 * 128], fmaf(times, s[0], P[j]));
         }
       }
-      float v = (P[0] + P[1]) + (P[2] + P[3]);
-      if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(A + (size_t)token * lda, W + (size_t)row * ldw, K);
-      C[(size_t)token * ldc + row] = v;
+      v = (P[0] + P[1]) + (P[2] + P[3]);
     }
+    for (unsigned again = __ballot_sync(0xffffffffu, !is_finite(v)); again; again &= again - 1) {
+      const int at = __ffs(again) - 1;
+      const float* w_row[1] = {W + (size_t)__shfl_sync(0xffffffffu, row, at) * ldw};
+      float s[1];
+      warp_dots<1, VEC>(A + (size_t)__shfl_sync(0xffffffffu, token, at) * lda, w_row, K, s);
+      if (lane == at) v = s[0];
+    }
+    if (there) C[(size_t)token * ldc + row] = v;
   }
 }
 

@@ -127,3 +127,30 @@ def test_error_beside_fma_sums(K, kind):
     if kind != "normal":
         assert abs(float(((out.double() - ref) / ref).mean())) <= 0.5e-7      # half a unit of float32 is 0.6e-7; measured 0.37e-7
     assert torch.equal(ops.gemm_f32_nt(a[:5].contiguous(), w), out[:5])
+
+
+@pytest.mark.parametrize("M", [3, 301])
+@pytest.mark.parametrize("what", ["nan", "inf"])
+def test_rows_that_are_not_finite_are_not_slow(M, what):
+    """One such row, and all of them: a thread a sum took 30 and 430 times as long as the finite product; now at most 6 and 40 times."""
+    N, K = 4096, 2048
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+
+    def seconds():
+        _form(a, w, 0)
+        times = []
+        for _ in range(5):
+            first, last = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            first.record()
+            for _ in range(4):
+                _form(a, w, 0)
+            last.record()
+            torch.cuda.synchronize()
+            times.append(first.elapsed_time(last))
+        return min(times)
+
+    fine = seconds()
+    a[0, 5] = float(what)
+    one = seconds()
+    a[:, 7] = float(what)
+    assert one < 12 * fine and seconds() < 80 * fine
