@@ -1538,12 +1538,14 @@ def moe_gather_scaled(x, sorted_token, sorted_pair, weights, out):
 
 def grouped_tc_takes(n_pairs: int, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
     """Whether the routed products of a prompt go to the tcgen05 kernel (csrc/grouped_gemm_tc.cu): bfloat16, rows that start on
-    16 bytes, and more than 16 rows an expert on average. Below, tiles of 16 rows without the gather cost less or as much
+    16 bytes, more than 256 pairs (up to there the down products stay float32 until their weighted sum, here they are rounded to
+    bfloat16), and more than 16 rows an expert on average. Below, tiles of 16 rows without the gather cost less or as much
     (sort to combine, tiles of 16 / this, us: 16 experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, 7.5 rows each 88 / 96, 16 rows 114 /
     96, 48 rows 179 / 99; 128 of 2 x 768 x 2,048, 8 rows 223 / 252, 16 rows 259 / 256; 64 of 2 x 1,408 x 2,048, 12 rows 201 / 215, 19
     rows 254 / 217)."""
     E = w_gate_up.shape[0]
-    return (w_gate_up.dtype == torch.bfloat16 and not routed_tiles_small(n_pairs, E, w_gate_up.dtype) and E <= 1024
+    return (w_gate_up.dtype == torch.bfloat16 and n_pairs > GROUPED_SMALL_ROWS * 4
+            and not routed_tiles_small(n_pairs, E, w_gate_up.dtype) and E <= 1024
             and w_gate_up.shape[2] % 8 == 0 and w_down.shape[2] % 8 == 0 and w_down.shape[1] % 8 == 0)
 
 

@@ -115,3 +115,35 @@ def test_a_block_that_gives_up_leaves_no_numbers(form):
         o.check_tc_status(torch.device(DEV, 0))
     assert bool(call(0).isfinite().all()) and (form == "batched" or bool((out[int(rows.sum()):] == 3.0).all()))
     o.check_tc_status(torch.device(DEV, 0))
+
+
+@pytest.mark.parametrize("experts", [4, 8, 16])
+@pytest.mark.parametrize("rows", [32, 33, 64, 65, 127, 128, 129, 400])
+def test_down_products_of_few_pairs_are_not_rounded(experts, rows):
+    """Routed experts around the sizes where their kernels change. Inputs and weights are small whole numbers, so everything up to
+    the down products is exact, and those are whole numbers that bfloat16 does not hold: up to 256 pairs only the weighted sum rounds."""
+    from test_parts_gpu import build
+    d, ff, top = 64, 32, 2
+    part, _ = build("feed_forward", "routed_experts", {"hidden": d, "n_experts": experts, "top": top, "expert_ff": ff,
+                                                       "activation": "relu", "router_bias": False}, "bfloat16", seed=1)
+    g = torch.Generator().manual_seed(rows)
+    whole = lambda lo, hi, *s: torch.randint(lo, hi + 1, s, generator=g).double()                    # noqa: E731
+    router, x = torch.randn(experts, d, generator=g).double() / 8, whole(-1, 1, rows, d)
+    gate, up = (whole(-1, 1, experts, ff, d) * (torch.rand(experts, ff, d, generator=g) < 0.1) for _ in range(2))
+    down = whole(-200, 200, experts, d, ff)
+    tensors = {"router": router.float()}
+    for e in range(experts):
+        tensors.update({f"e{e}.gate": gate[e], f"e{e}.up": up[e], f"e{e}.down": down[e]})
+    part.load({k: v.to(torch.float32 if k == "router" else torch.bfloat16).to(DEV) for k, v in tensors.items()})
+    got = part.forward(x.to(torch.bfloat16).to(DEV), None).cpu().double()
+    scores, ids = (x @ router.float().double().T).topk(top, 1)
+    weights = scores.softmax(1)
+    act = torch.einsum("td,efd->tef", x, gate).clamp(min=0) * torch.einsum("td,efd->tef", x, up)
+    assert float(act.abs().max()) <= 256
+    y = torch.einsum("tef,edf->ted", act, down)
+    assert float(y.abs().max()) > 512
+    y = y.gather(1, ids[:, :, None].expand(-1, -1, d))
+    want, size = (weights[:, :, None] * y).sum(1), (weights[:, :, None] * y.abs()).sum(1)
+    # float32 scores of 64 terms (their size times 2^-17 at most), exponentials, two products and a sum
+    bound = 1e-4 * size + 1e-6 if rows * top <= 256 else (1e-4 + U) * size + 1e-6
+    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / (size + 1)).max())
