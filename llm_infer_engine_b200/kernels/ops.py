@@ -734,6 +734,19 @@ def gemm_f32_tc_takes(n: int, k: int) -> bool:
     return n >= 128 and k >= 1024 and k % 128 == 0
 
 
+F32_PARTS_BYTES = 256 << 20      # of scratch that a float32 product may take for its rows' parts, 6 bytes a number
+
+
+def _f32_parts_rows(rows: int, k: int) -> int:
+    """Rows of a float32 product that one launch takes: all of them, or equal shares in whole tiles of 80 that keep to
+    F32_PARTS_BYTES. A row's bits do not depend on its launch."""
+    most = max(F32_PARTS_BYTES // (6 * k) // 80 * 80, 80)
+    if rows <= most:
+        return rows
+    launches = -(-rows // most)
+    return min(most, -(-rows // (launches * 80)) * 80)
+
+
 def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, stored: bool = False) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T in true float32, fixed summation order: a row's bits do not depend on the other rows.
     Large weights on the tensor cores, every number as the sum of three bfloat16 (csrc/gemm_f32_tc.cu; which weights are
@@ -748,11 +761,15 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     _need(out, "out", torch.float32, (M, N))
     _work(_nbytes(a, w) + a.shape[0] * w.shape[0] * 4, 2.0 * a.shape[0] * w.shape[0] * w.shape[1])
     if gemm_f32_tc_takes(N, K):
-        # scratch: the parts of `a`, which the kernel for few rows makes itself
-        parts = torch.empty(3 * M * K, dtype=torch.bfloat16, device=a.device) if M > 16 else None
+        # scratch: the parts of `a`, which the kernel for few rows makes itself; more rows than it may hold in several launches
+        rows = _f32_parts_rows(M, K)
+        parts = torch.empty(3 * rows * K, dtype=torch.bfloat16, device=a.device) if M > 16 else None
         f = _fn("gemm_f32_tc", "llmie_gemm_f32_tc", [_c_void_p] * 4 + [_c_int] * 7 + [_c_void_p] * 2)
-        _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(parts), M, N, K, K, K, N, 0 if stored else 1,
-                 tc_status_word(a.device).data_ptr(), _stream()), "gemm_f32_tc")
+        pa, pw, po, pp, status, s = (a.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(parts),
+                                     tc_status_word(a.device).data_ptr(), _stream())
+        for m in range(0, M, max(rows, 1)):
+            _check(f(pa + 4 * m * K, pw, po + 4 * m * N, pp, min(rows, M - m), N, K, K, K, N, 0 if stored else 1, status, s),
+                   "gemm_f32_tc")
         return out
     f = _fn("gemm_simt", "llmie_gemm_f32_nt", [_c_void_p] * 3 + [_c_int] * 6 + [_c_void_p])
     _check(f(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, _stream()), "gemm_f32_nt")

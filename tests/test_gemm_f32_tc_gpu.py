@@ -154,3 +154,20 @@ def test_rows_that_are_not_finite_are_not_slow(M, what):
     one = seconds()
     a[:, 7] = float(what)
     assert one < 12 * fine and seconds() < 80 * fine
+
+
+@pytest.mark.parametrize("M", [1, 17, 161, 400, 1000])
+def test_scratch_is_bounded(M, monkeypatch):
+    """More rows than the scratch for their parts holds: several launches, the same bits."""
+    from llm_infer_engine_b200.kernels import ops
+    K, N = 1152, 300
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    want = ops.gemm_f32_nt(a, w)
+    monkeypatch.setattr(ops, "F32_PARTS_BYTES", 6 * K * 170)
+    used = []
+    empty = torch.empty
+    monkeypatch.setattr(ops.torch, "empty", lambda *s, **kw: (used.append(s[0]) if kw.get("dtype") == torch.bfloat16 else None) or empty(*s, **kw))
+    got = ops.gemm_f32_nt(a, w)
+    monkeypatch.undo()
+    assert all(n * 2 <= 6 * K * 170 for n in used) and len(used) == (M > 16)
+    assert torch.equal(got, want)
