@@ -1,20 +1,27 @@
 // True float32 matrix product on the tensor cores: C[M, N] = A[M, K] * W[N, K]^T for large weights of the 32-bit path.
 //
-// A float32 number is the exact sum of three bfloat16 numbers, x = x1 + x2 + x3: x rounded, what is left rounded, the rest. A
-// product of two bfloat16 numbers is exact in float32. Of the nine products of parts the six with a weight of 2^-16 or more are
-// formed; the three left out are below 2^-25 of the product and of either sign (parts that were cut off instead of rounded
-// would leave out 3e-8 of one sign). w1 x1 has a sum of its own, G1; the other five share G2, which is 2^-8 of it, so that only
-// G1 is subject to the accumulator's rounding (it cuts off what does not fit), and that for 128 k only: then G1 + G2 joins a
-// float32 sum in registers. Relative error against 64-bit sums (2-norm; sums in packed FMAs, gemm_simt.cu, in brackets): 2,048
-// terms 1.3e-7 (2.1e-7), 8,192 terms 1.4e-7 (4.1e-7); an attention layer of 2,048 3.6e-7 (3.9e-7), a feed-forward of 2,048 /
-// 8,192 3.9e-7 (5.2e-7).
+// A float32 number from 2^-110 on is the exact sum of three bfloat16 numbers, x = x1 + x2 + x3: x rounded, what is left rounded, the
+// rest. (Below, the third part falls under bfloat16's least number, 2^-133; what is lost is 2^-134 at most.) A product of two bfloat16
+// numbers is exact in float32. Of the nine products of parts the six with a weight of 2^-16 or more are formed; the three left
+// out are below 2^-25 of the product (parts that were cut off instead of rounded would leave out 3e-8 of one sign). w1 x1 has a
+// sum of its own, G1; the other five share G2, which is 2^-8 of it, so that only G1 is subject to the accumulator's rounding.
+//
+// The accumulator cuts off what does not fit, towards zero. So it keeps 64 k at a time, then G1 + G2 joins a float32 sum in
+// registers; and slices go in pairs: the products of the second one are SUBTRACTED from where the first one ended. With sums of
+// one sign the accumulator goes up and comes back through the same range, and loses as much on the way back as on the way up: with
+// v1 after the first slice and v2 after the second one, 2 v1 - v2 is free of it. Relative error against 64-bit sums (2-norm, 1e-7;
+// without pairs, 128 k a slice; in brackets the packed FMAs of gemm_simt.cu), K of 1,024 / 2,048 / 8,192: normal numbers 1.1 / 1.2
+// / 1.5 (1.3 / 1.3 / 1.5) (1.6 / 2.1 / 4.1), their magnitudes 0.55 / 0.56 / 0.66 (1.73 / 1.72 / 1.74, all of it bias) (0.60 / 0.67 /
+// 1.01), 1 +- 0.01 0.45 / 0.47 / 0.57 (0.40 / 0.42 / 0.48) (0.55 / 0.61 / 0.88), equal numbers 0.25 / 0.25 / 1.2 (4.8 / 9.6 / 38).
+// Uniform numbers that rise along K have 0.57 / 0.57 / 0.71 (0.54 / 0.59 / 0.74): the one kind seen above the FMAs, by 5 % with 1,024.
 //
 // One summation order for every shape. K is cut into slices of 128; n slices make four chains, chain j the slices
-// [j n / 4, (j + 1) n / 4); a chain's sum P_j adds its slices in order, and the result is (P_0 + P_1) + (P_2 + P_3). A row's
-// result does not depend on which other rows share the launch, on the tile or on how the chains are shared among blocks.
+// [j n / 4, (j + 1) n / 4), in pairs from its first on (the last of an odd number has no partner); a chain's sum P_j adds the
+// halves of its slices in order, and the result is (P_0 + P_1) + (P_2 + P_3). A row's result does not depend on which other rows
+// share the launch, on the tile or on how the chains are shared among blocks.
 //
 // Sums that are not finite (an infinity or NaN among the inputs, whose parts are NaN, or an overflow, of a part too) are formed again by plain
-// FMAs over K, which give what IEEE arithmetic gives.
+// FMAs over K, a warp a sum, which give what IEEE arithmetic gives.
 //
 // A block makes 128 weight rows x NT tokens. The weights are the 128-row operand, in tensor memory; per 16 k five tcgen05.mma: w1
 // by [x1 x2] into [G1 G2], then w1 x3, w2 x1, w2 x2, w3 x1 into G2. Sixteen warps in four groups, a group a stage of 32 k, read
@@ -24,10 +31,8 @@
 // sums of finished chains in shared memory.
 //
 // What bounds it: the issue of the products, about 80 cycles each with 80 tokens, 56 with 16, of which the tensor cores work 48
-// (80 tokens). With the weights' parts in shared memory it was its bandwidth: 128 x 80 tokens x 32 k wrote and read 110 KB of it,
-// 890 cycles of the 926 they took (now 820). Products of 2,048 k (weights in shared memory; FMA): 301 x 16,384 141 us (149; 498),
-// 465 x 3,072 38 (40; 165), 301 x 2,048 x 8,192 k 70 (76; 275); a gated feed-forward of 2,048 / 8,192 at 301 rows 253 us (260; FMA
-// 784).
+// (80 tokens). With the weights' parts in shared memory it was its bandwidth. Products of 2,048 k (128 k a slice, no pairs; FMA): 301
+// x 16,384 158 us (151; 500), 301 x 2,048 x 8,192 k 75 (75; 279).
 #include "tcgen05.cuh"
 
 namespace llmie {
@@ -507,15 +512,21 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const float* A, co
 }
 
 // ------------------------------------------------------------------------------------------ up to 16 tokens
-// What bounds it is the weights' way from memory: 3 tokens, 16,384 x 2,048 27.7 us (4.8 TB/s; FMA from shared memory 29.5),
-// 32,000 x 2,048 47 (5.6 TB/s; 49.7), 2,048 x 8,192 19.7 (22.5), 3,072 x 2,048 9.3 (9.7), 1 token 2,048 x 2,048 7.4 (5.6); 16
-// tokens, 2,048 x 2,048 8.8 (15.5).
+// What bounds it: large weights, their way from memory; small ones, the chain of products on one another (40 of a turn share G2) behind the
+// loads. Microseconds one after another, weights from memory, FMA from shared memory (gemm_simt.cu) / this, 1, 4, 8 and 16 tokens:
+//
+//   128 x 1,024 k     2.5 / 2.9    3.3 / 2.9    4.9 / 3.8    8.3 / 4.8       2,048 x 8,192 k    16.4 / 18.0    23.5 / 18.8    36 / 20    50 / 26
+//   512 x 2,048 k     3.9 / 4.3    5.5 / 4.0    9.4 / 5.9    14.1 / 7.5      16,384 x 2,048 k   27.5 / 31.8    32.4 / 32.7    43 / 33    64 / 35
+//   2,048 x 2,048 k   5.9 / 6.7    7.8 / 6.7    11 / 7.6     15.5 / 8.8      32,000 x 2,048 k   46.6 / 51.0    52.8 / 52.8    74 / 54    120 / 65
+//   3,072 x 2,048 k   7.8 / 8.1    10.0 / 8.7   15 / 10.1    20.3 / 12.9     16,384 x 8,192 k   92 / 105       104 / 108      142 / 108  226 / 108
+//
+// So one token (two, of large weights) takes up to 20 % longer than by FMAs; the choice of kernel looks at the weight alone, or a row's
+// bits would depend on its step.
 //
 // The same sums by mma.sync, which rounds as tcgen05.mma does, whatever the order of the k inside a product (tests compare the
 // bits): weights go from memory into registers and are split there, so nothing stands between a load and the next one. A block
 // makes 16 weight rows; its warps take slices in turn, and a slice's sums meet in shared memory, where they are added in the
 // order of the chains. A lane's 16 bytes of a row are four neighbouring k of the sixteen of a product.
-constexpr int kFewWarps = 8;
 
 __device__ __forceinline__ void few_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -559,59 +570,90 @@ __device__ __forceinline__ int few_item(int item, int slices) {
   return at + 1 == n && (n & 1) ? 4 * item : 4 * item - 2 * (at & 1) + 1;
 }
 
-template <int T8, bool VEC>      // T8: eights of tokens
-__global__ void __launch_bounds__(kFewWarps * 32, 2)
-gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
-                    int w_written) {
-  extern __shared__ float sums[];         // [halves of slices][T8][4][32]
+// T8: eights of tokens, a block's tile has 16 weight rows; 0: up to four tokens and a tile of 8 weight rows. A product's rows are then
+// the 8 of one item over the 8 of the next one, its columns the tokens of the one beside those of the other, and two quarters of its
+// result are used: two items a warp at a time, where the chain of a product on the one before it is what there is to wait for.
+// VEC: rows on 16 bytes.
+//
+// Shared memory is kept small because the weights come through what it leaves of L1: with the tokens staged there, or their parts, 8,192 x
+// 4,096 k took 36 us instead of 32.
+template <int T8, bool VEC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+gemm_f32_few_rows_kernel(const float* A, const float* W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc,
+                         int w_written, int buffers) {
+  constexpr bool PAIR = T8 == 0;
+  constexpr int kX = PAIR ? 1 : T8, kRows = PAIR ? 8 : 16;
+  constexpr int kHalf = kSliceK / 2;
+  extern __shared__ __align__(16) float few_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int tiles = (N + 15) / 16, slices = K / kSliceK;
-  const float* a_src[T8];
-#pragma unroll
-  for (int i = 0; i < T8; ++i) a_src[i] = A + (size_t)min(g + 8 * i, M - 1) * lda + 4 * t;
-  const float *w_lo, *w_hi;               // of the item that is loaded
-  int w_to_b;                             // from where half `a` ends to half `b`
-  auto point = [&](int tile, int f) {
-    const float* w = W + (f >> 1) * (kSliceK / 2) + 4 * t;
-    w_lo = w + (size_t)min(tile * 16 + g, N - 1) * ldw;
-    w_hi = w + (size_t)min(tile * 16 + g + 8, N - 1) * ldw;
-    w_to_b = (f & 1) * (kSliceK / 2);
+  const int tiles = (N + kRows - 1) / kRows, slices = K / kSliceK, turns = PAIR ? (slices + 1) / 2 : slices;
+  // sums: [halves of slices][rows 8 to 15][odd tokens][pairs of tokens][8 rows]: a warp's stores are neighbours
+  constexpr int kPairs = PAIR ? 2 : 4 * T8, kOut = 2 * kPairs * kRows;
+  const int buffer = 2 * slices * kOut;
+  const float *w_lo, *w_hi;               // of the turn that is loaded
+  int lo_b, hi_b;                         // from where an item's first half ends to its second one
+  // the items of a turn: one, or two (after an odd number of them the last one twice)
+  auto item_lo = [&](int turn) { return few_item(PAIR ? 2 * turn : turn, slices); };
+  auto item_hi = [&](int turn) { return few_item(min(2 * turn + 1, slices - 1), slices); };
+  auto point = [&](int tile, int f_lo, int f_hi) {
+    const float* w = W + 4 * t;
+    w_lo = w + (size_t)min(tile * kRows + g, N - 1) * ldw + (f_lo >> 1) * kHalf;
+    w_hi = w + (size_t)min(tile * kRows + g + (PAIR ? 0 : 8), N - 1) * ldw + (f_hi >> 1) * kHalf;
+    lo_b = (f_lo & 1) * kHalf;
+    hi_b = (f_hi & 1) * kHalf;
   };
-  float4 lo[8], hi[8];                    // an item of this warp: eight products' worth of k
+  float4 lo[8], hi[8];                    // a turn of this warp: eight products' worth of k
   auto load = [&](int j) {
-    const int k = 16 * j + (j < 4 ? 0 : w_to_b);
-    lo[j] = few_load_w<VEC>(w_lo + k);
-    hi[j] = few_load_w<VEC>(w_hi + k);
+    lo[j] = few_load_w<VEC>(w_lo + 16 * j + (j < 4 ? 0 : lo_b));
+    hi[j] = few_load_w<VEC>(w_hi + 16 * j + (j < 4 ? 0 : hi_b));
   };
-  const int first = few_item(min(warp, slices - 1), slices);
-  point(blockIdx.x, first);
+  const int first = min(warp, turns - 1);
+  const int first_lo = item_lo(first), first_hi = PAIR ? item_hi(first) : first_lo;
+  point(blockIdx.x, first_lo, first_hi);
   if (w_written) pdl_wait();
+  if (warp < turns) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) load(j);
+    for (int j = 0; j < 8; ++j) load(j);
+  }
   pdl_wait();
+  int which = 0;                          // buffer of this tile's sums
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    int now = first;
+    float* sums = few_smem + which * buffer;
+    int f_lo = first_lo, f_hi = first_hi;
 #pragma unroll 1
-    for (int item = warp; item < slices; item += kFewWarps) {
-      float g1[T8][4], g2[T8][4];
-      // the next item of this tile, or this warp's first of the block's next tile
-      const bool more = item + kFewWarps < slices;
-      const int next = more ? few_item(item + kFewWarps, slices) : first;
-      point(more ? tile : min(tile + (int)gridDim.x, tiles - 1), next);
-      if (item == warp) __syncthreads();        // the sums of the tile before have been read
-      const unsigned minus = (unsigned)now << 31;
-      const int half = now >> 1;
+    for (int turn = warp; turn < turns; turn += WARPS) {
+      float g1[kX][4], g2[kX][4];
+      // the next turn of this tile, or this warp's first of the block's next tile
+      const bool more = turn + WARPS < turns;
+      const int next_lo = more ? item_lo(turn + WARPS) : first_lo;
+      const int next_hi = !PAIR ? next_lo : more ? item_hi(turn + WARPS) : first_hi;
+      point(more ? tile : min(tile + (int)gridDim.x, tiles - 1), next_lo, next_hi);
+      const unsigned minus = (unsigned)(PAIR && g >= 4 ? f_hi : f_lo) << 31;
+      auto store = [&](bool second) {
+        const int u_lo = (f_lo >> 1) + (second ? 1 + (f_lo & 1) : 0), u_hi = (f_hi >> 1) + (second ? 1 + (f_hi & 1) : 0);
+        if (PAIR) {
+          float* to = sums + (t < 2 ? u_lo : u_hi) * kOut + (t & 1) * 8 + g;
+          to[0] = t < 2 ? g1[0][0] + g2[0][0] : g1[0][2] + g2[0][2];
+          to[kPairs * 8] = t < 2 ? g1[0][1] + g2[0][1] : g1[0][3] + g2[0][3];
+        } else {
+#pragma unroll
+          for (int i = 0; i < kX; ++i) {
+            float* to = sums + u_lo * kOut + (4 * i + t) * 8 + g;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) to[e * kPairs * 8] = g1[i][e] + g2[i][e];
+          }
+        }
+      };
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
+        if (j == 4) store(false);
         if (j % 4 == 0) {
 #pragma unroll
-          for (int i = 0; i < T8; ++i)
+          for (int i = 0; i < kX; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if (j == 4) sums[((half * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
-              if (j == 0 || !minus) g1[i][e] = g2[i][e] = 0.f;
-            }
+            for (int e = 0; e < 4; ++e)
+              if (j == 0 || !((e < 2 ? f_lo : f_hi) & 1)) g1[i][e] = g2[i][e] = 0.f;
         }
         unsigned a[2][3][2];
         split_4(lo[j], a[0]);
@@ -626,9 +668,9 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
           w[p][3] = a[1][p][1];
         }
 #pragma unroll
-        for (int i = 0; i < T8; ++i) {
-          const float* x_at = a_src[i] + half * (kSliceK / 2) + 16 * j + (j < 4 ? 0 : (now & 1) * (kSliceK / 2));
-          float4 v = VEC ? *reinterpret_cast<const float4*>(x_at) : make_float4(x_at[0], x_at[1], x_at[2], x_at[3]);
+        for (int i = 0; i < kX; ++i) {
+          const int f = PAIR && g >= 4 ? f_hi : f_lo, token = min(PAIR ? g & 3 : g + 8 * i, M - 1);
+          float4 v = load_4<VEC>(A + (size_t)token * lda + ((f >> 1) + (j < 4 ? 0 : f & 1)) * kHalf + 16 * j + 4 * t);
           if (j >= 4) {                   // subtracted from the pair's first slice
             v.x = __uint_as_float(__float_as_uint(v.x) ^ minus);
             v.y = __uint_as_float(__float_as_uint(v.y) ^ minus);
@@ -645,56 +687,72 @@ gemm_f32_few_kernel(const float* A, const float* W, float* __restrict__ C, int M
           few_mma(g2[i], w[2], x[0][0], x[0][1]);
         }
       }
-#pragma unroll
-      for (int i = 0; i < T8; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sums[(((half + 1 + (now & 1)) * T8 + i) * 4 + e) * 32 + lane] = g1[i][e] + g2[i][e];
-      now = next;
+      store(true);
+      f_lo = next_lo;
+      f_hi = next_hi;
     }
     __syncthreads();
-    const int i = threadIdx.x >> 7, e = (threadIdx.x >> 5) & 3;
-    const int row = tile * 16 + g + (e >> 1) * 8, token = i * 8 + 2 * t + (e & 1);
-    const bool there = i < T8 && row < N && token < M;
-    float v = 0.f;
-    if (there) {
+    if (warp * 32 < kOut) {
+      // the four chains side by side; they differ by a slice at most
+      const float* from[kChains];
+      int n[kChains];
       float P[kChains];
 #pragma unroll
-      for (int j = 0; j < kChains; ++j) {
-        const int c0 = j * slices / kChains, n = (j + 1) * slices / kChains - c0;
-        const float* s = sums + ((size_t)2 * c0 * T8 * 4 + i * 4 + e) * 32 + lane;
-        P[j] = 0.f;
-        for (int k = 0; k < n; ++k, s += 2 * T8 * 128) {
-          const float times = k & 1 ? -1.f : k + 1 < n ? 2.f : 1.f;
-          P[j] = fmaf(times, s[T8 * 128], fmaf(times, s[0], P[j]));
+      for (int c = 0; c < kChains; ++c) {
+        const int c0 = c * slices / kChains;
+        n[c] = (c + 1) * slices / kChains - c0;
+        from[c] = sums + 2 * c0 * kOut + min((int)threadIdx.x, kOut - 1);
+        P[c] = 0.f;
+      }
+      const int most = (slices + kChains - 1) / kChains;
+#pragma unroll 2
+      for (int k = 0; k < most; ++k) {
+#pragma unroll
+        for (int c = 0; c < kChains; ++c) {
+          if (k < n[c]) {
+            const float times = k & 1 ? -1.f : k + 1 < n[c] ? 2.f : 1.f;
+            P[c] = fmaf(times, from[c][(2 * k + 1) * kOut], fmaf(times, from[c][2 * k * kOut], P[c]));
+          }
         }
       }
-      v = (P[0] + P[1]) + (P[2] + P[3]);
+      float v = (P[0] + P[1]) + (P[2] + P[3]);
+      const int part = (int)threadIdx.x / (8 * kPairs);
+      const int row = tile * kRows + (threadIdx.x & 7) + (part >> 1) * 8, token = 2 * ((threadIdx.x >> 3) % kPairs) + (part & 1);
+      const bool there = (int)threadIdx.x < kOut && row < N && token < M;
+      for (unsigned again = __ballot_sync(0xffffffffu, there && !is_finite(v)); again; again &= again - 1) {
+        const int at = __ffs(again) - 1;
+        const float* w_row[1] = {W + (size_t)__shfl_sync(0xffffffffu, row, at) * ldw};
+        float dot[1];
+        warp_dots<1, VEC>(A + (size_t)__shfl_sync(0xffffffffu, token, at) * lda, w_row, K, dot);
+        if (lane == at) v = dot[0];
+      }
+      if (there) C[(size_t)token * ldc + row] = v;
     }
-    for (unsigned again = __ballot_sync(0xffffffffu, !is_finite(v)); again; again &= again - 1) {
-      const int at = __ffs(again) - 1;
-      const float* w_row[1] = {W + (size_t)__shfl_sync(0xffffffffu, row, at) * ldw};
-      float s[1];
-      warp_dots<1, VEC>(A + (size_t)__shfl_sync(0xffffffffu, token, at) * lda, w_row, K, s);
-      if (lane == at) v = s[0];
-    }
-    if (there) C[(size_t)token * ldc + row] = v;
+    if (buffers == 2) which ^= 1;
+    else if (tile + (int)gridDim.x < tiles) __syncthreads();      // else the next tile's sums would meet this one's readers
   }
 }
 
-constexpr int kFewSmem = 200 * 1024;
+constexpr int kFewSmem = 200 * 1024;      // of a block that has an SM to itself; two of half of it
+constexpr int kFewSecond = 40 * 1024;     // up to here a block has two buffers of sums
+constexpr int few_out(int t8) { return t8 ? 128 * t8 : 32; }
+size_t few_sums(int K, int t8) { return (size_t)(K / kSliceK) * 2 * few_out(t8) * 4; }
 
-size_t few_smem(int K, int t8) { return (size_t)(K / kSliceK) * 2 * t8 * 128 * 4; }
-
-template <int T8, bool VEC>
+template <int T8, bool VEC, int WARPS>
 int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
                cudaStream_t stream) {
-  const size_t smem = few_smem(K, T8);
-  if (smem > kFewSmem) return LLMIE_ERR_UNSUPPORTED_SIZE;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<T8, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem);
+  constexpr size_t limit = kFewSmem / (16 / WARPS);
+  constexpr int kRows = T8 ? 16 : 8;
+  const int tiles = (N + kRows - 1) / kRows, slots = 148 * (16 / WARPS);
+  const size_t sums = few_sums(K, T8);
+  const int buffers = tiles > slots && 2 * sums <= kFewSecond ? 2 : 1;
+  const size_t smem = buffers * sums;
+  if (smem > limit) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  auto kernel = gemm_f32_few_rows_kernel<T8, VEC, WARPS>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
   if (e != cudaSuccess) return (int)e;
-  const int tiles = (N + 15) / 16;
-  launch_k(gemm_f32_few_kernel<T8, VEC>, dim3(tiles < 2 * 148 ? tiles : 2 * 148), dim3(kFewWarps * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc,
-           w_written);
+  launch_k(kernel, dim3(tiles < slots ? tiles : slots), dim3(WARPS * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc, w_written,
+           buffers);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
@@ -733,18 +791,28 @@ int launch_tc(const float* A, const float* W, float* C, void* parts, int M, int 
   return LLMIE_OK;
 }
 
+// One block an SM where there are no more, and turns enough for its warps; or where the sums of two leave too little (1 token, 4,096 x
+// 12,288 k 45 us against 53; 4,096 x 8,192 k 35 against 32).
+bool few_alone(int t8, int N, int K) {
+  return (t8 ? N <= 148 * 16 : N <= 148 * 8 && K > 16 * kSliceK) || few_sums(K, t8) > 80 * 1024;
+}
+// Whether a product of few rows fits the kernel: its sums, whose number follows K.
+bool few_takes(int t8, int K, bool alone) { return few_sums(K, t8) <= (alone ? kFewSmem : kFewSmem / 2); }
 template <int T8>
 int few_form(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
-             cudaStream_t stream) {
+             bool alone, cudaStream_t stream) {
   const bool vec = aligned16(A) && aligned16(W) && ((lda | ldw) & 3) == 0;
-  return vec ? launch_few<T8, true>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream)
-             : launch_few<T8, false>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream);
+#define LLMIE_FEW(vec_, warps_) launch_few<T8, vec_, warps_>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream)
+  if (alone) return vec ? LLMIE_FEW(true, 16) : LLMIE_FEW(false, 16);
+  return vec ? LLMIE_FEW(true, 8) : LLMIE_FEW(false, 8);
+#undef LLMIE_FEW
 }
 
 // 1 when the kernel takes a weight [N, K]. The answer depends on the weight alone: a row's bits are then the same in every step.
 bool takes(int N, int K) { return N >= 128 && K >= 1024 && K % kSliceK == 0; }
 
-// form: tokens a block (8: the kernel for up to 16 tokens; 16, 64, 80) + 1000 * split (blocks of a tile: 1, 2, 4), for tests: every form gives the same bits. 0:
+// form: tokens a block (8: the kernel for up to 16 tokens, 4: its form for up to 4; 16, 64, 80) + 1000 * split (blocks of a tile: 1, 2, 4;
+// of the kernel for few tokens 2: eight warps a block, 4: sixteen), for tests: every form gives the same bits. 0:
 // chosen by size. + 10000: every wait gives up at once (for tests of that path; the sums are then made by plain FMAs). `parts`: 3 M K bfloat16 of scratch, not needed for 16 tokens a block.
 int product(const float* A, const float* W, float* C, void* parts, int M, int N, int K, int lda, int ldw, int ldc, int form,
             int w_written, int* status, cudaStream_t stream) {
@@ -762,11 +830,14 @@ int product(const float* A, const float* W, float* C, void* parts, int M, int N,
       return tiles <= 33 ? 4 : tiles <= 74 ? 2 : 1;
     };
     if (M <= 16) {
-      // up to 8 tokens the stream of the weights bounds both; with 16 the splitting of both operands by every warp does, where
-      // there are many rows (16 tokens, microseconds: 2,048 x 2,048 8.8 against 11.6, 16,384 x 2,048 40.8 against 31.9)
-      // (two blocks an SM, or one where there are no more)
-      const bool few = few_smem(K, M <= 8 ? 1 : 2) <= (N <= 148 * 16 ? kFewSmem : kFewSmem / 2) && (M <= 8 || N < 8192);
-      nt = few ? 8 : 16;
+      // microseconds, the kernel for few rows / 16 tokens a block: 8 rows, 8,192 x 4,096 k 35.7 / 35.3, 16,384 x 4,096 k 64 / 60,
+      // 32,000 x 4,096 k 108 / 115; 16 rows, 3,072 x 1,024 k 8.0 / 9.5, x 2,048 k 12.8 / 12.9, x 4,096 k 23.0 / 19.5
+      const int t8 = M <= 8 ? 1 : 2;
+      const bool few = few_takes(t8, K, few_alone(t8, N, K)) &&
+                       (M <= 4 || (M <= 8 ? !(K >= 4096 && N >= 8192 && N <= 148 * kMt) : N <= 148 * 16 || (N < 8192 && K <= 1024)));
+      // two items at a time / one, 4 rows: 512 x 2,048 k 4.0 / 6.1, 2,048 x 2,048 k 6.7 / 7.5, 3,072 x 4,096 k 15.8 / 17.5,
+      // 4,096 x 4,096 k 18.9 / 18.8, 8,192 x 8,192 k 62 / 61
+      nt = M <= 4 && N <= 3072 && few_takes(0, K, few_alone(0, N, K)) ? 4 : few ? 8 : 16;
     } else {
       // a block's time does not follow its tokens (2,048 k: 35 us with 64, 37 with 80), so what counts is how many rounds of
       // blocks there are, and how many share a tile
@@ -780,10 +851,13 @@ int product(const float* A, const float* W, float* C, void* parts, int M, int N,
   }
   if (split != 1 && split != 2 && split != 4) return LLMIE_ERR_BAD_ARG;
   const bool wide = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 31) == 0 && ((lda | ldw) & 7) == 0;
-  if (nt == 8) {
-    if (M > 16) return LLMIE_ERR_UNSUPPORTED_SIZE;
-    return M <= 8 ? few_form<1>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream)
-                  : few_form<2>(A, W, C, M, N, K, lda, ldw, ldc, w_written, stream);
+  if (nt == 4 || nt == 8) {
+    const int t8 = nt == 4 ? 0 : M <= 8 ? 1 : 2;
+    const bool alone = form / 1000 > 1 ? split == 4 : few_alone(t8, N, K);
+    if (M > (nt == 4 ? 4 : 16) || !few_takes(t8, K, alone)) return LLMIE_ERR_UNSUPPORTED_SIZE;
+    return t8 == 0   ? few_form<0>(A, W, C, M, N, K, lda, ldw, ldc, w_written, alone, stream)
+           : t8 == 1 ? few_form<1>(A, W, C, M, N, K, lda, ldw, ldc, w_written, alone, stream)
+                     : few_form<2>(A, W, C, M, N, K, lda, ldw, ldc, w_written, alone, stream);
   }
 #define LLMIE_TC(nt_)                                                                                     \
   case nt_:                                                                                               \

@@ -51,6 +51,26 @@ def test_every_form_gives_the_same_bits(M, N, K, offset):
     ops.check_tc_status(torch.device(DEV, 0))
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(128, 1024), (1185, 1152), (300, 2048), (2369, 1408), (129, 2176), (640, 8192), (300, 14336), (130, 20480)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_two_items_at_a_time(M, N, K, offset):
+    """The form for up to four rows, with an odd number of slices too: the bits of the others, and what is not finite where it belongs."""
+    g = torch.Generator().manual_seed(M * 1000 + K)
+    a = torch.randn(M, K + offset, generator=g).to(DEV)[:, :K]
+    w = torch.randn(N, K + offset, generator=g).to(DEV)[:, :K]
+    status, want = _form(a, w, 1016)
+    for form in (1004, 1008, 0):
+        status, out = _form(a, w, form, ld_extra=3)
+        assert status == 0 and torch.equal(out, want), form
+    assert _form(torch.cat([a] * 5), w, 1004)[0] == -2
+    a[M - 1, K - 1], w[N - 1, 0] = float("inf"), float("nan")
+    ref, out = a.double() @ w.double().T, _form(a, w, 1004)[1].double()
+    fine = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(out[~fine & ~torch.isnan(ref)], ref[~fine & ~torch.isnan(ref)])
+    assert torch.equal(out[fine], want.double()[fine])
+
+
 def test_infinities_nan_overflow_and_nothing():
     torch.manual_seed(5)
     a, w = torch.randn(40, 1152, device=DEV), torch.randn(200, 1152, device=DEV)
