@@ -165,7 +165,10 @@ __device__ __forceinline__ int md_sequence(const int* seq_kvlen, int n_seqs, int
 // column lies HD / 2 columns on, which is the same lane's fragment KS / 2 k-steps on), and the one warp whose
 // half page holds the sequence's newest position rotates the new key, puts key and value into its staged tile
 // and (with write_kv) into the cache. Rotation in float32, one rounding to bfloat16, as the separate kernel.
-template <int HD, int WARPS, bool ROPE>
+// ORDERED: the longest sequences first. At head size 64 a kernel of its own: with the search for the order in every launch it lost 2 to 7 %
+// where there is nothing to order (registers). Head size 128 looks at its argument (opt.longest_first): there a kernel of its own costs
+// the others 2 to 4 %.
+template <int HD, int WARPS, bool ROPE, bool ORDERED>
 __global__ void __launch_bounds__(WARPS * 32, HD != 64 ? 1 : WARPS <= 4 ? 16 / WARPS : WARPS <= 6 ? 2 : 1)
 decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
                   const __nv_bfloat16* v_cache, float* part_m, float* part_l,
@@ -183,7 +186,7 @@ decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
   extern __shared__ __align__(16) unsigned char md_smem[];
   __shared__ int is_last;
 
-  const int run = blockIdx.x, seq = opt.longest_first ? md_sequence(seq_kvlen, gridDim.z, blockIdx.z) : blockIdx.z;
+  const int run = blockIdx.x, seq = (HD == 64 ? ORDERED : opt.longest_first) ? md_sequence(seq_kvlen, gridDim.z, blockIdx.z) : blockIdx.z;
   const int G = n_q / n_kv;
   const int chunks = (G + 15) / 16;
   const int hk = blockIdx.y / chunks;
@@ -526,7 +529,7 @@ decode_mma_kernel(const __nv_bfloat16* q, const __nv_bfloat16* k_cache,
   }
 }
 
-template <int HD, int WARPS, bool ROPE>
+template <int HD, int WARPS, bool ROPE, bool ORDERED>
 static int launch_mma(const void* q, const void* k_cache, const void* v_cache, float* part_m, float* part_l,
                       float* part_acc, const int* seq_slot, const int* seq_kvlen, const int* block_table, int max_pages,
                       int n_seqs, int n_q, int n_kv, float scale, int window, int pages_per_run, int n_runs,
@@ -536,11 +539,11 @@ static int launch_mma(const void* q, const void* k_cache, const void* v_cache, f
   const int chunks = (G + 15) / 16;
   constexpr size_t kSmem = (size_t)WARPS * 2 * kMdPage * (HD + 8) * sizeof(__nv_bfloat16);
   if (kSmem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(decode_mma_kernel<HD, WARPS, ROPE>,
+    cudaError_t e = cudaFuncSetAttribute(decode_mma_kernel<HD, WARPS, ROPE, ORDERED>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
     if (e != cudaSuccess) return (int)e;
   }
-  launch_k(decode_mma_kernel<HD, WARPS, ROPE>, dim3(n_runs, n_kv * chunks, n_seqs), dim3(WARPS * 32), kSmem, stream,
+  launch_k(decode_mma_kernel<HD, WARPS, ROPE, ORDERED>, dim3(n_runs, n_kv * chunks, n_seqs), dim3(WARPS * 32), kSmem, stream,
            (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache, part_m, part_l,
            part_acc, seq_slot, seq_kvlen, block_table, max_pages, n_q, n_kv, scale, window, pages_per_run, n_runs,
            counters, (__nv_bfloat16*)out, rope, table_len, q_ld, write_kv, opt);
@@ -640,25 +643,35 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
   const bool fill = 100 * blocks >= 85 * rounds_6 * slots_6;
   if (long_ones && blocks > 148 && (hd == 64 ? rounds_6 == 1 || (rounds_6 == 2 && fill) : fill && blocks <= 400)) best_w = 6;
   // (finding the order takes a block about half a microsecond; blocks that are all there at once gain nothing by it)
-  opt.longest_first = long_ones && n_seqs <= 64 && blocks > slots_of(best_w) ? 1 : 0;
-#define LLMIE_MMA(HD, W)                                                                                             \
-  return rope ? launch_mma<HD, W, true>(q, k_cache, v_cache, part_m, part_l, part_acc, seq_slot, seq_kvlen,          \
-                                        block_table, max_pages, n_seqs, n_q, n_kv, scale, window, pages_per_run,     \
-                                        n_runs, counters, out, rope, table_len, q_ld, write_kv, opt, stream)         \
-              : launch_mma<HD, W, false>(q, k_cache, v_cache, part_m, part_l, part_acc, seq_slot, seq_kvlen,         \
-                                         block_table, max_pages, n_seqs, n_q, n_kv, scale, window, pages_per_run,    \
-                                         n_runs, counters, out, nullptr, 0, 0, 0, opt, stream)
-  if (hd == 64) {
-    if (best_w == 8) LLMIE_MMA(64, 8);
-    if (best_w == 6) LLMIE_MMA(64, 6);
-    if (best_w == 4) LLMIE_MMA(64, 4);
-    if (best_w == 3) LLMIE_MMA(64, 3);
-    LLMIE_MMA(64, 2);
+  const bool ordered = long_ones && n_seqs <= 64 && blocks > slots_of(best_w);
+  opt.longest_first = ordered ? 1 : 0;
+#define LLMIE_MMA(HD, W, ORDERED)                                                                                    \
+  return rope ? launch_mma<HD, W, true, ORDERED>(q, k_cache, v_cache, part_m, part_l, part_acc, seq_slot, seq_kvlen, \
+                                                 block_table, max_pages, n_seqs, n_q, n_kv, scale, window,           \
+                                                 pages_per_run, n_runs, counters, out, rope, table_len, q_ld,        \
+                                                 write_kv, opt, stream)                                              \
+              : launch_mma<HD, W, false, ORDERED>(q, k_cache, v_cache, part_m, part_l, part_acc, seq_slot,           \
+                                                  seq_kvlen, block_table, max_pages, n_seqs, n_q, n_kv, scale,       \
+                                                  window, pages_per_run, n_runs, counters, out, nullptr, 0, 0, 0,    \
+                                                  opt, stream)
+  if (hd == 64 && ordered) {
+    if (best_w == 8) LLMIE_MMA(64, 8, true);
+    if (best_w == 6) LLMIE_MMA(64, 6, true);
+    if (best_w == 4) LLMIE_MMA(64, 4, true);
+    if (best_w == 3) LLMIE_MMA(64, 3, true);
+    LLMIE_MMA(64, 2, true);
   }
-  if (best_w == 6) LLMIE_MMA(128, 6);
-  if (best_w >= 4) LLMIE_MMA(128, 4);
-  if (best_w == 3) LLMIE_MMA(128, 3);
-  LLMIE_MMA(128, 2);
+  if (hd == 64) {
+    if (best_w == 8) LLMIE_MMA(64, 8, false);
+    if (best_w == 6) LLMIE_MMA(64, 6, false);
+    if (best_w == 4) LLMIE_MMA(64, 4, false);
+    if (best_w == 3) LLMIE_MMA(64, 3, false);
+    LLMIE_MMA(64, 2, false);
+  }
+  if (best_w == 6) LLMIE_MMA(128, 6, false);
+  if (best_w >= 4) LLMIE_MMA(128, 4, false);
+  if (best_w == 3) LLMIE_MMA(128, 3, false);
+  LLMIE_MMA(128, 2, false);
 #undef LLMIE_MMA
 }
 

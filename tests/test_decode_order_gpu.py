@@ -7,11 +7,9 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("n,longest", [(19, 2100), (36, 2113), (40, 2113), (49, 2100), (64, 2300), (65, 2200), (33, 1100)])
-def test_every_sequence_is_served(hd, n, longest):
+def _step(hd, n, longest, n_q=32, n_kv=8):
+    """A step of n sequences: the blocks' runs, and both entry points against the plain kernel."""
     from llm_infer_engine_b200.kernels import ops
-    n_q, n_kv = 32, 8
     g = torch.Generator().manual_seed(n * hd)
     lens = torch.randint(1, longest + 1, (n,), generator=g)
     lens[n // 2], lens[3], lens[n - 1], lens[5] = longest, lens[7], 1, lens[7]          # the longest, the shortest, equal ones
@@ -41,3 +39,22 @@ def test_every_sequence_is_served(hd, n, longest):
     assert torch.equal(got, want) and not bool(counters.any())
     # outputs and probabilities are bfloat16: as in the other tests of this kernel
     assert torch.allclose(want.float(), plain.float(), atol=2e-2, rtol=1.6e-2)
+    return runs
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("n,longest", [(19, 2100), (36, 2113), (40, 2113), (49, 2100), (64, 2300), (65, 2200), (33, 1100)])
+def test_every_sequence_is_served(hd, n, longest):
+    _step(hd, n, longest)
+
+
+@pytest.mark.parametrize("hd,n,longest,runs", [(128, 16, 4300, 2), (128, 15, 8300, 2), (128, 17, 4200, 2), (64, 9, 8300, 4)])
+def test_runs_that_meet(hd, n, longest, runs):
+    """Sequences in several runs, whose blocks meet by the counters, the longest first (head size 128: more blocks than SMs)."""
+    assert _step(hd, n, longest) == runs
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_a_key_head_for_every_query_head(hd):
+    """Many more blocks than fit at once: few warps a block, the longest sequences first."""
+    _step(hd, 40, 2100, 32, 32)
