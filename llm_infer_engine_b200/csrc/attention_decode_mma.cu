@@ -627,17 +627,23 @@ static int decode_mma_entry(const void* q, const void* k_cache, const void* v_ca
       best_w = w;
     }
   }
+  // (Six warps in this estimate, us without / with: head size 128, 8 KV heads, 1 sequence of 900 keys 13.5 / 11.6, 8 of 1,600 22.0 / 19.5, 16
+  // of 250 to 2,000 25.0 / 22.0; head size 64, 24 sequences of 900 14.1 / 11.2, of 2,000 26.9 / 20.3. In a captured step, whose estimate is
+  // made for a longer context than its sequences have, also the other way: head size 128, 8 of 60 keys 5.6 / 5.9; head size 64, 37 of
+  // 400 keys 9.0 / 9.9, of 600 11.7 / 11.1, of 1,500 23.2 / 21.2.)
+  //
   // That is right for sequences of one length. Lengths differ where batches are served, and then a long sequence's block with few
   // warps is what a launch ends with, however many others run beside it. Where some sequence is longer than 2,048 keys (a captured
   // step of shorter ones is sized for 2,048 at most): six warps a block (two blocks an SM; head size 128, one), served longest
-  // first where blocks have to queue, as long as equal lengths do not pay for it, which they do where the last round of such
-  // blocks fills the SMs badly. Measured, us, the choice above / this one, head size 64: 64 sequences of 700 to 3,900 keys 56.0 /
-  // 41.2, of 200 to 4,000 54.6 / 32.9, of 3,000 70.0 / 65.3; 24 of 200 to 4,000 37.4 / 29.5, of 3,000 38.1 / 29.4; 48 (left as they
-  // were) of 200 to 4,000 42.2 / 31.8, of 3,000 53.3 / 59.0. Head size 128: 48 of 200 to 4,000 77.9 / 48.8, of 3,000 104 / 101, 50 of
-  // 2,000 to 2,400 about 76 / 80; 32 of 200 to 4,000 58.5 / 36.1, of 3,000 70.6 / 67.6; 24 (left) 53.5 / 34.0 and 57.2 / 63.7; 64
-  // (three warps, longest first) of 200 to 4,000 86.6 / 69.8, of 3,000 124 / 124, with six warps 66.6 and 134. With shorter ones six
-  // warps cost more where lengths are equal (64 of 512, 14.2 / 19.4) than they give where not. A window or a chunk makes the work
-  // of long sequences alike.
+  // first where blocks have to queue, as long as equal lengths do not pay much for it, which they do where the last round of such
+  // blocks fills the SMs badly. Measured, us, the choice above / this one, head size 64: 64 sequences of 200 to 4,000 keys 61 / 45, of
+  // 2,600 61.5 / 59.7; 24 of 200 to 4,000 40.1 / 32.0, of 3,000 37.6 / 29.6; 48 (left) of 200 to 4,000 42.2 / 31.8, of 3,000 53.3 / 59.0.
+  // Head size 128: 48 of 200 to 4,000 95.6 / 73.9, of 2,100 74.5 / 76.2, of 3,400 116 / 112; 32 of 200 to 4,000 69.4 / 56.6, of 2,100 50.8 /
+  // 51.4; 37 of 200 to 4,000 70.3 / 54.5, of 2,100 56.2 / 58.5 (the worst seen), of 3,400 86.7 / 88.2; 24 (left) of 200 to 4,000 53.5 /
+  // 34.0, of 3,000 57.2 / 63.7; 64 (three warps, longest first) of 200 to 4,000 103 / 86.5, of 2,100 92.1 / 93.2. With shorter ones six
+  // warps cost more where lengths are equal (64 of 512, 14.2 / 19.4) than they give where not. A window or a chunk makes the work of
+  // long sequences alike. (Leaving out counts whose blocks fill the last round of the choice above, 33 to 37 and 49, gave 2 to 4 % where
+  // all have 2,100 and took 12 to 30 % where lengths differ.)
   const bool long_ones = window == 0 && pages_per_run > 32;
   const long long slots_6 = slots_of(6), rounds_6 = (blocks + slots_6 - 1) / slots_6;
   const bool fill = 100 * blocks >= 85 * rounds_6 * slots_6;
