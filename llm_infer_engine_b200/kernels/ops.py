@@ -1369,7 +1369,9 @@ def batched_gemm_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, a_group
         _work(_nbytes(w) + T * G * (K * a.element_size() + N * out.element_size()), 2.0 * T * G * N * K)
     pa, pw, po = a.data_ptr(), w.data_ptr(), out.data_ptr()
     if (T >= BATCHED_TC_FROM and a.dtype is torch.bfloat16 and out.dtype is torch.bfloat16 and G <= 1024
-            and not (K & 63 or (N | lda | ldc | a_group_cols | out_group_cols) & 7 or (pa | pw | po) & 15)):
+            and not (K & 63 or (N | lda | ldc | a_group_cols | out_group_cols) & 7 or (pa | pw | po) & 15)
+            and lda >= (G - 1) * a_group_cols + K and ldc >= (G - 1) * out_group_cols + N         # rows that do not overlap
+            and a_group_cols >= 0 and out_group_cols >= 0 and G * N < 2 ** 30 and lda < 2 ** 31):
         f = _fn("grouped_gemm_tc", "llmie_grouped_gemm_tc", _GROUPED_TC_ARGS)
         _check(f(pa, lda, a_group_cols, pw, po, ldc, out_group_cols, None, G, T, N, K, 0, 0,
                  tc_status_word(a.device).data_ptr(), _stream()), "batched_gemm_nt")

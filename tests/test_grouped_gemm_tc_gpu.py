@@ -69,6 +69,21 @@ def test_batched(T, G, N, K):
         assert bool(((mine[:64, :N] - f).abs() <= 2 * b[:64] + 2 * U * (s[:64].abs() + b[:64])).all())
 
 
+@pytest.mark.parametrize("T", [128, 300])
+def test_batched_rows_that_overlap(T):
+    """One row for all (stride 0), and windows of a sequence: what the kernel of fewer rows takes, whatever their number."""
+    o = ops()
+    G, N, K = 3, 64, 64
+    w = torch.randn(G, N, K, device=DEV).to(torch.bfloat16)
+    flat = torch.randn(T * 8 + G * K, device=DEV).to(torch.bfloat16)
+    for a in (flat[:G * K].expand(T, G * K), flat.as_strided((T, G * K), (8, 1))):
+        out = torch.zeros(T, G * N, dtype=torch.bfloat16, device=DEV)
+        o.batched_gemm_nt(a, w, out, K, N, K)
+        want = torch.zeros_like(out)
+        o.batched_gemm_nt(a.contiguous(), w, want, K, N, K)
+        assert torch.equal(out, want)
+
+
 def test_no_finite_value_crosses_rows_or_groups():
     o = ops()
     a = torch.ones(256, 72, dtype=torch.bfloat16, device=DEV)
