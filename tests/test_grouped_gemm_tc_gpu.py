@@ -84,6 +84,24 @@ def test_batched_rows_that_overlap(T):
         assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("G,N,K", [(3, 64, 64), (2, 72, 128), (5, 8, 64), (2, 264, 192), (32, 256, 64), (40, 64, 256), (2, 512, 1024)])
+@pytest.mark.parametrize("spread", [0.0, 3.0])
+def test_batched_rows_do_not_depend_on_the_step(G, N, K, spread):
+    """A row's bits in a step of few rows (tiles of 16, of 64) and of many (tcgen05); numbers alike, and over many powers of two."""
+    o, T = ops(), 400
+    g = torch.Generator().manual_seed(G + N + K)
+    a = (torch.randn(T, G * K, generator=g) * torch.exp(spread * torch.randn(T, G * K, generator=g))).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(G, N, K, generator=g) * torch.exp(spread * torch.randn(G, N, K, generator=g))).to(torch.bfloat16).to(DEV)
+
+    def product(rows):
+        out = torch.zeros(rows, G * N, dtype=torch.bfloat16, device=DEV)
+        return o.batched_gemm_nt(a[:rows], w, out, K, N, K)
+
+    many = product(T)
+    for rows in (1, 16, 64, 65, 127, 128):
+        assert torch.equal(product(rows), many[:rows]), rows
+
+
 def test_no_finite_value_crosses_rows_or_groups():
     o = ops()
     a = torch.ones(256, 72, dtype=torch.bfloat16, device=DEV)
