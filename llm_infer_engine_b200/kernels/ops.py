@@ -987,12 +987,16 @@ _TC_STATUS_TEXT = {1: "a TMA load did not arrive", 2: "the tensor cores did not 
 
 
 def tc_status_word(device) -> torch.Tensor:
-    """One int32 per device that the tensor-core kernels set when a bounded wait gives up."""
+    """One int32 per device that the tensor-core kernels set when a bounded wait gives up. While a graph is captured that no call
+    outside a graph has come before, a word of its own: it lies in graph memory, unset until a replay, and is never read."""
     key = (device if type(device) is torch.device else torch.device(device)).index or 0
     t = _tc_status.get(key)
     if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=device)
-        _tc_status[key] = t
+        if torch.device(device).type == "cuda" and torch.cuda.is_current_stream_capturing():
+            key = ("captured", key)
+        t = _tc_status.get(key)
+        if t is None:
+            t = _tc_status[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return t
 
 

@@ -191,3 +191,21 @@ def test_scratch_is_bounded(M, monkeypatch):
     monkeypatch.undo()
     assert all(n * 2 <= 6 * K * 170 for n in used) and len(used) == (M > 16)
     assert torch.equal(got, want)
+
+
+def test_first_call_under_capture(monkeypatch):
+    """A call that a graph captures first leaves nothing behind that is read before a replay has set it."""
+    from llm_infer_engine_b200.kernels import ops
+    a, w = torch.randn(40, 1024, device=DEV), torch.randn(256, 1024, device=DEV)
+    want = ops.gemm_f32_nt(a, w)
+    monkeypatch.setattr(ops, "_tc_status", {})
+    out = torch.zeros_like(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.gemm_f32_nt(a, w, out)
+    captured = [t for t in ops._tc_status.values()]
+    word = ops.tc_status_word(torch.device(DEV, 0))
+    assert len(captured) == 1 and all(word is not t for t in captured) and int(word) == 0
+    graph.replay()
+    ops.check_tc_status(torch.device(DEV, 0))
+    assert torch.equal(out, want)
