@@ -741,15 +741,15 @@ size_t few_sums(int K, int t8) { return (size_t)(K / kSliceK) * 2 * few_out(t8) 
 template <int T8, bool VEC, int WARPS>
 int launch_few(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int w_written,
                cudaStream_t stream) {
-  constexpr size_t limit = kFewSmem / (16 / WARPS);
+  constexpr int kLimit = kFewSmem / (16 / WARPS);
   constexpr int kRows = T8 ? 16 : 8;
   const int tiles = (N + kRows - 1) / kRows, slots = 148 * (16 / WARPS);
   const size_t sums = few_sums(K, T8);
   const int buffers = tiles > slots && 2 * sums <= kFewSecond ? 2 : 1;
   const size_t smem = buffers * sums;
-  if (smem > limit) return LLMIE_ERR_UNSUPPORTED_SIZE;
+  if (smem > kLimit) return LLMIE_ERR_UNSUPPORTED_SIZE;
   auto kernel = gemm_f32_few_rows_kernel<T8, VEC, WARPS>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit);
   if (e != cudaSuccess) return (int)e;
   launch_k(kernel, dim3(tiles < slots ? tiles : slots), dim3(WARPS * 32), smem, stream, A, W, C, M, N, K, lda, ldw, ldc, w_written,
            buffers);
