@@ -11,17 +11,23 @@
 //
 // One block per SM walks over the tiles (128 rows x BN weight rows; the row tiles of one slice of weights follow one another,
 // so the slice comes from memory once). Warp 0 loads (TMA, 128-byte swizzle, a ring of stages of 64 k), warp 1 multiplies,
-// warps 2 to 9 take the sums out of tensor memory, two tiles of sums in turn, while the next tile is multiplied. Every wait is
+// warps 2 to 9 (to 17 with a gate) take the sums out of tensor memory, two tiles of sums in turn, while the next tile is multiplied. Every wait is
 // bounded; one that gives up records a status, what the block has not finished becomes NaN (C may hold something else that
 // looks like a result: the routed experts' second product writes over their gathered inputs), and the block waits for its copies
 // and products, frees its tensor memory and returns.
 //
 // What bounds it: many rows, shared memory (a stage of 48 KB is written and read once for 512 cycles of products); few, the
 // weights' way from memory; one short K (attention heads), the way of the results out of tensor memory, hence eight warps for
-// it (four: 15.5 us where eight take 13.4) and stores of 64 bytes a row (a thread storing its own row: 17.5). Measured, us, the
-// vendor's grouped products with the activation by itself / this: 16 experts of 2 x 2,048 x 2,048 and 2,048 x 2,048, 600 pairs 75.4 +
-// 38.3 / 50.8 + 27.3, 5,331 pairs 117 + 56.1 / 97.7 + 51.1, 16,384 pairs 260 + 115 / 226 + 120; 8 of 2 x 1,408 x 4,096, 5,331 pairs
-// 118 + 57.1 / 117 + 63.4, 16,384 pairs 304 + 137 / 279 + 157; 128 of 2 x 768 x 2,048, 3,000 pairs 188 + 93.3 / 142 + 71.1. Heads, the
+// it (four: 15.5 us where eight take 13.4) and stores of 64 bytes a row (a thread storing its own row: 17.5). With a gate, the
+// activation of the tile that a block ends with: its divisions wait for one another, so sixteen warps (eight, silu: 16 experts of 2 x
+// 2,048 x 2,048, 600 pairs 59 us where sixteen take 54; 8 of 2 x 1,408 x 4,096, 2,400 pairs 87 / 79).
+//
+// Measured, us, the vendor's grouped products with the activation (silu) by itself / this, gate and up with it + down: 16 experts of 2 x 2,048
+// x 2,048 and 2,048 x 2,048, 600 pairs 71 + 39 / 53 + 27, 2,400 pairs 72 + 36 / 72 + 36, 5,331 pairs 114 + 54 / 97 + 49, 16,384 pairs 250 +
+// 113 / 221 + 126; 8 of 2 x 1,408 x 4,096, 600 pairs 76 + 33 / 46 + 18, 5,331 pairs 114 + 56 / 117 + 62, 16,384 pairs 301 + 135 / 279 + 151;
+// 128 of 2 x 768 x 2,048, 3,000 pairs 171 + 93 / 139 + 67; 32 of 2 x 1,024 x 2,880, 2,400 pairs 99 + 56 / 71 + 39, 5,331 pairs 95 + 50 / 99 +
+// 54. So from some 500 rows an expert on the down product takes up to 13 % longer, both together up to 5 % (8 of 1,408 x 4,096 with 670
+// rows each, 32 of 1,024 x 2,880 with 170: tiles of 128 rows that are two thirds full, rounds of blocks that are nearly empty). Heads, the
 // mma.sync kernel / this: 32 of 256 x 64, 2,130 rows 22.8 / 13.4; of 64 x 256, 19.9 / 9.3.
 #include "tcgen05.cuh"
 
@@ -33,7 +39,8 @@ namespace {
 constexpr int kRows = 128, kK = 64;
 constexpr int kRing = 192 * 1024;                 // bytes of the ring of stages
 constexpr int kMostGroups = 1024;
-constexpr int kThreads = 320;
+template <bool DUAL> constexpr int kEpilogueWarps = DUAL ? 16 : 8;
+template <bool DUAL> constexpr int kThreads = 64 + 32 * kEpilogueWarps<DUAL>;
 constexpr int kStaged = 8 * 32 * 64;              // 32 rows x 32 columns of results for each epilogue warp, on their way to memory
 constexpr int kSmem = kRing + kStaged + 1024 + 2 * (kMostGroups + 1) * 4;
 
@@ -57,11 +64,12 @@ __device__ __forceinline__ void give_up(volatile int* abort, int* status, int co
 
 // LIMIT: polls before a wait gives up, a constant as in attention_latent_tc.cu.
 template <int BN, bool DUAL, unsigned LIMIT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads<DUAL>, 1)
 grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Args p) {
   constexpr int kStageBytes = (kRows + BN) * kK * 2;
   constexpr int kStages = kRing / kStageBytes;            // 4 at BN 256, 6 at 128, 8 at 64
   constexpr int kCols = DUAL ? BN / 2 : BN;               // columns of C a tile covers
+  constexpr int kParts = kEpilogueWarps<DUAL> / 4, kChunk = DUAL ? 16 : 32, kPieces = kChunk / 8;
   extern __shared__ uint8_t smem_raw[];
   __shared__ Shared sh;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -78,7 +86,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh.acc_full[b], 1);
-      mbar_init(&sh.acc_empty[b], 8);
+      mbar_init(&sh.acc_empty[b], kEpilogueWarps<DUAL>);
     }
     mbar_init(&sh.drained, 1);
     sh.abort = sh.loaded = 0;
@@ -185,7 +193,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else {
     const int quarter = warp & 3;                          // the tensor memory lanes this warp may read
-    const int c_first = warp < 6 ? 0 : kCols / 2;          // and its half of the columns
+    const int c_first = (warp - 2) / 4 * (kCols / kParts);    // and its part of the columns
     int e = 0, i = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < n_all; t += gridDim.x, ++i) {
@@ -199,49 +207,51 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (!ok) {                                           // neither this tile nor those behind it have a result
         give_up(abort, p.status, kStatusTimeoutMma);
         const uint4 nan8 = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
-        for (int at = lane; at < 32 * (kCols / 16); at += 32) {
-          const int rr = at / (kCols / 16), col = c_first + at % (kCols / 16) * 8;
+        for (int at = lane; at < 32 * (kCols / kParts / 8); at += 32) {
+          const int rr = at / (kCols / kParts / 8), col = c_first + at % (kCols / kParts / 8) * 8;
           if (row + rr < end && n0 + col < p.N) *reinterpret_cast<uint4*>(dst + (size_t)rr * p.ldc + col) = nan8;
         }
         continue;
       }
       tc_fence_after_sync();
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + buf * BN;
-      uint8_t* staged = ring + kRing + (warp - 2) * (32 * 64);
+      uint8_t* staged = ring + kRing + (warp - 2) * (32 * kChunk * 2);
 #pragma unroll 1
-      for (int c = c_first; c < c_first + kCols / 2; c += 32) {
-        float v[4][8];
-        uint32_t g[32];
-        tmem_ld_32x32(acc + c, g);
-        if (DUAL) {
-          uint32_t u[32];
-          tmem_ld_32x32(acc + BN / 2 + c, u);
+      for (int c = c_first; c < c_first + kCols / kParts; c += kChunk) {
+        float v[kPieces][8];
+        uint32_t g[kChunk];
+        if constexpr (DUAL) {
+          uint32_t u[kChunk];
+          tmem_ld_32x16(acc + c, g);
+          tmem_ld_32x16(acc + BN / 2 + c, u);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
+          for (int j = 0; j < kChunk; ++j)
             v[j >> 3][j & 7] = apply_act(__bfloat162float(__float2bfloat16(__uint_as_float(g[j]))), p.act) *
                                __bfloat162float(__float2bfloat16(__uint_as_float(u[j])));
         } else {
+          tmem_ld_32x32(acc + c, g);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j >> 3][j & 7] = __uint_as_float(g[j]);
+          for (int j = 0; j < kChunk; ++j) v[j >> 3][j & 7] = __uint_as_float(g[j]);
           if (p.act) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
+            for (int j = 0; j < kChunk; ++j)
               v[j >> 3][j & 7] = apply_act(__bfloat162float(__float2bfloat16(v[j >> 3][j & 7])), p.act);
           }
         }
-        // a thread has a row: through shared memory (the four 16-byte pieces of a row in swizzled order) to stores in which
+        // a thread has a row: through shared memory (the 16-byte pieces of a row in swizzled order) to stores in which
         // neighbours write neighbouring pieces
+        const int swizzle = kPieces - 1;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          store8(reinterpret_cast<__nv_bfloat16*>(staged + lane * 64 + ((j ^ (lane >> 1 & 3)) << 4)), v[j]);
+        for (int j = 0; j < kPieces; ++j)
+          store8(reinterpret_cast<__nv_bfloat16*>(staged + lane * (kChunk * 2) + ((j ^ (lane * kPieces / 8 & swizzle)) << 4)), v[j]);
         __syncwarp();
-        const int piece = lane & 3, col = c + piece * 8;
+        const int piece = lane % kPieces, col = c + piece * 8;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int rr = j * 8 + (lane >> 2);
-          const uint4 x = *reinterpret_cast<const uint4*>(staged + rr * 64 + ((piece ^ (rr >> 1 & 3)) << 4));
+        for (int j = 0; j < kPieces; ++j) {
+          const int rr = j * (32 / kPieces) + lane / kPieces;
+          const uint4 x = *reinterpret_cast<const uint4*>(staged + rr * (kChunk * 2) + ((piece ^ (rr * kPieces / 8 & swizzle)) << 4));
           if (row + rr < end && n0 + col < p.N) *reinterpret_cast<uint4*>(dst + (size_t)rr * p.ldc + col) = x;
         }
         __syncwarp();
@@ -283,7 +293,7 @@ int launch(const CUtensorMap& map_a, const void* W, const Args& p, bool no_wait,
   const long long n_tiles = (p.N + kCols - 1) / kCols, m_tiles = (p.M + kRows - 1) / kRows;
   const long long most = n_tiles * (p.group_end ? m_tiles + p.groups : m_tiles * p.groups);
   if (most > 0x3fffffff) return LLMIE_ERR_UNSUPPORTED_SIZE;
-  launch_k(kernel, dim3((unsigned)(most < 148 ? most : 148)), dim3(kThreads), kSmem, stream, map_a, map_w, p);
+  launch_k(kernel, dim3((unsigned)(most < 148 ? most : 148)), dim3(kThreads<DUAL>), kSmem, stream, map_a, map_w, p);
   LLMIE_LAUNCH_CHECK();
   return LLMIE_OK;
 }
