@@ -31,8 +31,9 @@
 // sums of finished chains in shared memory.
 //
 // What bounds it: the issue of the products, about 80 cycles each with 80 tokens, 56 with 16, of which the tensor cores work 48
-// (80 tokens). With the weights' parts in shared memory it was its bandwidth. Products of 2,048 k (128 k a slice, no pairs; FMA): 301
-// x 16,384 158 us (151; 500), 301 x 2,048 x 8,192 k 75 (75; 279).
+// (80 tokens), and the weights' way through L1, a lane its row (301 x 16,384: tensor pipe 48 % of the active cycles, L1 80 %). With the
+// weights' parts in shared memory it was its bandwidth. Products of 2,048 k (128 k a slice, no pairs; FMA): 301 x 16,384 158 us (151;
+// 500), 301 x 2,048 x 8,192 k 75 (75; 279).
 #include "tcgen05.cuh"
 
 namespace llmie {
